@@ -311,7 +311,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     plan_bidiag(b1, m, n, ldw, nctas, kind, &pl.bw);
     b1.take<char>(gsc);
     Arena b2 = a;
-    DDC_TRY(dc_sigma(ctx, n, nullptr, nullptr, nullptr, nullptr, nullptr, b2, true));
+    DDC_TRY(dc_sigma(ctx, n, nullptr, nullptr, nullptr, nullptr, nullptr, b2, true, false));
     Arena b3 = a;
     DDC_TRY(bd_vectors(ctx, n, (long long)n * n, nullptr, nullptr, nullptr, nullptr, nullptr, b3, true));
     Arena b4 = a, b5 = a;  // stage 5 (its buffers are in region a when it overlaps stages 2-4)
@@ -384,7 +384,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
   // ---- stage 2
   {
     Arena b = a;
-    DDC_TRY(dc_sigma(ctx, n, P.b1, P.b2, pl.sig_slot, &P.H, P.dints, b, false));
+    DDC_TRY(dc_sigma(ctx, n, P.b1, P.b2, pl.sig_slot, &P.H, P.dints, b, false, false));
   }
   DDC_TRY(stage_event(ctx, 2));
   // ---- stages 3-4: X straight into V, Y into the top of U (ascending order)
@@ -782,7 +782,7 @@ static int bd_standalone(ddcsvd_context* h, int N, const double* dB1, const doub
     a.take<char>(PB.blob_bytes);
     a.take<double>(N + 4);
     Arena b = a, c = a;
-    DDC_TRY(dc_sigma(h, N, nullptr, nullptr, nullptr, nullptr, nullptr, b, true));
+    DDC_TRY(dc_sigma(h, N, nullptr, nullptr, nullptr, nullptr, nullptr, b, true, true));
     if (dX) DDC_TRY(bd_vectors(h, N, (long long)N * N, nullptr, nullptr, nullptr, nullptr, nullptr, c, true));
     c.take<int>(N + 8);
     need = std::max(b.off, c.off);
@@ -810,7 +810,7 @@ static int bd_standalone(ddcsvd_context* h, int N, const double* dB1, const doub
     DDC_CUDA_TRY(cudaMemcpyAsync(sig_slot, dSigmaIn, sizeof(double) * N, cudaMemcpyDeviceToDevice, h->stream));
   } else {
     Arena b = a;
-    DDC_TRY(dc_sigma(h, N, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false));
+    DDC_TRY(dc_sigma(h, N, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true));
   }
   if (dX) {
     Arena c = a;

@@ -641,7 +641,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
     Arena a;
     layout(a, &W, &d, &e, &tq, &tp, &dt, &dord, &counter, &blob, &sig_slot, &sig);
     Arena b = a, c = a;
-    DDC_TRY(dc_sigma(h, Ntot, nullptr, nullptr, nullptr, nullptr, nullptr, b, true));
+    DDC_TRY(dc_sigma(h, Ntot, nullptr, nullptr, nullptr, nullptr, nullptr, b, true, true));
     DDC_TRY(bd_vectors(h, Ntot, PB.store, nullptr, nullptr, nullptr, nullptr, nullptr, c, true));
     need = std::max(b.off, c.off);
   }
@@ -727,7 +727,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
   // ---- stages 2-4
   {
     Arena b = a;
-    DDC_TRY(dc_sigma(h, Ntot, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false));
+    DDC_TRY(dc_sigma(h, Ntot, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true));
   }
   {
     Arena c = a;

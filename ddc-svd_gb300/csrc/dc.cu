@@ -59,17 +59,90 @@ struct DcParams {
   double* L[2];
   double *ds, *zs, *hfs, *hls;
   double *dq, *zq, *fq, *lq;
-  float *dqf, *zqf;  // FP32 copies of dq, zq for the first phase of the root solver
+  float2* dqf;       // dq as a pair of floats (hi + lo), for the FP32 phase of the root solver
+  float* zqf;        // FP32 copy of zq
   double *dd, *fd, *ld;  // deflated entries (ascending d)
-  double *tau, *zh, *rS, *rF, *rL;
-  int* org;
+  double *tau, *dor, *zh, *rS, *rF, *rL;  // root i: sigma^2 = dor^2 + tau, dor its origin pole
   int* defl;
   int* nq;
   double *zz, *phi, *psi;
-  double* out;
   GridBarrier* bar;
   DevStatus* st;
 };
+
+// ---------------------------------------------------------------- FP64 arithmetic
+// GB300's FP64 pipe bounds this stage: one FP64 instruction of a warp holds it
+// for 64 cycles (19 per SM when four warps or more share the SM), against one
+// for FP32 and integer instructions, and comparisons, fmin / fmax take a turn
+// in it like an addition.  Measured per warp (one warp per scheduler): add,
+// multiply, FMA 64-66 cycles, a compare and an add 176, a division 566, hypot
+// 1059; the approximate reciprocal and the conversions to and from FP32 do not
+// use the pipe (9 and 2 cycles).  So divisions are formed from the approximate
+// reciprocal by one cubic Newton step (four FP64 instructions instead of
+// about nine), values of known sign are compared through their bit patterns,
+// and whatever does not need 53 bits is FP32.
+
+// a / x to about an ulp for normal x: with r ~ 1/x and e = 1 - x r,
+// 1/x = r (1 + e + e^2 + ...); |e| < 2^-18, so e^3 is below rounding.  x = 0
+// or subnormal gives NaN (callers fall back or had an infinity there before).
+__device__ __forceinline__ double rcp_approx(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+}
+__device__ __forceinline__ double quot(double a, double x) {
+  const double r = rcp_approx(x);
+  const double e = fma(-x, r, 1.0);
+  const double y = fma(e, e, e);
+  const double t = a * r;
+  return fma(t, y, t);
+}
+// a / x rounded to nearest, as the division operator gives it, in six FP64
+// instructions: the reciprocal as above, q = a r, and the correction by the
+// exact remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990).  Operands outside 2^+-500 take the
+// operator.
+__device__ __forceinline__ double quot_rn(double a, double x) {
+  const unsigned ea = (unsigned)__double2hiint(a) & 0x7ff00000u, ex = (unsigned)__double2hiint(x) & 0x7ff00000u;
+  constexpr unsigned lo = 523u << 20, span = 1000u << 20;
+  if (ea - lo > span || ex - lo > span) return a / x;
+  double r = rcp_approx(x);
+  const double e = fma(-x, r, 1.0);
+  r = fma(r, fma(e, e, e), r);
+  const double q = a * r;
+  return fma(fma(-x, q, a), r, q);
+}
+
+// Two versions of the stage's arithmetic.  kBits = true keeps every FP64
+// rounding of the plain formulas (division operator, hypot, sqrt, a fixed
+// order of sums): the twisted vectors' signs follow from a twist index that
+// rounding decides among the large components, so one last-bit change of a
+// sigma may flip its vectors.  The entry points that hand back what a stored
+// bidiagonal or batch gave before run with it.  kBits = false (single SVDs,
+// whose FP32 reduction rounds by the launch knobs anyway) spends fewer FP64
+// instructions on results of the same accuracy.
+template <bool kBits>
+__device__ __forceinline__ double quotient(double a, double x) {
+  return kBits ? quot_rn(a, x) : quot(a, x);
+}
+
+// order of non-negative values = order of their bit patterns
+__device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
+// |x|'s bits for a maximum that ignores NaN, as fmax does
+__device__ __forceinline__ long long max_bits(double x) {
+  const long long b = abs_bits(x);
+  return b <= 0x7ff0000000000000ll ? b : 0ll;
+}
+// p = m 2^e with |m| in [1, 2): keeps the mantissa, adds e to ex (zero,
+// subnormal and non-finite values stay as they are)
+__device__ __forceinline__ double take_exponent(double p, int& ex) {
+  const int hi = __double2hiint(p);
+  const int e = (hi >> 20) & 0x7ff;
+  if (e == 0 || e == 0x7ff) return p;
+  ex += e - 1023;
+  return __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(p));
+}
 
 // ---------------------------------------------------------------- leaves
 __device__ void dc_leaf(int nn, const double* b1, const double* b2, double* sig, double* fr,
@@ -134,15 +207,21 @@ __device__ int block_exscan(int v, int* sh, int* tot) {
   return r;
 }
 
-__device__ double block_max(double v, double* sh) {
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+__device__ __forceinline__ long long warp_max_ll(long long v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+__device__ long long block_max_ll(long long v, double* sh) {
+  long long* shl = reinterpret_cast<long long*>(sh);
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+  v = warp_max_ll(v);
   __syncthreads();
-  if (lane == 0) sh[wid] = v;
+  if (lane == 0) shl[wid] = v;
   __syncthreads();
-  double r = 0.0;
-  for (int w = 0; w < nw; w++) r = fmax(r, sh[w]);
+  long long r = 0;
+  for (int w = 0; w < nw; w++) r = max(r, shl[w]);
   __syncthreads();
   return r;
 }
@@ -153,10 +232,28 @@ __device__ double block_sumd(double v, double* sh) {
   __syncthreads();
   if (lane == 0) sh[wid] = v;
   __syncthreads();
-  double r = 0.0;
-  for (int w = 0; w < nw; w++) r += sh[w];
+  if (t == 0) {  // one thread: every warp adding them would queue at the FP64 pipe
+    double r = 0.0;
+    for (int w = 0; w < nw; w++) r += sh[w];
+    sh[0] = r;
+  }
+  __syncthreads();
+  const double r = sh[0];
   __syncthreads();
   return r;
+}
+
+// 1 / sqrt(a + a1^2) and 1 / sqrt(b + b1^2), or 1 where that is not positive,
+// in lanes 0 and 1 of one warp (one pass of the FP64 pipe for both)
+__device__ __forceinline__ double lane_inv_norm(double a, double a1, double b, double b1, int lane) {
+  const double v = (lane == 0) ? a : b, w = (lane == 0) ? a1 : b1;
+  const double n2 = v + w * w;
+  return (n2 > 0.0) ? rsqrt(n2) : 1.0;
+}
+// sqrt(a + a1^2) and sqrt(b + b1^2) likewise
+__device__ __forceinline__ double lane_norm(double a, double a1, double b, double b1, int lane) {
+  const double v = (lane == 0) ? a : b, w = (lane == 0) ? a1 : b1;
+  return sqrt(v + w * w);
 }
 
 // Cooperation policies for the per-node phases: a whole CTA for large nodes,
@@ -169,20 +266,31 @@ struct CtaGroup {
   __device__ int rank() const { return threadIdx.x; }
   __device__ int size() const { return blockDim.x; }
   __device__ void sync() const { __syncthreads(); }
-  __device__ double max(double v) const { return block_max(v, shd); }
+  __device__ long long maxbits(long long v) const { return block_max_ll(v, shd); }
   __device__ double sum(double v) const { return block_sumd(v, shd); }
   __device__ int exscan(int v, int* tot) const { return block_exscan(v, shi, tot); }
   __device__ int any(int v) const { return __syncthreads_or(v); }
+  // lane_inv_norm / lane_norm of the pair, computed by one warp and shared
+  // (every warp computing them would queue at the FP64 pipe)
+  __device__ void inv_norms(double* a, double a1, double* b, double b1) const { pair<true>(a, a1, b, b1); }
+  __device__ void norms(double* a, double a1, double* b, double b1) const { pair<false>(a, a1, b, b1); }
+  template <bool kInv>
+  __device__ void pair(double* a, double a1, double* b, double b1) const {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const double r = kInv ? lane_inv_norm(*a, a1, *b, b1, threadIdx.x) : lane_norm(*a, a1, *b, b1, threadIdx.x);
+      if (threadIdx.x < 2) shd[threadIdx.x] = r;
+    }
+    __syncthreads();
+    *a = shd[0];
+    *b = shd[1];
+  }
 };
 struct WarpGroup {
   __device__ int rank() const { return threadIdx.x & 31; }
   __device__ int size() const { return 32; }
   __device__ void sync() const { __syncwarp(); }
-  __device__ double max(double v) const {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-  }
+  __device__ long long maxbits(long long v) const { return warp_max_ll(v); }
   __device__ double sum(double v) const { return warp_sum(v); }
   __device__ int exscan(int v, int* tot) const {
     const int lane = threadIdx.x & 31;
@@ -196,22 +304,33 @@ struct WarpGroup {
     return x - v;
   }
   __device__ int any(int v) const { return __any_sync(0xffffffffu, v); }
+  __device__ void inv_norms(double* a, double a1, double* b, double b1) const { pair<true>(a, a1, b, b1); }
+  __device__ void norms(double* a, double a1, double* b, double b1) const { pair<false>(a, a1, b, b1); }
+  template <bool kInv>
+  __device__ void pair(double* a, double a1, double* b, double b1) const {
+    const int lane = threadIdx.x & 31;
+    const double r = kInv ? lane_inv_norm(*a, a1, *b, b1, lane) : lane_norm(*a, a1, *b, b1, lane);
+    *a = __shfl_sync(0xffffffffu, r, 0);
+    *b = __shfl_sync(0xffffffffu, r, 1);
+  }
 };
 
-// number of a[0..n) < v (strict) or <= v
+// number of a[0..n) < v (strict) or <= v, all values non-negative
 __device__ __forceinline__ int count_lt(const double* a, int n, double v) {
+  const long long vb = bits(v);
   int lo = 0, hi = n;
-  while (lo < hi) { int mid = (lo + hi) >> 1; if (a[mid] < v) lo = mid + 1; else hi = mid; }
+  while (lo < hi) { int mid = (lo + hi) >> 1; if (bits(a[mid]) < vb) lo = mid + 1; else hi = mid; }
   return lo;
 }
 __device__ __forceinline__ int count_le(const double* a, int n, double v) {
+  const long long vb = bits(v);
   int lo = 0, hi = n;
-  while (lo < hi) { int mid = (lo + hi) >> 1; if (a[mid] <= v) lo = mid + 1; else hi = mid; }
+  while (lo < hi) { int mid = (lo + hi) >> 1; if (bits(a[mid]) <= vb) lo = mid + 1; else hi = mid; }
   return lo;
 }
 
 // ---------------------------------------------------------------- P1 merge set-up
-template <class Grp>
+template <bool kBits, class Grp>
 __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& grp) {
   const int t = grp.rank(), nt = grp.size();
   const int nn = p.nd_nn[node], slot = p.nd_slot[node], K = p.nd_K[node], r0 = p.nd_r0[node];
@@ -226,43 +345,55 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
   const double* l2 = p.L[cp] + slot + K + 1;
   const double bk1 = p.b1[r0 + K], bk2 = p.b2[r0 + K];
   const double phi1 = p.phi[c1], psi1 = p.psi[c1], phi2 = p.phi[c2], psi2 = p.psi[c2];
-  const double r = hypot(bk1 * psi1, bk2 * phi2);  // Calculations-Parallel.c:769-771
-  const double c0 = (r > 0.0) ? bk1 * psi1 / r : 1.0;
-  const double s0 = (r > 0.0) ? bk2 * phi2 / r : 0.0;
+  // r = hypot(x, y), (c0, s0) = (x, y) / r  (Calculations-Parallel.c:769-771)
+  const double rx = bk1 * psi1, ry = bk2 * phi2;
+  const double r2 = fma(rx, rx, ry * ry);
+  double r, c0, s0;
+  if (!kBits && bits(r2) > bits(1e-280) && bits(r2) < bits(1e280)) {
+    const double ri = rsqrt(r2);
+    r = r2 * ri;
+    c0 = rx * ri;
+    s0 = ry * ri;
+  } else {
+    r = hypot(rx, ry);
+    c0 = (r > 0.0) ? quot_rn(rx, r) : 1.0;
+    s0 = (r > 0.0) ? quot_rn(ry, r) : 0.0;
+  }
   double* ds = p.ds + slot;
   double* zs = p.zs + slot;
   double* hfs = p.hfs + slot;
   double* hls = p.hls + slot;
   // parallel merge of [0] ++ child1 ++ child2 by value (ties: entry 0, then child1)
-  double dmax = 0.0, zmax = 0.0;
+  long long zb = 0;  // max |z|, as bits
   if (t == 0) {
     ds[0] = 0.0; zs[0] = r; hfs[0] = c0 * phi1; hls[0] = s0 * psi2;
-    zmax = fabs(r);
+    zb = max_bits(r);
   }
   for (int k = t; k < n1; k += nt) {
     const double v = s1[k];
     const int pos = 1 + k + count_lt(s2, n2, v);
     const double z = bk1 * l1[k];
     ds[pos] = v; zs[pos] = z; hfs[pos] = f1[k]; hls[pos] = 0.0;
-    dmax = fmax(dmax, fabs(v)); zmax = fmax(zmax, fabs(z));
+    zb = max(zb, max_bits(z));
   }
   for (int k = t; k < n2; k += nt) {
     const double v = s2[k];
     const int pos = 1 + k + count_le(s1, n1, v);
     const double z = bk2 * f2[k];
     ds[pos] = v; zs[pos] = z; hfs[pos] = 0.0; hls[pos] = l2[k];
-    dmax = fmax(dmax, fabs(v)); zmax = fmax(zmax, fabs(z));
+    zb = max(zb, max_bits(z));
   }
-  dmax = grp.max(dmax);
-  zmax = grp.max(zmax);
-  const double tol = 8.0 * DBL_EPSILON * fmax(dmax, zmax);
+  // the children's values ascend, so the largest d is one of their last
+  zb = max(grp.maxbits(zb), max(n1 > 0 ? max_bits(s1[n1 - 1]) : 0ll, n2 > 0 ? max_bits(s2[n2 - 1]) : 0ll));
+  const double tol = 8.0 * DBL_EPSILON * __longlong_as_double(zb);
+  const long long tolb = bits(tol);
   grp.sync();
   // deflation 1: negligible z
   const int per = ceil_div(nn, nt);
   const int lo = min(nn, t * per), hi = min(nn, lo + per);
   int cnt = 0;
   for (int k = lo; k < hi; k++) {
-    int dfl = fabs(zs[k]) <= tol;
+    int dfl = abs_bits(zs[k]) <= tolb;
     p.defl[slot + k] = dfl;
     cnt += !dfl;
   }
@@ -275,7 +406,7 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
   // deflation 2 needed?  (adjacent non-deflated values within tol)
   int close = 0;
   for (int k = 1 + t; k < tot; k += nt)
-    if (p.dq[slot + k] - p.dq[slot + k - 1] <= tol) close = 1;
+    if (bits(p.dq[slot + k] - p.dq[slot + k - 1]) <= tolb) close = 1;
   const int need2 = grp.any(close);
   if (need2 && t == 0) {
     int prev = -1;
@@ -302,7 +433,9 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
   for (int k = lo; k < hi; k++) {
     if (!p.defl[slot + k]) {
       p.dq[slot + off] = ds[k]; p.zq[slot + off] = zs[k];
-      p.dqf[slot + off] = (float)ds[k]; p.zqf[slot + off] = (float)zs[k];
+      const float dh = (float)ds[k];
+      p.dqf[slot + off] = make_float2(dh, (float)(ds[k] - (double)dh));
+      p.zqf[slot + off] = (float)zs[k];
       p.fq[slot + off] = hfs[k]; p.lq[slot + off] = hls[k];
       zzl += zs[k] * zs[k];
       off++;
@@ -355,7 +488,7 @@ __device__ __forceinline__ void sec_eval(int q, const double* d, const double* z
   for (int j = g.lg; j < q; j += g.G) {
     const double dj = d[j];
     const double del = (dj - dorg) * (dj + dorg) - tau;
-    const double tt = z[j] / del;
+    const double tt = quot_rn(z[j], del);
     if (j <= split) { ps += z[j] * tt; dps += tt * tt; }
     else { ph += z[j] * tt; dph += tt * tt; }
   }
@@ -363,25 +496,69 @@ __device__ __forceinline__ void sec_eval(int q, const double* d, const double* z
   f = 1.0 + psi + phi;
 }
 
-// FP32 twin of sec_eval on the FP32 copies of d and z.
-__device__ __forceinline__ void sec_eval32(int q, const float* d, const float* z, float dorg, float tau, int split,
+// FP32 reciprocal to an ulp or so (range ends flush to 0 or infinity)
+__device__ __forceinline__ float rcp32(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// d_j - d_o from the float pairs: the heads' difference is exact when they are
+// close, so it keeps FP32's relative accuracy down to gaps of 2^-24 |d| (from
+// the heads alone, a gap of |d| / 1000 had only 14 good bits, and the FP64
+// phase then needed a second evaluation for most roots)
+__device__ __forceinline__ float pair_diff(float2 a, float2 b) { return (a.x - b.x) + (a.y - b.y); }
+
+// FP32 twin of sec_eval on the float copies of d and z (kBits: the heads and
+// the division operator only).
+template <bool kBits>
+__device__ __forceinline__ void sec_eval32(int q, const float2* d, const float* z, float2 dorg, float tau, int split,
                                            const LaneGroup& g, float& f, float& psi, float& dpsi, float& phi,
                                            float& dphi) {
   float ps = 0.f, dps = 0.f, ph = 0.f, dph = 0.f;
   for (int j = g.lg; j < q; j += g.G) {
-    const float dj = d[j];
-    const float del = (dj - dorg) * (dj + dorg) - tau;
-    const float tt = z[j] / del;
-    if (j <= split) { ps += z[j] * tt; dps += tt * tt; }
-    else { ph += z[j] * tt; dph += tt * tt; }
+    const float2 dj = d[j];
+    const float zj = z[j];
+    const float del = (kBits ? dj.x - dorg.x : pair_diff(dj, dorg)) * (dj.x + dorg.x) - tau;
+    const float tt = kBits ? zj / del : zj * rcp32(del);
+    if (j <= split) { ps += zj * tt; dps += tt * tt; }
+    else { ph += zj * tt; dph += tt * tt; }
   }
   psi = gsum(ps, g); dpsi = gsum(dps, g); phi = gsum(ph, g); dphi = gsum(dph, g);
   f = 1.f + psi + phi;
 }
 
+// One FP64 evaluation for the third-order step: f, f' = sum (z / del)^2, and
+// in FP32 the second-derivative sum g2 = sum (z / del)^2 (tau / del), which
+// only forms the correction term.  Nine FP64 instructions per pole.
+__device__ __forceinline__ void sec_eval_newton(int q, const double* d, const double* z, double dorg, double tau,
+                                                const LaneGroup& g, double& f, double& fp, float& g2) {
+  const float t32 = (float)tau;
+  double s = 0.0, sp = 0.0;
+  float sg = 0.f;
+  for (int j = g.lg; j < q; j += g.G) {
+    const double dj = d[j], zj = z[j];
+    const double del = fma(dj - dorg, dj + dorg, -tau);
+    const double r = rcp_approx(del);
+    const double e = fma(-del, r, 1.0);
+    const double y = fma(e, e, e);
+    const double t = zj * r;
+    const double tt = fma(t, y, t);
+    s = fma(zj, tt, s);
+    sp = fma(tt, tt, sp);
+    const float tf = (float)tt;
+    sg += tf * tf * ((float)r * t32);
+  }
+  f = 1.0 + gsum(s, g);
+  fp = gsum(sp, g);
+  g2 = gsum(sg, g);
+}
+
 // One safeguarded step of the root iteration (two-pole rational model for an
 // interior root, one pole for the last root), shared by the FP32 and FP64
 // phases.  Returns true when converged.
+__device__ __forceinline__ float step_quot(float a, float x) { return a / x; }
+__device__ __forceinline__ double step_quot(double a, double x) { return quot_rn(a, x); }
+
 template <typename T>
 __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T dphi, T da0, T db0, T eps,
                                          T& lo, T& hi, T& tau) {
@@ -394,18 +571,18 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
   if (last) {
     const T da = -tau;
     const T s1 = da * da * dpsi;
-    const T c = f - s1 / da;
-    tn = (c != T(0)) ? tau + da + s1 / c : T(0.5) * (lo + hi);
+    const T c = f - step_quot(s1, da);
+    tn = (c != T(0)) ? tau + da + step_quot(s1, c) : T(0.5) * (lo + hi);
   } else {
     const T da = da0 - tau, db = db0 - tau;
     const T s1 = da * da * dpsi, s2 = db * db * dphi;
-    const T c = f - s1 / da - s2 / db;
+    const T c = f - step_quot(s1, da) - step_quot(s2, db);
     const T aq = c, bq = c * (da + db) + s1 + s2, cq = da * db * f;
     const T disc = sqrt(fabs(bq * bq - T(4) * aq * cq));
     T eta;
-    if (aq == T(0)) eta = cq / bq;
-    else if (bq <= T(0)) eta = (bq - disc) / (T(2) * aq);
-    else eta = T(2) * cq / (bq + disc);
+    if (aq == T(0)) eta = step_quot(cq, bq);
+    else if (bq <= T(0)) eta = step_quot(bq - disc, T(2) * aq);
+    else eta = step_quot(T(2) * cq, bq + disc);
     tn = tau + eta;
   }
   if (!(tn > lo && tn < hi)) tn = T(0.5) * (lo + hi);
@@ -413,37 +590,35 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
   return false;
 }
 
-// Root i of the node's secular equation; returns origin (local index) and tau.
-// Phase 1 iterates in FP32 (GB300's FP64 pipe is narrow and these sums are
-// the D&C's dominant cost) to about single precision; phase 2 continues in
-// FP64 from that point inside the FP64 bracket, typically for 1-3 steps, to
-// full accuracy.  A poor FP32 start (clustered poles, range trouble) only
-// costs more FP64 steps: the FP64 phase keeps its own bisection safeguard.
 #ifdef DDCSVD_PHASE_TRACE
 __device__ unsigned g_dc_iters[64 * 84];  // [depth][FP64 iterations 0..80, 81: FP32 phase gave up early]
 #endif
 
-// f at the midpoint of (d_i, d_i+1) on the FP32 copies, with a bound on its
-// error: the copies carry relative error eps32, so the difference
-// del_j = (d_j - d_o)(d_j + d_o) - tau is off by about
-// 3 eps32 ((|d_j| + |d_o|)^2 + |tau|); term j is off by its size times that
-// over |del_j| (plus a few roundings), and the sum by q eps32 of the total.
-// A term whose del_j may change sign, or lies near the FP32 subnormal range
-// (where the copies lose relative precision), makes the bound infinite.
-__device__ __forceinline__ void sec_mid32(int q, const float* d, const float* z, float dorg, float tau,
+// f at the midpoint of (d_i, d_i+1) on the float pairs, with a bound on its
+// error: del_j = (d_j - d_o)(d_j + d_o) - tau carries a relative error of a few
+// eps32 on the product and on tau, plus 2^-47 of |d| in each difference (the
+// pairs' own rounding; tau comes from such a difference too); term j is off by
+// its size times that over |del_j| (plus a few roundings), and the sum by
+// q eps32 of the total.  A term whose del_j may change sign, or lies near the
+// FP32 subnormal range (where the copies lose relative precision), makes the
+// bound infinite.
+__device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z, float2 dorg, float tau,
                                           const LaneGroup& g, float& f, float& err) {
   constexpr float e32 = FLT_EPSILON;
   float s = 0.f, sa = 0.f, ea = 0.f;
   for (int j = g.lg; j < q; j += g.G) {
-    const float dj = d[j];
-    const float del = (dj - dorg) * (dj + dorg) - tau;
-    const float tt = z[j] * z[j] / del;
-    const float ad = fabsf(dj) + fabsf(dorg);
-    const float ed = 3.f * e32 * (ad * ad + fabsf(tau));
-    const float at = fabsf(tt);
+    const float2 dj = d[j];
+    const float ad = fabsf(dj.x) + fabsf(dorg.x);
+    const float dif = pair_diff(dj, dorg);
+    const float del = dif * (dj.x + dorg.x) - tau;
+    const float ir = rcp32(del);
+    const float tt = z[j] * z[j] * ir;
+    const float ed = 4.f * e32 * (fabsf(dif) * ad + fabsf(tau)) + 0x1p-44f * ad * ad;
+    const float at = fabsf(tt), adel = fabsf(del);
     s += tt;
     sa += at;
-    ea += (ed < 0.5f * fabsf(del) && fabsf(del) >= 0x1p-100f) ? at * (2.f * ed / fabsf(del) + 4.f * e32) : INFINITY;
+    ea += (ed < 0.5f * adel && adel >= 0x1p-100f && adel <= 0x1p100f) ? at * (2.5f * ed * fabsf(ir) + 6.f * e32)
+                                                                     : INFINITY;
   }
   s = gsum(s, g);
   sa = gsum(sa, g);
@@ -452,53 +627,113 @@ __device__ __forceinline__ void sec_mid32(int q, const float* d, const float* z,
   err = ea + (float)(q + 2) * e32 * (1.f + sa);
 }
 
-__device__ bool sec_root(int q, const double* d, const double* z, const float* df, const float* zf, double zz,
+// Root i of the node's secular equation; returns its origin pole (local index)
+// and tau = sigma^2 - d_o^2.
+// Phase 1 iterates in FP32 to about single precision.  Phase 2 evaluates f and
+// f' once in FP64 at that point and takes the step x = -u (1 + g u), u = f/f',
+// g = sum z^2/del^3 / f' (Chebyshev's method, third order): with |u / tau| near
+// 1e-6 what is left is below FP64 resolution, so no second evaluation is
+// needed to confirm it.  The estimate of the third-order rest decides; a root
+// it does not clear (clustered poles, range trouble) goes through the
+// safeguarded FP64 iteration from there.  The corrected step counts as two
+// iterations against the caller's cap.
+// kBits iterates both phases with the two-pole model alone.
+template <bool kBits>
+__device__ bool sec_root(int q, const double* d, const double* z, const float2* df, const float* zf, double zz,
                          int i, const LaneGroup& g, int maxit, int* origin, double* tau_out, int* iters = nullptr) {
   double f, psi, dpsi, phi, dphi;
   const bool last = (i == q - 1);
+  const int split = last ? q - 1 : i;
   int o;
-  double lo, hi, tau, da0 = 0.0, db0 = 0.0;
+  float dd32 = 0.f;
+  double dd = 0.0;
   if (!last) {
-    const double dd = (d[i + 1] - d[i]) * (d[i + 1] + d[i]);
-    // origin = nearer pole, from the sign of f at the midpoint: from the FP32
+    // origin = nearer pole, from the sign of f at the midpoint: from the float
     // copies when f clears twice its error bound, else in FP64 (an FP32 sign
     // taken without the bound picked the wrong half on close poles of a
     // batch forest, and the root then lies outside the bracket)
+    const float2 a = df[i], b = df[i + 1];
+    dd32 = pair_diff(b, a) * (b.x + a.x);
     float f32, e32;
-    sec_mid32(q, df, zf, df[i], (float)(0.5 * dd), g, f32, e32);
-    if (fabsf(f32) > 2.f * e32 && fabsf(f32) < INFINITY) {
+    sec_mid32(q, df, zf, a, 0.5f * dd32, g, f32, e32);
+    const bool sure = fabsf(f32) > 2.f * e32 && fabsf(f32) < INFINITY;
+    if (kBits || !sure) dd = (d[i + 1] - d[i]) * (d[i + 1] + d[i]);
+    if (sure) {
       o = (f32 >= 0.f) ? i : i + 1;
     } else {
       sec_eval(q, d, z, d[i], 0.5 * dd, i, g, f, psi, dpsi, phi, dphi);
       o = (f >= 0.0) ? i : i + 1;
     }
-    const double dorg = d[o];
-    if (o == i) { lo = 0.0; hi = 0.5 * dd; tau = 0.5 * dd; }
+  } else {
+    o = q - 1;
+  }
+  *origin = o;
+  const double dorg = d[o];
+  const float2 od = df[o];
+  const bool left = (o == i);  // tau > 0
+  // ---- phase 1: FP32
+  float lo32, hi32, t32, da32, db32;
+  if (kBits) {
+    const double hd = last ? 0.5 * zz : 0.5 * dd;
+    lo32 = left ? 0.f : (float)-hd;
+    hi32 = last ? (float)zz : left ? (float)hd : 0.f;
+    t32 = left ? (float)hd : (float)-hd;
+    da32 = (last || left) ? 0.f : (float)((d[i] - dorg) * (d[i] + dorg));
+    db32 = (last || !left) ? 0.f : (float)((d[i + 1] - dorg) * (d[i + 1] + dorg));
+  } else {
+    lo32 = left ? 0.f : -0.5f * dd32;
+    hi32 = last ? (float)zz : left ? 0.5f * dd32 : 0.f;
+    t32 = last ? 0.5f * hi32 : left ? hi32 : lo32;
+    da32 = (last || left) ? 0.f : -dd32;
+    db32 = (last || !left) ? 0.f : dd32;
+  }
+  bool fine = false;
+  for (int it = 0; it < 40; it++) {
+    float f3, ps3, dps3, ph3, dph3;
+    sec_eval32<kBits>(q, df, zf, od, t32, split, g, f3, ps3, dps3, ph3, dph3);
+    if (!(fabsf(f3) < INFINITY) || !(dps3 < INFINITY) || !(dph3 < INFINITY)) break;
+    if (sec_step<float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32)) {
+      if (!kBits) {
+        const float tn = t32 - f3 / (dps3 + dph3);  // the evaluation's own Newton step is free
+        if (tn > lo32 && tn < hi32) t32 = tn;
+      }
+      fine = true;
+      break;
+    }
+  }
+  // ---- phase 2: one FP64 evaluation and a third-order step
+  if (!kBits && fine && maxit >= 2) {
+    double fp;
+    float g2;
+    const double t0 = (double)t32;
+    sec_eval_newton(q, d, z, dorg, t0, g, f, fp, g2);
+    const double u = quot(f, fp);
+    const float uf = (float)u, un = uf / t32, gr = g2 / (float)fp;
+    const float corr = uf * gr * un;
+    const float rest = fabsf(uf) * un * un * (2.f * gr * gr + 1.f);  // size of the third-order term
+    const double tau = t0 - (u + (double)corr);
+    const float tf = left ? (float)tau : -(float)tau;
+    const float far32 = last ? 1.001f * (float)zz : 0.501f * dd32;
+    if (fabsf(un) <= 1e-3f && rest <= 0x1p-55f * (od.x * od.x + t32) && tf > 0.f && tf <= far32) {
+      if (iters) *iters = 1;
+      *tau_out = tau;
+      return true;
+    }
+  }
+  // ---- the safeguarded FP64 iteration.  A step below 1e-10 |tau| is accepted
+  // without another evaluation: the rational model converges at least
+  // quadratically, so the remaining error is far below FP64 resolution.
+  double lo, hi, tau, da0 = 0.0, db0 = 0.0;
+  if (!last) {
+    if (!kBits) dd = (d[i + 1] - d[i]) * (d[i + 1] + d[i]);
+    if (left) { lo = 0.0; hi = 0.5 * dd; tau = 0.5 * dd; }
     else { lo = -0.5 * dd; hi = 0.0; tau = -0.5 * dd; }
     da0 = (d[i] - dorg) * (d[i] + dorg);
     db0 = (d[i + 1] - dorg) * (d[i + 1] + dorg);
   } else {
-    o = q - 1;
     lo = 0.0; hi = zz; tau = 0.5 * zz;
   }
-  const double dorg = d[o];
-  const int split = last ? q - 1 : i;
-  // ---- phase 1: FP32
-  {
-    float lo32 = (float)lo, hi32 = (float)hi, t32 = (float)tau;
-    const float d32 = df[o], da32 = (float)da0, db32 = (float)db0;
-    for (int it = 0; it < 40; it++) {
-      float f3, ps3, dps3, ph3, dph3;
-      sec_eval32(q, df, zf, d32, t32, split, g, f3, ps3, dps3, ph3, dph3);
-      if (!(fabsf(f3) < INFINITY) || !(dps3 < INFINITY) || !(dph3 < INFINITY)) break;
-      if (sec_step<float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32)) break;
-    }
-    const double t = (double)t32;
-    if (t > lo && t < hi) tau = t;
-  }
-  // ---- phase 2: FP64.  A step below 1e-10 |tau| is accepted without another
-  // evaluation: the rational model converges at least quadratically, so the
-  // remaining error is far below FP64 resolution.
+  if ((double)t32 > lo && (double)t32 < hi) tau = (double)t32;
   bool conv = false;
   int it = 0;
   for (; it < maxit; it++) {
@@ -514,9 +749,105 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float* d
     }
   }
   if (iters) *iters = it;
-  *origin = o;
   *tau_out = tau;
   return conv;
+}
+
+// ---------------------------------------------------------------- P2 - P4, one lane group per root
+// root i = pos - slot of the node at `slot` with q poles
+template <bool kBits>
+__device__ __forceinline__ void dc_root(const DcParams& p, int node, int slot, int pos, int q, int d,
+                                        const LaneGroup& g) {
+  int o, its = 0;
+  double tau;
+  const bool ok = sec_root<kBits>(q, p.dq + slot, p.zq + slot, p.dqf + slot, p.zqf + slot, p.zz[node], pos - slot, g,
+                           p.maxit, &o, &tau, &its);
+#ifdef DDCSVD_PHASE_TRACE
+  if (g.lg == 0 && d < 64) atomicAdd(&g_dc_iters[d * 84 + min(its, 80)], 1u);
+#else
+  (void)its;
+  (void)d;
+#endif
+  if (g.lg == 0) {
+    const double dorg = p.dq[slot + o];
+    p.tau[pos] = tau;
+    p.dor[pos] = dorg;
+    p.rS[pos] = sqrt(dorg * dorg + tau);
+    if (!ok) set_error(p.st, DDCSVD_ERR_NOCONV, pos);
+  }
+}
+
+// z-hat component j = pos - slot (Gu-Eisenstat): the product of
+// (sigma_k^2 - d_j^2) / (d_k^2 - d_j^2).  Without kBits numerators and
+// denominators are multiplied apart with their exponents in an integer (eight
+// FP64 instructions per term; a division in each makes it 13, and the
+// operator's 16).
+template <bool kBits>
+__device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, int q, const LaneGroup& g) {
+  const int j = pos - slot;
+  const double* dq = p.dq + slot;
+  const double* tau = p.tau + slot;
+  const double* dor = p.dor + slot;
+  const double dj = dq[j];
+  double prod, pn = 1.0, pd = 1.0;
+  int en = 0, ed = 0;
+  for (int k = g.lg; k < q - 1; k += g.G) {
+    const double dk = dor[k], dd = dq[(k < j) ? k : k + 1];
+    const double num = tau[k] - (dj - dk) * (dj + dk);
+    const double den = (dd - dj) * (dd + dj);
+    if (kBits) {
+      pn *= quot_rn(num, den);
+    } else {
+      pn = take_exponent(pn * num, en);
+      pd = take_exponent(pd * den, ed);
+    }
+  }
+  prod = gprod(kBits ? pn : quot(pn, pd), g);
+  int ex = kBits ? 0 : gsum(en - ed, g);
+  if (g.lg == 0) {
+    const double dk = dor[q - 1];
+    prod *= tau[q - 1] - (dj - dk) * (dj + dk);
+    double a;
+    if (kBits) {
+      a = sqrt(fabs(prod));
+    } else {
+      prod = take_exponent(prod, ex);
+      if (ex & 1) { prod *= 2.0; ex -= 1; }
+      a = ldexp(sqrt(fabs(prod)), ex / 2);
+    }
+    p.zh[pos] = (p.zq[pos] >= 0.0) ? a : -a;
+  }
+}
+
+// first / last rows of the merged right vector of root i = pos - slot
+template <bool kBits>
+__device__ __forceinline__ void dc_rows(const DcParams& p, int slot, int pos, int q, const LaneGroup& g) {
+  const double* dq = p.dq + slot;
+  const double* zh = p.zh + slot;
+  const double* fq = p.fq + slot;
+  const double* lq = p.lq + slot;
+  const double dorg = p.dor[pos], ti = p.tau[pos];
+  double nv = 0.0, sf = 0.0, sl = 0.0;
+  for (int j = g.lg; j < q; j += g.G) {
+    const double dj = dq[j];
+    const double del = (dj - dorg) * (dj + dorg) - ti;
+    const double v = quotient<kBits>(zh[j], del);
+    nv += v * v;
+    sf += v * fq[j];
+    sl += v * lq[j];
+  }
+  nv = gsum(nv, g); sf = gsum(sf, g); sl = gsum(sl, g);
+  if (g.lg == 0) {
+    if (kBits) {
+      nv = sqrt(nv);
+      p.rF[pos] = quot_rn(sf, nv);
+      p.rL[pos] = quot_rn(sl, nv);
+    } else {
+      nv = rsqrt(nv);
+      p.rF[pos] = sf * nv;
+      p.rL[pos] = sl * nv;
+    }
+  }
 }
 
 // merge node at depth d containing slot position pos (or -1)
@@ -534,7 +865,7 @@ __device__ __forceinline__ int find_node(const DcParams& p, int d, int pos) {
 }
 
 // ---------------------------------------------------------------- P5 final merge
-template <class Grp>
+template <bool kBits, class Grp>
 __device__ void dc_finish_node(const DcParams& p, int node, int par, bool rows, const Grp& grp) {
   const int t = grp.rank(), nt = grp.size();
   const int nn = p.nd_nn[node], slot = p.nd_slot[node];
@@ -544,32 +875,63 @@ __device__ void dc_finish_node(const DcParams& p, int node, int par, bool rows, 
   double* sig = p.sig[par] + slot;
   double* F = p.F[par] + slot;
   double* L = p.L[par] + slot;
+  double nf = 1.0, nl = 1.0;
+  if (rows && !kBits) {  // the norms first, then one write of the scaled rows
+    double sf = 0.0, sl = 0.0;
+    for (int k = t; k < q; k += nt) {
+      const double f = p.rF[slot + k], l = p.rL[slot + k];
+      sf += f * f;
+      sl += l * l;
+    }
+    for (int k = t; k < nd; k += nt) {
+      const double f = p.fd[slot + k], l = p.ld[slot + k];
+      sf += f * f;
+      sl += l * l;
+    }
+    nf = grp.sum(sf);
+    nl = grp.sum(sl);
+    const double ph = p.phi[node], ps = p.psi[node];
+    grp.inv_norms(&nf, ph, &nl, ps);
+    if (t == 0) {
+      p.phi[node] = ph * nf;
+      p.psi[node] = ps * nl;
+    }
+  }
   for (int k = t; k < q; k += nt) {
     const int pos = k + count_lt(dd, nd, rs[k]);
     sig[pos] = rs[k];
-    if (rows) { F[pos] = p.rF[slot + k]; L[pos] = p.rL[slot + k]; }
+    if (rows) {
+      const double f = p.rF[slot + k], l = p.rL[slot + k];
+      F[pos] = kBits ? f : f * nf;
+      L[pos] = kBits ? l : l * nl;
+    }
   }
   for (int k = t; k < nd; k += nt) {
     const int pos = k + count_le(rs, q, dd[k]);
     sig[pos] = dd[k];
-    if (rows) { F[pos] = p.fd[slot + k]; L[pos] = p.ld[slot + k]; }
+    if (rows) {
+      const double f = p.fd[slot + k], l = p.ld[slot + k];
+      F[pos] = kBits ? f : f * nf;
+      L[pos] = kBits ? l : l * nl;
+    }
   }
-  if (!rows) return;
+  if (!rows || !kBits) return;
+  // kBits: the sums over the merged order, square roots and divisions
   grp.sync();
   double sf = 0.0, sl = 0.0;
   for (int k = t; k < nn; k += nt) { sf += F[k] * F[k]; sl += L[k] * L[k]; }
   sf = grp.sum(sf);
   sl = grp.sum(sl);
   const double ph = p.phi[node], ps = p.psi[node];
-  const double nf = sqrt(sf + ph * ph), nl = sqrt(sl + ps * ps);
+  grp.norms(&sf, ph, &sl, ps);
   for (int k = t; k < nn; k += nt) {
-    if (nf > 0.0) F[k] /= nf;
-    if (nl > 0.0) L[k] /= nl;
+    if (sf > 0.0) F[k] = quot_rn(F[k], sf);
+    if (sl > 0.0) L[k] = quot_rn(L[k], sl);
   }
   grp.sync();
   if (t == 0) {
-    if (nf > 0.0) p.phi[node] = ph / nf;
-    if (nl > 0.0) p.psi[node] = ps / nl;
+    if (sf > 0.0) p.phi[node] = quot_rn(ph, sf);
+    if (sl > 0.0) p.psi[node] = quot_rn(ps, sl);
   }
 }
 
@@ -590,13 +952,16 @@ __device__ unsigned long long g_dc_trace[64 * 16];
   } while (0)
 #endif
 
+template <bool kBits>
 __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
   __shared__ int shi[40];
   __shared__ double shd[40];
   const int t = threadIdx.x, lane = t & 31;
-  const int gw = (blockIdx.x * blockDim.x + t) >> 5;
+  // warps numbered across the CTAs first: a depth with fewer lane groups than
+  // the grid holds puts one warp on every scheduler before a second on any
+  const int gw = (t >> 5) * gridDim.x + blockIdx.x;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int gt = blockIdx.x * blockDim.x + t, nthreads = gridDim.x * blockDim.x;
+  const int gt = gw * 32 + lane, nthreads = gridDim.x * blockDim.x;
   for (int d = p.maxdepth; d >= 0; d--) {
     const int par = d & 1;
     const bool rows = d > 0;
@@ -614,43 +979,27 @@ __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
     {
       const CtaGroup cg{shi, shd};
       for (int mi = p.dm_start[d] + blockIdx.x; mi < p.dm_start[d + 1]; mi += gridDim.x)
-        if (p.nd_nn[p.depth_merge[mi]] > kWarpNode) dc_setup_node(p, p.depth_merge[mi], par, cg);
+        if (p.nd_nn[p.depth_merge[mi]] > kWarpNode) dc_setup_node<kBits>(p, p.depth_merge[mi], par, cg);
       const WarpGroup wg;
       for (int mi = p.dm_start[d] + gw; mi < p.dm_start[d + 1]; mi += nwarps)
-        if (p.nd_nn[p.depth_merge[mi]] <= kWarpNode) dc_setup_node(p, p.depth_merge[mi], par, wg);
+        if (p.nd_nn[p.depth_merge[mi]] <= kWarpNode) dc_setup_node<kBits>(p, p.depth_merge[mi], par, wg);
     }
     if (p.dm_start[d + 1] == p.dm_start[d]) {  // only leaves at this depth
       if (d > 0 && !grid_sync(p.bar, p.P, p.st, 600 + d)) return;
       continue;
     }
+    const LaneGroup g = make_group(p.dgroup[d], lane);
+    const int gid = gt / g.G, ngroups = nthreads / g.G;
+    const int node0 = gid < p.N ? find_node(p, d, gid) : -1;  // the forest does not change: ahead of the barrier
     DMARK(1);
     if (!grid_sync(p.bar, p.P, p.st, 100 + d)) return;
     DMARK(2);
     // ---- P2 secular roots (lane group per root)
-    const LaneGroup g = make_group(p.dgroup[d], lane);
-    const int gid = gt / g.G, ngroups = nthreads / g.G;
     for (int pos = gid; pos < p.N; pos += ngroups) {
-      const int node = find_node(p, d, pos);
+      const int node = (pos == gid) ? node0 : find_node(p, d, pos);
       if (node < 0) continue;
-      const int slot = p.nd_slot[node], i = pos - slot, q = p.nq[node];
-      if (i >= q) continue;
-      int o;
-      double tau;
-      int its = 0;
-      bool ok = sec_root(q, p.dq + slot, p.zq + slot, p.dqf + slot, p.zqf + slot, p.zz[node], i, g, p.maxit, &o,
-                         &tau, &its);
-#ifdef DDCSVD_PHASE_TRACE
-      if (g.lg == 0 && d < 64) atomicAdd(&g_dc_iters[d * 84 + min(its, 80)], 1u);
-#else
-      (void)its;
-#endif
-      if (g.lg == 0) {
-        p.org[pos] = o;
-        p.tau[pos] = tau;
-        const double dorg = p.dq[slot + o];
-        p.rS[pos] = sqrt(dorg * dorg + tau);
-        if (!ok) set_error(p.st, DDCSVD_ERR_NOCONV, pos);
-      }
+      const int slot = p.nd_slot[node], q = p.nq[node];
+      if (pos - slot < q) dc_root<kBits>(p, node, slot, pos, q, d, g);
     }
     DMARK(3);
     if (rows) {
@@ -658,56 +1007,20 @@ __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
       DMARK(4);
       // ---- P3 z-hat (lane group per component)
       for (int pos = gid; pos < p.N; pos += ngroups) {
-        const int node = find_node(p, d, pos);
+        const int node = (pos == gid) ? node0 : find_node(p, d, pos);
         if (node < 0) continue;
-        const int slot = p.nd_slot[node], j = pos - slot, q = p.nq[node];
-        if (j >= q) continue;
-        const double* dq = p.dq + slot;
-        const double* tau = p.tau + slot;
-        const int* org = p.org + slot;
-        const double dj = dq[j];
-        double prod = 1.0;
-        for (int k = g.lg; k < q - 1; k += g.G) {
-          const int ok = org[k];
-          const double num = tau[k] - (dj - dq[ok]) * (dj + dq[ok]);
-          const int kk = (k < j) ? k : k + 1;
-          const double den = (dq[kk] - dj) * (dq[kk] + dj);
-          prod *= num / den;
-        }
-        prod = gprod(prod, g);
-        if (g.lg == 0) {
-          const int ol = org[q - 1];
-          prod *= tau[q - 1] - (dj - dq[ol]) * (dj + dq[ol]);
-          const double a = sqrt(fabs(prod));
-          p.zh[pos] = (p.zq[pos] >= 0.0) ? a : -a;
-        }
+        const int slot = p.nd_slot[node], q = p.nq[node];
+        if (pos - slot < q) dc_zhat<kBits>(p, slot, pos, q, g);
       }
       DMARK(5);
       if (!grid_sync(p.bar, p.P, p.st, 300 + d)) return;
       DMARK(6);
       // ---- P4 rows of the merged right vectors (lane group per root)
       for (int pos = gid; pos < p.N; pos += ngroups) {
-        const int node = find_node(p, d, pos);
+        const int node = (pos == gid) ? node0 : find_node(p, d, pos);
         if (node < 0) continue;
-        const int slot = p.nd_slot[node], i = pos - slot, q = p.nq[node];
-        if (i >= q) continue;
-        const double* dq = p.dq + slot;
-        const double dorg = dq[p.org[pos]], ti = p.tau[pos];
-        double nv = 0.0, sf = 0.0, sl = 0.0;
-        for (int j = g.lg; j < q; j += g.G) {
-          const double dj = dq[j];
-          const double del = (dj - dorg) * (dj + dorg) - ti;
-          const double v = p.zh[slot + j] / del;
-          nv += v * v;
-          sf += v * p.fq[slot + j];
-          sl += v * p.lq[slot + j];
-        }
-        nv = gsum(nv, g); sf = gsum(sf, g); sl = gsum(sl, g);
-        if (g.lg == 0) {
-          nv = sqrt(nv);
-          p.rF[pos] = sf / nv;
-          p.rL[pos] = sl / nv;
-        }
+        const int slot = p.nd_slot[node], q = p.nq[node];
+        if (pos - slot < q) dc_rows<kBits>(p, slot, pos, q, g);
       }
     }
     DMARK(7);
@@ -717,10 +1030,10 @@ __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
     {
       const CtaGroup cg{shi, shd};
       for (int mi = p.dm_start[d] + blockIdx.x; mi < p.dm_start[d + 1]; mi += gridDim.x)
-        if (p.nd_nn[p.depth_merge[mi]] > kWarpNode) dc_finish_node(p, p.depth_merge[mi], par, rows, cg);
+        if (p.nd_nn[p.depth_merge[mi]] > kWarpNode) dc_finish_node<kBits>(p, p.depth_merge[mi], par, rows, cg);
       const WarpGroup wg;
       for (int mi = p.dm_start[d] + gw; mi < p.dm_start[d + 1]; mi += nwarps)
-        if (p.nd_nn[p.depth_merge[mi]] <= kWarpNode) dc_finish_node(p, p.depth_merge[mi], par, rows, wg);
+        if (p.nd_nn[p.depth_merge[mi]] <= kWarpNode) dc_finish_node<kBits>(p, p.depth_merge[mi], par, rows, wg);
     }
     DMARK(9);
     if (d > 0 && !grid_sync(p.bar, p.P, p.st, 500 + d)) return;
@@ -792,10 +1105,10 @@ __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, 
       {
         const CtaGroup cg{shi, shd};
         for (int x = lo; x < mid; x++)
-          if (p.nd_nn[tr.nodes[x]] > kWarpNode) dc_setup_node(p, tr.nodes[x], par, cg);
+          if (p.nd_nn[tr.nodes[x]] > kWarpNode) dc_setup_node<true>(p, tr.nodes[x], par, cg);
         const WarpGroup wg;
         for (int x = lo + wid; x < mid; x += nw)
-          if (p.nd_nn[tr.nodes[x]] <= kWarpNode) dc_setup_node(p, tr.nodes[x], par, wg);
+          if (p.nd_nn[tr.nodes[x]] <= kWarpNode) dc_setup_node<true>(p, tr.nodes[x], par, wg);
       }
       __syncthreads();
       const LaneGroup g = make_group(tr.seg_G[k], lane);
@@ -806,19 +1119,8 @@ __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, 
       for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
         const int node = seg_find(p, tr.nodes, lo, mid, pos);
         if (node < 0) continue;
-        const int slot = p.nd_slot[node], i = pos - slot, q = p.nq[node];
-        if (i >= q) continue;
-        int o;
-        double tau;
-        const bool ok =
-            sec_root(q, p.dq + slot, p.zq + slot, p.dqf + slot, p.zqf + slot, p.zz[node], i, g, p.maxit, &o, &tau);
-        if (g.lg == 0) {
-          p.org[pos] = o;
-          p.tau[pos] = tau;
-          const double dorg = p.dq[slot + o];
-          p.rS[pos] = sqrt(dorg * dorg + tau);
-          if (!ok) set_error(p.st, DDCSVD_ERR_NOCONV, pos);
-        }
+        const int slot = p.nd_slot[node], q = p.nq[node];
+        if (pos - slot < q) dc_root<true>(p, node, slot, pos, q, d, g);
       }
       __syncthreads();
       if (rows) {
@@ -826,52 +1128,16 @@ __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, 
         for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
           const int node = seg_find(p, tr.nodes, lo, mid, pos);
           if (node < 0) continue;
-          const int slot = p.nd_slot[node], j = pos - slot, q = p.nq[node];
-          if (j >= q) continue;
-          const double* dq = p.dq + slot;
-          const double* tau = p.tau + slot;
-          const int* org = p.org + slot;
-          const double dj = dq[j];
-          double prod = 1.0;
-          for (int kk = g.lg; kk < q - 1; kk += g.G) {
-            const int ok = org[kk];
-            const double num = tau[kk] - (dj - dq[ok]) * (dj + dq[ok]);
-            const int k2 = (kk < j) ? kk : kk + 1;
-            const double den = (dq[k2] - dj) * (dq[k2] + dj);
-            prod *= num / den;
-          }
-          prod = gprod(prod, g);
-          if (g.lg == 0) {
-            const int ol = org[q - 1];
-            prod *= tau[q - 1] - (dj - dq[ol]) * (dj + dq[ol]);
-            const double a = sqrt(fabs(prod));
-            p.zh[pos] = (p.zq[pos] >= 0.0) ? a : -a;
-          }
+          const int slot = p.nd_slot[node], q = p.nq[node];
+          if (pos - slot < q) dc_zhat<true>(p, slot, pos, q, g);
         }
         __syncthreads();
         // ---- rows of the merged right vectors (lane group per root)
         for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
           const int node = seg_find(p, tr.nodes, lo, mid, pos);
           if (node < 0) continue;
-          const int slot = p.nd_slot[node], i = pos - slot, q = p.nq[node];
-          if (i >= q) continue;
-          const double* dq = p.dq + slot;
-          const double dorg = dq[p.org[pos]], ti = p.tau[pos];
-          double nv = 0.0, sf = 0.0, sl = 0.0;
-          for (int j = g.lg; j < q; j += g.G) {
-            const double dj = dq[j];
-            const double del = (dj - dorg) * (dj + dorg) - ti;
-            const double v = p.zh[slot + j] / del;
-            nv += v * v;
-            sf += v * p.fq[slot + j];
-            sl += v * p.lq[slot + j];
-          }
-          nv = gsum(nv, g); sf = gsum(sf, g); sl = gsum(sl, g);
-          if (g.lg == 0) {
-            nv = sqrt(nv);
-            p.rF[pos] = sf / nv;
-            p.rL[pos] = sl / nv;
-          }
+          const int slot = p.nd_slot[node], q = p.nq[node];
+          if (pos - slot < q) dc_rows<true>(p, slot, pos, q, g);
         }
         __syncthreads();
       }
@@ -879,18 +1145,14 @@ __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, 
       {
         const CtaGroup cg{shi, shd};
         for (int x = lo; x < mid; x++)
-          if (p.nd_nn[tr.nodes[x]] > kWarpNode) dc_finish_node(p, tr.nodes[x], par, rows, cg);
+          if (p.nd_nn[tr.nodes[x]] > kWarpNode) dc_finish_node<true>(p, tr.nodes[x], par, rows, cg);
         const WarpGroup wg;
         for (int x = lo + wid; x < mid; x += nw)
-          if (p.nd_nn[tr.nodes[x]] <= kWarpNode) dc_finish_node(p, tr.nodes[x], par, rows, wg);
+          if (p.nd_nn[tr.nodes[x]] <= kWarpNode) dc_finish_node<true>(p, tr.nodes[x], par, rows, wg);
       }
       __syncthreads();
     }
   }
-}
-
-__global__ void dc_copy_out(int N, const double* s, double* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) out[i] = s[i];
 }
 
 // ---------------------------------------------------------------- host: forest
@@ -1044,12 +1306,12 @@ size_t dc_max_ints(int N) { return 9 * (size_t)(2 * N + 8) + 2 * 64 + 16 + 2 * (
 
 
 int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, double* sigma,
-             const DcHost* H, const int* dints, Arena& a, bool plan_only) {
+             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits) {
   if (N <= 0) return DDCSVD_ERR_ARG;
   const int maxnodes = 2 * N + 8;
-  int* scratch_ints = a.take<int>((size_t)N * 2 + maxnodes);
+  int* scratch_ints = a.take<int>((size_t)N + maxnodes);
   double* dbl = a.take<double>((size_t)N * 25 + 3 * (size_t)maxnodes + 8);
-  float* flt = a.take<float>((size_t)N * 2 + 8);
+  float* flt = a.take<float>((size_t)N * 3 + 8);
   GridBarrier* bar = a.take<GridBarrier>(4);
   if (plan_only) return DDCSVD_OK;
   const int nnodes = H->nnodes, md = H->maxdepth;
@@ -1067,19 +1329,19 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
   p.dm_start = dints + o; o += md + 2;
   p.depth_merge = dints + o; o += H->ndm;
   p.dgroup = dints + o; o += md + 2;
-  p.org = scratch_ints;
-  p.defl = scratch_ints + N;
-  p.nq = scratch_ints + 2 * (size_t)N;
+  p.defl = scratch_ints;
+  p.nq = scratch_ints + N;
   p.b1 = b1; p.b2 = b2;
   double* q = dbl;
-  for (int k = 0; k < 2; k++) { p.sig[k] = q; q += N; p.F[k] = q; q += N; p.L[k] = q; q += N; }
+  p.sig[0] = sigma;  // depth 0 writes the result in place
+  p.sig[1] = q; q += N;
+  for (int k = 0; k < 2; k++) { p.F[k] = q; q += N; p.L[k] = q; q += N; }
   p.ds = q; q += N; p.zs = q; q += N; p.hfs = q; q += N; p.hls = q; q += N;
   p.dq = q; q += N; p.zq = q; q += N; p.fq = q; q += N; p.lq = q; q += N;
   p.dd = q; q += N; p.fd = q; q += N; p.ld = q; q += N;
-  p.tau = q; q += N; p.zh = q; q += N; p.rS = q; q += N; p.rF = q; q += N; p.rL = q; q += N;
+  p.tau = q; q += N; p.dor = q; q += N; p.zh = q; q += N; p.rS = q; q += N; p.rF = q; q += N; p.rL = q; q += N;
   p.zz = q; q += maxnodes; p.phi = q; q += maxnodes; p.psi = q; q += maxnodes;
-  p.dqf = flt; p.zqf = flt + N;
-  p.out = sigma;
+  p.dqf = reinterpret_cast<float2*>(flt); p.zqf = flt + 2 * (size_t)N;
   p.bar = bar;
   p.st = ctx->d_status;
   // a forest of many small trees: whole trees per CTA, no grid barriers
@@ -1104,27 +1366,24 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
     dc_tree_kernel<<<grid, kDcTreeThreads, 0, ctx->stream>>>(p, tr);
     ktimer_end(ctx);
     count_launch();
-    dc_copy_out<<<std::min(ceil_div(N, 256), 1024), 256, 0, ctx->stream>>>(N, p.sig[0], sigma);
-    count_launch();
     DDC_CUDA_TRY(cudaGetLastError());
     return DDCSVD_OK;
   }
   int occ = 0;
-  DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dc_kernel, kDcThreads, 0));
+  const void* kern = keep_bits ? (const void*)dc_kernel<true> : (const void*)dc_kernel<false>;
+  DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kDcThreads, 0));
   if (occ < 1) {
     set_last_error("dc_kernel cannot be resident");
     return DDCSVD_ERR_CUDA;
   }
-  const int P = std::min(ctx->num_sms, std::max(1, ceil_div(N, 16)));
+  const int P = std::min(ctx->num_sms, std::max(1, ceil_div(N, 4)));
   p.P = P;
   DDC_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), ctx->stream));
   void* argv[] = {&p};
   ktimer_begin(ctx, KC_DC);
-  DDC_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)dc_kernel, dim3(P), dim3(kDcThreads), argv, 0,
+  DDC_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(P), dim3(kDcThreads), argv, 0,
                                            ctx->stream));
   ktimer_end(ctx);
-  count_launch();
-  dc_copy_out<<<std::min(ceil_div(N, 256), 1024), 256, 0, ctx->stream>>>(N, p.sig[0], sigma);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;

@@ -197,8 +197,9 @@ struct DcHost {
 };
 void dc_build_host(int N, const std::vector<int>& block_starts, DcHost& H, int terms_per_lane = 8);
 size_t dc_max_ints(int N);
+// keep_bits: every FP64 rounding of the plain formulas kept (dc.cu says why)
 int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, double* sigma,
-             const DcHost* H, const int* dints, Arena& a, bool plan_only);
+             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits);
 
 // Splits the N x N bidiagonal (host copies a[N], b[N]) at |b_i| <= 4 eps max|B|:
 // zeroes those b_i (and b[N-1]), fills block_starts (ascending, ends with N)
