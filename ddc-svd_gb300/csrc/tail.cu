@@ -1,399 +1,485 @@
 // tail.cu -- the last columns of the blocked bidiagonalisation on one
-// thread-block cluster.
+// thread-block cluster, the trailing block in registers.
 //
 // Once the trailing block W[k0:m, k0:n] of the panel factorisation is small
-// enough to live in the distributed shared memory of one cluster (C CTAs,
-// C = 16 where the GPU can co-schedule that many, else 8), the remaining
-// columns no longer pay the grid-wide costs of the panel kernel (two grid
-// barriers and two reductions over 152 partial records per column, ~9 us at
-// any size).  Here CTA k holds columns k, k + C, k + 2C, ... of the trailing
-// block (cyclic, so the work stays even while columns retire), all rows, in
-// its shared memory and the algorithm is the unblocked one of
-// the reference (bidiag_par.c:310-397, left_update_mat.cl / right_update_mat.cl):
-// per column a left reflector and its rank-1 update, then a right reflector
-// and its rank-1 update, exchanged through distributed shared memory with
-// one hardware cluster barrier per column: the right reflector's products
-// x = A' v are gathered unscaled (v = e_1 + s * row, so x = A'(:, i+1) +
-// s * A'(:, i+2:) row(i+2:)) right after the left update, every CTA adds the
-// C partials for all rows itself, and since column i+1 after the right update
-// is A'(:, i+1) - tau * x, every CTA also forms the next left reflector
-// itself instead of waiting for the column's owner.  Reflector conventions, FP32 compensated
-// norms and the LAPACK-form storage are those of the panel kernel, so the
-// back-transformation reads the result unchanged.
+// enough, the remaining columns no longer pay the grid-wide costs of the panel
+// kernel (two grid barriers and two reductions over 152 partial records per
+// column, ~9 us at any size).  One cluster of C CTAs (up to 16) holds the whole
+// block: row r belongs to one warp (row r to warp r mod 8C of the cluster, so
+// the work stays even while rows retire), lane l of the warp holds its columns
+// l, l + 32, ... in registers.  The algorithm is the unblocked one of the
+// reference (bidiag_par.c:310-397, left_update_mat.cl / right_update_mat.cl): per
+// column a left reflector and its rank-1 update, then a right reflector and its
+// rank-1 update.  Reflector conventions, FP32 compensated norms and the
+// LAPACK-form storage are those of the panel kernel.
 //
-// The unblocked form rewrites the trailing block every column at the shared-
-// memory bandwidth of C SMs, so it only beats the 152-SM panel kernel once
-// the block is small: measured on 4096^2 / 2048^2 / 1024^2 SVDs, handing over
-// the last 512 columns is best (77.4 -> 75.9, 30.2 -> 28.8, 14.8 -> 13.3 ms;
-// the last 384 or 640 columns slightly worse, every column that fits -- ~900
-// at 4096^2 -- slower than none).  A 512 x 256 problem runs here entirely
-// (4.5 -> 3.7 ms).
+// Per column i the block is read and written once, in registers: the left
+// update with (u, tau y), the row's product with v, the right update, and the
+// unscaled products sum_r x_r A[r, c] of the next column x with every column.
+// Between columns the CTAs exchange vectors along c only (the row-shaped
+// vectors never leave their warps):
+//   1. each CTA adds its warps' products and sends them, slice by slice (CTA k
+//      owns the columns 32 k .. 32 k + 31), to the slice's owner, with the
+//      squared norm of its part of x; the warp of row i sends that row;
+//   2. each CTA adds the C partial products of its slice, forms the left
+//      reflector (every CTA the same one, from the same C norms), tau y and the
+//      new row w of its columns, and sends both to every CTA with the slice's
+//      part of ||w||^2; every warp then forms the right reflector.
+// Both exchanges are remote asynchronous stores that complete on the receiver's
+// mbarrier (one way, 340-490 cycles for 2-16 CTAs; stores followed by a hardware
+// cluster barrier, whose release waits for their acknowledgement, measured
+// 690-1200), and a CTA receives 2 nt floats per column.
+//
+// What bounds it: the chain of the two exchanges and of the two norms (sums of
+// records, a square root and quotients each) -- not arithmetic: a 512 x 512
+// block is 32 elements a thread.  The former kernel kept columns instead of
+// rows, in shared memory, and let every CTA read all C partial row-vectors
+// (64 mt bytes per CTA and column through distributed shared memory at ~8
+// bytes a clock).  Us per column, before and now: 64 x 48 3.5 and 1.5, 512 x 256
+// 5.3 and 1.9, 900 x 250 8.5 and 2.3, 1000 x 490 9 and 2.8.
 #include <cooperative_groups.h>
 
+#include "async.cuh"
 #include "internal.hpp"
 
 namespace cg = cooperative_groups;
 
 namespace ddcsvd {
 
-constexpr int kTailThreads = 512;
-
-// phase marks (trace builds): CTA 0, every 8th column, one row per column
-#ifdef DDCSVD_PHASE_TRACE
-__device__ unsigned long long g_tail_trace[128 * 16];
-#define TMARK(slot)                                                                  \
-  do {                                                                               \
-    if (rank == 0 && threadIdx.x == 0 && (i & 7) == 0 && (i >> 3) < 128)             \
-      g_tail_trace[(i >> 3) * 16 + (slot)] = global_ns();                            \
-  } while (0)
-#else
-#define TMARK(slot) \
-  do {              \
-  } while (0)
-#endif
+constexpr int kTailThreads = 256;
+constexpr int kTailWarps = kTailThreads / 32;
+constexpr int kTailMaxC = 16;
 
 struct TailParams {
-  int mt, nt;     // trailing block: rows, columns (mt >= nt)
-  int ncb;        // columns per CTA (at most)
-  float* W;       // trailing block (its row 0 / column 0 = the first tail column)
+  int mt, nt;  // trailing block: rows, columns (mt >= nt)
+  float* W;    // trailing block (its row 0 / column 0 = the first tail column)
   int ldw;
   float *d, *e, *tauq, *taup;  // offset to the first tail column
+  DevStatus* st;
 };
 
-// Shared-memory layout (floats, every section 16-byte aligned): A [mt x ncb]
-// (column-major, ld mt), u, x, xp[2], pc[2] [mt each; xp and pc, the ones
-// other CTAs read, double-buffered by column parity], vrow [ncb], red [32 FF],
-// scal [8], nrm [2 FF].
-__host__ __device__ inline size_t tail_vec_floats(int mt) { return (size_t)((mt + 4 + 3) & ~3); }
-__host__ __device__ inline size_t tail_smem_floats(int mt, int ncb) {
-  return (((size_t)mt * ncb + 3) & ~(size_t)3) + 6 * tail_vec_floats(mt) + (((size_t)ncb + 3) & ~(size_t)3) +
-         64 + 8 + 4;
+// Compensated sums without the final renormalisation of ff_add: the heads by
+// two-sum, the errors added to the tails.  Head, error and tail do not depend
+// on the operands' order, so lanes that add the same pair agree bit for bit.
+__device__ __forceinline__ FF ff_acc(FF a, FF b) {
+  const float s = __fadd_rn(a.hi, b.hi);
+  const float bb = __fsub_rn(s, a.hi);
+  const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));
+  return FF{s, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
+}
+__device__ __forceinline__ FF ff_square(float x) {
+  const float p = __fmul_rn(x, x);
+  return FF{p, __fmaf_rn(x, x, -p)};
+}
+// sum over aligned groups of N lanes
+template <int N>
+__device__ __forceinline__ FF ff_lanes(FF v) {
+#pragma unroll
+  for (int o = N >> 1; o > 0; o >>= 1)
+    v = ff_acc(v, FF{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+  return v;
 }
 
-// CTA-wide compensated sum (fixed order: warp trees, then warps in order).
-__device__ __forceinline__ FF tail_sum_ff(FF v, FF* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  v = warp_sum_ff(v);
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    FF s = lane < nw ? red[lane] : FF{0.f, 0.f};
-    s = warp_sum_ff(s);
-    if (lane == 0) red[0] = s;
-  }
-  __syncthreads();
-  return red[0];
+__device__ __forceinline__ float rcp_approx_f32(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
-// Right update of the own columns l >= lr with (tp, x, row i of A) and then
-// their left update with (tq, u), rows > i, one warp per column: x and u for
-// the lane's rows (i + 1 + lane + 32 j) in registers, each column read and
-// written once.  Row i + 1 of the columns >= the local index lv is gathered
-// into vrow for the next step.  Needs mt - i - 1 <= 32 KR.
-template <int KR>
-__device__ __forceinline__ void tail_fused_update(float* A, int mt, int i, int lr, int nown, float tp, float tq,
-                                                  const float* x, const float* u, float* vrow, int lv) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int rb = i + 1 + lane;
-  float uc[KR], xc[KR];
-#pragma unroll
-  for (int j = 0; j < KR; j++) {
-    const int r = rb + 32 * j;
-    uc[j] = r < mt ? u[r] : 0.f;
-    xc[j] = (r < mt && tp != 0.f) ? x[r] : 0.f;  // x is not formed when tp = 0
-  }
-  for (int l = lr + wid; l < nown; l += nw) {
-    float* col = A + (size_t)l * mt;
-    const float f = tp * col[i];
-    float c[KR];
-    float y = 0.f;
-#pragma unroll
-    for (int j = 0; j < KR; j++) {
-      const int r = rb + 32 * j;
-      c[j] = r < mt ? col[r] - f * xc[j] : 0.f;
-      y += uc[j] * c[j];
+// Remote stores that complete on the target CTA's mbarrier (addresses in the
+// shared::cluster window, from mapa).
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_async(uint32_t dst, float v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
+               "r"(__float_as_uint(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t dst, float a, float b, uint32_t bar) {
+  const unsigned long long v = (unsigned long long)__float_as_uint(b) << 32 | __float_as_uint(a);
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(v), "r"(bar)
+               : "memory");
+}
+// householder_ff with approximate reciprocal and reciprocal square root and one
+// Newton correction each (within an ulp or so; the square root's from the
+// compensated sum itself) in place of the IEEE square root and quotients, whose
+// ~300 cycles stood twice in every column's chain.
+__device__ __forceinline__ void householder_fast(float x0, FF t2, float* alpha, float* tau, float* scale) {
+  const FF n2 = ff_add_sq(t2, x0);
+  const float s = n2.hi;
+  const float r = rsqrtf(s);
+  float nrm = s * r;
+  const float d2 = __fadd_rn(__fmaf_rn(-nrm, nrm, s), n2.lo);
+  nrm = fmaf(0.5f * r, d2, nrm);
+  const float ax = fabsf(x0), den = ax + nrm;
+  float q = rcp_approx_f32(den);
+  q = fmaf(q, fmaf(-den, q, 1.f), q);
+  float ri = r;  // 1 / nrm
+  ri = fmaf(ri, fmaf(-nrm, ri, 1.f), ri);
+  const float sg = x0 < 0.f ? -1.f : 1.f;
+  const bool zero = !(s > 0.f);
+  *alpha = zero ? 0.f : -sg * nrm;
+  *tau = zero ? 0.f : fmaf(ax, ri, 1.f);
+  *scale = zero ? 0.f : sg * q;
+}
+
+// Waits for the phase of the given parity.  Bounded: after kTailWaitNs the
+// status word holds DDCSVD_ERR_TIMEOUT, `dead` stays set in this thread and no
+// later wait of it waits (the column loop runs out with meaningless values).
+constexpr unsigned long long kTailWaitNs = 2000000000ull;
+__device__ __forceinline__ void tail_wait(uint32_t bar, unsigned parity, bool& dead, DevStatus* st) {
+  unsigned long long t0 = 0;
+  for (unsigned polls = 0; !dead; polls++) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n"
+        " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return;
+    if ((polls & 63u) == 63u) {
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kTailWaitNs) {
+        set_error(st, DDCSVD_ERR_TIMEOUT, 700);
+        dead = true;
+      }
     }
-    y = warp_sum(y) * tq;
-#pragma unroll
-    for (int j = 0; j < KR; j++) {
-      const int r = rb + 32 * j;
-      c[j] -= y * uc[j];
-      if (r < mt) col[r] = c[j];
-    }
-    if (lane == 0 && l >= lv) vrow[l - lv] = c[0];
   }
 }
 
+// Sums v[q0 .. q0 + R) over the warp; every lane gets all of them (R a power
+// of two).
+template <int R, int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N], int q0, int lane) {
+  float s[R];
+#pragma unroll
+  for (int q = 0; q < R; q++) s[q] = v[q0 + q];
+#pragma unroll
+  for (int nv = R, off = 16; nv > 1; nv >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int h = 0; h < nv / 2; h++) {
+      const float send = up ? s[h] : s[h + nv / 2];
+      const float keep = up ? s[h + nv / 2] : s[h];
+      s[h] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+#pragma unroll
+  for (int off = 16 / R; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+#pragma unroll
+  for (int q = 0; q < R; q++) v[q0 + q] = __shfl_sync(0xffffffffu, s[0], q * (32 / R));
+}
+
+// R rows per warp, K columns per lane: blocks of up to 8 C R rows and 32 K
+// columns.
+template <int R, int K>
 __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams p) {
-  extern __shared__ __align__(16) float sm[];
+  constexpr int H = R < 4 ? R : 4;   // rows, and columns per lane, whose work is skipped together
+  constexpr int KC = K < 4 ? K : K == 8 ? 8 : 4;  // once they have retired
+  constexpr int NS = (K + 7) / 8;    // slices a warp sends to: wid and wid + 8
+  constexpr int NT = kTailMaxC / kTailWarps;  // CTAs a warp sends to: the same
+  __shared__ float s_part[kTailWarps][32 * K];  // per warp: products of the next column with every column
+  __shared__ FF s_nw[kTailWarps];               // per warp: ||x||^2 of the own rows
+  __shared__ float s_own[32 * K];               // row i, in the CTA that holds it
+  // exchange 1, by column parity: a CTA may send column i + 1's records while
+  // a slower one still reads column i's (never i + 2's: it has then received
+  // something that every CTA sends after its last read of column i)
+  __shared__ __align__(16) float s_in[2][kTailMaxC][32];  // partial products of the own slice by sender
+  __shared__ __align__(16) float s_row[2][32];            // row i of the own slice
+  __shared__ __align__(16) FF s_n1[2][kTailMaxC];         // ||x||^2 by sender
+  __shared__ float s_x0[2];                               // A[i, i]
+  // exchange 2 (sent after exchange 1 has completed, so after every read of
+  // the previous column's)
+  __shared__ __align__(16) float2 s_yw[32 * K];  // (tau y, w) of every column
+  __shared__ __align__(16) FF s_n2[kTailMaxC];   // ||w||^2 over the columns > i + 1 by slice
+  __shared__ __align__(8) uint64_t s_bar[2];
   cg::cluster_group cluster = cg::this_cluster();
-  const int C = (int)cluster.num_blocks();
-  const int rank = (int)cluster.block_rank();
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5, nt_ = blockDim.x;
-  const int mt = p.mt, ncols = p.nt, ncb = p.ncb;
-  // own columns: c = rank + l * C, l < nown (local index l)
-  const int nown = rank < ncols ? (ncols - rank + C - 1) / C : 0;
-  // first local index whose column is >= c
-  auto lfirst = [&](int c) { return c <= rank ? 0 : (c - rank + C - 1) / C; };
-  const size_t vec = tail_vec_floats(mt);
-  float* A = sm;
-  float* u = A + (((size_t)mt * ncb + 3) & ~(size_t)3);
-  float* x = u + vec;
-  float* xp = x + vec;      // [2][vec]
-  float* pc = xp + 2 * vec;  // [2][vec]
-  float* vrow = pc + 2 * vec;
-  FF* red = reinterpret_cast<FF*>(vrow + ((ncb + 3) & ~3));
-  float* scal = reinterpret_cast<float*>(red + 32);
-  FF* nrm = reinterpret_cast<FF*>(scal + 8);  // [2]
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int mt = p.mt, nt = p.nt, ldw = p.ldw;
+  const int GW = kTailWarps * C, gw = wid * C + rank;  // row r: warp r mod GW, slot r / GW
+  const int c_own = 32 * rank + lane;                  // the lane's column of the CTA's slice
+  const int slice_cols = min(32, nt - 32 * rank);      // (<= 0: no slice)
+  const uint32_t bar1 = smem_u32(&s_bar[0]), bar2 = smem_u32(&s_bar[1]);
+  // a shared address of this CTA plus such a difference is the same place in
+  // CTA lane's / CTA (wid + 8 j)'s shared memory
+  const uint32_t to_lane = map_rank(bar1, min(lane, C - 1)) - bar1;
+  uint32_t to_cta[NT];
+#pragma unroll
+  for (int j = 0; j < NT; j++) to_cta[j] = map_rank(bar1, min(wid + 8 * j, C - 1)) - bar1;
+  bool dead = false;
 
-  // Left reflector of column j from u[j..mt) (the column after every earlier
-  // update).  Every CTA forms it from the same values in the same order, so
-  // all hold the same u; the owner of column j also stores it there.
-  auto form_left = [&](int j) {
-    FF s2{0.f, 0.f};
-    for (int r = j + 1 + t; r < mt; r += nt_) s2 = ff_add_sq(s2, u[r]);
-    s2 = tail_sum_ff(s2, red);
-    float alpha, tq, sq;
-    householder_ff(u[j], s2, &alpha, &tq, &sq);
-    __syncthreads();  // u[j] read by every thread before it is overwritten
-    const bool own = j % C == rank;
-    float* col = A + (size_t)(j / C) * mt;
-    for (int r = j + t; r < mt; r += nt_) {
-      const float v = (r == j) ? 1.f : u[r] * sq;
-      u[r] = v;
-      if (own) col[r] = v;
+  float A[R][K];
+#pragma unroll
+  for (int s = 0; s < R; s++)
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const int r = s * GW + gw, c = lane + 32 * k;
+      A[s][k] = (r < mt && c < nt) ? p.W[r + (size_t)c * ldw] : 0.f;
     }
-    if (own && t == 0) {
-      p.d[j] = alpha;
-      p.tauq[j] = tq;
-    }
-    __syncthreads();
-    return tq;
-  };
+  float x[R];  // the current column's entries of the own rows (zero for retired rows)
+#pragma unroll
+  for (int s = 0; s < R; s++) {
+    const float v = __shfl_sync(0xffffffffu, A[s][0], 0);
+    x[s] = (s * GW + gw > 0) ? v : 0.f;
+  }
+  float acc[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    acc[k] = 0.f;
+#pragma unroll
+    for (int s = 0; s < R; s++) acc[k] += x[s] * A[s][k];
+  }
+  // records of absent CTAs and columns read as zero
+  for (int q = t; q < 2 * kTailMaxC * 32; q += kTailThreads) (&s_in[0][0][0])[q] = 0.f;
+  if (t < 2 * kTailMaxC) (&s_n1[0][0])[t] = FF{0.f, 0.f};
+  if (t == 0) {
+    mbar_init(&s_bar[0], 1);
+    mbar_init(&s_bar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster.sync();  // every CTA runs and is ready before the first remote store
 
-  // Left update of the own columns > j with u (warp per column, in shared
-  // memory); row j of the columns > j + 1 gathered into vrow.
-  auto left_update = [&](int j, float tq) {
-    const int l1 = lfirst(j + 1), l2 = lfirst(j + 2);
-    for (int l = l1 + wid; l < nown; l += nw) {
-      float* col = A + (size_t)l * mt;
-      if (tq != 0.f) {
-        float y = 0.f;
-        for (int r = j + lane; r < mt; r += 32) y += u[r] * col[r];
-        y = warp_sum(y) * tq;
-        for (int r = j + lane; r < mt; r += 32) col[r] -= y * u[r];
-      }
-      if (lane == 0 && l >= l2) vrow[l - l2] = col[j];
-    }
-    __syncthreads();
-  };
-
-  // own columns into shared memory; column 0 to every CTA
-  for (int l = 0; l < nown; l++)
-    for (int r = t; r < mt; r += nt_) A[r + (size_t)l * mt] = p.W[r + (size_t)(rank + l * C) * p.ldw];
-  for (int r = t; r < mt; r += nt_) u[r] = p.W[r];
-  __syncthreads();
-  left_update(0, form_left(0));
-  cluster.sync();
-
-  // step i: right reflector of row i, then the left reflector of column i + 1
-  for (int i = 0; i + 1 < ncols; i++) {
+  int islot = 0, iwarp = 0;  // slot and warp of row i
+  for (int i = 0; i < nt; i++) {
     const int b = i & 1;
-    float* xpb = xp + b * vec;
-    float* pcb = pc + b * vec;
-    const int l1 = lfirst(i + 1), l2 = lfirst(i + 2);
-    const int own_next = (i + 1) % C;  // rank owning column i + 1
-    TMARK(0);
-    // ---- B: per row r > i the unscaled partial product of the right
-    // reflector's x over the own columns >= i + 2, the partial squared norm of
-    // row i over them, and column i + 1 copied (its owner replaces it in C
-    // while the other CTAs still read it)
+    const unsigned ph = (unsigned)(i & 1);  // both barriers complete one phase per column
+    const int kf = (i + 1) >> 5;            // first slice with a column > i
+    const bool mine = gw == iwarp;          // this warp holds row i
+    // ---- exchange 1: products of column i, its norm, row i
+    if (t == 0) {
+      unsigned bytes = 8u * C + 4u;
+      if (rank >= kf && slice_cols > 0) bytes += 4u * (C + 1) * slice_cols;
+      mbar_arrive_expect_tx(&s_bar[0], bytes);
+      if (i < nt - 1)
+        mbar_arrive_expect_tx(&s_bar[1], 8u * (unsigned)((nt + 31) / 32 - kf) + 8u * (unsigned)(nt - 32 * kf));
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) s_part[wid][lane + 32 * k] = acc[k];
     {
-      const int nz = nown - l2;
-      const float* cnext = A + (size_t)((i + 1) / C) * mt;
-      for (int r = i + 1 + t; r < mt; r += nt_) {
-        const float* ar = A + r + (size_t)l2 * mt;
-        float z = 0.f;
-        for (int j = 0; j < nz; j++) z += ar[(size_t)j * mt] * vrow[j];
-        xpb[r] = z;
-      }
-      if (rank == own_next)
-        for (int r = i + t; r < mt; r += nt_) pcb[r] = cnext[r];
-      if (wid == nw - 1) {
-        FF s{0.f, 0.f};
-        for (int j = lane; j < nz; j += 32) s = ff_add_sq(s, vrow[j]);
-        s = warp_sum_ff(s);
-        if (lane == 0) nrm[b] = s;
+      FF n[R];
+#pragma unroll
+      for (int s = 0; s < R; s++) n[s] = ff_square(x[s]);
+#pragma unroll
+      for (int m = R; m > 1; m = (m + 1) / 2)
+#pragma unroll
+        for (int s = 0; s < m / 2; s++) n[s] = ff_acc(n[s], n[s + (m + 1) / 2]);
+      if (lane == 0) s_nw[wid] = n[0];
+    }
+    if (mine) {
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        if (r == islot) {
+#pragma unroll
+          for (int k = 0; k < K; k++) s_own[lane + 32 * k] = A[r][k];
+        }
+    }
+    __syncthreads();
+    const bool holds = rank == (iwarp & (C - 1));  // row i is in this CTA
+#pragma unroll
+    for (int j = 0; j < NS; j++) {
+      const int c = t + kTailThreads * j;  // warp wid: slice wid + 8 j
+      if (c >= 32 * kf && c < nt) {
+        float v[kTailWarps];
+#pragma unroll
+        for (int w = 0; w < kTailWarps; w++) v[w] = s_part[w][c];
+        if (holds) st_async(smem_u32(&s_row[b][lane]) + to_cta[j], s_own[c], bar1 + to_cta[j]);
+        const float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        st_async(smem_u32(&s_in[b][rank][lane]) + to_cta[j], sum, bar1 + to_cta[j]);
       }
     }
-    TMARK(1);
-    cluster.sync();  // partial norms, partial products and column i + 1 published
-    TMARK(2);
-    // ---- C: right reflector from row i (every CTA forms it; warp 0), and
-    // x = a'(:, i+1) + sp * (sum of the C partial products) with the next
-    // column a'(:, i+1) - tp * x, for all rows in every CTA: rows in aligned
-    // groups of four (the vectors are padded past mt), four lanes per group
-    // adding a quarter of the partials each
-    const float* pn = cluster.map_shared_rank(pcb, own_next);
-    const int r0 = (i + 1) & ~3;
-    const int ngr = (mt - r0 + 3) >> 2;
-    const int part = t & 3;
-    auto right_reflector = [&](FF v, float x0) {  // warp 0; v: lane t < C holds CTA t's norm partial
-      const FF tot = warp_sum_ff(v);
-      float beta, tpv, spv;
-      if (i < ncols - 2) {
-        householder_ff(x0, tot, &beta, &tpv, &spv);
-      } else {  // one element left: no reflection (bidiag.c:125-129)
-        beta = x0;
-        tpv = 0.f;
-        spv = 0.f;
+    if (wid == kTailWarps - 1) {
+      const FF n = ff_lanes<kTailWarps>(s_nw[lane & (kTailWarps - 1)]);
+      if (lane < C) {
+        st_async(smem_u32(&s_n1[b][rank]) + to_lane, n.hi, n.lo, bar1 + to_lane);
+        if (holds) st_async(smem_u32(&s_x0[b]) + to_lane, s_own[i], bar1 + to_lane);
       }
-      if (t == 0) {
-        if (rank == 0) {
-          p.e[i] = beta;
-          p.taup[i] = tpv;
-        }
-        scal[1] = tpv;
-        scal[2] = spv;
+    }
+    tail_wait(bar1, ph, dead, p.st);
+    // ---- left reflector, and exchange 2: tau y and the new row of the own
+    // slice (every warp forms them; warp w sends them to the CTAs w, w + 8)
+    float alpha, tq, sq, w = 0.f;
+    {
+      const FF n1 = ff_lanes<kTailMaxC>(s_n1[b][lane & (kTailMaxC - 1)]);
+      const bool in = c_own < nt && c_own > i;
+      float v[kTailMaxC];
+#pragma unroll
+      for (int q = 0; q < kTailMaxC; q++) v[q] = s_in[b][q][lane];
+#pragma unroll
+      for (int h = kTailMaxC / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int q = 0; q < h; q++) v[q] += v[q + h];
+      const float row = s_row[b][lane];
+      householder_fast(s_x0[b], n1, &alpha, &tq, &sq);
+      const float ty = in ? tq * (row + sq * v[0]) : 0.f;
+      w = in ? row - ty : 0.f;
+      if (i < nt - 1 && rank >= kf && slice_cols > 0) {
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+          if (c_own < nt && wid + 8 * j < C)
+            st_async(smem_u32(&s_yw[c_own]) + to_cta[j], ty, w, bar2 + to_cta[j]);
+        const FF n2 = ff_lanes<32>(c_own > i + 1 ? ff_square(w) : FF{0.f, 0.f});
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+          if (lane == 0 && wid + 8 * j < C)
+            st_async(smem_u32(&s_n2[rank]) + to_cta[j], n2.hi, n2.lo, bar2 + to_cta[j]);
       }
-    };
-    auto zsum = [&](int r, bool load) {  // the group's rows summed over the C partials (all four lanes)
-      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (load) {
-        for (int k = part; k < C; k += 4) {
-          const float4 q = *reinterpret_cast<const float4*>(cluster.map_shared_rank(xpb, k) + r);
-          z.x += q.x;
-          z.y += q.y;
-          z.z += q.z;
-          z.w += q.w;
-        }
+    }
+    if (rank == 0 && t == 0) {
+      p.d[i] = alpha;
+      p.tauq[i] = tq;
+    }
+    // column i of W: 1 on the diagonal, u below
+    {
+      float v = 0.f;
+#pragma unroll
+      for (int s = 0; s < R; s++) {
+        x[s] *= sq;  // now u
+        if (lane == s) v = x[s];
+      }
+      const int r = lane * GW + gw;
+      if (lane < R && r >= i && r < mt) p.W[r + (size_t)i * ldw] = (r == i) ? 1.f : v;
+    }
+    if (i == nt - 1) break;
+    tail_wait(bar2, ph, dead, p.st);
+    // ---- right reflector (every warp); row i of W
+    float tp = 0.f, sp = 0.f;
+    {
+      const float w1 = s_yw[i + 1].y;
+      float beta = w1;  // one element left: no reflection (bidiag.c:125-129)
+      if (i < nt - 2) {
+        const int q = lane & (kTailMaxC - 1);
+        const FF n2 = ff_lanes<kTailMaxC>((q >= kf && 32 * q < nt) ? s_n2[q] : FF{0.f, 0.f});
+        householder_fast(w1, n2, &beta, &tp, &sp);
+      }
+      if (rank == 0 && t == 0) {
+        p.e[i] = beta;
+        p.taup[i] = tp;
+      }
+      if (wid == 1 && c_own > i && c_own < nt)
+        p.W[i + (size_t)c_own * ldw] = (c_own == i + 1) ? (tp != 0.f ? 1.f : 0.f) : sp * w;
+    }
+    // ---- left update, products with v = (1, sp w), per row
+    float z[R], nx[R];
+#pragma unroll
+    for (int s = 0; s < R; s++) z[s] = nx[s] = 0.f;
+    auto vcol = [&](int c, float wv) { return (c == i + 1) ? 1.f : (c > i + 1 && c < nt) ? sp * wv : 0.f; };
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += KC) {
+      if (k0 + KC <= kf) continue;
+      float ty[KC], v[KC];
+#pragma unroll
+      for (int k = 0; k < KC; k++) {
+        const int c = lane + 32 * (k0 + k);
+        const float2 yw = s_yw[c];
+        ty[k] = (c > i && c < nt) ? yw.x : 0.f;
+        v[k] = vcol(c, yw.y);
       }
 #pragma unroll
-      for (int o = 1; o <= 2; o <<= 1) {  // sums commute: the four lanes agree bit for bit
-        z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
-        z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
-        z.z += __shfl_xor_sync(0xffffffffu, z.z, o);
-        z.w += __shfl_xor_sync(0xffffffffu, z.w, o);
+      for (int h = 0; h < R; h += H) {
+        if ((h + H - 1) * GW + gw <= i) continue;
+#pragma unroll
+        for (int s = h; s < h + H; s++)
+#pragma unroll
+          for (int k = 0; k < KC; k++) {
+            A[s][k0 + k] -= x[s] * ty[k];
+            z[s] += A[s][k0 + k] * v[k];
+          }
       }
-      return z;
-    };
-    auto finish = [&](int r, float4 a, float4 z, float tp, float sp) {  // x and the next column, rows r..r+3
-      if (tp != 0.f) {
-        const float4 xv = make_float4(a.x + sp * z.x, a.y + sp * z.y, a.z + sp * z.z, a.w + sp * z.w);
-        *reinterpret_cast<float4*>(x + r) = xv;
-        *reinterpret_cast<float4*>(u + r) =
-            make_float4(a.x - tp * xv.x, a.y - tp * xv.y, a.z - tp * xv.z, a.w - tp * xv.w);
-      } else {
-        *reinterpret_cast<float4*>(u + r) = a;
-      }
-    };
-    auto scale_row = [&](float tp, float sp) {  // row i of the own columns > i: the stored right reflector
-      for (int l = l1 + t; l < nown; l += nt_) {
-        float* a = A + i + (size_t)l * mt;
-        *a = (rank + l * C == i + 1) ? (tp != 0.f ? 1.f : 0.f) : *a * sp;
-      }
-    };
-    if (ngr <= (nt_ >> 2)) {
-      // one group per four lanes covers every row: the partial sums are loaded
-      // together with the reflector's inputs and wait in registers for tp and sp
-      FF v{0.f, 0.f};
-      float x0 = 0.f;
-      if (t < 32) {
-        if (t < C) v = cluster.map_shared_rank(nrm, t)[b];
-        x0 = *cluster.map_shared_rank(pcb + i, own_next);
-      }
-      const int g = t >> 2;
-      const bool act = g < ngr;
-      const int r = r0 + 4 * g;
-      const float4 z = zsum(r, act);
-      const float4 a = (act && part == 0) ? *reinterpret_cast<const float4*>(pn + r) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (t < 32) right_reflector(v, x0);
-      __syncthreads();
-      TMARK(3);
-      const float tp = scal[1], sp = scal[2];
-      scale_row(tp, sp);
-      if (act && part == 0) finish(r, a, z, tp, sp);
-    } else {
-      if (t < 32) {
-        const FF v = t < C ? cluster.map_shared_rank(nrm, t)[b] : FF{0.f, 0.f};
-        right_reflector(v, *cluster.map_shared_rank(pcb + i, own_next));
-      }
-      __syncthreads();
-      TMARK(3);
-      const float tp = scal[1], sp = scal[2];
-      scale_row(tp, sp);
-      for (int g0 = 0; g0 < ngr; g0 += nt_ >> 2) {
-        const int g = g0 + (t >> 2);
-        const bool act = g < ngr;
-        const int r = r0 + 4 * g;
-        const float4 z = zsum(r, act && tp != 0.f);
-        if (act && part == 0) finish(r, *reinterpret_cast<const float4*>(pn + r), z, tp, sp);
-      }
-    }
-    __syncthreads();
-    TMARK(4);
-    const float tp = scal[1];
-    const float tq = form_left(i + 1);
-    TMARK(5);
-    // ---- D: right update of the own columns > i + 1 (column i + 1 now holds
-    // its left reflector), then their left update with it
-    const int lr = lfirst(i + 2);
-    const int rows = mt - i - 1;
-    if (rows <= 32 * 16) {
-      // one pass per column, x and u held in registers (the fewest per lane that hold the rows)
-      const int lv = lfirst(i + 3);
-      if (rows <= 32 * 4)
-        tail_fused_update<4>(A, mt, i, lr, nown, tp, tq, x, u, vrow, lv);
-      else if (rows <= 32 * 8)
-        tail_fused_update<8>(A, mt, i, lr, nown, tp, tq, x, u, vrow, lv);
-      else
-        tail_fused_update<16>(A, mt, i, lr, nown, tp, tq, x, u, vrow, lv);
-      __syncthreads();
-    } else {
-      if (tp != 0.f) {
-        for (int r = i + 1 + t; r < mt; r += nt_) {
-          const float f = tp * x[r];
-          for (int l = lr; l < nown; l++) A[r + (size_t)l * mt] -= f * A[i + (size_t)l * mt];
+#pragma unroll
+      for (int k = 0; k < KC; k++)
+        if (k0 + k == kf) {
+#pragma unroll
+          for (int s = 0; s < R; s++) nx[s] = A[s][k0 + k];
         }
-      }
-      __syncthreads();
-      left_update(i + 1, tq);
     }
-    TMARK(6);
+    {
+      constexpr int P = R < 8 ? R : (R & 8) ? 8 : 16;  // R = 2, 4 or a sum of 16s, 8s and a 4
+#pragma unroll
+      for (int q = 0; q + P <= R; q += P) warp_sums<P>(z, q, lane);
+      if (R % P) warp_sums<(R % P) ? R % P : 1>(z, R - R % P, lane);
+    }
+#pragma unroll
+    for (int s = 0; s < R; s++) {
+      z[s] *= tp;
+      const float v = __shfl_sync(0xffffffffu, nx[s], (i + 1) & 31) - z[s];
+      x[s] = (s * GW + gw > i + 1) ? v : 0.f;
+    }
+    // ---- right update and the products of the next column
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += KC) {
+      if (k0 + KC <= kf) continue;
+      float v[KC];
+#pragma unroll
+      for (int k = 0; k < KC; k++) {
+        const int c = lane + 32 * (k0 + k);
+        v[k] = vcol(c, s_yw[c].y);
+        acc[k0 + k] = 0.f;
+      }
+#pragma unroll
+      for (int h = 0; h < R; h += H) {
+        if ((h + H - 1) * GW + gw <= i) continue;
+#pragma unroll
+        for (int s = h; s < h + H; s++)
+#pragma unroll
+          for (int k = 0; k < KC; k++) {
+            A[s][k0 + k] -= z[s] * v[k];
+            acc[k0 + k] += x[s] * A[s][k0 + k];
+          }
+      }
+    }
+    if (++iwarp == GW) {
+      iwarp = 0;
+      islot++;
+    }
   }
-  // reflectors and the bidiagonal's neighbourhood back to the working matrix
+  if (dead) __nanosleep(100000);  // remote stores still under way land before any CTA leaves
   cluster.sync();
-  for (int l = 0; l < nown; l++)
-    for (int r = t; r < mt; r += nt_) p.W[r + (size_t)(rank + l * C) * p.ldw] = A[r + (size_t)l * mt];
+}
+
+// The kernel for R rows per warp and K columns per lane (at most 192
+// registers of the block per thread; the three largest tiles spill a few
+// hundred bytes and still beat the panel kernel, whose trailing updates would
+// also cost accuracy on tall blocks: a tensor-core GEMM rounds towards zero).
+static const void* tail_kernel(int R, int K) {
+#define DDC_TAIL(r, k) \
+  if (R == r && K == k) return (const void*)bidiag_tail_kernel<r, k>
+  DDC_TAIL(2, 2); DDC_TAIL(4, 2); DDC_TAIL(8, 2); DDC_TAIL(16, 2); DDC_TAIL(24, 2);
+  DDC_TAIL(2, 4); DDC_TAIL(4, 4); DDC_TAIL(8, 4); DDC_TAIL(16, 4); DDC_TAIL(24, 4);
+  DDC_TAIL(2, 8); DDC_TAIL(4, 8); DDC_TAIL(8, 8); DDC_TAIL(16, 8); DDC_TAIL(24, 8);
+  DDC_TAIL(4, 12); DDC_TAIL(8, 12); DDC_TAIL(12, 12); DDC_TAIL(16, 12);
+  DDC_TAIL(4, 16); DDC_TAIL(8, 16); DDC_TAIL(12, 16);
+#undef DDC_TAIL
+  return nullptr;
 }
 
 // Cluster size the device can co-schedule (16, else 8, else 0), cached.
 static int tail_cluster_size(ddcsvd_context* ctx) {
   if (ctx->tail_cluster >= 0) return ctx->tail_cluster;
   int best = 0;
-  if (cudaFuncSetAttribute((const void*)bidiag_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-      cudaSuccess) {
-    const int smem = (int)(ctx->smem_optin > 1024 ? ctx->smem_optin - 1024 : ctx->smem_optin);
-    cudaFuncSetAttribute((const void*)bidiag_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    for (int c : {16, 8}) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(c);
-      cfg.blockDim = dim3(kTailThreads);
-      cfg.dynamicSmemBytes = smem;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = c;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      int nclusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, (const void*)bidiag_tail_kernel, &cfg) == cudaSuccess &&
-          nclusters >= 1) {
-        best = c;
-        break;
-      }
+  for (int c : {16, 8}) {
+    const void* fn = tail_kernel(8, 16);
+    if (c > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) continue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kTailThreads);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int nclusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) == cudaSuccess && nclusters >= 1) {
+      best = c;
+      break;
     }
   }
   cudaGetLastError();  // a refused attribute or query only means no cluster tail
@@ -401,55 +487,72 @@ static int tail_cluster_size(ddcsvd_context* ctx) {
   return best;
 }
 
+// Cluster size and register tile for an mt x nt block (C = 0: it does not fit):
+// the fewest CTAs that leave two rows a warp, else the largest cluster.  The
+// exchanges cost nearly the same for any C, the rows' work shrinks with it
+// (us per column: 64 x 48 C = 4 1.52, C = 2 1.61; 256^2 C = 16 1.74, C = 8 1.87;
+// 512 x 256 C = 16 1.89, C = 8 2.25).
+struct TailConfig {
+  int C, R, K;
+};
+static TailConfig tail_config(int mt, int nt, int cmax) {
+  TailConfig g{0, 0, 0};
+  for (int K : {2, 4, 8, 12, 16})
+    if (32 * K >= nt) {
+      g.K = K;
+      break;
+    }
+  if (g.K == 0) return g;
+  int C = 1;
+  while (32 * C < nt) C *= 2;  // a slice of columns is at most one warp wide
+  for (; C <= cmax; C *= 2)
+    for (int R : {2, 4, 8, 12, 16, 24})
+      if (kTailWarps * C * R >= mt && tail_kernel(R, g.K) && (R <= 2 || C == cmax)) {
+        g.C = C;
+        g.R = R;
+        return g;
+      }
+  return g;
+}
+
 int bidiag_tail_columns(ddcsvd_context* ctx, int m, int n, int k0) {
   const int cap = ctx->tune[TK_PANEL_TAIL];
   const int mt = m - k0, nt = n - k0;
   if (cap <= 0 || nt > cap || nt <= 0 || mt < nt) return 0;
-  const int C = tail_cluster_size(ctx);
-  if (C == 0) return 0;
-  const int ncb = ceil_div(nt, C);
-  const size_t bytes = tail_smem_floats(mt, ncb) * sizeof(float);
-  return (bytes + 1024 <= ctx->smem_optin) ? nt : 0;
+  return tail_config(mt, nt, tail_cluster_size(ctx)).C > 0 ? nt : 0;
 }
 
 int bidiag_tail(ddcsvd_context* ctx, int m, int n, int k0, float* W, int ldw, float* d, float* e, float* tauq,
                 float* taup) {
-  const int C = tail_cluster_size(ctx);
-  if (C == 0) return DDCSVD_ERR_UNSUPPORTED;
   TailParams p;
   p.mt = m - k0;
   p.nt = n - k0;
-  p.ncb = ceil_div(p.nt, C);
+  const TailConfig g = tail_config(p.mt, p.nt, tail_cluster_size(ctx));
+  if (g.C == 0) return DDCSVD_ERR_UNSUPPORTED;
   p.W = W + k0 + (size_t)k0 * ldw;
   p.ldw = ldw;
   p.d = d + k0;
   p.e = e + k0;
   p.tauq = tauq + k0;
   p.taup = taup + k0;
-  const size_t smem = tail_smem_floats(p.mt, p.ncb) * sizeof(float);
-  DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)bidiag_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+  p.st = ctx->d_status;
+  const void* fn = tail_kernel(g.R, g.K);
+  if (g.C > 8) DDC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C);
+  cfg.gridDim = dim3(g.C);
   cfg.blockDim = dim3(kTailThreads);
-  cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.x = g.C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  DDC_CUDA_TRY(cudaLaunchKernelEx(&cfg, bidiag_tail_kernel, p));
+  void* args[] = {&p};
+  DDC_CUDA_TRY(cudaLaunchKernelExC(&cfg, fn, args));
   count_launch();
   return DDCSVD_OK;
 }
 
 }  // namespace ddcsvd
-
-#ifdef DDCSVD_PHASE_TRACE
-extern "C" int ddcsvd_tail_trace_read(unsigned long long* out) {
-  return (int)cudaMemcpyFromSymbol(out, ddcsvd::g_tail_trace, sizeof(ddcsvd::g_tail_trace));
-}
-#endif
