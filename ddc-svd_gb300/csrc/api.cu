@@ -211,13 +211,14 @@ __global__ void copy2d_kernel(int rows, int cols, const float* __restrict__ src,
 
 // The tensor-core back-transformation reads U and V through TMA, which needs
 // 16-byte aligned bases and leading dimensions; other layouts go through
-// aligned staging buffers.
+// aligned staging buffers (except small problems, whose columns are read and
+// written by plain accesses).
 static int svd_core(ddcsvd_context* ctx, int m, int n, const float* dA, int lda, float* dS, float* dU,
                     int ldu, float* dV, int ldv, int mode, bool check_finite) {
   const bool tcmode = (mode >= DDCSVD_MODE_BLOCKED_TF32X3);
   auto ok = [](const float* p, int ld) { return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && (ld % 4 == 0); };
   const bool tall = use_tall_qr(ctx, m, n, mode);
-  if (!tcmode || (ok(dU, ldu) && ok(dV, ldv)))
+  if (!tcmode || (ok(dU, ldu) && ok(dV, ldv)) || (!tall && bx_direct_ok(m, n)))
     return tall ? svd_tall_qr(ctx, m, n, dA, lda, dS, dU, ldu, dV, ldv, mode, check_finite)
                 : svd_core_impl(ctx, m, n, dA, lda, dS, dU, ldu, dV, ldv, mode, check_finite);
   const int lu = (int)round_up(m, 4), lv = (int)round_up(n, 4);
@@ -285,8 +286,10 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
   // that leaves most of the GPU idle); their buffers then get a region of
   // their own instead of sharing the one that stages 2-4 use.  Stage timing
   // keeps everything on one stream so that the stage events mean what they say.
+  const bool direct = !plain && kind != GEMM_SIMT && bx_direct_ok(m, n);
   const bool overlap = !plain && kind != GEMM_SIMT && !ctx->timing;
   BxPrepared bxl, bxr;
+  BxDirect bxd;
   auto region_a = [&](Arena& a, Plan& pl) {
     pl.W = a.take<float>((size_t)ldw * n);
     pl.d = a.take<float>(n + 4);
@@ -296,7 +299,9 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     pl.sig_slot = a.take<double>(n + 4);
     pl.sig = a.take<double>(n + 4);
     pl.blob = a.take<char>(prep_bounds({n}).blob_bytes);
-    if (overlap) {
+    if (direct) {
+      bx_direct_plan(m, n, a, &bxd);
+    } else if (overlap) {
       bx_plan(m, n, n, kind, a, &bxl);
       bx_plan(n, std::max(0, n - 2), n, kind, a, &bxr);
     }
@@ -315,7 +320,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     Arena b3 = a;
     DDC_TRY(bd_vectors(ctx, n, (long long)n * n, nullptr, nullptr, nullptr, nullptr, nullptr, b3, true));
     Arena b4 = a, b5 = a;  // stage 5 (its buffers are in region a when it overlaps stages 2-4)
-    if (!overlap) {
+    if (!overlap && !direct) {
       DDC_TRY(apply_left_reflectors(ctx, m, n, nullptr, ldw, nullptr, dU, ldu, n, kind, plain, b4, true));
       DDC_TRY(apply_right_reflectors(ctx, n, std::max(0, n - 2), nullptr, ldw, nullptr, dV, ldv, n, kind, plain, b5,
                                      true));
@@ -351,8 +356,13 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
   SideWork side(ctx);
   if (overlap) {
     DDC_TRY(side.fork());
-    int rc = bx_prepare(ctx, 0, m, n, pl.W, ldw, pl.tauq, bxl);
-    if (rc == DDCSVD_OK) rc = bx_prepare(ctx, 1, n, std::max(0, n - 2), pl.W, ldw, pl.taup, bxr);
+    int rc;
+    if (direct) {
+      rc = bx_direct_prepare(ctx, m, n, pl.W, ldw, pl.tauq, pl.taup, bxd);
+    } else {
+      rc = bx_prepare(ctx, 0, m, n, pl.W, ldw, pl.tauq, bxl);
+      if (rc == DDCSVD_OK) rc = bx_prepare(ctx, 1, n, std::max(0, n - 2), pl.W, ldw, pl.taup, bxr);
+    }
     side.back();
     DDC_TRY(rc);
   }
@@ -392,7 +402,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     Arena b = a;
     DDC_TRY(bd_vectors(ctx, n, P.store, P.b1, P.b2, pl.sig_slot, &P.L, pl.sig, b, false));
   }
-  if (m > n) {
+  if (m > n && !direct) {
     zero_rows_kernel<<<dim3(std::min(ceil_div(m - n, 256), 64), n), 256, 0, ctx->stream>>>(n, m, n, dU, ldu);
     count_launch();
   }
@@ -407,7 +417,14 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     }
     return DDCSVD_OK;
   };
-  if (overlap) {
+  if (direct) {
+    if (overlap) DDC_TRY(side.join());
+    ktimer_begin(ctx, KC_BACKXFORM);
+    if (!overlap) DDC_TRY(bx_direct_prepare(ctx, m, n, pl.W, ldw, pl.tauq, pl.taup, bxd));
+    DDC_TRY(bx_direct_apply(ctx, m, n, bxd, dU, ldu, dV, ldv));
+    ktimer_end(ctx);
+    DDC_TRY(v_done());
+  } else if (overlap) {
     DDC_TRY(side.join());
     ktimer_begin(ctx, KC_BACKXFORM);
     DDC_TRY(bx_apply(ctx, n, std::max(0, n - 2), bxr, dV, ldv, n, kind));

@@ -648,6 +648,242 @@ int bx_apply(ddcsvd_context* ctx, int rows_total, int nref, const BxPrepared& w,
   return DDCSVD_OK;
 }
 
+// ---------------------------------------------------------------- small problems
+// Up to kDirectCols columns the WY machinery costs more than it saves: at
+// 512 x 256 its preparation (Gram matrices, T factors, U T on a handful of CTAs)
+// took 0.75 ms beside 0.6 ms of stages 2-4 that hide it, and the four products
+// another 0.12 ms.  Instead a CTA holds four columns of U or V in registers (thread t rows t, t + 128, ...) and applies the reflectors in groups
+// of four, I - U4 T4 U4^T with the 4 x 4 triangular T4 formed beforehand.  A
+// thread needs only its own rows of a reflector, so they go straight from L2 to
+// registers, a group ahead; the dot products of a group share one reduction over
+// the CTA.  Bound by that reduction's latency (n / 4 groups in a chain).  A first
+// form with a column per warp and the reflectors in shared memory read each of
+// them four times a CTA and took up to twice as long; eight columns a CTA were
+// slower too.  0.64-0.85 us per group: 47 us at 512 x 256, 63 us at 1100 x 300,
+// 123 us at 1024 x 512.  FP32 throughout.
+constexpr int kDirectCols = 512;   // columns n
+constexpr int kDirectRows = 2048;  // rows m
+constexpr int kDirectThreads = 128;
+constexpr int kDirectW = 4;  // columns per CTA
+
+bool bx_direct_ok(int m, int n) { return n <= kDirectCols && m <= kDirectRows; }
+
+// T4 of reflectors 4 q .. 4 q + 3 of one side (warp per group): Gram products
+// by the warp, then T[l, l] = tau_l, T[0:l, l] = -tau_l T[0:l, 0:l] G[0:l, l].
+// 16 floats per group, row-major, zero below the diagonal and beyond nref.
+__global__ void __launch_bounds__(128) bx_t4_kernel(int rowsL, int nrefL, const float* __restrict__ UcL, int lduL,
+                                                    const float* __restrict__ tauL, int rowsR, int nrefR,
+                                                    const float* __restrict__ UcR, int lduR,
+                                                    const float* __restrict__ tauR, float* T4) {
+  const int nqL = ceil_div(nrefL, 4), nqR = ceil_div(nrefR, 4);
+  const int g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (g >= nqL + nqR) return;
+  const bool left = g < nqL;
+  const int j0 = 4 * (left ? g : g - nqL), rows = left ? rowsL : rowsR, nref = left ? nrefL : nrefR;
+  const int ldu = left ? lduL : lduR;
+  const float* U = (left ? UcL : UcR) + (size_t)j0 * ldu;
+  const float* tau = (left ? tauL : tauR) + j0;
+  float G[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // 01 02 12 03 13 23
+  for (int r = (j0 & ~31) + lane; r < rows; r += 32) {
+    float u[4];
+#pragma unroll
+    for (int l = 0; l < 4; l++) u[l] = (j0 + l < nref) ? U[r + (size_t)l * ldu] : 0.f;
+    G[0] += u[0] * u[1];
+    G[1] += u[0] * u[2];
+    G[2] += u[1] * u[2];
+    G[3] += u[0] * u[3];
+    G[4] += u[1] * u[3];
+    G[5] += u[2] * u[3];
+  }
+#pragma unroll
+  for (int q = 0; q < 6; q++) G[q] = warp_sum(G[q]);
+  if (lane == 0) {
+    float t[4], T[4][4];
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+      t[l] = (j0 + l < nref) ? tau[l] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) T[l][k] = (k == l) ? t[l] : 0.f;
+    }
+    T[0][1] = -t[1] * (T[0][0] * G[0]);
+    T[0][2] = -t[2] * (T[0][0] * G[1] + T[0][1] * G[2]);
+    T[1][2] = -t[2] * (T[1][1] * G[2]);
+    T[0][3] = -t[3] * (T[0][0] * G[3] + T[0][1] * G[4] + T[0][2] * G[5]);
+    T[1][3] = -t[3] * (T[1][1] * G[4] + T[1][2] * G[5]);
+    T[2][3] = -t[3] * (T[2][2] * G[5]);
+    float4* out = reinterpret_cast<float4*>(T4 + (size_t)g * 16);
+#pragma unroll
+    for (int l = 0; l < 4; l++) out[l] = make_float4(T[l][0], T[l][1], T[l][2], T[l][3]);
+  }
+}
+
+// registers per thread that hold a column of `rows` entries
+__host__ __device__ inline int direct_regs(int rows) {
+  const int k = ceil_div(rows, kDirectThreads);
+  return k <= 4 ? k : k <= 6 ? 6 : k <= 8 ? 8 : k <= 10 ? 10 : 16;
+}
+
+struct BxSide {
+  int rows, nref, off;  // reflector j starts at row j + off
+  int vrows;            // rows of C that hold values on entry (zero below)
+  int ncols, ldu, ldc;
+  const float *Uc, *T4;
+  float* C;
+};
+
+// One CTA: kDirectW columns of C from column c0, their rows in KR registers a thread.
+template <int KR>
+__device__ void bx_direct_cta(const BxSide& p, int c0, float (*red)[kDirectThreads / 32][4 * kDirectW]) {
+  constexpr int CW = kDirectW;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  float c[CW][KR];
+#pragma unroll
+  for (int q = 0; q < CW; q++)
+#pragma unroll
+    for (int k = 0; k < KR; k++) {
+      const int r = t + kDirectThreads * k;
+      c[q][k] = (c0 + q < p.ncols && r < p.vrows) ? p.C[r + (size_t)(c0 + q) * p.ldc] : 0.f;
+    }
+  // the next D groups' entries of the own rows, and their T4 (a group takes
+  // about half of the L2 round trip at the small end)
+  constexpr int D = KR <= 4 ? 2 : 1;
+  float ur[D][KR][4];
+  float4 tr[D][4];
+  auto fetch = [&](int g, float (&un)[KR][4], float4 (&tn)[4]) {
+    if (g < 0) return;
+#pragma unroll
+    for (int k = 0; k < KR; k++)
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        const int r = t + kDirectThreads * k, j = 4 * g + l;
+        un[k][l] = (r < p.ldu && j < p.nref) ? __ldg(p.Uc + r + (size_t)j * p.ldu) : 0.f;
+      }
+#pragma unroll
+    for (int l = 0; l < 4; l++) tn[l] = __ldg(reinterpret_cast<const float4*>(p.T4 + (size_t)g * 16) + l);
+  };
+  const int nq = ceil_div(p.nref, 4);
+#pragma unroll
+  for (int s = 0; s < D; s++) fetch(nq - 1 - s, ur[s], tr[s]);
+  auto step = [&](int g, float (&un)[KR][4], float4 (&tn)[4]) {
+    float u[KR][4];
+    const float4 t0 = tn[0], t1 = tn[1], t2 = tn[2], t3 = tn[3];
+#pragma unroll
+    for (int k = 0; k < KR; k++)
+#pragma unroll
+      for (int l = 0; l < 4; l++) u[k][l] = un[k][l];
+    fetch(g - D, un, tn);
+    float d[4 * CW];
+#pragma unroll
+    for (int q = 0; q < CW; q++)
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < KR; k++) s += u[k][l] * c[q][k];
+        d[4 * q + l] = s;
+      }
+    // sums over the CTA: lane v of a warp ends with its value v (pairs of lanes
+    // with one, for 16 values), then the four warps' through shared memory
+    constexpr int N = 4 * CW, G = 32 / N;
+#pragma unroll
+    for (int nv = N, off = 16; nv > 1; nv >>= 1, off >>= 1) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int h = 0; h < nv / 2; h++) {
+        const float send = up ? d[h] : d[h + nv / 2];
+        const float keep = up ? d[h + nv / 2] : d[h];
+        d[h] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+#pragma unroll
+    for (int off = G / 2; off > 0; off >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], off);
+    float(*rg)[N] = red[g & 1];  // two buffers: one barrier per group
+    if (lane % G == 0) rg[wid][lane / G] = d[0];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < CW; q++) {
+      float4 e = *reinterpret_cast<const float4*>(&rg[0][4 * q]);
+#pragma unroll
+      for (int w = 1; w < kDirectThreads / 32; w++) {
+        const float4 f = *reinterpret_cast<const float4*>(&rg[w][4 * q]);
+        e.x += f.x;
+        e.y += f.y;
+        e.z += f.z;
+        e.w += f.w;
+      }
+      const float w0 = t0.x * e.x + t0.y * e.y + t0.z * e.z + t0.w * e.w;
+      const float w1 = t1.y * e.y + t1.z * e.z + t1.w * e.w;
+      const float w2 = t2.z * e.z + t2.w * e.w;
+      const float w3 = t3.w * e.w;
+#pragma unroll
+      for (int k = 0; k < KR; k++)
+        c[q][k] -= (u[k][0] * w0 + u[k][1] * w1) + (u[k][2] * w2 + u[k][3] * w3);
+    }
+  };
+  for (int g = nq - 1; g >= 0; g -= D)
+#pragma unroll
+    for (int s = 0; s < D; s++)
+      if (g - s >= 0) step(g - s, ur[s], tr[s]);
+#pragma unroll
+  for (int q = 0; q < CW; q++)
+#pragma unroll
+    for (int k = 0; k < KR; k++) {
+      const int r = t + kDirectThreads * k;
+      if (c0 + q < p.ncols && r < p.rows) p.C[r + (size_t)(c0 + q) * p.ldc] = c[q][k];
+    }
+}
+
+__global__ void __launch_bounds__(kDirectThreads) bx_direct_kernel(BxSide left, BxSide right, int ctas_left) {
+  __shared__ __align__(16) float red[2][kDirectThreads / 32][4 * kDirectW];
+  const bool l = (int)blockIdx.x < ctas_left;
+  const BxSide p = l ? left : right;
+  const int c0 = kDirectW * (l ? blockIdx.x : blockIdx.x - ctas_left);
+  switch (direct_regs(p.rows)) {
+    case 1: bx_direct_cta<1>(p, c0, red); break;
+    case 2: bx_direct_cta<2>(p, c0, red); break;
+    case 3: bx_direct_cta<3>(p, c0, red); break;
+    case 4: bx_direct_cta<4>(p, c0, red); break;
+    case 6: bx_direct_cta<6>(p, c0, red); break;
+    case 8: bx_direct_cta<8>(p, c0, red); break;
+    case 10: bx_direct_cta<10>(p, c0, red); break;
+    default: bx_direct_cta<16>(p, c0, red); break;
+  }
+}
+
+void bx_direct_plan(int m, int n, Arena& a, BxDirect* out) {
+  out->lduL = (int)round_up(m, 32);
+  out->lduR = (int)round_up(n, 32);
+  out->UcL = a.take<float>((size_t)out->lduL * n);
+  out->UcR = a.take<float>((size_t)out->lduR * n);
+  out->T4 = a.take<float>(16 * (size_t)(2 * ceil_div(n, 4)) + 16);
+}
+
+int bx_direct_prepare(ddcsvd_context* ctx, int m, int n, const float* W, int ldw, const float* tauq,
+                      const float* taup, const BxDirect& w) {
+  const int nr = std::max(0, n - 2);
+  build_reflectors_kernel<<<dim3(ceil_div(w.lduL, 32), ceil_div(n, 32)), dim3(32, 8), 0, ctx->stream>>>(
+      0, m, n, W, ldw, tauq, w.UcL, w.lduL);
+  if (nr > 0)
+    build_reflectors_kernel<<<dim3(ceil_div(w.lduR, 32), ceil_div(nr, 32)), dim3(32, 8), 0, ctx->stream>>>(
+        1, n, nr, W, ldw, taup, w.UcR, w.lduR);
+  bx_t4_kernel<<<ceil_div(ceil_div(n, 4) + ceil_div(nr, 4), 4), 128, 0, ctx->stream>>>(
+      m, n, w.UcL, w.lduL, tauq, n, nr, w.UcR, w.lduR, taup, w.T4);
+  count_launch(nr > 0 ? 3 : 2);
+  DDC_CUDA_TRY(cudaGetLastError());
+  return DDCSVD_OK;
+}
+
+int bx_direct_apply(ddcsvd_context* ctx, int m, int n, const BxDirect& w, float* U, int ldu, float* V, int ldv) {
+  const int nr = std::max(0, n - 2);
+  const BxSide left{m, n, 0, n, n, w.lduL, ldu, w.UcL, w.T4, U};
+  const BxSide right{n, nr, 1, n, n, w.lduR, ldv, w.UcR, w.T4 + 16 * (size_t)ceil_div(n, 4), V};
+  const int ctas = ceil_div(n, kDirectW), ctas_r = nr > 0 ? ctas : 0;
+  bx_direct_kernel<<<ctas + ctas_r, kDirectThreads, 0, ctx->stream>>>(left, right, ctas);
+  count_launch();
+  DDC_CUDA_TRY(cudaGetLastError());
+  return DDCSVD_OK;
+}
+
 static int apply_blocked_tc(ddcsvd_context* ctx, int side, int rows_total, int nref, const float* W, int ldw,
                             const float* tau, float* C, int ldc, int ncols, GemmKind kind, Arena& a,
                             bool plan_only) {

@@ -249,6 +249,21 @@ int bx_prepare(ddcsvd_context* ctx, int side, int rows_total, int nref, const fl
 int bx_apply(ddcsvd_context* ctx, int rows_total, int nref, const BxPrepared& w, float* C, int ldc, int ncols,
              GemmKind kind);
 
+// The back-transformation of small problems (bx_direct_ok): columns of U and V
+// in registers, the reflectors streamed through shared memory in fours.
+// bx_direct_prepare may run on the side stream, like bx_prepare; then one
+// launch turns [Y; 0] (rows n.. of U need not be set) into U and X into V.
+struct BxDirect {
+  float *UcL = nullptr, *UcR = nullptr;  // explicit reflectors of the two sides
+  float *T4 = nullptr;                   // 4 x 4 triangular factors, left then right
+  int lduL = 0, lduR = 0;
+};
+bool bx_direct_ok(int m, int n);
+void bx_direct_plan(int m, int n, Arena& a, BxDirect* out);
+int bx_direct_prepare(ddcsvd_context* ctx, int m, int n, const float* W, int ldw, const float* tauq,
+                      const float* taup, const BxDirect& w);
+int bx_direct_apply(ddcsvd_context* ctx, int m, int n, const BxDirect& w, float* U, int ldu, float* V, int ldv);
+
 // UT = Vp T (or Vp T^T) of one QR panel (nb <= kPanel reflectors), row-major with kPanel columns.
 int wy_prepare_block(ddcsvd_context* ctx, int rows, int nb, const float* Vp, int ldv, const float* tau, float* UT,
                      bool transT, float* scratch);

@@ -153,29 +153,6 @@ __device__ __forceinline__ void tail_wait(uint32_t bar, unsigned parity, bool& d
   }
 }
 
-// Sums v[q0 .. q0 + R) over the warp; every lane gets all of them (R a power
-// of two).
-template <int R, int N>
-__device__ __forceinline__ void warp_sums(float (&v)[N], int q0, int lane) {
-  float s[R];
-#pragma unroll
-  for (int q = 0; q < R; q++) s[q] = v[q0 + q];
-#pragma unroll
-  for (int nv = R, off = 16; nv > 1; nv >>= 1, off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int h = 0; h < nv / 2; h++) {
-      const float send = up ? s[h] : s[h + nv / 2];
-      const float keep = up ? s[h + nv / 2] : s[h];
-      s[h] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-#pragma unroll
-  for (int off = 16 / R; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
-#pragma unroll
-  for (int q = 0; q < R; q++) v[q0 + q] = __shfl_sync(0xffffffffu, s[0], q * (32 / R));
-}
-
 // R rows per warp, K columns per lane: blocks of up to 8 C R rows and 32 K
 // columns.
 template <int R, int K>
