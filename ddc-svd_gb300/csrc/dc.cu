@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "fp64.cuh"
 #include "internal.hpp"
 
 namespace ddcsvd {
@@ -70,49 +71,6 @@ struct DcParams {
   DevStatus* st;
 };
 
-// ---------------------------------------------------------------- FP64 arithmetic
-// GB300's FP64 pipe bounds this stage: one FP64 instruction of a warp holds it
-// for 64 cycles (19 per SM when four warps or more share the SM), against one
-// for FP32 and integer instructions, and comparisons, fmin / fmax take a turn
-// in it like an addition.  Measured per warp (one warp per scheduler): add,
-// multiply, FMA 64-66 cycles, a compare and an add 176, a division 566, hypot
-// 1059; the approximate reciprocal and the conversions to and from FP32 do not
-// use the pipe (9 and 2 cycles).  So divisions are formed from the approximate
-// reciprocal by one cubic Newton step (four FP64 instructions instead of
-// about nine), values of known sign are compared through their bit patterns,
-// and whatever does not need 53 bits is FP32.
-
-// a / x to about an ulp for normal x: with r ~ 1/x and e = 1 - x r,
-// 1/x = r (1 + e + e^2 + ...); |e| < 2^-18, so e^3 is below rounding.  x = 0
-// or subnormal gives NaN (callers fall back or had an infinity there before).
-__device__ __forceinline__ double rcp_approx(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  return r;
-}
-__device__ __forceinline__ double quot(double a, double x) {
-  const double r = rcp_approx(x);
-  const double e = fma(-x, r, 1.0);
-  const double y = fma(e, e, e);
-  const double t = a * r;
-  return fma(t, y, t);
-}
-// a / x rounded to nearest, as the division operator gives it, in six FP64
-// instructions: the reciprocal as above, q = a r, and the correction by the
-// exact remainder (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990).  Operands outside 2^+-500 take the
-// operator.
-__device__ __forceinline__ double quot_rn(double a, double x) {
-  const unsigned ea = (unsigned)__double2hiint(a) & 0x7ff00000u, ex = (unsigned)__double2hiint(x) & 0x7ff00000u;
-  constexpr unsigned lo = 523u << 20, span = 1000u << 20;
-  if (ea - lo > span || ex - lo > span) return a / x;
-  double r = rcp_approx(x);
-  const double e = fma(-x, r, 1.0);
-  r = fma(r, fma(e, e, e), r);
-  const double q = a * r;
-  return fma(fma(-x, q, a), r, q);
-}
-
 // Two versions of the stage's arithmetic.  kBits = true keeps every FP64
 // rounding of the plain formulas (division operator, hypot, sqrt, a fixed
 // order of sums): the twisted vectors' signs follow from a twist index that
@@ -126,14 +84,6 @@ __device__ __forceinline__ double quotient(double a, double x) {
   return kBits ? quot_rn(a, x) : quot(a, x);
 }
 
-// order of non-negative values = order of their bit patterns
-__device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
-// |x|'s bits for a maximum that ignores NaN, as fmax does
-__device__ __forceinline__ long long max_bits(double x) {
-  const long long b = abs_bits(x);
-  return b <= 0x7ff0000000000000ll ? b : 0ll;
-}
 // p = m 2^e with |m| in [1, 2): keeps the mantissa, adds e to ex (zero,
 // subnormal and non-finite values stay as they are)
 __device__ __forceinline__ double take_exponent(double p, int& ex) {

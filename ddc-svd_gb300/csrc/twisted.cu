@@ -22,6 +22,7 @@
 // access of a warp is one contiguous 256-byte segment.
 #include <vector>
 
+#include "fp64.cuh"
 #include "internal.hpp"
 #include "prep.hpp"
 
@@ -74,104 +75,179 @@ constexpr int kTwWarps = 4;
 
 // 32 vectors per CTA, one per lane; kTwWarps warps share the work of each
 // vector: the stationary and progressive transforms run concurrently (warps
-// 0 and 1), the twist search and ||B z|| are split over index segments
+// 0 and 1), the twist search and the norms are split over index segments
 // (warp w takes segment w), and the two halves of the solve run concurrently
 // (warp 0 below the twist, warp 1 above).
+// Bound by the two transforms' chains: nine FP64 instructions a step, each 64
+// cycles for a warp whatever its active lanes (fp64.cuh); the division was half
+// of them.  Every rounding of S, P and of the division is that of the plain
+// formulas: the twist index, and with it the vector's sign, follows from them.
+// Loads are a batch of steps ahead.  N = 3000: 2.18 -> 1.59 ms, of which the
+// transforms 1.15 (745 cycles a step); the batch of 2048 1.26 -> 1.09 ms.
+// A warp whose vectors share one block (uni: every warp of a single unreduced
+// bidiagonal) walks it in step: whole batches without per-lane bounds, the
+// operand ranges of the short division checked once a batch (a batch that
+// fails is done again with the general one), and coalesced solves.
+constexpr int kTwB = 8;  // steps per batch of the transforms
+struct TwIn {
+  double x[3][kTwB];
+};
+
+// kF: steps per batch of the other phases, whose steps are shorter: 16 of them
+// cover the L2 round trip (N = 3000: 1.67 -> 1.59 ms); blocks of a few dozen
+// entries end before that pays (the 2048-problem batch: 8 1.09, 16 1.23 ms).
+template <int kF>
 __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
   __shared__ double s_val[kTwWarps][32];
+  __shared__ double s_nrm[kTwWarps][32];
   __shared__ int s_idx[kTwWarps][32];
-  __shared__ double s_nrm[2][32];
   __shared__ int s_r[32];
+  constexpr int kB = kTwB;
   const int N = p.N;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
-  const bool act = k < N;
-  const int lo = act ? p.L.blo[k] : 0, hi = act ? p.L.bhi[k] : 0;
+  const bool act = blockIdx.x * 32 + lane < N;
+  const int k = min(blockIdx.x * 32 + lane, N - 1);  // lanes beyond N repeat the last vector (the same stores)
+  const int lo = p.L.blo[k], hi = p.L.bhi[k];
   const int nb = hi - lo;
-  const long long base = act ? p.L.base[k] + (k - lo) : 0;  // element i at base + (i - lo) * nb
+  const int lo0 = __shfl_sync(0xffffffffu, lo, 0), hi0 = __shfl_sync(0xffffffffu, hi, 0);
+  const bool uni = __all_sync(0xffffffffu, lo == lo0 && hi == hi0);
+  const long long base = p.L.base[k] + (k - lo);  // element i at base + (i - lo) * nb
   auto at = [&](int i) { return base + (long long)(i - lo) * nb; };
-  const double lam = act ? p.sigma[k] * p.sigma[k] : 0.0;
+  const double lam = p.sigma[k] * p.sigma[k];
   const double tiny = DBL_MIN / DBL_EPSILON;
-  // The recurrences below are serial in their FP64 values but not in their
-  // loads: every loop fetches its next kB inputs before the dependent chain
-  // (one loop iteration per step waited a full memory round trip per step).
-  constexpr int kB = 8;
   if (w == 0) {
     // stationary qd on the block: L D L^T - lam = L+ D+ L+^T, s_lo = -lam
     double s = -lam;
-    for (int i0 = lo; i0 < hi - 1; i0 += kB) {
-      double ddv[kB], dlv[kB], llv[kB];
+    auto load = [&](TwIn& v, int i0) {
 #pragma unroll
       for (int u = 0; u < kB; u++) {
-        const int i = min(i0 + u, hi - 2);
-        ddv[u] = p.dd[i];
-        dlv[u] = p.dl[i];
-        llv[u] = p.ll[i];
+        const int i = max(lo, min(i0 + u, hi - 2));
+        v.x[0][u] = p.dd[i];
+        v.x[1][u] = p.dl[i];
+        v.x[2][u] = p.ll[i];
       }
+    };
+    auto work = [&](const TwIn& v, int i0) {
+      if (uni && i0 + kB <= hi - 1) {
+        const double s0 = s;
+        bool ok = true;
 #pragma unroll
+        for (int u = 0; u < kB; u++) {
+          const double dp = v.x[0][u] + s;
+          ok = ok && mid_range(dp) && mid_range(v.x[1][u]);
+          const double L = quot_mid(v.x[1][u], dp);
+          p.Lp[at(i0 + u)] = L;
+          p.S[at(i0 + u)] = s;
+          s = L * v.x[2][u] * s - lam;
+        }
+        if (__all_sync(0xffffffffu, ok)) return;
+        s = s0;
+      }
+#pragma unroll 1
       for (int u = 0; u < kB; u++) {
         const int i = i0 + u;
         if (i < hi - 1) {
-          double dp = ddv[u] + s;
-          if (fabs(dp) < tiny) dp = -tiny;
-          const double L = dlv[u] / dp;
+          double dp = p.dd[i] + s;
+          if (abs_bits(dp) < bits(tiny)) dp = -tiny;
+          const double L = quot_rn(p.dl[i], dp);
           p.Lp[at(i)] = L;
           p.S[at(i)] = s;
-          s = L * llv[u] * s - lam;
+          s = L * p.ll[i] * s - lam;
         }
       }
+    };
+    TwIn A, B;
+    if (lo < hi - 1) load(A, lo);
+    for (int i0 = lo; i0 < hi - 1; i0 += 2 * kB) {
+      load(B, i0 + kB);
+      work(A, i0);
+      load(A, i0 + 2 * kB);
+      work(B, i0 + kB);
     }
-    if (hi > lo) p.S[at(hi - 1)] = s;
-  } else if (w == 1 && hi > lo) {
+    p.S[at(hi - 1)] = s;
+  } else if (w == 1) {
     // progressive qd on the block: L D L^T - lam = U- D- U-^T, p_{hi-1} = d_{hi-1} - lam
     double pv = p.dd[hi - 1] - lam;
     p.Pp[at(hi - 1)] = pv;
-    for (int i0 = hi - 2; i0 >= lo; i0 -= kB) {
-      double dllv[kB], ddv[kB], llv[kB];
+    auto load = [&](TwIn& v, int i0) {
 #pragma unroll
       for (int u = 0; u < kB; u++) {
         const int i = max(i0 - u, lo);
-        dllv[u] = p.dll[i];
-        ddv[u] = p.dd[i];
-        llv[u] = p.ll[i];
+        v.x[0][u] = p.dll[i];
+        v.x[1][u] = p.dd[i];
+        v.x[2][u] = p.ll[i];
       }
+    };
+    auto work = [&](const TwIn& v, int i0) {
+      if (uni && i0 - kB + 1 >= lo) {
+        const double p0 = pv;
+        bool ok = true;
 #pragma unroll
+        for (int u = 0; u < kB; u++) {
+          const double dm = v.x[0][u] + pv;
+          ok = ok && mid_range(dm) && mid_range(v.x[1][u]);
+          const double tt = quot_mid(v.x[1][u], dm);
+          p.Um[at(i0 - u)] = v.x[2][u] * tt;
+          pv = pv * tt - lam;
+          p.Pp[at(i0 - u)] = pv;
+        }
+        if (__all_sync(0xffffffffu, ok)) return;
+        pv = p0;
+      }
+#pragma unroll 1
       for (int u = 0; u < kB; u++) {
         const int i = i0 - u;
         if (i >= lo) {
-          double dm = dllv[u] + pv;
-          if (fabs(dm) < tiny) dm = -tiny;
-          const double tt = ddv[u] / dm;
-          p.Um[at(i)] = llv[u] * tt;
+          double dm = p.dll[i] + pv;
+          if (abs_bits(dm) < bits(tiny)) dm = -tiny;
+          const double tt = quot_rn(p.dd[i], dm);
+          p.Um[at(i)] = p.ll[i] * tt;
           pv = pv * tt - lam;
           p.Pp[at(i)] = pv;
         }
       }
+    };
+    TwIn A, B;
+    load(A, hi - 2);
+    for (int i0 = hi - 2; i0 >= lo; i0 -= 2 * kB) {
+      load(B, i0 - kB);
+      work(A, i0);
+      load(A, i0 - 2 * kB);
+      work(B, i0 - kB);
     }
   }
   __syncthreads();
+  const int seg = (nb + kTwWarps - 1) / kTwWarps;
+  const int sa = lo + w * seg, sb = min(hi, sa + seg);  // this warp's indices of the split phases
   // ---- twist index r = argmin |gamma_i|, gamma_i = s_i + p_i + lam; ties -> larger i
   {
-    const int seg = (nb + kTwWarps - 1) / kTwWarps;
-    const int a = lo + w * seg, b = min(hi, a + seg);
     double best = INFINITY;
     int bi = -1;
-    for (int i0 = b - 1; i0 >= a; i0 -= kB) {  // downward scan, strict <: keeps the larger index on ties
-      double sv[kB], pvv[kB];
+    double v[2][2][kF];
+    auto load = [&](double (&x)[2][kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) {
-        const int i = max(i0 - u, a);
-        sv[u] = p.S[at(i)];
-        pvv[u] = p.Pp[at(i)];
+      for (int u = 0; u < kF; u++) {
+        const long long q = at(min(hi - 1, max(i0 - u, sa)));
+        x[0][u] = p.S[q];
+        x[1][u] = p.Pp[q];
       }
+    };
+    auto work = [&](const double (&x)[2][kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) {
+      for (int u = 0; u < kF; u++) {
         const int i = i0 - u;
-        if (i >= a) {
-          const double g = fabs(sv[u] + pvv[u] + lam);
-          if (g < best) { best = g; bi = i; }
+        if (i >= sa) {
+          const double g = fabs(x[0][u] + x[1][u] + lam);
+          if (bits(g) < bits(best)) { best = g; bi = i; }
         }
       }
+    };
+    if (sb > sa) load(v[0], sb - 1);
+    for (int i0 = sb - 1; i0 >= sa; i0 -= 2 * kF) {  // downward scan, strict <: keeps the larger index on ties
+      load(v[1], i0 - kF);
+      work(v[0], i0);
+      load(v[0], i0 - 2 * kF);
+      work(v[1], i0 - kF);
     }
     s_val[w][lane] = best;
     s_idx[w][lane] = bi;
@@ -181,71 +257,106 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
     double best = INFINITY;
     int r = hi - 1;
     for (int q = kTwWarps - 1; q >= 0; q--) {  // segments from the top: the same order as one downward scan
-      if (s_idx[q][lane] >= 0 && s_val[q][lane] < best) { best = s_val[q][lane]; r = s_idx[q][lane]; }
+      if (s_idx[q][lane] >= 0 && bits(s_val[q][lane]) < bits(best)) { best = s_val[q][lane]; r = s_idx[q][lane]; }
     }
-    s_r[lane] = act ? r : 0;
+    s_r[lane] = r;
   }
   __syncthreads();
   const int r = s_r[lane];
-  // ---- solve N_r z = gamma_r e_r with z_r = 1, outwards from r (two directions in parallel)
-  if (act && w == 0) {
-    double z = 1.0, nrm = 1.0;
-    p.Z[at(r)] = 1.0;
-    for (int i0 = r - 1; i0 >= lo; i0 -= kB) {
-      double lv[kB];
+  // ---- solve N_r z = gamma_r e_r with z_r = 1, outwards from r (two directions
+  // in parallel); in step from the outermost r of a warp that shares its block
+  if (w == 0) {
+    const int top = uni ? __reduce_max_sync(0xffffffffu, r) : r;
+    double z = 1.0;
+    double v[2][kF];
+    auto load = [&](double (&x)[kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) lv[u] = p.Lp[at(max(i0 - u, lo))];
+      for (int u = 0; u < kF; u++) x[u] = p.Lp[at(max(min(i0 - u, hi - 2), lo))];
+    };
+    auto work = [&](const double (&x)[kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) {
+      for (int u = 0; u < kF; u++) {
         const int i = i0 - u;
-        if (i >= lo) {
-          z = -lv[u] * z;
-          p.Z[at(i)] = z;
-          nrm += z * z;
-        }
+        if (i < r) z = -x[u] * z;
+        if (i >= lo && i <= r) p.Z[at(i)] = z;
       }
+    };
+    if (nb > 1) load(v[0], top);
+    for (int i0 = top; i0 >= lo; i0 -= 2 * kF) {
+      if (nb > 1) load(v[1], i0 - kF);
+      work(v[0], i0);
+      if (nb > 1) load(v[0], i0 - 2 * kF);
+      work(v[1], i0 - kF);
     }
-    s_nrm[0][lane] = nrm;
-  } else if (act && w == 1) {
-    double z = 1.0, nrm = 0.0;
-    for (int i0 = r + 1; i0 < hi; i0 += kB) {
-      double uv[kB];
+  } else if (w == 1) {
+    const int bot = uni ? __reduce_min_sync(0xffffffffu, r) : r;
+    double z = 1.0;
+    double v[2][kF];
+    auto load = [&](double (&x)[kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) uv[u] = p.Um[at(min(i0 + u, hi - 1) - 1)];
+      for (int u = 0; u < kF; u++) x[u] = p.Um[at(max(min(i0 + u, hi - 1) - 1, lo))];
+    };
+    auto work = [&](const double (&x)[kF], int i0) {
 #pragma unroll
-      for (int u = 0; u < kB; u++) {
+      for (int u = 0; u < kF; u++) {
         const int i = i0 + u;
-        if (i < hi) {
-          z = -uv[u] * z;
-          p.Z[at(i)] = z;
-          nrm += z * z;
-        }
+        if (i > r) z = -x[u] * z;
+        if (i < hi && i > r) p.Z[at(i)] = z;
       }
+    };
+    load(v[0], bot + 1);
+    for (int i0 = bot + 1; i0 < hi; i0 += 2 * kF) {
+      load(v[1], i0 + kF);
+      work(v[0], i0);
+      load(v[0], i0 + 2 * kF);
+      work(v[1], i0 + kF);
     }
-    s_nrm[1][lane] = nrm;
   }
   __syncthreads();
-  // ---- ||B z||^2 for the left vector, split by segment (b is zero at the block end)
+  // ---- ||z||^2, and ||B z||^2 for the left vector, split by segment (b is zero at the block end)
   {
-    double by = 0.0;
-    if (act) {
-      const int seg = (nb + kTwWarps - 1) / kTwWarps;
-      const int a = lo + w * seg, b = min(hi, a + seg);
-#pragma unroll 8
-      for (int i = a; i < b; i++) {
-        const double zi = p.Z[at(i)];
-        const double zn = (i + 1 < hi) ? p.Z[at(i + 1)] : 0.0;
-        const double y = p.a[i] * zi + ((i + 1 < hi) ? p.b[i] * zn : 0.0);
-        by += y * y;
+    double by = 0.0, nrm = 0.0;
+    double zn = sa < sb ? p.Z[at(sa)] : 0.0;
+    constexpr int kH = kTwB;
+    double v[2][3][kH];
+    auto load = [&](double (&x)[3][kH], int i0) {
+#pragma unroll
+      for (int u = 0; u < kH; u++) {
+        const int i = max(sa, min(i0 + u, sb - 1));
+        x[0][u] = (i + 1 < hi) ? p.Z[at(i + 1)] : 0.0;
+        x[1][u] = p.a[i];
+        x[2][u] = (i + 1 < hi) ? p.b[i] : 0.0;
       }
+    };
+    auto work = [&](const double (&x)[3][kH], int i0) {
+#pragma unroll
+      for (int u = 0; u < kH; u++)
+        if (i0 + u < sb) {
+          const double zi = zn;
+          zn = x[0][u];
+          const double y = x[1][u] * zi + x[2][u] * zn;
+          by += y * y;
+          nrm += zi * zi;
+        }
+    };
+    if (sa < sb) load(v[0], sa);
+    for (int i0 = sa; i0 < sb; i0 += 2 * kH) {
+      load(v[1], i0 + kH);
+      work(v[0], i0);
+      load(v[0], i0 + 2 * kH);
+      work(v[1], i0 + kH);
     }
     s_val[w][lane] = by;
+    s_nrm[w][lane] = nrm;
   }
   __syncthreads();
   if (w == 0 && act) {
-    double by = 0.0;
-    for (int q = 0; q < kTwWarps; q++) by += s_val[q][lane];
-    p.xinv[k] = 1.0 / sqrt(s_nrm[0][lane] + s_nrm[1][lane]);
+    double by = 0.0, nrm = 0.0;
+    for (int q = 0; q < kTwWarps; q++) {
+      by += s_val[q][lane];
+      nrm += s_nrm[q][lane];
+    }
+    p.xinv[k] = 1.0 / sqrt(nrm);
     p.yinv[k] = (by > 0.0) ? 1.0 / sqrt(by) : 0.0;
   }
 }
@@ -444,16 +555,16 @@ constexpr int kRankTile = 1024;
 
 __global__ void __launch_bounds__(kRankThreads) tw_rank_count_kernel(int N, const double* __restrict__ sigma,
                                                                    VecLayout L, int* rank, int seg) {
-  __shared__ double tile[kRankTile];
+  __shared__ long long tile[kRankTile];  // bit patterns: order as the (non-negative) values do
   __shared__ int s_lo, s_hi;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   int glo = N, ghi = 0;
-  double v = 0.0;
+  long long v = 0;
   if (k < N) {
     const int g = L.grp[k];
     glo = L.g_lo[g];
     ghi = glo + L.g_n[g];
-    v = sigma[k];
+    v = bits(sigma[k]);
   }
   if (threadIdx.x == 0) {
     s_lo = N;
@@ -469,11 +580,11 @@ __global__ void __launch_bounds__(kRankThreads) tw_rank_count_kernel(int N, cons
   int cnt = 0;
   for (int t0 = j0; t0 < j1; t0 += kRankTile) {
     const int t1 = min(j1, t0 + kRankTile);
-    for (int j = t0 + threadIdx.x; j < t1; j += blockDim.x) tile[j - t0] = sigma[j];
+    for (int j = t0 + threadIdx.x; j < t1; j += blockDim.x) tile[j - t0] = bits(sigma[j]);
     __syncthreads();
     const int a = max(t0, glo), b = min(t1, ghi);
     for (int j = a; j < b; j++) {
-      const double u = tile[j - t0];
+      const long long u = tile[j - t0];
       cnt += (u < v) || (u == v && j < k);
     }
     __syncthreads();
@@ -607,7 +718,10 @@ int bd_vectors(ddcsvd_context* ctx, int N, long long store, const double* a, con
   tw_absmax_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, amax);
   tw_setup_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, amax, dd, ll, dl, dll);
   count_launch(2);
-  twisted_kernel<<<ceil_div(N, 32), 32 * kTwWarps, 0, ctx->stream>>>(p);
+  if (store / N >= 256)  // mean block size, weighted by its vectors
+    twisted_kernel<16><<<ceil_div(N, 32), 32 * kTwWarps, 0, ctx->stream>>>(p);
+  else
+    twisted_kernel<8><<<ceil_div(N, 32), 32 * kTwWarps, 0, ctx->stream>>>(p);
   count_launch();
   tw_cluster_kernel<<<std::min(ceil_div(N, kClThreads), 2 * ctx->num_sms), kClThreads, 0, ctx->stream>>>(p);
   count_launch();
