@@ -9,22 +9,47 @@
 // + (I - U U^T) gU S^-1 V^T.  (The reference has no derivative; this is the
 // standard SVD adjoint.)  Any of gU, gs, gV may be null (zero).
 //
-// Four kernels per call: a batched tiled GEMM for J and K, an elementwise
-// kernel for M, the batched GEMM for U M (+ gU S^-1 as its C input) and for
-// (U M + gU S^-1) V^T.
+// Four launches per call: J and K together, an elementwise kernel for M, then
+// P = U M + gU S^-1 and gA = P V^T, all batched products of any strides.  FP32
+// products run on the FP32 pipe; FP64 ones on the tensor cores, exactly on
+// digits (ozgemm_kernel), because GB300's FP64 pipe is 1/64 of FP32's.
 #include <cudaTypedefs.h>
 
+#include <cuda_fp16.h>
+
 #include "ctx_cache.hpp"
+#include "fp64.cuh"
 #include "internal.hpp"
 
 namespace ddcsvd {
 
-// C[b] (M x N, col-major, ldc) = beta * C[b] + alpha * A[b] B[b], element
-// (r, k) of A[b] at A + b*as + r*ars + k*acs, element (k, c) of B[b] at
-// B + b*bs + k*brs + c*bcs.  64 x 64 tiles, 256 threads with 4 x 4 outputs
-// each (rows ty + 16 a, columns tx + 16 c), K in slabs of 16.  Tile loads
-// walk the operand's unit-stride index fastest, so either layout of A and B
-// (the adjoint reads U, V transposed and not) is read in coalesced segments.
+__device__ __forceinline__ float adj_quot(float a, float x) { return a / x; }
+__device__ __forceinline__ double adj_quot(double a, double x) { return quot_rn(a, x); }
+
+// A matrix of every problem: element (r, c) of problem b at p + b*b_ + r*r_ + c*c_.
+template <typename T>
+struct BMat {
+  const T* p;
+  long long r, c, b;
+};
+
+// C[b] (M x N, column-major, ldc) = A[b] B[b] + X[b] diag(s[b])^-1 (X.p may be null).
+template <typename T>
+struct BGemm {
+  int M, N, K;
+  BMat<T> A, B, X;
+  const T* s;
+  long long sb;
+  T* C;
+  int ldc;
+  long long cb;
+};
+
+// 64 x 64 tiles, 256 threads with 4 x 4 outputs each (rows ty + 16 a, columns
+// tx + 16 c), K in slabs of 16.  Tile loads walk the operand's unit-stride index
+// fastest, so either layout of A and B (the adjoint reads U, V transposed and
+// not) is read in coalesced segments.  blockIdx.z: problem, first of g0, then of
+// g1.
 constexpr int kBgTile = 64, kBgK = 16;
 
 template <typename T>
@@ -42,25 +67,25 @@ __device__ __forceinline__ void bgemm_load(T (*dst)[kBgTile + 1], const T* __res
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) bgemm_kernel(int M, int N, int K, const T* __restrict__ A, long long ars,
-                                                    long long acs, long long as, const T* __restrict__ B,
-                                                    long long brs, long long bcs, long long bs, T* C, int ldc,
-                                                    long long cs, T alpha, T beta) {
+__global__ void __launch_bounds__(256) bgemm_kernel(BGemm<T> g0, BGemm<T> g1, int batch) {
   __shared__ T At[kBgK][kBgTile + 1];
   __shared__ T Bt[kBgK][kBgTile + 1];
-  const int b = blockIdx.z;
+  const bool first = (int)blockIdx.z < batch;
+  const BGemm<T> g = first ? g0 : g1;
+  const int b = first ? blockIdx.z : blockIdx.z - batch;
   const int r0 = blockIdx.x * kBgTile, c0 = blockIdx.y * kBgTile;
+  if (r0 >= g.M || c0 >= g.N) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const T* Ab = A + b * as;
-  const T* Bb = B + b * bs;
+  const T* Ab = g.A.p + b * g.A.b;
+  const T* Bb = g.B.p + b * g.B.b;
   T acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; a++)
 #pragma unroll
     for (int c = 0; c < 4; c++) acc[a][c] = T(0);
-  for (int k0 = 0; k0 < K; k0 += kBgK) {
-    bgemm_load<T>(At, Ab, ars, acs, r0, M, k0, K);
-    bgemm_load<T>(Bt, Bb, bcs, brs, c0, N, k0, K);
+  for (int k0 = 0; k0 < g.K; k0 += kBgK) {
+    bgemm_load<T>(At, Ab, g.A.r, g.A.c, r0, g.M, k0, g.K);
+    bgemm_load<T>(Bt, Bb, g.B.c, g.B.r, c0, g.N, k0, g.K);
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < kBgK; kk++) {
@@ -77,102 +102,394 @@ __global__ void __launch_bounds__(256) bgemm_kernel(int M, int N, int K, const T
     }
     __syncthreads();
   }
-  T* Cb = C + b * cs;
+  T* Cb = g.C + b * g.cb;
 #pragma unroll
   for (int a = 0; a < 4; a++)
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int r = r0 + ty + 16 * a, cc = c0 + tx + 16 * c;
-      if (r < M && cc < N) {
-        T* p = Cb + r + (size_t)cc * ldc;
-        *p = (beta == T(0) ? T(0) : beta * *p) + alpha * acc[a][c];
+      if (r < g.M && cc < g.N) {
+        T v = acc[a][c];
+        if (g.X.p) v += adj_quot(g.X.p[b * g.X.b + r * g.X.r + cc * g.X.c], g.s[b * g.sb + cc]);
+        Cb[r + (size_t)cc * g.ldc] = v;
       }
     }
 }
 
-// M (k x k per problem) from J, K, s, gs; P := gU S^-1 (m x k) in the same pass.
+// ---------------------------------------------------------------- FP64 products on the tensor cores
+// The Ozaki scheme (Ozaki, Ogita, Oishi, Rump, "Error-free transformations of
+// matrix multiplication", Numer. Algorithms 59, 2012; on FP16 tensor cores:
+// Mukunoki, Ozaki, Ogita, Imamura, ISC 2020): every row of A and column of B is
+// scaled by a power of two and rounded to a 54-bit integer, the integer written
+// in seven signed base-256 digits, and each pair of digit matrices multiplied in
+// FP16 with FP32 accumulation.  Digits are at most 128 in magnitude, so a sum of
+// up to seven pairs over K = 128 stays below 2^24 and every accumulation is
+// exact; the 34 pairs of weight 256^12 .. 256^5 are kept and put together in
+// 64-bit integers.  What is lost is the rounding to 54 bits of a row's or
+// column's largest entry and the pairs below, together below the rounding
+// errors of an FP64 sum of the same products (against quadruple precision, the
+// adjoint of 128 x 64, 200 x 100 and 16 x 16 problems is 2.7e-16, 3.0e-16 and
+// 2.2e-16 off, where FP64 sums gave 5.3e-16, 6.5e-16 and 2.8e-16).  Rows or columns that hold Inf or NaN take plain
+// FP64 sums.  The FP64 pipe bounded the direct form (0.98 ms for the four
+// products of 256 x (128 x 64), 0.85 ms at cuBLAS's DGEMM rate); this one is
+// bound by the tensor pipe and the digit extraction (integer instructions).
+//
+// 64 x 32 tile per CTA, eight warps of 16 x 16, two CTAs per SM (one extracts
+// digits while the other multiplies), K in slabs of 32 through two stages.
+constexpr int kOzThreads = 256;
+constexpr int kOzM = 64, kOzN = 32, kOzK = 32;           // tile, slab
+constexpr int kOzD = 7, kOzS = 8;                        // digits, diagonals
+constexpr int kOzLd = kOzK + 8;                          // halves per staged row: ldmatrix rows on distinct banks
+constexpr int kOzChunk = 128;                            // K per exact accumulation
+constexpr int kOzStage = kOzD * (kOzM + kOzN) * kOzLd;   // halves per stage: A's digits, then B's
+constexpr int kOzSmem = 2 * kOzStage * (int)sizeof(__half);
+
+// One operand of the tile: R rows (of A, or columns of B) by K.
+struct OzOp {
+  const double* p;  // problem's matrix at the tile's first row
+  long long s_r, s_k;
+  int rows;  // valid rows
+  int K;
+  bool k_fast;  // K has the unit stride
+};
+// Unit u of an R x 32 slab: eight consecutive k of one row (a 16-byte store per
+// digit); consecutive threads walk the operand's unit stride.
+template <int R>
+__device__ __forceinline__ void oz_place(const OzOp& o, int u, int& r, int& k) {
+  if (o.k_fast) {
+    r = u >> 2;
+    k = 8 * (u & 3);
+  } else {
+    r = u % R;
+    k = 8 * (u / R);
+  }
+}
+template <int R>
+__device__ __forceinline__ void oz_load(const OzOp& o, int k0, int u, double (&v)[8]) {
+  int r, k;
+  oz_place<R>(o, u, r, k);
+  k += k0;
+  const double* q = o.p + r * o.s_r + k * o.s_k;
+#pragma unroll
+  for (int h = 0; h < 8; h++) v[h] = (r < o.rows && k + h < o.K) ? q[h * o.s_k] : 0.0;
+}
+template <int R>
+__device__ __forceinline__ bool oz_max(const OzOp& o, int* e) {  // exponents of the largest entries; any non-finite?
+  bool bad = false;
+  for (int u = threadIdx.x; u < 4 * R; u += kOzThreads) {
+    int ex = 1, r, k;
+    oz_place<R>(o, u, r, k);
+#pragma unroll 2
+    for (int k0 = 0; k0 < o.K; k0 += kOzK) {
+      double v[8];
+      oz_load<R>(o, k0, u, v);
+#pragma unroll
+      for (int h = 0; h < 8; h++) ex = max(ex, (__double2hiint(v[h]) >> 20) & 0x7ff);
+    }
+    atomicMax(&e[r], ex);
+    bad = bad || ex == 0x7ff;
+  }
+  return bad;
+}
+// v 2^(54 - e) rounded to an integer, where |v| < 2^e, plus 128 in each of the
+// seven low bytes: byte t is then digit t + 128
+__device__ __forceinline__ unsigned long long oz_digits(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+  if (ex) m |= 0x10000000000000ull;
+  const int sh = (ex ? ex : 1) - 1075 + 54 - e;  // at most 1
+  unsigned long long x;
+  if (sh >= 0) x = m << sh;
+  else if (sh > -64) x = (m + (1ull << (-sh - 1))) >> -sh;
+  else x = 0;
+  return (b < 0 ? 0ull - x : x) + 0x0080808080808080ull;
+}
+// digits of one slab into a stage: digit d (0 = most significant) of row r at
+// dst + (d R + r) kOzLd + k
+template <int R>
+__device__ __forceinline__ void oz_stage(const OzOp& o, const int* e, int k0, __half* dst) {
+  for (int u = threadIdx.x; u < 4 * R; u += kOzThreads) {
+    double v[8];
+    oz_load<R>(o, k0, u, v);
+    int r, k;
+    oz_place<R>(o, u, r, k);
+    const int er = e[r];
+    unsigned long long y[8];
+#pragma unroll
+    for (int h = 0; h < 8; h++) y[h] = oz_digits(v[h], er);
+    __half* q = dst + r * kOzLd + k;
+#pragma unroll
+    for (int d = 0; d < kOzD; d++) {
+      const int t = kOzD - 1 - d;  // byte
+      const unsigned by = t & 3;
+      unsigned w[4];
+#pragma unroll
+      for (int h = 0; h < 4; h++) {
+        const unsigned w0 = t < 4 ? (unsigned)y[2 * h] : (unsigned)(y[2 * h] >> 32);
+        const unsigned w1 = t < 4 ? (unsigned)y[2 * h + 1] : (unsigned)(y[2 * h + 1] >> 32);
+        // halves 1024 + (digit + 128) from the bytes, minus 1152
+        const unsigned x = (__byte_perm(w0, w1, by | (4 + by) << 8) & 0x00ff00ffu) | 0x64006400u;
+        const __half2 hv = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2half2(__ushort_as_half(0x6480)));
+        w[h] = *reinterpret_cast<const unsigned*>(&hv);
+      }
+      *reinterpret_cast<uint4*>(q + d * R * kOzLd) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+__device__ __forceinline__ void ldsm4(unsigned (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p))
+               : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0, BGemm<double> g1, int batch) {
+  extern __shared__ __align__(16) __half ozm[];  // [stage][A digits, B digits]
+  __shared__ int s_ea[kOzM], s_eb[kOzN];         // exponent bound of each row of A / column of B
+  __shared__ double s_rs[kOzN];                  // 1 / s of each column
+  __shared__ int s_bad;
+  const bool first = (int)blockIdx.z < batch;
+  const BGemm<double>& g = first ? g0 : g1;
+  const int b = first ? blockIdx.z : blockIdx.z - batch;
+  const int r0 = blockIdx.x * kOzM, c0 = blockIdx.y * kOzN;
+  if (r0 >= g.M || c0 >= g.N) return;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const OzOp A{g.A.p + b * g.A.b + r0 * g.A.r, g.A.r, g.A.c, min(kOzM, g.M - r0), g.K, g.A.c == 1};
+  const OzOp B{g.B.p + b * g.B.b + c0 * g.B.c, g.B.c, g.B.r, min(kOzN, g.N - c0), g.K, g.B.r == 1};
+  // ---- exponent of the largest entry of each row / column
+  if (t < kOzM) s_ea[t] = 1;
+  if (t < kOzN) s_eb[t] = 1;
+  if (t == 0) s_bad = 0;
+  __syncthreads();
+  const bool bada = oz_max<kOzM>(A, s_ea), badb = oz_max<kOzN>(B, s_eb);
+  if (bada || badb) s_bad = 1;
+  if (g.X.p && t < B.rows) s_rs[t] = adj_quot(1.0, g.s[b * g.sb + c0 + t]);
+  __syncthreads();
+  const bool bad = s_bad != 0;
+  if (t < kOzM) s_ea[t] -= 1022;  // |v| < 2^(exponent - 1022)
+  if (t < kOzN) s_eb[t] -= 1022;
+  __syncthreads();
+  const int wm = (wid & 3) * 16, wn = (wid >> 2) * 16;  // the warp's part of the tile
+  // value x of the lane: row (lane >> 2) + 8 ((x >> 1) & 1), column 8 (x >> 2) + 2 (lane & 3) + (x & 1)
+  const int lr = wm + (lane >> 2), lc = wn + 2 * (lane & 3);
+  double run[8];
+#pragma unroll
+  for (int x = 0; x < 8; x++) run[x] = 0.0;
+  if (bad) {
+    for (int k = 0; k < g.K; k++)
+#pragma unroll
+      for (int x = 0; x < 8; x++) {
+        const int r = lr + 8 * ((x >> 1) & 1), c = lc + 8 * (x >> 2) + (x & 1);
+        if (r < A.rows && c < B.rows) run[x] += A.p[r * A.s_r + k * A.s_k] * B.p[c * B.s_r + k * B.s_k];
+      }
+  } else {
+    auto stage = [&](int s, int op) { return ozm + (size_t)s * kOzStage + op * kOzD * kOzM * kOzLd; };
+    oz_stage<kOzM>(A, s_ea, 0, stage(0, 0));
+    oz_stage<kOzN>(B, s_eb, 0, stage(0, 1));
+    float acc[kOzS][2][4];
+#pragma unroll
+    for (int s = 0; s < kOzS; s++)
+#pragma unroll
+      for (int x = 0; x < 8; x++) acc[s][x >> 2][x & 3] = 0.f;
+    int buf = 0;
+    for (int k0 = 0; k0 < g.K; k0 += kOzK, buf ^= 1) {
+      const bool more = k0 + kOzK < g.K;
+      __syncthreads();  // stage `buf` written; the other one's readers are done
+      const __half* sa = stage(buf, 0) + (wm + (lane & 15)) * kOzLd + 8 * (lane >> 4);
+      const __half* sb = stage(buf, 1) + (wn + (lane & 7) + 8 * (lane >> 4)) * kOzLd + 8 * ((lane >> 3) & 1);
+#pragma unroll
+      for (int kk = 0; kk < kOzK; kk += 16) {
+        unsigned bf[kOzD][4];
+#pragma unroll
+        for (int j = 0; j < kOzD; j++) ldsm4(bf[j], sb + j * kOzN * kOzLd + kk);
+#pragma unroll
+        for (int i = 0; i < kOzD; i++) {
+          unsigned af[4];
+          ldsm4(af, sa + i * kOzM * kOzLd + kk);
+#pragma unroll
+          for (int j = 0; j < kOzD; j++) {
+            if (i + j >= kOzS) continue;
+            mma16816(acc[i + j][0], af, bf[j][0], bf[j][1]);
+            mma16816(acc[i + j][1], af, bf[j][2], bf[j][3]);
+          }
+        }
+      }
+      if (more) {
+        oz_stage<kOzM>(A, s_ea, k0 + kOzK, stage(buf ^ 1, 0));
+        oz_stage<kOzN>(B, s_eb, k0 + kOzK, stage(buf ^ 1, 1));
+      }
+      if (!more || (k0 + kOzK) % kOzChunk == 0) {
+        // the exact sums of this chunk, weights 2^96 .. 2^72 and 2^64 .. 2^40; each
+        // half is below 2^49, so an integer added to the bits of 1.5 2^52 is its double
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+          double w[2];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            long long q = 0;
+#pragma unroll
+            for (int s = 4 * h; s < 4 * h + 4; s++) {
+              float& f = acc[s][x >> 2][x & 3];
+              q = q * 256 + __float2int_rn(f);
+              f = 0.f;
+            }
+            w[h] = __longlong_as_double(0x4338000000000000ll + q) - 6755399441055744.0;
+          }
+          const double v = fma(w[0], 4294967296.0, w[1]);
+          run[x] = k0 < kOzChunk ? v : run[x] + v;
+        }
+      }
+    }
+  }
+  double* Cb = g.C + b * g.cb;
+#pragma unroll
+  for (int x = 0; x < 8; x++) {
+    const int r = lr + 8 * ((x >> 1) & 1), c = lc + 8 * (x >> 2) + (x & 1);
+    if (r < A.rows && c < B.rows) {
+      double v = run[x];
+      if (!bad) {  // v 2^(e_r + e_c - 68), in the exponent field where both ends are normal
+        const int sh = s_ea[r] + s_eb[c] - 68, ex = (__double2hiint(v) >> 20) & 0x7ff;
+        if (ex != 0 && ex + sh > 0 && ex + sh < 0x7ff)
+          v = __hiloint2double(__double2hiint(v) + (sh << 20), __double2loint(v));
+        else
+          v = scalbn(v, sh);
+      }
+      if (g.X.p) {
+        const double xv = g.X.p[b * g.X.b + (r0 + r) * g.X.r + (c0 + c) * g.X.c];
+        const double rs = s_rs[c];
+        v += mid_range(rs) ? xv * rs : adj_quot(xv, g.s[b * g.sb + c0 + c]);
+      }
+      Cb[(r0 + r) + (size_t)(c0 + c) * g.ldc] = v;
+    }
+  }
+}
+
+// M (k x k per problem) from J, K, s, gs.  The pair (i, j), (j, i) shares
+// F_ij (J_ij - J_ji) and F_ij (K_ij - K_ji), which do not change under exchange.
+// Columns a and k - 1 - a of the upper triangle hold k + 1 entries together, so
+// the pairs fill a rectangle and no lane idles through an FP64 instruction.
+constexpr int kCoreCols = 512;
+__device__ __forceinline__ bool adj_mid(double x) { return mid_range(x); }
+__device__ __forceinline__ bool adj_mid(float) { return false; }  // FP32 divisions cost nothing that matters here
+
 template <typename T>
-__global__ void adjoint_core_kernel(int k, int m, const T* __restrict__ J, const T* __restrict__ Kv,
-                                    const T* __restrict__ s, const T* __restrict__ gs, const T* __restrict__ gU,
-                                    T* Mo, T* P) {
+__global__ void __launch_bounds__(256) adjoint_core_kernel(int k, const T* __restrict__ J, const T* __restrict__ Kv,
+                                                           const T* __restrict__ s, const T* __restrict__ gs, T* Mo) {
   const int b = blockIdx.y;
   const T* Jb = J ? J + (size_t)b * k * k : nullptr;
   const T* Kb = Kv ? Kv + (size_t)b * k * k : nullptr;
   const T* sb = s + (size_t)b * k;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < k * k; idx += gridDim.x * blockDim.x) {
-    const int i = idx % k, j = idx / k;
+  T* Mb = Mo + (size_t)b * k * k;
+  // 1 / s of every column once per CTA; columns whose reciprocal leaves the
+  // normal range (or beyond the table) divide
+  __shared__ T s_rs[kCoreCols];
+  for (int c = threadIdx.x; c < min(k, kCoreCols); c += blockDim.x) s_rs[c] = adj_quot(T(1), sb[c]);
+  __syncthreads();
+  auto over = [&](T x, int c) {  // x / s_c
+    return (c < kCoreCols && adj_mid(s_rs[c])) ? x * s_rs[c] : adj_quot(x, sb[c]);
+  };
+  const int half = (k + 1) / 2;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < half * (k + 1); idx += gridDim.x * blockDim.x) {
+    const int a = idx / (k + 1), c = idx % (k + 1);
+    const int i = c <= a ? c : c - a - 1, j = c <= a ? a : k - 1 - a;
+    if (c > a && 2 * a + 1 == k) continue;  // odd k: the middle column once
     const T si = sb[i], sj = sb[j];
-    T v = T(0);
+    const int ij = i + j * k, ji = j + i * k;
     if (i == j) {
-      if (gs) v += gs[(size_t)b * k + i];
-    } else {
-      const T f = T(1) / ((sj - si) * (sj + si));
-      if (Jb) v += f * (Jb[i + (size_t)j * k] - Jb[j + (size_t)i * k]) * sj;
-      if (Kb) v += si * f * (Kb[i + (size_t)j * k] - Kb[j + (size_t)i * k]);
+      T v = gs ? gs[(size_t)b * k + i] : T(0);
+      if (Jb) v -= over(Jb[ij], j);
+      Mb[ij] = v;
+      continue;
     }
-    if (Jb) v -= Jb[i + (size_t)j * k] / sj;
-    Mo[(size_t)b * k * k + idx] = v;
-  }
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < m * k; idx += gridDim.x * blockDim.x) {
-    const int j = idx / m;
-    P[(size_t)b * m * k + idx] = gU ? gU[(size_t)b * m * k + idx] / sb[j] : T(0);
+    const T f = adj_quot(T(1), (sj - si) * (sj + si));
+    T vij = T(0), vji = T(0);
+    if (Jb) {
+      const T x = Jb[ij], y = Jb[ji], fj = f * (x - y);
+      vij += fj * sj - over(x, j);
+      vji += fj * si - over(y, i);
+    }
+    if (Kb) {
+      const T fk = f * (Kb[ij] - Kb[ji]);
+      vij += si * fk;
+      vji += sj * fk;
+    }
+    Mb[ij] = vij;
+    Mb[ji] = vji;
   }
 }
 
-template <typename T>
-static int bgemm(ddcsvd_context* ctx, int batch, int M, int N, int K, const T* A, long long ars, long long acs,
-                 long long as, const T* B, long long brs, long long bcs, long long bs, T* C, int ldc, long long cs,
-                 T alpha, T beta) {
-  dim3 grid(ceil_div(M, kBgTile), ceil_div(N, kBgTile), batch);
-  bgemm_kernel<T><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, ars, acs, as, B, brs, bcs, bs, C, ldc, cs, alpha,
-                                                 beta);
+static int bgemm(ddcsvd_context* ctx, int batch, const BGemm<float>& g0, const BGemm<float>* g1) {
+  const int M = std::max(g0.M, g1 ? g1->M : 0), N = std::max(g0.N, g1 ? g1->N : 0);
+  dim3 grid(ceil_div(M, kBgTile), ceil_div(N, kBgTile), batch * (g1 ? 2 : 1));
+  bgemm_kernel<float><<<grid, 256, 0, ctx->stream>>>(g0, g1 ? *g1 : g0, batch);
+  count_launch();
+  DDC_CUDA_TRY(cudaGetLastError());
+  return DDCSVD_OK;
+}
+static int bgemm(ddcsvd_context* ctx, int batch, const BGemm<double>& g0, const BGemm<double>* g1) {
+  const int M = std::max(g0.M, g1 ? g1->M : 0), N = std::max(g0.N, g1 ? g1->N : 0);
+  dim3 grid(ceil_div(M, kOzM), ceil_div(N, kOzN), batch * (g1 ? 2 : 1));
+  DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)ozgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem));
+  ozgemm_kernel<<<grid, kOzThreads, kOzSmem, ctx->stream>>>(g0, g1 ? *g1 : g0, batch);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;
 }
 
-// The four launches of one adjoint on intermediates J, Kv, Mm (k x k per
-// problem) and P (m x k per problem).  Launch grids carry the batch in
-// gridDim.z / gridDim.y (at most 65535), so larger batches go in chunks.
-constexpr int kBatchChunk = 65535;
+// The launches of one adjoint on intermediates J, Kv, Mm (k x k per problem)
+// and P (m x k per problem).  Launch grids carry the batch in gridDim.z /
+// gridDim.y (at most 65535, two products in one launch), so larger batches go
+// in chunks.  Inputs by strides (column-major for the C entry points).
+constexpr int kBatchChunk = 32767;
 
 template <typename T>
-static int adjoint_enqueue(ddcsvd_context* h, int batch, int m, int n, const T* U, const T* S, const T* V,
-                           const T* gU, const T* gS, const T* gV, T* gA, T* J, T* Kv, T* Mm, T* P) {
+static int adjoint_enqueue(ddcsvd_context* h, int batch, int m, int n, BMat<T> U, const T* S, BMat<T> V, BMat<T> gU,
+                           const T* gS, BMat<T> gV, T* gA, T* J, T* Kv, T* Mm, T* P) {
   const int k = n;
-  const long long sU = (long long)m * k, sV = (long long)n * k, sK = (long long)k * k, sA = (long long)m * n;
+  const long long sP = (long long)m * k, sK = (long long)k * k, sA = (long long)m * n;
+  auto tr = [](BMat<T> x) { return BMat<T>{x.p, x.c, x.r, x.b}; };
+  const BMat<T> none{nullptr, 0, 0, 0};
   for (int b0 = 0; b0 < batch; b0 += kBatchChunk) {
     const int nb = std::min(kBatchChunk, batch - b0);
-    const T* Ub = U + b0 * sU;
-    const T* Vb = V + b0 * sV;
+    auto at = [&](BMat<T> x) { return BMat<T>{x.p ? x.p + b0 * x.b : nullptr, x.r, x.c, x.b}; };
+    const BMat<T> Ub = at(U), Vb = at(V), gUb = at(gU), gVb = at(gV);
     const T* Sb = S + b0 * (long long)k;
-    const T* gUb = gU ? gU + b0 * sU : nullptr;
-    const T* gVb = gV ? gV + b0 * sV : nullptr;
-    const T* gSb = gS ? gS + b0 * (long long)k : nullptr;
     T* Jb = J + b0 * sK;
     T* Kb = Kv + b0 * sK;
     T* Mb = Mm + b0 * sK;
-    T* Pb = P + b0 * sU;
+    T* Pb = P + b0 * sP;
     // J = U^T gU, K = V^T gV
-    if (gUb) DDC_TRY(bgemm<T>(h, nb, k, k, m, Ub, m, 1, sU, gUb, 1, m, sU, Jb, k, sK, T(1), T(0)));
-    if (gVb) DDC_TRY(bgemm<T>(h, nb, k, k, n, Vb, n, 1, sV, gVb, 1, n, sV, Kb, k, sK, T(1), T(0)));
-    dim3 g2(std::max(1, std::min(64, ceil_div(std::max(k * k, m * k), 256))), nb);
-    adjoint_core_kernel<T><<<g2, 256, 0, h->stream>>>(k, m, gUb ? Jb : nullptr, gVb ? Kb : nullptr, Sb, gSb, gUb,
-                                                      Mb, Pb);
+    const BGemm<T> gj{k, k, m, tr(Ub), gUb, none, nullptr, 0, Jb, k, sK};
+    const BGemm<T> gk{k, k, n, tr(Vb), gVb, none, nullptr, 0, Kb, k, sK};
+    if (gUb.p && gVb.p) DDC_TRY(bgemm(h, nb, gj, &gk));
+    else if (gUb.p) DDC_TRY(bgemm(h, nb, gj, nullptr));
+    else if (gVb.p) DDC_TRY(bgemm(h, nb, gk, nullptr));
+    dim3 g2(std::max(1, std::min(64, ceil_div((k + 1) / 2 * (k + 1), 256))), nb);
+    adjoint_core_kernel<T><<<g2, 256, 0, h->stream>>>(k, gUb.p ? Jb : nullptr, gVb.p ? Kb : nullptr, Sb,
+                                                      gS ? gS + b0 * (long long)k : nullptr, Mb);
     count_launch();
     DDC_CUDA_TRY(cudaGetLastError());
-    // P += U M
-    DDC_TRY(bgemm<T>(h, nb, m, k, k, Ub, 1, m, sU, Mb, 1, k, sK, Pb, m, sU, T(1), T(1)));
+    // P = U M + gU S^-1
+    const BGemm<T> gp{m, k, k, Ub, BMat<T>{Mb, 1, k, sK}, gUb, Sb, k, Pb, m, sP};
+    DDC_TRY(bgemm(h, nb, gp, nullptr));
     // gA = P V^T
-    DDC_TRY(bgemm<T>(h, nb, m, n, k, Pb, 1, m, sU, Vb, n, 1, sV, gA + b0 * sA, m, sA, T(1), T(0)));
+    const BGemm<T> ga{m, n, k, BMat<T>{Pb, 1, m, sP}, tr(Vb), none, nullptr, 0, gA + b0 * sA, m, sA};
+    DDC_TRY(bgemm(h, nb, ga, nullptr));
   }
   return DDCSVD_OK;
 }
 
 template <typename T>
-static int svd_backward(ddcsvd_context* h, int batch, int m, int n, const T* U, const T* S, const T* V, const T* gU,
-                        const T* gS, const T* gV, T* gA) {
-  if (!h || batch <= 0 || m <= 0 || n <= 0 || m < n || !U || !S || !V || !gA) return DDCSVD_ERR_ARG;
+static int svd_backward(ddcsvd_context* h, int batch, int m, int n, BMat<T> U, const T* S, BMat<T> V, BMat<T> gU,
+                        const T* gS, BMat<T> gV, T* gA) {
+  if (!h || batch <= 0 || m <= 0 || n <= 0 || m < n || !U.p || !S || !V.p || !gA) return DDCSVD_ERR_ARG;
   std::lock_guard<std::mutex> g(h->mu);
   DDC_CUDA_TRY(cudaSetDevice(h->device));
   const int k = n;
@@ -193,6 +510,11 @@ static int svd_backward(ddcsvd_context* h, int batch, int m, int n, const T* U, 
   DDC_TRY(reset_status(h));
   DDC_TRY(adjoint_enqueue<T>(h, batch, m, n, U, S, V, gU, gS, gV, gA, J, Kv, Mm, P));
   return check_status(h, "svd_backward");
+}
+// column-major matrices of `rows` rows, one after another
+template <typename T>
+static BMat<T> colmajor(const T* p, int rows, int cols) {
+  return BMat<T>{p, 1, rows, (long long)rows * cols};
 }
 
 // ---------------------------------------------------------------- allocation-free variant
@@ -304,7 +626,8 @@ static int svd_backward_f64_noalloc(cudaStream_t stream, int batch, int m, int n
   // overwritten before they are read, so nothing needs clearing.  The call
   // only enqueues: kernels of the same stream run in order, and a caller
   // reads gA after synchronising the stream.
-  DDC_TRY(adjoint_enqueue<double>(&ctx, batch, m, n, U, S, V, gU, gS, gV, gA, J, Kv, Mm, P));
+  DDC_TRY(adjoint_enqueue<double>(&ctx, batch, m, n, colmajor(U, m, n), S, colmajor(V, n, n), colmajor(gU, m, n), gS,
+                                  colmajor(gV, n, n), gA, J, Kv, Mm, P));
   return DDCSVD_OK;
 }
 }  // namespace ddcsvd
@@ -320,11 +643,34 @@ extern "C" int ddcsvd_svd_backward_f64_noalloc(void* stream, int batch, int m, i
 extern "C" int ddcsvd_svd_backward_f64_device(ddcsvd_handle_t h, int batch, int m, int n, const double* dU,
                                               const double* dS, const double* dV, const double* gU,
                                               const double* gS, const double* gV, double* gA) {
-  return svd_backward<double>(h, batch, m, n, dU, dS, dV, gU, gS, gV, gA);
+  return svd_backward<double>(h, batch, m, n, colmajor(dU, m, n), dS, colmajor(dV, n, n), colmajor(gU, m, n), gS,
+                              colmajor(gV, n, n), gA);
 }
 
 extern "C" int ddcsvd_svd_backward_f32_device(ddcsvd_handle_t h, int batch, int m, int n, const float* dU,
                                               const float* dS, const float* dV, const float* gU, const float* gS,
                                               const float* gV, float* gA) {
-  return svd_backward<float>(h, batch, m, n, dU, dS, dV, gU, gS, gV, gA);
+  return svd_backward<float>(h, batch, m, n, colmajor(dU, m, n), dS, colmajor(dV, n, n), colmajor(gU, m, n), gS,
+                             colmajor(gV, n, n), gA);
+}
+
+template <typename T>
+static int svd_backward_strided(ddcsvd_context* h, int batch, int m, int n, const T* U, const T* S, const T* V,
+                                const T* gU, const T* gS, const T* gV, const long long* strides, T* gA) {
+  if (!strides) return DDCSVD_ERR_ARG;
+  auto mat = [&](const T* p, int q) { return BMat<T>{p, strides[3 * q], strides[3 * q + 1], strides[3 * q + 2]}; };
+  return svd_backward<T>(h, batch, m, n, mat(U, 0), S, mat(V, 1), mat(gU, 2), gS, mat(gV, 3), gA);
+}
+
+extern "C" int ddcsvd_svd_backward_f64_strided(ddcsvd_handle_t h, int batch, int m, int n, const double* dU,
+                                               const double* dS, const double* dV, const double* gU,
+                                               const double* gS, const double* gV, const long long* strides,
+                                               double* gA) {
+  return svd_backward_strided<double>(h, batch, m, n, dU, dS, dV, gU, gS, gV, strides, gA);
+}
+
+extern "C" int ddcsvd_svd_backward_f32_strided(ddcsvd_handle_t h, int batch, int m, int n, const float* dU,
+                                               const float* dS, const float* dV, const float* gU, const float* gS,
+                                               const float* gV, const long long* strides, float* gA) {
+  return svd_backward_strided<float>(h, batch, m, n, dU, dS, dV, gU, gS, gV, strides, gA);
 }

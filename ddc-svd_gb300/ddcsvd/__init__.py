@@ -403,17 +403,19 @@ def svd_backward_device(U, S, V, gU, gS, gV, handle: Handle | None = None):
     Bt, m, k = U.shape
     n = V.shape[1]
     dt = U.dtype
-    fn = load().ddcsvd_svd_backward_f64_device if dt == torch.float64 else load().ddcsvd_svd_backward_f32_device
-
-    def cm(x):  # (B, r, c) -> column-major per matrix
-        return None if x is None else x.transpose(1, 2).contiguous()
-
-    Uc, Vc = cm(U), cm(V)
-    gUc, gVc = cm(gU), cm(gV)
+    fn = load().ddcsvd_svd_backward_f64_strided if dt == torch.float64 else load().ddcsvd_svd_backward_f32_strided
+    # the matrices are read by their strides, whatever their layout (a lazily
+    # negated view is the one form whose memory does not hold its values)
+    U, V, gU, gV = (None if x is None else x.resolve_neg() for x in (U, V, gU, gV))
+    strides = (ctypes.c_longlong * 12)()
+    for q, x in enumerate((U, V, gU, gV)):
+        if x is not None:
+            sb, sr, sc = x.stride()
+            strides[3 * q:3 * q + 3] = (sr, sc, sb)
     Sc = S.contiguous()
     gSc = None if gS is None else gS.contiguous()
     gA = torch.empty((Bt, n, m), dtype=dt, device=U.device)
     ptr = lambda x: 0 if x is None else x.data_ptr()  # noqa: E731
-    check(fn(h.ptr, Bt, m, n, ptr(Uc), ptr(Sc), ptr(Vc), ptr(gUc), ptr(gSc), ptr(gVc), gA.data_ptr()),
-          "svd_backward")
+    check(fn(h.ptr, Bt, m, n, ptr(U), ptr(Sc), ptr(V), ptr(gU), ptr(gSc), ptr(gV), ctypes.addressof(strides),
+             gA.data_ptr()), "svd_backward")
     return gA.transpose(1, 2)

@@ -41,6 +41,8 @@ _SIGS = {
     "ddcsvd_svd_batched_f32_device": (c_int, [P, c_int, P, P, P, P, P, P, P, P, P, P]),
     "ddcsvd_svd_backward_f64_device": (c_int, [P, c_int, c_int, c_int, P, P, P, P, P, P, P]),
     "ddcsvd_svd_backward_f32_device": (c_int, [P, c_int, c_int, c_int, P, P, P, P, P, P, P]),
+    "ddcsvd_svd_backward_f64_strided": (c_int, [P, c_int, c_int, c_int, P, P, P, P, P, P, P, P]),
+    "ddcsvd_svd_backward_f32_strided": (c_int, [P, c_int, c_int, c_int, P, P, P, P, P, P, P, P]),
     "ddcsvd_svd_backward_f64_noalloc": (c_int, [P, c_int, c_int, c_int, P, P, P, P, P, P, P]),
     "ddcsvd_gemm_f32_device": (c_int, [P, c_int, c_int, c_int, c_int, P, c_int, P, c_int, P, c_int, c_float,
                                        c_float]),

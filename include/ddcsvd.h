@@ -200,6 +200,17 @@ int ddcsvd_svd_backward_f32_device(ddcsvd_handle_t handle, int batch, int m, int
                                    const float *dU, const float *dS, const float *dV,
                                    const float *gU, const float *gS, const float *gV, float *gA);
 
+/* The same on matrices of any layout: element (r, c) of problem b of dU, dV, gU
+ * and gV is at base + r*strides[3q] + c*strides[3q+1] + b*strides[3q+2] with
+ * q = 0, 1, 2, 3 in that order (host array of 12, in elements; entries of null
+ * matrices are not read).  dS, gS and gA as above. */
+int ddcsvd_svd_backward_f64_strided(ddcsvd_handle_t handle, int batch, int m, int n, const double *dU,
+                                    const double *dS, const double *dV, const double *gU, const double *gS,
+                                    const double *gV, const long long *strides, double *gA);
+int ddcsvd_svd_backward_f32_strided(ddcsvd_handle_t handle, int batch, int m, int n, const float *dU,
+                                    const float *dS, const float *dV, const float *gU, const float *gS,
+                                    const float *gV, const long long *strides, float *gA);
+
 /* No counterpart in the reference.  The FP64 adjoint above for callers that
  * must not allocate device memory when they call it -- code working inside
  * another framework's memory pool or a fixed, pre-planned memory budget, or a
