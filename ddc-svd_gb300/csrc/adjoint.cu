@@ -443,6 +443,129 @@ static int bgemm(ddcsvd_context* ctx, int batch, const BGemm<double>& g0, const 
   return DDCSVD_OK;
 }
 
+// ---------------------------------------------------------------- FP32, one CTA per problem
+// Small FP32 problems are bound by the launches and by each product's load
+// latency per slab, not by arithmetic (300 x (97 x 41): three products of ~21 us
+// for 5 us worth of FMAs), so a CTA keeps its whole problem in shared memory and
+// forms J, K, M, P and gA there: one round trip to memory in and one out, 71 -> 41
+// us of kernels with cold caches (bound by shared-memory reads), the call 111 ->
+// 78 us.  Rows of every matrix are an odd number of floats apart, so
+// walks along rows and along columns both spread over the banks.
+constexpr int kFusedThreads = 256;
+static size_t fused_floats(int m, int n) {
+  const size_t ld = (size_t)(n | 1);
+  return 2 * m * ld + 4 * n * ld + n;
+}
+
+// out(i, j) for i < MI, j < NJ in 4 x 4 register tiles: sum over q < K of a(i, q) b(q, j)
+template <typename FA, typename FB, typename FO>
+__device__ __forceinline__ void fused_product(int MI, int NJ, int K, int t0, int nt, FA a, FB b, FO out) {
+  const int TI = (MI + 3) >> 2, TJ = (NJ + 3) >> 2;
+  for (int t = t0; t < TI * TJ; t += nt) {
+    const int ti = t % TI, tj = t / TI;
+    int ri[4], cj[4];
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      ri[x] = min(ti + TI * x, MI - 1);
+      cj[x] = min(tj + TJ * x, NJ - 1);
+    }
+    float acc[4][4];
+#pragma unroll
+    for (int x = 0; x < 16; x++) acc[x >> 2][x & 3] = 0.f;
+#pragma unroll 4
+    for (int q = 0; q < K; q++) {
+      float u[4], v[4];
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        u[x] = a(ri[x], q);
+        v[x] = b(q, cj[x]);
+      }
+#pragma unroll
+      for (int x = 0; x < 16; x++) acc[x >> 2][x & 3] += u[x >> 2] * v[x & 3];
+    }
+#pragma unroll
+    for (int x = 0; x < 16; x++) {
+      const int i = ti + TI * (x >> 2), j = tj + TJ * (x & 3);
+      if (i < MI && j < NJ) out(i, j, acc[x >> 2][x & 3]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kFusedThreads) adjoint_fused_kernel(int m, int n, BMat<float> U, const float* S,
+                                                                      BMat<float> V, BMat<float> gU, const float* gS,
+                                                                      BMat<float> gV, float* gA) {
+  extern __shared__ __align__(16) float fsm[];
+  const int t = threadIdx.x, ld = n | 1;
+  const long long b = blockIdx.x;
+  float* sU = fsm;
+  float* sP = sU + m * ld;  // gU, then P
+  float* sV = sP + m * ld;
+  float* sW = sV + n * ld;  // gV
+  float* sJ = sW + n * ld;  // J, then M
+  float* sK = sJ + n * ld;
+  float* ss = sK + n * ld;
+  auto load = [&](float* dst, const BMat<float>& x, int rows) {
+    if (!x.p) return;
+    const float* p = x.p + b * x.b;
+    const bool rfast = x.r == 1 && x.c != 1;
+    for (int idx = t; idx < rows * n; idx += kFusedThreads) {
+      const int r = rfast ? idx % rows : idx / n, c = rfast ? idx / rows : idx % n;
+      dst[r * ld + c] = p[r * x.r + c * x.c];
+    }
+  };
+  load(sU, U, m);
+  load(sP, gU, m);
+  load(sV, V, n);
+  load(sW, gV, n);
+  for (int c = t; c < n; c += kFusedThreads) ss[c] = S[b * n + c];
+  __syncthreads();
+  // J = U^T gU on one half of the threads, K = V^T gV on the other
+  constexpr int h = kFusedThreads / 2;
+  if (t < h) {
+    if (gU.p)
+      fused_product(n, n, m, t, h, [&](int i, int q) { return sU[q * ld + i]; },
+                    [&](int q, int j) { return sP[q * ld + j]; }, [&](int i, int j, float v) { sJ[i * ld + j] = v; });
+  } else if (gV.p) {
+    fused_product(n, n, n, t - h, h, [&](int i, int q) { return sV[q * ld + i]; },
+                  [&](int q, int j) { return sW[q * ld + j]; }, [&](int i, int j, float v) { sK[i * ld + j] = v; });
+  }
+  __syncthreads();
+  for (int idx = t; idx < n * n; idx += kFusedThreads) {  // M in place of J, a pair at a time
+    const int i = idx / n, j = idx % n;
+    if (i > j) continue;
+    const float si = ss[i], sj = ss[j];
+    if (i == j) {
+      float v = gS ? gS[b * n + i] : 0.f;
+      if (gU.p) v -= sJ[i * ld + i] / sj;
+      sJ[i * ld + i] = v;
+      continue;
+    }
+    const float f = 1.f / ((sj - si) * (sj + si));
+    float vij = 0.f, vji = 0.f;
+    if (gU.p) {
+      const float x = sJ[i * ld + j], y = sJ[j * ld + i], fj = f * (x - y);
+      vij += fj * sj - x / sj;
+      vji += fj * si - y / si;
+    }
+    if (gV.p) {
+      const float fk = f * (sK[i * ld + j] - sK[j * ld + i]);
+      vij += si * fk;
+      vji += sj * fk;
+    }
+    sJ[i * ld + j] = vij;
+    sJ[j * ld + i] = vji;
+  }
+  __syncthreads();
+  fused_product(m, n, n, t, kFusedThreads, [&](int i, int q) { return sU[i * ld + q]; },
+                [&](int q, int j) { return sJ[q * ld + j]; },
+                [&](int i, int j, float v) { sP[i * ld + j] = gU.p ? v + sP[i * ld + j] / ss[j] : v; });
+  __syncthreads();
+  float* out = gA + b * m * n;
+  fused_product(m, n, n, t, kFusedThreads, [&](int i, int q) { return sP[i * ld + q]; },
+                [&](int q, int j) { return sV[j * ld + q]; },
+                [&](int i, int j, float v) { out[i + (size_t)j * m] = v; });
+}
+
 // The launches of one adjoint on intermediates J, Kv, Mm (k x k per problem)
 // and P (m x k per problem).  Launch grids carry the batch in gridDim.z /
 // gridDim.y (at most 65535, two products in one launch), so larger batches go
@@ -509,6 +632,22 @@ static int svd_backward(ddcsvd_context* h, int batch, int m, int n, BMat<T> U, c
   T* P = a.take<T>(mk);
   DDC_TRY(reset_status(h));
   DDC_TRY(adjoint_enqueue<T>(h, batch, m, n, U, S, V, gU, gS, gV, gA, J, Kv, Mm, P));
+  return check_status(h, "svd_backward");
+}
+// FP32 problems whose six matrices fit one CTA's shared memory: one launch
+static int svd_backward_f32(ddcsvd_context* h, int batch, int m, int n, BMat<float> U, const float* S, BMat<float> V,
+                            BMat<float> gU, const float* gS, BMat<float> gV, float* gA) {
+  if (!h || batch <= 0 || m <= 0 || n <= 0 || m < n || !U.p || !S || !V.p || !gA) return DDCSVD_ERR_ARG;
+  const size_t bytes = fused_floats(m, n) * sizeof(float);
+  if (bytes > h->smem_optin - 1024) return svd_backward<float>(h, batch, m, n, U, S, V, gU, gS, gV, gA);
+  std::lock_guard<std::mutex> g(h->mu);
+  DDC_CUDA_TRY(cudaSetDevice(h->device));
+  DDC_TRY(reset_status(h));
+  DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)adjoint_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)bytes));
+  adjoint_fused_kernel<<<batch, kFusedThreads, bytes, h->stream>>>(m, n, U, S, V, gU, gS, gV, gA);
+  count_launch();
+  DDC_CUDA_TRY(cudaGetLastError());
   return check_status(h, "svd_backward");
 }
 // column-major matrices of `rows` rows, one after another
@@ -650,27 +789,28 @@ extern "C" int ddcsvd_svd_backward_f64_device(ddcsvd_handle_t h, int batch, int 
 extern "C" int ddcsvd_svd_backward_f32_device(ddcsvd_handle_t h, int batch, int m, int n, const float* dU,
                                               const float* dS, const float* dV, const float* gU, const float* gS,
                                               const float* gV, float* gA) {
-  return svd_backward<float>(h, batch, m, n, colmajor(dU, m, n), dS, colmajor(dV, n, n), colmajor(gU, m, n), gS,
-                             colmajor(gV, n, n), gA);
+  return svd_backward_f32(h, batch, m, n, colmajor(dU, m, n), dS, colmajor(dV, n, n), colmajor(gU, m, n), gS,
+                          colmajor(gV, n, n), gA);
 }
 
 template <typename T>
-static int svd_backward_strided(ddcsvd_context* h, int batch, int m, int n, const T* U, const T* S, const T* V,
-                                const T* gU, const T* gS, const T* gV, const long long* strides, T* gA) {
-  if (!strides) return DDCSVD_ERR_ARG;
-  auto mat = [&](const T* p, int q) { return BMat<T>{p, strides[3 * q], strides[3 * q + 1], strides[3 * q + 2]}; };
-  return svd_backward<T>(h, batch, m, n, mat(U, 0), S, mat(V, 1), mat(gU, 2), gS, mat(gV, 3), gA);
+static BMat<T> strided(const T* p, const long long* st) {
+  return BMat<T>{p, st[0], st[1], st[2]};
 }
 
 extern "C" int ddcsvd_svd_backward_f64_strided(ddcsvd_handle_t h, int batch, int m, int n, const double* dU,
                                                const double* dS, const double* dV, const double* gU,
                                                const double* gS, const double* gV, const long long* strides,
                                                double* gA) {
-  return svd_backward_strided<double>(h, batch, m, n, dU, dS, dV, gU, gS, gV, strides, gA);
+  if (!strides) return DDCSVD_ERR_ARG;
+  return svd_backward<double>(h, batch, m, n, strided(dU, strides), dS, strided(dV, strides + 3),
+                              strided(gU, strides + 6), gS, strided(gV, strides + 9), gA);
 }
 
 extern "C" int ddcsvd_svd_backward_f32_strided(ddcsvd_handle_t h, int batch, int m, int n, const float* dU,
                                                const float* dS, const float* dV, const float* gU, const float* gS,
                                                const float* gV, const long long* strides, float* gA) {
-  return svd_backward_strided<float>(h, batch, m, n, dU, dS, dV, gU, gS, gV, strides, gA);
+  if (!strides) return DDCSVD_ERR_ARG;
+  return svd_backward_f32(h, batch, m, n, strided(dU, strides), dS, strided(dV, strides + 3),
+                          strided(gU, strides + 6), gS, strided(gV, strides + 9), gA);
 }
