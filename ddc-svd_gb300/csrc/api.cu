@@ -108,7 +108,7 @@ int ensure_pinned(ddcsvd_context* ctx, size_t bytes) {
 // Clears the error code and writes the handle's limits (kernel arguments, so
 // the host values may change right after the launch).
 __global__ void status_init_kernel(DevStatus* st, unsigned wait_us, unsigned extra) {
-  if (threadIdx.x == 0) *st = DevStatus{0, 0, wait_us, extra};
+  if (threadIdx.x == 0) *st = DevStatus{0, 0, wait_us, extra, 0, {0, 0, 0}};
 }
 
 int reset_status(ddcsvd_context* ctx) {
@@ -153,19 +153,30 @@ static int resolve_mode(int mode) {
 
 // ---------------------------------------------------------------- small kernels
 // W = A with zero rows m .. ldw-1; with `st` set, a non-finite entry also
-// records DDCSVD_ERR_NONFINITE (the input check rides on the copy's read).
-__global__ void copy_pad_kernel(int m, int n, const float* __restrict__ A, int lda, float* W, int ldw,
-                                DevStatus* st = nullptr) {
+// records DDCSVD_ERR_NONFINITE, and with `amax` set the largest |a| is taken (bit
+// pattern; NaN ignored): the input check and the range scan ride on the copy's
+// read.
+__global__ void __launch_bounds__(256) copy_pad_kernel(int m, int n, const float* __restrict__ A, int lda, float* W,
+                                                       int ldw, DevStatus* st, unsigned* amax) {
+  __shared__ float red[8];
   const int c = blockIdx.y;
+  float mx = 0.f;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < ldw; r += gridDim.x * blockDim.x) {
     const float v = (r < m) ? A[r + (size_t)c * lda] : 0.f;
     if (st && !isfinite(v)) set_error(st, DDCSVD_ERR_NONFINITE, (int)((r + (size_t)c * m) % 2147483647));
     W[r + (size_t)c * ldw] = v;
+    mx = fmaxf(mx, fabsf(v));
   }
-}
-
-__global__ void sigma_out_kernel(int n, const double* s, float* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = (float)s[i];
+  if (!amax) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+    const unsigned b = __float_as_uint(mx);
+    if (b > *reinterpret_cast<volatile unsigned*>(amax)) atomicMax(amax, b);  // most blocks only read
+  }
 }
 
 __global__ void zero_rows_kernel(int r0, int r1, int ncols, float* C, int ldc) {
@@ -290,6 +301,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
   const bool overlap = !plain && kind != GEMM_SIMT && !ctx->timing;
   BxPrepared bxl, bxr;
   BxDirect bxd;
+  const PrepBounds PB = prep_bounds({n});
   auto region_a = [&](Arena& a, Plan& pl) {
     pl.W = a.take<float>((size_t)ldw * n);
     pl.d = a.take<float>(n + 4);
@@ -298,7 +310,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     pl.taup = a.take<float>(n + 4);
     pl.sig_slot = a.take<double>(n + 4);
     pl.sig = a.take<double>(n + 4);
-    pl.blob = a.take<char>(prep_bounds({n}).blob_bytes);
+    pl.blob = a.take<char>(PB.blob_bytes);
     if (direct) {
       bx_direct_plan(m, n, a, &bxd);
     } else if (overlap) {
@@ -338,19 +350,20 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     ctx->kused = 0;
   }
   DDC_TRY(stage_event(ctx, 0));
-  copy_pad_kernel<<<dim3(ceil_div(ldw, 256), n), 256, 0, ctx->stream>>>(m, n, dA, lda, pl.W, ldw,
-                                                                      check_finite ? ctx->d_status : nullptr);
-  count_launch();
-  DDC_CUDA_TRY(cudaGetLastError());
   {
     Arena b = a;
     plan_bidiag(b, m, n, ldw, nctas, kind, &pl.bw);
+    if (!plain) DDC_CUDA_TRY(cudaMemsetAsync(pl.bw.amax, 0, sizeof(unsigned), ctx->stream));
+    copy_pad_kernel<<<dim3(std::min(ceil_div(ldw, 256), 4), n), 256, 0, ctx->stream>>>(
+        m, n, dA, lda, pl.W, ldw, check_finite ? ctx->d_status : nullptr, plain ? nullptr : pl.bw.amax);
+    count_launch();
+    DDC_CUDA_TRY(cudaGetLastError());
     Arena sc;
     sc.base = b.take<char>(gsc);
     sc.plan = false;
     sc.cap = gsc;
     if (plain) DDC_TRY(bidiag_plain(ctx, m, n, pl.W, ldw, pl.d, pl.e, pl.tauq, pl.taup, pl.bw));
-    else DDC_TRY(bidiag_blocked(ctx, m, n, pl.W, ldw, pl.d, pl.e, pl.tauq, pl.taup, pl.bw, kind, &sc));
+    else DDC_TRY(bidiag_blocked(ctx, m, n, pl.W, ldw, pl.d, pl.e, pl.tauq, pl.taup, pl.bw, kind, &sc, true));
   }
   DDC_TRY(stage_event(ctx, 1));
   SideWork side(ctx);
@@ -366,40 +379,51 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     side.back();
     DDC_TRY(rc);
   }
-  // ---- bidiagonal read-back: split at negligible superdiagonal entries and
-  //      build the D&C forest and vector layout on the host (2n floats down, one blob up)
-  const PrepBounds PB = prep_bounds({n});
+  // ---- hand-over to stages 2-4.  While stage 1 runs the host lays out the D&C
+  // forest and the vector stage for one unreduced block and sends them; the
+  // device turns (d, e) into the FP64 bidiagonal and looks for negligible
+  // superdiagonal entries.  Only the status word comes back: a stage-1 failure
+  // (non-finite input, a wait that ran out) ends the call here, and a bidiagonal
+  // that splits is laid out anew from its values.
   Prep P;
   {
     const size_t rb = (size_t)round_up(sizeof(float) * 2 * (n + 4), 256);
     const size_t ab = (size_t)round_up(sizeof(double) * 2 * (n + 4), 256);
     DDC_TRY(ensure_pinned(ctx, rb + ab + PB.blob_bytes));
-    float* hd = (float*)ctx->pinned;
-    float* he = hd + n + 4;
-    DDC_CUDA_TRY(cudaMemcpyAsync(hd, pl.d, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    if (n > 1)
-      DDC_CUDA_TRY(cudaMemcpyAsync(he, pl.e, sizeof(float) * (n - 1), cudaMemcpyDeviceToHost, ctx->stream));
-    // the status word rides along: a stage-1 failure (non-finite input, a
-    // wait that ran out) ends the call here instead of feeding stages 2-5
-    DDC_TRY(check_status(ctx, "bidiagonalisation"));
-    double* a64 = (double*)((char*)ctx->pinned + rb);
-    double* b64 = a64 + n + 4;
-    for (int i = 0; i < n; i++) {
-      a64[i] = hd[i];
-      b64[i] = (i < n - 1) ? (double)he[i] : 0.0;  // beta[N-1] := 0 (square case)
-    }
     char* hb = (char*)ctx->pinned + rb + ab;
-    DDC_TRY(prep_build(ctx, {n}, {GroupOut{dV, ldv, dU, ldu}}, a64, b64, FLT_EPSILON, false, hb, pl.blob, &P));
+    const std::vector<GroupOut> out{GroupOut{dV, ldv, dU, ldu}};
+    DDC_TRY(prep_layout(ctx, {n}, out, {0, n}, hb, pl.blob, &P));
+    DDC_TRY(prep_upload(P, hb, pl.blob, ctx->stream));
+    DDC_TRY(prep_values(ctx, P, 1, pl.d, pl.e, plain ? nullptr : pl.bw.amax, FLT_EPSILON));
+    P.L.amax = P.amax;
+    DDC_TRY(check_status(ctx, "bidiagonalisation"));
+    if (ctx->h_status->split) {
+      float* hd = (float*)ctx->pinned;
+      float* he = hd + n + 4;
+      DDC_CUDA_TRY(cudaMemcpyAsync(hd, pl.d, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
+      if (n > 1)
+        DDC_CUDA_TRY(cudaMemcpyAsync(he, pl.e, sizeof(float) * (n - 1), cudaMemcpyDeviceToHost, ctx->stream));
+      DDC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+      double* a64 = (double*)((char*)ctx->pinned + rb);
+      double* b64 = a64 + n + 4;
+      for (int i = 0; i < n; i++) {
+        a64[i] = hd[i];
+        b64[i] = (i < n - 1) ? (double)he[i] : 0.0;  // beta[N-1] := 0 (square case)
+      }
+      DDC_TRY(prep_build(ctx, {n}, out, a64, b64, FLT_EPSILON, false, hb, pl.blob, &P));
+      P.L.amax = nullptr;  // (the upload cleared it)
+    }
   }
   // ---- stage 2
   {
     Arena b = a;
-    DDC_TRY(dc_sigma(ctx, n, P.b1, P.b2, pl.sig_slot, &P.H, P.dints, b, false, false));
+    DDC_TRY(dc_sigma(ctx, n, P.b1, P.b2, pl.sig_slot, &P.H, P.dints, b, false, false, P.bar));
   }
   DDC_TRY(stage_event(ctx, 2));
   // ---- stages 3-4: X straight into V, Y into the top of U (ascending order)
   {
     Arena b = a;
+    P.L.sigma32 = dS;
     DDC_TRY(bd_vectors(ctx, n, P.store, P.b1, P.b2, pl.sig_slot, &P.L, pl.sig, b, false));
   }
   if (m > n && !direct) {
@@ -438,8 +462,6 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     Arena b = a;
     DDC_TRY(apply_left_reflectors(ctx, m, n, pl.W, ldw, pl.tauq, dU, ldu, n, kind, plain, b, false));
   }
-  sigma_out_kernel<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(n, pl.sig, dS);
-  count_launch();
   DDC_TRY(stage_event(ctx, 4));
   DDC_CUDA_TRY(cudaGetLastError());
   int rc = check_status(ctx, "svd");
@@ -493,8 +515,8 @@ static int svd_tall_qr(ddcsvd_context* ctx, int m, int n, const float* dA, int l
   do {
     if ((rc = reset_status(ctx))) break;
     ctx->kused = 0;
-    copy_pad_kernel<<<dim3(ceil_div(ldq, 256), n), 256, 0, ctx->stream>>>(m, n, dA, lda, Wq, ldq,
-                                                                          check_finite ? ctx->d_status : nullptr);
+    copy_pad_kernel<<<dim3(std::min(ceil_div(ldq, 256), 4), n), 256, 0, ctx->stream>>>(
+        m, n, dA, lda, Wq, ldq, check_finite ? ctx->d_status : nullptr, nullptr);
     count_launch();
     if ((rc = range_scale_matrix(ctx, m, n, Wq, ldq, amax))) break;
     if ((rc = qr_blocked(ctx, m, n, Wq, ldq, tau, qw, kind))) break;
@@ -822,12 +844,18 @@ static int bd_standalone(ddcsvd_context* h, int N, const double* dB1, const doub
   DDC_TRY(prep_build(h, {N}, {GroupOut{dX, N, dY, N}}, a64, b64, DBL_EPSILON, !square, (char*)h->pinned + ab, blob,
                      &P));
   DDC_TRY(reset_status(h));
+  if (!dX && P.L.sorted) {  // the only values wanted, and already ascending
+    Arena b = a;
+    DDC_TRY(dc_sigma(h, N, P.b1, P.b2, dSigmaOut, &P.H, P.dints, b, false, true, P.bar));
+    return check_status(h, "bdsdc");
+  }
   if (dX && P.single_block && dSigmaIn) {
     // one unreduced block: the caller's ascending sigma is already in slot order
     DDC_CUDA_TRY(cudaMemcpyAsync(sig_slot, dSigmaIn, sizeof(double) * N, cudaMemcpyDeviceToDevice, h->stream));
+    P.L.sorted = false;  // (ranked all the same, should the caller's not ascend)
   } else {
     Arena b = a;
-    DDC_TRY(dc_sigma(h, N, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true));
+    DDC_TRY(dc_sigma(h, N, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true, P.bar));
   }
   if (dX) {
     Arena c = a;
@@ -1012,13 +1040,16 @@ int svd_gpu_ex(int m, int n, double* A, double* sigma, double* U, double* V, int
   std::lock_guard<std::mutex> g(h->mu);
   const int k = std::min(m, n);
   const size_t na = (size_t)m * n, nu = (size_t)m * k, nv = (size_t)n * k;
-  // at least what the bidiagonal read-back inside the call asks for, so the
-  // buffer is never reallocated under pa / pu / pv
+  // behind what the pipeline itself stages at the front of the buffer (it writes
+  // there while the copy of pa may still be under way), and never reallocated
+  // under pa / pu / pv
   const size_t own = sizeof(float) * (na + k + nu + nv + 64);
-  const size_t readback = (size_t)round_up(sizeof(float) * 2 * (k + 4), 256) +
-                          (size_t)round_up(sizeof(double) * 2 * (k + 4), 256) + prep_bounds({k}).blob_bytes;
-  DDC_TRY(ensure_pinned(h, std::max(own, readback)));
-  float* pa = (float*)h->pinned;
+  const size_t front = (size_t)round_up(
+      (long long)((size_t)round_up(sizeof(float) * 2 * (k + 4), 256) +
+                  (size_t)round_up(sizeof(double) * 2 * (k + 4), 256) + prep_bounds({k}).blob_bytes),
+      256);
+  DDC_TRY(ensure_pinned(h, front + own));
+  float* pa = (float*)((char*)h->pinned + front);
   float* ps = pa + na;
   float* pu = ps + k;
   float* pv = pu + nu;

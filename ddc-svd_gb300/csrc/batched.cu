@@ -688,13 +688,10 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   // ---- bidiagonal read-back and preparation (one forest, one group per problem)
-  float* hd = (float*)(pin + tb);
-  float* he = hd + Ntot + 8;
-  DDC_CUDA_TRY(cudaMemcpyAsync(hd, d, sizeof(float) * Ntot, cudaMemcpyDeviceToHost, h->stream));
-  DDC_CUDA_TRY(cudaMemcpyAsync(he, e, sizeof(float) * Ntot, cudaMemcpyDeviceToHost, h->stream));
-  DDC_CUDA_TRY(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->stream));
-  // while stage 1 runs: the D&C forest and vector layout for one block per
-  // problem (a split inside a problem is rare; prep_build lays out anew then)
+  // While stage 1 runs: the D&C forest and vector layout for one block per
+  // problem, sent on the side stream.  The device then forms the FP64
+  // bidiagonals and looks for splits; a split inside a problem is rare, and
+  // everything is laid out anew from the values then.
   Prep P;
   {
     std::vector<int> starts0;
@@ -706,28 +703,36 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
     }
     starts0.push_back(off);
     DDC_TRY(prep_layout(h, gn, gout, starts0, pin + tb + rb + ab, blob, &P));
+    DDC_TRY(prep_upload(P, pin + tb + rb + ab, blob, h->side));
+    DDC_CUDA_TRY(cudaEventRecord(h->join_ev, h->side));
+    DDC_CUDA_TRY(cudaStreamWaitEvent(h->stream, h->join_ev, 0));
   }
-  DDC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  if (h->h_status->code != 0) {  // a stage-1 failure ends the call before stages 2-5
-    set_last_error("batched bidiagonalisation: device status %d (detail %d)", h->h_status->code,
-                   h->h_status->detail);
-    return h->h_status->code;
-  }
-  double* a64 = (double*)(pin + tb + rb);
-  double* b64 = a64 + Ntot + 8;
-  for (int b = 0; b < batch; b++) {
-    const long long o = tasks[b].offD;
-    const int nb = tasks[b].n;
-    for (int i = 0; i < nb; i++) {
-      a64[o + i] = hd[o + i];
-      b64[o + i] = (i < nb - 1) ? (double)he[o + i] : 0.0;
+  DDC_TRY(prep_values(h, P, batch, d, e, nullptr, FLT_EPSILON));
+  P.L.amax = P.amax;
+  DDC_TRY(check_status(h, "batched bidiagonalisation"));  // a stage-1 failure ends the call before stages 2-5
+  if (h->h_status->split) {
+    float* hd = (float*)(pin + tb);
+    float* he = hd + Ntot + 8;
+    DDC_CUDA_TRY(cudaMemcpyAsync(hd, d, sizeof(float) * Ntot, cudaMemcpyDeviceToHost, h->stream));
+    DDC_CUDA_TRY(cudaMemcpyAsync(he, e, sizeof(float) * Ntot, cudaMemcpyDeviceToHost, h->stream));
+    DDC_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    double* a64 = (double*)(pin + tb + rb);
+    double* b64 = a64 + Ntot + 8;
+    for (int b = 0; b < batch; b++) {
+      const long long o = tasks[b].offD;
+      const int nb = tasks[b].n;
+      for (int i = 0; i < nb; i++) {
+        a64[o + i] = hd[o + i];
+        b64[o + i] = (i < nb - 1) ? (double)he[o + i] : 0.0;
+      }
     }
+    DDC_TRY(prep_build(h, gn, gout, a64, b64, FLT_EPSILON, false, pin + tb + rb + ab, blob, &P));
+    P.L.amax = nullptr;  // (the upload cleared it)
   }
-  DDC_TRY(prep_build(h, gn, gout, a64, b64, FLT_EPSILON, false, pin + tb + rb + ab, blob, &P));
   // ---- stages 2-4
   {
     Arena b = a;
-    DDC_TRY(dc_sigma(h, Ntot, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true));
+    DDC_TRY(dc_sigma(h, Ntot, P.b1, P.b2, sig_slot, &P.H, P.dints, b, false, true, P.bar));
   }
   {
     Arena c = a;
@@ -745,7 +750,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
       dt, dord, batch, counter + 1, W, tq, tp, dU, dV, smem_floats);
   count_launch();
   ktimer_end(h);
-  batch_sigma_out_kernel<<<std::min(batch, 1024), 128, 0, h->stream>>>(dt, batch, sig, dSigma);
+  batch_sigma_out_kernel<<<std::min(batch, 1024), 128, 0, h->stream>>>(dt, batch, P.L.sorted ? sig_slot : sig, dSigma);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   const int rc = check_status(h, "svd_batched");

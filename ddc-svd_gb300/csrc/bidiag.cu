@@ -1239,14 +1239,17 @@ static int launch_coop(const void* fn, int P, int threads, size_t smem, void* ar
 }
 
 int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d, float* e,
-                   float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch) {
+                   float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch, bool scanned) {
   if (m < n || n <= 0) return DDCSVD_ERR_ARG;
   const int P = w.P;
   const int sg = std::min(n, 4 * ctx->num_sms);
-  DDC_CUDA_TRY(cudaMemsetAsync(w.amax, 0, sizeof(unsigned), ctx->stream));
-  range_scan_kernel<<<sg, 256, 0, ctx->stream>>>(m, n, W, ldw, w.amax);
+  if (!scanned) {
+    DDC_CUDA_TRY(cudaMemsetAsync(w.amax, 0, sizeof(unsigned), ctx->stream));
+    range_scan_kernel<<<sg, 256, 0, ctx->stream>>>(m, n, W, ldw, w.amax);
+    count_launch();
+  }
   range_apply_kernel<<<sg, 256, 0, ctx->stream>>>(m, n, W, ldw, w.amax);
-  count_launch(2);
+  count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   for (int k0 = 0; k0 < n; k0 += kPanel) {
     // the remaining columns on one thread-block cluster once they fit
@@ -1331,8 +1334,10 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
       ktimer_end(ctx);
     }
   }
-  range_unscale_kernel<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(n, d, e, w.amax);
-  count_launch();
+  if (!scanned) {
+    range_unscale_kernel<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(n, d, e, w.amax);
+    count_launch();
+  }
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;
 }

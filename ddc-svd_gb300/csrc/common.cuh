@@ -34,6 +34,8 @@ struct __align__(16) DevStatus {
   unsigned extra;    // fault injection: arrivals that the first grid barrier of a cooperative
                      // launch waits for beyond its own CTAs (0 in normal use; > 0 makes that
                      // barrier's waits run out, which tests the timeout path)
+  unsigned split;    // set when a bidiagonal splits (prep.cu): its layout has to be made from its values
+  unsigned pad[3];
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {

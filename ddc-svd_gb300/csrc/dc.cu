@@ -1256,7 +1256,7 @@ size_t dc_max_ints(int N) { return 9 * (size_t)(2 * N + 8) + 2 * 64 + 16 + 2 * (
 
 
 int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, double* sigma,
-             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits) {
+             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits, GridBarrier* zeroed) {
   if (N <= 0) return DDCSVD_ERR_ARG;
   const int maxnodes = 2 * N + 8;
   int* scratch_ints = a.take<int>((size_t)N + maxnodes);
@@ -1292,6 +1292,8 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
   p.tau = q; q += N; p.dor = q; q += N; p.zh = q; q += N; p.rS = q; q += N; p.rF = q; q += N; p.rL = q; q += N;
   p.zz = q; q += maxnodes; p.phi = q; q += maxnodes; p.psi = q; q += maxnodes;
   p.dqf = reinterpret_cast<float2*>(flt); p.zqf = flt + 2 * (size_t)N;
+  if (zeroed) bar = zeroed;
+  else DDC_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), ctx->stream));
   p.bar = bar;
   p.st = ctx->d_status;
   // a forest of many small trees: whole trees per CTA, no grid barriers
@@ -1311,7 +1313,6 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
     int occ = 0;
     DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dc_tree_kernel, kDcTreeThreads, 0));
     const int grid = std::max(1, std::min(nt, ctx->num_sms * std::max(occ, 1)));
-    DDC_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), ctx->stream));
     ktimer_begin(ctx, KC_DC);
     dc_tree_kernel<<<grid, kDcTreeThreads, 0, ctx->stream>>>(p, tr);
     ktimer_end(ctx);
@@ -1328,7 +1329,6 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
   }
   const int P = std::min(ctx->num_sms, std::max(1, ceil_div(N, 4)));
   p.P = P;
-  DDC_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), ctx->stream));
   void* argv[] = {&p};
   ktimer_begin(ctx, KC_DC);
   DDC_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(P), dim3(kDcThreads), argv, 0,

@@ -170,7 +170,8 @@ constexpr int kFusedRows = 8192; // fused panel pass: rows (from the first stage
 constexpr int kBidiagThreads = 512;
 void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWork* w);
 int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d, float* e,
-                   float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch);
+                   float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch, bool scanned = false);
+// (scanned: w.amax already holds the largest |a|, and the caller scales d and e back)
 int bidiag_plain(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d, float* e,
                  float* tauq, float* taup, BidiagWork& w);
 int bidiag_coop_ctas(ddcsvd_context* ctx, int m, int n);
@@ -199,7 +200,7 @@ void dc_build_host(int N, const std::vector<int>& block_starts, DcHost& H, int t
 size_t dc_max_ints(int N);
 // keep_bits: every FP64 rounding of the plain formulas kept (dc.cu says why)
 int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, double* sigma,
-             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits);
+             const DcHost* H, const int* dints, Arena& a, bool plan_only, bool keep_bits, GridBarrier* zeroed = nullptr);
 
 // Splits the N x N bidiagonal (host copies a[N], b[N]) at |b_i| <= 4 eps max|B|:
 // zeroes those b_i (and b[N-1]), fills block_starts (ascending, ends with N)

@@ -11,6 +11,7 @@
 
 #include <vector>
 
+#include "fp64.cuh"
 #include "internal.hpp"
 #include "prep.hpp"
 
@@ -37,7 +38,7 @@ PrepBounds prep_bounds(const std::vector<int>& gn) {
   o = align256(o + sizeof(void*) * 2 * G);    // g_X, g_Y
   o = align256(o + sizeof(int4) * tiles);     // tiles
   o = align256(o + sizeof(int) * dc_max_ints((int)N));
-  B.blob_bytes = o + 256;
+  B.blob_bytes = o + 512;
   B.store = store;
   B.N = (int)N;
   return B;
@@ -109,7 +110,13 @@ int prep_layout(ddcsvd_context* ctx, const std::vector<int>& gn, const std::vect
   const size_t o_gp = put(gp.data(), sizeof(float*) * 2 * G);
   const size_t o_tiles = put(tiles.data(), sizeof(int4) * tiles.size());
   const size_t o_ints = put(P->H.ints.data(), sizeof(int) * P->H.ints.size());
+  const size_t o_zero = o;  // stage 2's barrier and the largest entry
+  memset(hblob + o, 0, 256);
+  o = align256(o + 256);
   P->used = o;
+  P->bar = reinterpret_cast<GridBarrier*>(dblob + o_zero);
+  P->amax = reinterpret_cast<unsigned long long*>(dblob + o_zero + 128);
+  P->o_rest = o_base;
   P->o_b1 = o_b1;
   P->o_b2 = o_b2;
   P->starts = starts;
@@ -131,8 +138,57 @@ int prep_layout(ddcsvd_context* ctx, const std::vector<int>& gn, const std::vect
   L.g_Y = L.g_X + G;
   L.tiles = reinterpret_cast<const int4*>(dblob + o_tiles);
   L.ntiles = (int)tiles.size();
+  int ngroups = 0;
+  for (int n : gn) ngroups += n > 0;
+  L.sorted = (int)starts.size() - 1 == ngroups;
+  L.amax = nullptr;
   P->single_block = (starts.size() == 2);
   P->laid_out = true;
+  return DDCSVD_OK;
+}
+
+int prep_upload(const Prep& P, const char* hblob, char* dblob, cudaStream_t stream) {
+  DDC_CUDA_TRY(cudaMemcpyAsync(dblob + P.o_rest, hblob + P.o_rest, P.used - P.o_rest, cudaMemcpyHostToDevice, stream));
+  return DDCSVD_OK;
+}
+
+// One CTA per group.
+__global__ void prep_values_kernel(VecLayout L, float* d, float* e, double* b1, double* b2, const unsigned* amax32,
+                                   double eps4, unsigned long long* amax, DevStatus* st) {
+  __shared__ long long red[32];
+  const int g = blockIdx.x, lo = L.g_lo[g], n = L.g_n[g], t = threadIdx.x;
+  const float s = amax32 ? range_scale(*amax32) : 1.f;
+  const float inv = 1.f / s;
+  long long mx = 0;
+  for (int i = t; i < n; i += blockDim.x) {
+    float di = d[lo + i], ei = i < n - 1 ? e[lo + i] : 0.f;
+    if (s != 1.f) {
+      d[lo + i] = di *= inv;
+      if (i < n - 1) e[lo + i] = ei *= inv;
+    }
+    b1[lo + i] = di;
+    b2[lo + i] = ei;
+    mx = max(mx, max(max_bits(di), max_bits(ei)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((t & 31) == 0) red[t >> 5] = mx;
+  __syncthreads();
+  mx = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); w++) mx = max(mx, red[w]);
+  const long long tol = bits(eps4 * __longlong_as_double(mx));
+  bool split = false;
+  for (int i = t; i < n - 1; i += blockDim.x) split = split || abs_bits(b2[lo + i]) <= tol;
+  if (__syncthreads_or(split) && t == 0) st->split = 1;
+  if (t == 0 && mx > 0) atomicMax(amax, (unsigned long long)mx);
+}
+
+int prep_values(ddcsvd_context* ctx, const Prep& P, int groups, float* d, float* e, const unsigned* amax32,
+                double eps) {
+  prep_values_kernel<<<groups, groups == 1 ? 1024 : 128, 0, ctx->stream>>>(
+      P.L, d, e, const_cast<double*>(P.b1), const_cast<double*>(P.b2), amax32, 4.0 * eps, P.amax, ctx->d_status);
+  count_launch();
+  DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;
 }
 

@@ -26,6 +26,9 @@ struct VecLayout {
   const int* g_ldy;
   const int4* tiles;  // finalize tiles: (block lo, nb, k0, i0)
   int ntiles;
+  bool sorted;                      // every group is one block: slots are in ascending order already
+  const unsigned long long* amax;   // largest |entry| of the bidiagonal (bits of the double), or null
+  float* sigma32 = nullptr;         // FP32 copy of the sorted values (one group), or null
 };
 
 struct GroupOut {
@@ -50,6 +53,9 @@ struct Prep {
   long long store;
   size_t used;
   size_t o_b1 = 0, o_b2 = 0;  // blob offsets of the bidiagonal
+  size_t o_rest = 0;          // and of everything behind it
+  GridBarrier* bar = nullptr; // zeroed with the blob, for stage 2's launch
+  unsigned long long* amax = nullptr;
   int N;
   bool single_block;
   bool laid_out = false;      // prep_layout ran for `starts`
@@ -71,5 +77,15 @@ int prep_build(ddcsvd_context* ctx, const std::vector<int>& group_sizes, const s
 // GPU; prep_build then reuses it when the splits agree (else lays out anew).
 int prep_layout(ddcsvd_context* ctx, const std::vector<int>& group_sizes, const std::vector<GroupOut>& out,
                 const std::vector<int>& starts, char* hblob, char* dblob, Prep* P);
+
+// Sends what prep_layout wrote.
+int prep_upload(const Prep& P, const char* hblob, char* dblob, cudaStream_t stream);
+
+// The bidiagonal's values on the device, for a layout of one block per group:
+// FP64 copies of d and e (scaled back by the range scale behind `amax32`, if
+// given; e's last entry of a group reads as zero) into b1 and b2, their largest
+// magnitude, and the status word's split flag when a superdiagonal entry is
+// negligible in its group (4 eps max|entry|, as split_bidiagonal).
+int prep_values(ddcsvd_context* ctx, const Prep& P, int groups, float* d, float* e, const unsigned* amax32, double eps);
 
 }  // namespace ddcsvd

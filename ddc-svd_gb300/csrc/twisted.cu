@@ -67,7 +67,7 @@ struct TwParams {
   double *Lp, *Um, *S, *Pp;  // compact block layout
   double* Z;
   double *xinv, *yinv;  // per vector
-  int* rank;            // position of each vector within its group (ascending sigma)
+  int* rank;            // position of each vector within its group (ascending sigma); null: its slot's
   const double *a, *b;
 };
 
@@ -624,6 +624,10 @@ __global__ void tw_finalize_kernel(TwParams p) {
   const int lo = T.x, nb = T.y, k0 = lo + T.z, i0 = lo + T.w, hi = lo + nb;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   const long long base = p.L.base[lo];
+  if (p.L.sigma32 && T.w == 0 && ty == 0 && k0 + tx < hi) {
+    const int k = k0 + tx;
+    p.L.sigma32[p.rank ? p.rank[k] : k - p.L.g_lo[p.L.grp[k]]] = (float)p.sigma[k];
+  }
   for (int rr = ty; rr < 33; rr += 8) {
     const int i = i0 + rr, k = k0 + tx;
     tile[rr][tx] = (i < hi && k < hi) ? p.Z[base + (long long)(i - lo) * nb + (k - lo)] : 0.0;
@@ -634,7 +638,7 @@ __global__ void tw_finalize_kernel(TwParams p) {
     if (k >= hi || i >= hi) continue;
     const int g = p.L.grp[k];
     const int g0 = p.L.g_lo[g];
-    const int col = p.rank[k];
+    const int col = p.rank ? p.rank[k] : k - g0;
     const double xi = tile[tx][kk], xn = tile[tx + 1][kk];
     p.L.g_X[g][(i - g0) + (size_t)col * p.L.g_ldx[g]] = (float)(xi * p.xinv[k]);
     const double y = p.a[i] * xi + ((i + 1 < hi) ? p.b[i] * xn : 0.0);
@@ -708,16 +712,19 @@ int bd_vectors(ddcsvd_context* ctx, int N, long long store, const double* a, con
   p.yinv = small + 5 * (size_t)N;
   p.sigma = sigma;
   p.L = *L;
-  p.rank = rank;
+  p.rank = L->sorted ? nullptr : rank;
   p.a = a;
   p.b = b;
   p.Lp = big; p.Um = big + store; p.S = big + 2 * store; p.Pp = big + 3 * store; p.Z = big + 4 * store;
   ktimer_begin(ctx, KC_VECTORS);
   const int sg = std::min(ceil_div(N, 256), 4 * ctx->num_sms);
-  DDC_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long), ctx->stream));
-  tw_absmax_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, amax);
-  tw_setup_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, amax, dd, ll, dl, dll);
-  count_launch(2);
+  if (!L->amax) {
+    DDC_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long), ctx->stream));
+    tw_absmax_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, amax);
+    count_launch();
+  }
+  tw_setup_kernel<<<sg, 256, 0, ctx->stream>>>(N, a, b, L->amax ? L->amax : amax, dd, ll, dl, dll);
+  count_launch();
   if (store / N >= 256)  // mean block size, weighted by its vectors
     twisted_kernel<16><<<ceil_div(N, 32), 32 * kTwWarps, 0, ctx->stream>>>(p);
   else
@@ -725,11 +732,13 @@ int bd_vectors(ddcsvd_context* ctx, int N, long long store, const double* a, con
   count_launch();
   tw_cluster_kernel<<<std::min(ceil_div(N, kClThreads), 2 * ctx->num_sms), kClThreads, 0, ctx->stream>>>(p);
   count_launch();
-  DDC_TRY(rank_values(ctx, N, sigma, p.L, rank, sigma_sorted));
+  if (!L->sorted) DDC_TRY(rank_values(ctx, N, sigma, p.L, rank, sigma_sorted));
   tw_finalize_kernel<<<L->ntiles, dim3(32, 8), 0, ctx->stream>>>(p);
   count_launch();
-  tw_zero_outside_kernel<<<std::min(N, 16 * ctx->num_sms), 128, 0, ctx->stream>>>(N, p);
-  count_launch();
+  if (!L->sorted) {  // (one block per group leaves no row outside)
+    tw_zero_outside_kernel<<<std::min(N, 16 * ctx->num_sms), 128, 0, ctx->stream>>>(N, p);
+    count_launch();
+  }
   ktimer_end(ctx);
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;
