@@ -42,6 +42,7 @@ constexpr int kDcThreads = 512;
 
 struct DcParams {
   int N, nnodes, maxdepth, P;
+  int terms;  // terms per lane that the depths' lane groups were sized for
   int maxit;  // FP64 iterations per secular root (the handle's limit, 80 by default)
   const int* nd_r0;
   const int* nd_nn;
@@ -407,42 +408,67 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
 // The per-root phases run one group of G lanes (G = 1, 2, ..., 32, chosen per
 // depth from its largest node) per root: small nodes of a batch forest would
 // otherwise leave most of a warp idle and pay five shuffle rounds per sum.
+// kG fixes the group's size at compile time: a whole warp (32) reduces in five
+// rounds with a constant mask, several sums to a round.  With the size and mask
+// read at run time and one loop per sum, the four sums of one FP32 evaluation
+// took most of its 2900 cycles (48 to 128 poles).  kG = 0: any size up to 16.
+template <int kG>
 struct LaneGroup {
   int G;          // lanes per group
   int lg;         // lane within the group
   unsigned mask;  // lanes of this group within the warp
+  __device__ __forceinline__ int size() const { return kG ? kG : G; }
 };
-__device__ __forceinline__ LaneGroup make_group(int G, int lane) {
-  LaneGroup g;
-  g.G = G;
-  g.lg = lane & (G - 1);
-  g.mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
+template <int kG>
+__device__ __forceinline__ LaneGroup<kG> make_group(int G, int lane) {
+  LaneGroup<kG> g;
+  g.G = kG ? kG : G;
+  g.lg = lane & (g.size() - 1);
+  g.mask = (kG == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
   return g;
 }
-template <typename T>
-__device__ __forceinline__ T gsum(T v, const LaneGroup& g) {
-  for (int o = g.G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(g.mask, v, o);
-  return v;
+// every v becomes its sum over the group (the same order of additions for each kG)
+template <int kG, typename... T>
+__device__ __forceinline__ void gsum(const LaneGroup<kG>& g, T&... v) {
+  if constexpr (kG == 32) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ((v += __shfl_xor_sync(0xffffffffu, v, o)), ...);
+  } else {
+    for (int o = g.G >> 1; o > 0; o >>= 1) ((v += __shfl_xor_sync(g.mask, v, o)), ...);
+  }
 }
-template <typename T>
-__device__ __forceinline__ T gprod(T v, const LaneGroup& g) {
-  for (int o = g.G >> 1; o > 0; o >>= 1) v *= __shfl_xor_sync(g.mask, v, o);
-  return v;
+// the product of v and the sum of e over the group
+template <int kG>
+__device__ __forceinline__ void gprod(const LaneGroup<kG>& g, double& v, int& e) {
+  if constexpr (kG == 32) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v *= __shfl_xor_sync(0xffffffffu, v, o);
+      e += __shfl_xor_sync(0xffffffffu, e, o);
+    }
+  } else {
+    for (int o = g.G >> 1; o > 0; o >>= 1) {
+      v *= __shfl_xor_sync(g.mask, v, o);
+      e += __shfl_xor_sync(g.mask, e, o);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- secular roots
+template <int kG>
 __device__ __forceinline__ void sec_eval(int q, const double* d, const double* z, double dorg,
-                                         double tau, int split, const LaneGroup& g, double& f, double& psi,
+                                         double tau, int split, const LaneGroup<kG>& g, double& f, double& psi,
                                          double& dpsi, double& phi, double& dphi) {
   double ps = 0.0, dps = 0.0, ph = 0.0, dph = 0.0;
-  for (int j = g.lg; j < q; j += g.G) {
+  for (int j = g.lg; j < q; j += g.size()) {
     const double dj = d[j];
     const double del = (dj - dorg) * (dj + dorg) - tau;
     const double tt = quot_rn(z[j], del);
     if (j <= split) { ps += z[j] * tt; dps += tt * tt; }
     else { ph += z[j] * tt; dph += tt * tt; }
   }
-  psi = gsum(ps, g); dpsi = gsum(dps, g); phi = gsum(ph, g); dphi = gsum(dph, g);
+  gsum(g, ps, dps, ph, dph);
+  psi = ps; dpsi = dps; phi = ph; dphi = dph;
   f = 1.0 + psi + phi;
 }
 
@@ -460,12 +486,12 @@ __device__ __forceinline__ float pair_diff(float2 a, float2 b) { return (a.x - b
 
 // FP32 twin of sec_eval on the float copies of d and z (kBits: the heads and
 // the division operator only).
-template <bool kBits>
+template <bool kBits, int kG>
 __device__ __forceinline__ void sec_eval32(int q, const float2* d, const float* z, float2 dorg, float tau, int split,
-                                           const LaneGroup& g, float& f, float& psi, float& dpsi, float& phi,
+                                           const LaneGroup<kG>& g, float& f, float& psi, float& dpsi, float& phi,
                                            float& dphi) {
   float ps = 0.f, dps = 0.f, ph = 0.f, dph = 0.f;
-  for (int j = g.lg; j < q; j += g.G) {
+  for (int j = g.lg; j < q; j += g.size()) {
     const float2 dj = d[j];
     const float zj = z[j];
     const float del = (kBits ? dj.x - dorg.x : pair_diff(dj, dorg)) * (dj.x + dorg.x) - tau;
@@ -473,19 +499,21 @@ __device__ __forceinline__ void sec_eval32(int q, const float2* d, const float* 
     if (j <= split) { ps += zj * tt; dps += tt * tt; }
     else { ph += zj * tt; dph += tt * tt; }
   }
-  psi = gsum(ps, g); dpsi = gsum(dps, g); phi = gsum(ph, g); dphi = gsum(dph, g);
+  gsum(g, ps, dps, ph, dph);
+  psi = ps; dpsi = dps; phi = ph; dphi = dph;
   f = 1.f + psi + phi;
 }
 
 // One FP64 evaluation for the third-order step: f, f' = sum (z / del)^2, and
 // in FP32 the second-derivative sum g2 = sum (z / del)^2 (tau / del), which
 // only forms the correction term.  Nine FP64 instructions per pole.
+template <int kG>
 __device__ __forceinline__ void sec_eval_newton(int q, const double* d, const double* z, double dorg, double tau,
-                                                const LaneGroup& g, double& f, double& fp, float& g2) {
+                                                const LaneGroup<kG>& g, double& f, double& fp, float& g2) {
   const float t32 = (float)tau;
   double s = 0.0, sp = 0.0;
   float sg = 0.f;
-  for (int j = g.lg; j < q; j += g.G) {
+  for (int j = g.lg; j < q; j += g.size()) {
     const double dj = d[j], zj = z[j];
     const double del = fma(dj - dorg, dj + dorg, -tau);
     const double r = rcp_approx(del);
@@ -498,18 +526,32 @@ __device__ __forceinline__ void sec_eval_newton(int q, const double* d, const do
     const float tf = (float)tt;
     sg += tf * tf * ((float)r * t32);
   }
-  f = 1.0 + gsum(s, g);
-  fp = gsum(sp, g);
-  g2 = gsum(sg, g);
+  gsum(g, s, sp, sg);
+  f = 1.0 + s;
+  fp = sp;
+  g2 = sg;
 }
 
 // One safeguarded step of the root iteration (two-pole rational model for an
 // interior root, one pole for the last root), shared by the FP32 and FP64
 // phases.  Returns true when converged.
-__device__ __forceinline__ float step_quot(float a, float x) { return a / x; }
+// (without kBits the FP32 steps use approximate quotients and roots: the test of
+// f decides when to stop, so a step need not be rounded correctly)
+__device__ __forceinline__ float sqrt32(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+template <bool kBits>
+__device__ __forceinline__ float step_quot(float a, float x) { return kBits ? a / x : a * rcp32(x); }
+template <bool kBits>
 __device__ __forceinline__ double step_quot(double a, double x) { return quot_rn(a, x); }
+template <bool kBits>
+__device__ __forceinline__ float step_sqrt(float x) { return kBits ? sqrtf(x) : sqrt32(x); }
+template <bool kBits>
+__device__ __forceinline__ double step_sqrt(double x) { return sqrt(x); }
 
-template <typename T>
+template <bool kBits, typename T>
 __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T dphi, T da0, T db0, T eps,
                                          T& lo, T& hi, T& tau) {
   const T err = last ? T(8) * (T(1) + fabs(psi)) + fabs(tau) * dpsi
@@ -521,18 +563,18 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
   if (last) {
     const T da = -tau;
     const T s1 = da * da * dpsi;
-    const T c = f - step_quot(s1, da);
-    tn = (c != T(0)) ? tau + da + step_quot(s1, c) : T(0.5) * (lo + hi);
+    const T c = f - step_quot<kBits>(s1, da);
+    tn = (c != T(0)) ? tau + da + step_quot<kBits>(s1, c) : T(0.5) * (lo + hi);
   } else {
     const T da = da0 - tau, db = db0 - tau;
     const T s1 = da * da * dpsi, s2 = db * db * dphi;
-    const T c = f - step_quot(s1, da) - step_quot(s2, db);
+    const T c = f - step_quot<kBits>(s1, da) - step_quot<kBits>(s2, db);
     const T aq = c, bq = c * (da + db) + s1 + s2, cq = da * db * f;
-    const T disc = sqrt(fabs(bq * bq - T(4) * aq * cq));
+    const T disc = step_sqrt<kBits>(fabs(bq * bq - T(4) * aq * cq));
     T eta;
-    if (aq == T(0)) eta = step_quot(cq, bq);
-    else if (bq <= T(0)) eta = step_quot(bq - disc, T(2) * aq);
-    else eta = step_quot(T(2) * cq, bq + disc);
+    if (aq == T(0)) eta = step_quot<kBits>(cq, bq);
+    else if (bq <= T(0)) eta = step_quot<kBits>(bq - disc, T(2) * aq);
+    else eta = step_quot<kBits>(T(2) * cq, bq + disc);
     tn = tau + eta;
   }
   if (!(tn > lo && tn < hi)) tn = T(0.5) * (lo + hi);
@@ -552,11 +594,12 @@ __device__ unsigned g_dc_iters[64 * 84];  // [depth][FP64 iterations 0..80, 81: 
 // q eps32 of the total.  A term whose del_j may change sign, or lies near the
 // FP32 subnormal range (where the copies lose relative precision), makes the
 // bound infinite.
+template <int kG>
 __device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z, float2 dorg, float tau,
-                                          const LaneGroup& g, float& f, float& err) {
+                                          const LaneGroup<kG>& g, float& f, float& err) {
   constexpr float e32 = FLT_EPSILON;
   float s = 0.f, sa = 0.f, ea = 0.f;
-  for (int j = g.lg; j < q; j += g.G) {
+  for (int j = g.lg; j < q; j += g.size()) {
     const float2 dj = d[j];
     const float ad = fabsf(dj.x) + fabsf(dorg.x);
     const float dif = pair_diff(dj, dorg);
@@ -570,9 +613,7 @@ __device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z
     ea += (ed < 0.5f * adel && adel >= 0x1p-100f && adel <= 0x1p100f) ? at * (2.5f * ed * fabsf(ir) + 6.f * e32)
                                                                      : INFINITY;
   }
-  s = gsum(s, g);
-  sa = gsum(sa, g);
-  ea = gsum(ea, g);
+  gsum(g, s, sa, ea);
   f = 1.f + s;
   err = ea + (float)(q + 2) * e32 * (1.f + sa);
 }
@@ -588,14 +629,15 @@ __device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z
 // safeguarded FP64 iteration from there.  The corrected step counts as two
 // iterations against the caller's cap.
 // kBits iterates both phases with the two-pole model alone.
-template <bool kBits>
+template <bool kBits, int kG>
 __device__ bool sec_root(int q, const double* d, const double* z, const float2* df, const float* zf, double zz,
-                         int i, const LaneGroup& g, int maxit, int* origin, double* tau_out, int* iters = nullptr) {
+                         int i, const LaneGroup<kG>& g, int maxit, int* origin, double* tau_out, int* iters = nullptr) {
   double f, psi, dpsi, phi, dphi;
   const bool last = (i == q - 1);
   const int split = last ? q - 1 : i;
   int o;
-  float dd32 = 0.f;
+  float dd32 = 0.f, f32 = 0.f;
+  bool sure = false;
   double dd = 0.0;
   if (!last) {
     // origin = nearer pole, from the sign of f at the midpoint: from the float
@@ -604,9 +646,9 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
     // batch forest, and the root then lies outside the bracket)
     const float2 a = df[i], b = df[i + 1];
     dd32 = pair_diff(b, a) * (b.x + a.x);
-    float f32, e32;
+    float e32;
     sec_mid32(q, df, zf, a, 0.5f * dd32, g, f32, e32);
-    const bool sure = fabsf(f32) > 2.f * e32 && fabsf(f32) < INFINITY;
+    sure = fabsf(f32) > 2.f * e32 && fabsf(f32) < INFINITY;
     if (kBits || !sure) dd = (d[i + 1] - d[i]) * (d[i + 1] + d[i]);
     if (sure) {
       o = (f32 >= 0.f) ? i : i + 1;
@@ -636,13 +678,38 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
     t32 = last ? 0.5f * hi32 : left ? hi32 : lo32;
     da32 = (last || left) ? 0.f : -dd32;
     db32 = (last || !left) ? 0.f : dd32;
+    // Start from the root of c + (the two poles next to the interval), c what the
+    // other poles and 1 add up to where f is known already (the midpoint; half
+    // the bracket for the last root).  A root that a small z leaves at 1e-20 of
+    // the gap from its pole starts there; from the midpoint the bracket was
+    // halved up to 40 times, and the warps with such a root held up the barrier
+    // by three times the common root's time.
+    if (last) {
+      float e32;
+      const int far = max(i - 1, 0);
+      const float gap = (q > 1) ? pair_diff(od, df[far]) * (od.x + df[far].x) : 1.f;
+      const float wn = zf[i] * zf[i], wf = (q > 1) ? zf[far] * zf[far] : 0.f;
+      sec_mid32(q, df, zf, od, t32, g, f32, e32);
+      const float c = f32 + wf * rcp32(gap + t32) + wn * rcp32(t32);
+      const float b = c * gap - wf - wn, r = sqrt32(b * b + 4.f * c * wn * gap);
+      const float t = (b > 0.f) ? 2.f * wn * gap * rcp32(b + r) : (r - b) * rcp32(2.f * c);
+      if (c > 0.f && t > lo32 && t < hi32) t32 = t;
+    } else if (sure) {
+      const float zi = zf[i] * zf[i], zj = zf[i + 1] * zf[i + 1];
+      const float wn = left ? zi : zj, wf = left ? zj : zi;
+      const float c = f32 + 2.f * (zi - zj) * rcp32(dd32), cs = (left ? c : -c) * dd32;
+      const float b = cs + wn + wf, h = cs - wn + wf, r = sqrt32(h * h + 4.f * wn * wf);
+      const float t = (b > 0.f) ? 2.f * wn * dd32 * rcp32(b + r) : (b - r) * dd32 * rcp32(2.f * cs);
+      const float ts = left ? t : -t;
+      if (ts > lo32 && ts < hi32) t32 = ts;
+    }
   }
   bool fine = false;
   for (int it = 0; it < 40; it++) {
     float f3, ps3, dps3, ph3, dph3;
     sec_eval32<kBits>(q, df, zf, od, t32, split, g, f3, ps3, dps3, ph3, dph3);
     if (!(fabsf(f3) < INFINITY) || !(dps3 < INFINITY) || !(dph3 < INFINITY)) break;
-    if (sec_step<float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32)) {
+    if (sec_step<kBits, float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32)) {
       if (!kBits) {
         const float tn = t32 - f3 / (dps3 + dph3);  // the evaluation's own Newton step is free
         if (tn > lo32 && tn < hi32) t32 = tn;
@@ -689,7 +756,7 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
   for (; it < maxit; it++) {
     sec_eval(q, d, z, dorg, tau, split, g, f, psi, dpsi, phi, dphi);
     const double prev = tau;
-    if (sec_step<double>(last, f, psi, dpsi, phi, dphi, da0, db0, DBL_EPSILON, lo, hi, tau)) {
+    if (sec_step<kBits, double>(last, f, psi, dpsi, phi, dphi, da0, db0, DBL_EPSILON, lo, hi, tau)) {
       conv = true;
       break;
     }
@@ -705,9 +772,9 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
 
 // ---------------------------------------------------------------- P2 - P4, one lane group per root
 // root i = pos - slot of the node at `slot` with q poles
-template <bool kBits>
+template <bool kBits, int kG>
 __device__ __forceinline__ void dc_root(const DcParams& p, int node, int slot, int pos, int q, int d,
-                                        const LaneGroup& g) {
+                                        const LaneGroup<kG>& g) {
   int o, its = 0;
   double tau;
   const bool ok = sec_root<kBits>(q, p.dq + slot, p.zq + slot, p.dqf + slot, p.zqf + slot, p.zz[node], pos - slot, g,
@@ -732,8 +799,8 @@ __device__ __forceinline__ void dc_root(const DcParams& p, int node, int slot, i
 // denominators are multiplied apart with their exponents in an integer (eight
 // FP64 instructions per term; a division in each makes it 13, and the
 // operator's 16).
-template <bool kBits>
-__device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, int q, const LaneGroup& g) {
+template <bool kBits, int kG>
+__device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, int q, const LaneGroup<kG>& g) {
   const int j = pos - slot;
   const double* dq = p.dq + slot;
   const double* tau = p.tau + slot;
@@ -741,7 +808,7 @@ __device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, in
   const double dj = dq[j];
   double prod, pn = 1.0, pd = 1.0;
   int en = 0, ed = 0;
-  for (int k = g.lg; k < q - 1; k += g.G) {
+  for (int k = g.lg; k < q - 1; k += g.size()) {
     const double dk = dor[k], dd = dq[(k < j) ? k : k + 1];
     const double num = tau[k] - (dj - dk) * (dj + dk);
     const double den = (dd - dj) * (dd + dj);
@@ -752,8 +819,9 @@ __device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, in
       pd = take_exponent(pd * den, ed);
     }
   }
-  prod = gprod(kBits ? pn : quot(pn, pd), g);
-  int ex = kBits ? 0 : gsum(en - ed, g);
+  prod = kBits ? pn : quot(pn, pd);
+  int ex = en - ed;  // (0 with kBits)
+  gprod(g, prod, ex);
   if (g.lg == 0) {
     const double dk = dor[q - 1];
     prod *= tau[q - 1] - (dj - dk) * (dj + dk);
@@ -770,15 +838,15 @@ __device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, in
 }
 
 // first / last rows of the merged right vector of root i = pos - slot
-template <bool kBits>
-__device__ __forceinline__ void dc_rows(const DcParams& p, int slot, int pos, int q, const LaneGroup& g) {
+template <bool kBits, int kG>
+__device__ __forceinline__ void dc_rows(const DcParams& p, int slot, int pos, int q, const LaneGroup<kG>& g) {
   const double* dq = p.dq + slot;
   const double* zh = p.zh + slot;
   const double* fq = p.fq + slot;
   const double* lq = p.lq + slot;
   const double dorg = p.dor[pos], ti = p.tau[pos];
   double nv = 0.0, sf = 0.0, sl = 0.0;
-  for (int j = g.lg; j < q; j += g.G) {
+  for (int j = g.lg; j < q; j += g.size()) {
     const double dj = dq[j];
     const double del = (dj - dorg) * (dj + dorg) - ti;
     const double v = quotient<kBits>(zh[j], del);
@@ -786,7 +854,7 @@ __device__ __forceinline__ void dc_rows(const DcParams& p, int slot, int pos, in
     sf += v * fq[j];
     sl += v * lq[j];
   }
-  nv = gsum(nv, g); sf = gsum(sf, g); sl = gsum(sl, g);
+  gsum(g, nv, sf, sl);
   if (g.lg == 0) {
     if (kBits) {
       nv = sqrt(nv);
@@ -902,6 +970,23 @@ __device__ unsigned long long g_dc_trace[64 * 16];
   } while (0)
 #endif
 
+// P2 (phase 0), P3 (1) and P4 (2) of one depth, one lane group per root
+template <bool kBits, int kG>
+__device__ __forceinline__ void dc_phase(const DcParams& p, int phase, int d, int G, int lane, int gt, int nthreads,
+                                         int node0) {
+  const LaneGroup<kG> g = make_group<kG>(G, lane);
+  const int gid = gt / g.size(), ngroups = nthreads / g.size();
+  for (int pos = gid; pos < p.N; pos += ngroups) {
+    const int node = (pos == gid) ? node0 : find_node(p, d, pos);
+    if (node < 0) continue;
+    const int slot = p.nd_slot[node], q = p.nq[node];
+    if (pos - slot >= q) continue;
+    if (phase == 0) dc_root<kBits>(p, node, slot, pos, q, d, g);
+    else if (phase == 1) dc_zhat<kBits>(p, slot, pos, q, g);
+    else dc_rows<kBits>(p, slot, pos, q, g);
+  }
+}
+
 template <bool kBits>
 __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
   __shared__ int shi[40];
@@ -938,40 +1023,33 @@ __global__ void __launch_bounds__(kDcThreads, 1) dc_kernel(DcParams p) {
       if (d > 0 && !grid_sync(p.bar, p.P, p.st, 600 + d)) return;
       continue;
     }
-    const LaneGroup g = make_group(p.dgroup[d], lane);
-    const int gid = gt / g.G, ngroups = nthreads / g.G;
+    int G = p.dgroup[d];
+    if (!kBits) {
+      // wider groups while every one still finds a scheduler to itself: an FP64
+      // instruction of a lone warp takes 64 cycles, so a lane's chain of terms is
+      // the phase's time (kBits: the order of the sums is the host's choice)
+      const int wide = min(32, G * p.terms);
+      while (G < wide && (long long)p.N * 2 * G <= 128ll * gridDim.x) G *= 2;
+    }
+    const int gid = gt / G;
     const int node0 = gid < p.N ? find_node(p, d, gid) : -1;  // the forest does not change: ahead of the barrier
+    auto phase = [&](int ph) {
+      if (G == 32) dc_phase<kBits, 32>(p, ph, d, G, lane, gt, nthreads, node0);
+      else dc_phase<kBits, 0>(p, ph, d, G, lane, gt, nthreads, node0);
+    };
     DMARK(1);
     if (!grid_sync(p.bar, p.P, p.st, 100 + d)) return;
     DMARK(2);
-    // ---- P2 secular roots (lane group per root)
-    for (int pos = gid; pos < p.N; pos += ngroups) {
-      const int node = (pos == gid) ? node0 : find_node(p, d, pos);
-      if (node < 0) continue;
-      const int slot = p.nd_slot[node], q = p.nq[node];
-      if (pos - slot < q) dc_root<kBits>(p, node, slot, pos, q, d, g);
-    }
+    phase(0);  // ---- P2 secular roots
     DMARK(3);
     if (rows) {
       if (!grid_sync(p.bar, p.P, p.st, 200 + d)) return;
       DMARK(4);
-      // ---- P3 z-hat (lane group per component)
-      for (int pos = gid; pos < p.N; pos += ngroups) {
-        const int node = (pos == gid) ? node0 : find_node(p, d, pos);
-        if (node < 0) continue;
-        const int slot = p.nd_slot[node], q = p.nq[node];
-        if (pos - slot < q) dc_zhat<kBits>(p, slot, pos, q, g);
-      }
+      phase(1);  // ---- P3 z-hat
       DMARK(5);
       if (!grid_sync(p.bar, p.P, p.st, 300 + d)) return;
       DMARK(6);
-      // ---- P4 rows of the merged right vectors (lane group per root)
-      for (int pos = gid; pos < p.N; pos += ngroups) {
-        const int node = (pos == gid) ? node0 : find_node(p, d, pos);
-        if (node < 0) continue;
-        const int slot = p.nd_slot[node], q = p.nq[node];
-        if (pos - slot < q) dc_rows<kBits>(p, slot, pos, q, g);
-      }
+      phase(2);  // ---- P4 rows of the merged right vectors
     }
     DMARK(7);
     if (!grid_sync(p.bar, p.P, p.st, 400 + d)) return;
@@ -1022,11 +1100,29 @@ __device__ __forceinline__ int seg_find(const DcParams& p, const int* nodes, int
   return (pos < p.nd_slot[node] + p.nd_nn[node]) ? node : -1;
 }
 
+template <int kG>
+__device__ __forceinline__ void dc_tree_phase(const DcParams& p, const int* nodes, int lo, int mid, int phase, int d,
+                                              int G) {
+  const LaneGroup<kG> g = make_group<kG>(G, threadIdx.x & 31);
+  const int ngroups = blockDim.x / g.size();
+  const int pos0 = p.nd_slot[nodes[lo]];
+  const int pos1 = p.nd_slot[nodes[mid - 1]] + p.nd_nn[nodes[mid - 1]];
+  for (int pos = pos0 + threadIdx.x / g.size(); pos < pos1; pos += ngroups) {
+    const int node = seg_find(p, nodes, lo, mid, pos);
+    if (node < 0) continue;
+    const int slot = p.nd_slot[node], q = p.nq[node];
+    if (pos - slot >= q) continue;
+    if (phase == 0) dc_root<true>(p, node, slot, pos, q, d, g);
+    else if (phase == 1) dc_zhat<true>(p, slot, pos, q, g);
+    else dc_rows<true>(p, slot, pos, q, g);
+  }
+}
+
 __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, DcTrees tr) {
   __shared__ int shi[40];
   __shared__ double shd[40];
   __shared__ int s_tree;
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+  const int t = threadIdx.x, wid = t >> 5, nw = blockDim.x >> 5;
   while (true) {
     if (t == 0) s_tree = atomicAdd(tr.counter, 1);
     __syncthreads();
@@ -1061,34 +1157,10 @@ __global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, 
           if (p.nd_nn[tr.nodes[x]] <= kWarpNode) dc_setup_node<true>(p, tr.nodes[x], par, wg);
       }
       __syncthreads();
-      const LaneGroup g = make_group(tr.seg_G[k], lane);
-      const int gid = t / g.G, ngroups = blockDim.x / g.G;
-      const int pos0 = p.nd_slot[tr.nodes[lo]];
-      const int pos1 = p.nd_slot[tr.nodes[mid - 1]] + p.nd_nn[tr.nodes[mid - 1]];
-      // ---- secular roots (lane group per root)
-      for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
-        const int node = seg_find(p, tr.nodes, lo, mid, pos);
-        if (node < 0) continue;
-        const int slot = p.nd_slot[node], q = p.nq[node];
-        if (pos - slot < q) dc_root<true>(p, node, slot, pos, q, d, g);
-      }
-      __syncthreads();
-      if (rows) {
-        // ---- z-hat (lane group per component)
-        for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
-          const int node = seg_find(p, tr.nodes, lo, mid, pos);
-          if (node < 0) continue;
-          const int slot = p.nd_slot[node], q = p.nq[node];
-          if (pos - slot < q) dc_zhat<true>(p, slot, pos, q, g);
-        }
-        __syncthreads();
-        // ---- rows of the merged right vectors (lane group per root)
-        for (int pos = pos0 + gid; pos < pos1; pos += ngroups) {
-          const int node = seg_find(p, tr.nodes, lo, mid, pos);
-          if (node < 0) continue;
-          const int slot = p.nd_slot[node], q = p.nq[node];
-          if (pos - slot < q) dc_rows<true>(p, slot, pos, q, g);
-        }
+      const int G = tr.seg_G[k];
+      for (int ph = 0; ph < (rows ? 3 : 1); ph++) {  // secular roots, z-hat, rows
+        if (G == 32) dc_tree_phase<32>(p, tr.nodes, lo, mid, ph, d, G);
+        else dc_tree_phase<0>(p, tr.nodes, lo, mid, ph, d, G);
         __syncthreads();
       }
       // ---- final merge + normalisation
@@ -1267,6 +1339,7 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
   const int nnodes = H->nnodes, md = H->maxdepth;
   DcParams p;
   p.N = N; p.nnodes = nnodes; p.maxdepth = md;
+  p.terms = std::max(1, ctx->tune[TK_DC_TERMS]);
   p.maxit = ctx->sec_maxit;
   size_t o = 0;
   p.nd_r0 = dints + o; o += nnodes;
