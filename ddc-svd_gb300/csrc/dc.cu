@@ -177,16 +177,24 @@ __device__ long long block_max_ll(long long v, double* sh) {
   return r;
 }
 
+// (kOrdered: the warps' parts are added in order)
+template <bool kOrdered>
 __device__ double block_sumd(double v, double* sh) {
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
   v = warp_sum(v);
   __syncthreads();
   if (lane == 0) sh[wid] = v;
   __syncthreads();
-  if (t == 0) {  // one thread: every warp adding them would queue at the FP64 pipe
+  if (t < 32) {  // one warp: every warp adding them would queue at the FP64 pipe
     double r = 0.0;
-    for (int w = 0; w < nw; w++) r += sh[w];
-    sh[0] = r;
+    if (kOrdered) {
+      if (t == 0)
+        for (int w = 0; w < nw; w++) r += sh[w];
+    } else {
+      r = warp_sum(t < nw ? sh[t] : 0.0);
+    }
+    __syncwarp();
+    if (t == 0) sh[0] = r;
   }
   __syncthreads();
   const double r = sh[0];
@@ -207,6 +215,15 @@ __device__ __forceinline__ double lane_norm(double a, double a1, double b, doubl
   return sqrt(v + w * w);
 }
 
+// Both sums over the warp.
+__device__ __forceinline__ void warp_sum2(double& a, double& b) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+}
+
 // Cooperation policies for the per-node phases: a whole CTA for large nodes,
 // one warp for nodes of at most kWarpNode entries (a batch forest has
 // thousands of those per depth; a CTA each would mostly wait at barriers).
@@ -218,19 +235,35 @@ struct CtaGroup {
   __device__ int size() const { return blockDim.x; }
   __device__ void sync() const { __syncthreads(); }
   __device__ long long maxbits(long long v) const { return block_max_ll(v, shd); }
-  __device__ double sum(double v) const { return block_sumd(v, shd); }
+  template <bool kOrdered>
+  __device__ double sum(double v) const { return block_sumd<kOrdered>(v, shd); }
   __device__ int exscan(int v, int* tot) const { return block_exscan(v, shi, tot); }
   __device__ int any(int v) const { return __syncthreads_or(v); }
-  // lane_inv_norm / lane_norm of the pair, computed by one warp and shared
-  // (every warp computing them would queue at the FP64 pipe)
-  __device__ void inv_norms(double* a, double a1, double* b, double b1) const { pair<true>(a, a1, b, b1); }
-  __device__ void norms(double* a, double a1, double* b, double b1) const { pair<false>(a, a1, b, b1); }
+  // lane_inv_norm / lane_norm of the two sums, taken by one warp and shared
+  // (every warp computing them would queue at the FP64 pipe); kInv adds the
+  // warps' parts in a tree, else in order
   template <bool kInv>
-  __device__ void pair(double* a, double a1, double* b, double b1) const {
+  __device__ void norms(double* a, double a1, double* b, double b1) const {
+    const int t = threadIdx.x, lane = t & 31, nw = blockDim.x >> 5;
+    warp_sum2(*a, *b);
     __syncthreads();
-    if (threadIdx.x < 32) {
-      const double r = kInv ? lane_inv_norm(*a, a1, *b, b1, threadIdx.x) : lane_norm(*a, a1, *b, b1, threadIdx.x);
-      if (threadIdx.x < 2) shd[threadIdx.x] = r;
+    if (lane == 0) {
+      shd[t >> 5] = *a;
+      shd[20 + (t >> 5)] = *b;
+    }
+    __syncthreads();
+    if (t < 32) {
+      double v = 0.0;
+      if (kInv) {
+        if ((lane >> 1) < nw) v = shd[20 * (lane & 1) + (lane >> 1)];
+#pragma unroll
+        for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      } else if (lane < 2) {
+        for (int w = 0; w < nw; w++) v += shd[20 * lane + w];
+      }
+      const double r = kInv ? lane_inv_norm(v, a1, v, b1, lane) : lane_norm(v, a1, v, b1, lane);
+      __syncwarp();
+      if (lane < 2) shd[lane] = r;
     }
     __syncthreads();
     *a = shd[0];
@@ -242,6 +275,7 @@ struct WarpGroup {
   __device__ int size() const { return 32; }
   __device__ void sync() const { __syncwarp(); }
   __device__ long long maxbits(long long v) const { return warp_max_ll(v); }
+  template <bool kOrdered>
   __device__ double sum(double v) const { return warp_sum(v); }
   __device__ int exscan(int v, int* tot) const {
     const int lane = threadIdx.x & 31;
@@ -255,11 +289,10 @@ struct WarpGroup {
     return x - v;
   }
   __device__ int any(int v) const { return __any_sync(0xffffffffu, v); }
-  __device__ void inv_norms(double* a, double a1, double* b, double b1) const { pair<true>(a, a1, b, b1); }
-  __device__ void norms(double* a, double a1, double* b, double b1) const { pair<false>(a, a1, b, b1); }
   template <bool kInv>
-  __device__ void pair(double* a, double a1, double* b, double b1) const {
+  __device__ void norms(double* a, double a1, double* b, double b1) const {
     const int lane = threadIdx.x & 31;
+    warp_sum2(*a, *b);
     const double r = kInv ? lane_inv_norm(*a, a1, *b, b1, lane) : lane_norm(*a, a1, *b, b1, lane);
     *a = __shfl_sync(0xffffffffu, r, 0);
     *b = __shfl_sync(0xffffffffu, r, 1);
@@ -295,44 +328,46 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
   const double* f2 = p.F[cp] + slot + K + 1;
   const double* l2 = p.L[cp] + slot + K + 1;
   const double bk1 = p.b1[r0 + K], bk2 = p.b2[r0 + K];
-  const double phi1 = p.phi[c1], psi1 = p.psi[c1], phi2 = p.phi[c2], psi2 = p.psi[c2];
-  // r = hypot(x, y), (c0, s0) = (x, y) / r  (Calculations-Parallel.c:769-771)
-  const double rx = bk1 * psi1, ry = bk2 * phi2;
-  const double r2 = fma(rx, rx, ry * ry);
-  double r, c0, s0;
-  if (!kBits && bits(r2) > bits(1e-280) && bits(r2) < bits(1e280)) {
-    const double ri = rsqrt(r2);
-    r = r2 * ri;
-    c0 = rx * ri;
-    s0 = ry * ri;
-  } else {
-    r = hypot(rx, ry);
-    c0 = (r > 0.0) ? quot_rn(rx, r) : 1.0;
-    s0 = (r > 0.0) ? quot_rn(ry, r) : 0.0;
-  }
   double* ds = p.ds + slot;
   double* zs = p.zs + slot;
   double* hfs = p.hfs + slot;
   double* hls = p.hls + slot;
   // parallel merge of [0] ++ child1 ++ child2 by value (ties: entry 0, then child1)
   long long zb = 0;  // max |z|, as bits
-  if (t == 0) {
-    ds[0] = 0.0; zs[0] = r; hfs[0] = c0 * phi1; hls[0] = s0 * psi2;
-    zb = max_bits(r);
+  for (int k = t; k < max(n1, n2); k += nt) {  // one of each child at a time: their loads and searches overlap
+    const bool h1 = k < n1, h2 = k < n2;
+    double va = 0.0, la = 0.0, fa = 0.0, vb = 0.0, fb = 0.0, lb = 0.0;
+    if (h1) { va = s1[k]; la = l1[k]; fa = f1[k]; }
+    if (h2) { vb = s2[k]; fb = f2[k]; lb = l2[k]; }
+    const int pa = 1 + k + (h1 ? count_lt(s2, n2, va) : 0);
+    const int pb = 1 + k + (h2 ? count_le(s1, n1, vb) : 0);
+    const double za = bk1 * la, zc = bk2 * fb;
+    if (h1) { ds[pa] = va; zs[pa] = za; hfs[pa] = fa; hls[pa] = 0.0; }
+    if (h2) { ds[pb] = vb; zs[pb] = zc; hfs[pb] = 0.0; hls[pb] = lb; }
+    zb = max(zb, max(max_bits(za), max_bits(zc)));
   }
-  for (int k = t; k < n1; k += nt) {
-    const double v = s1[k];
-    const int pos = 1 + k + count_lt(s2, n2, v);
-    const double z = bk1 * l1[k];
-    ds[pos] = v; zs[pos] = z; hfs[pos] = f1[k]; hls[pos] = 0.0;
-    zb = max(zb, max_bits(z));
-  }
-  for (int k = t; k < n2; k += nt) {
-    const double v = s2[k];
-    const int pos = 1 + k + count_le(s1, n1, v);
-    const double z = bk2 * f2[k];
-    ds[pos] = v; zs[pos] = z; hfs[pos] = 0.0; hls[pos] = l2[k];
-    zb = max(zb, max_bits(z));
+  if (t < 32) {  // one warp: each further one would queue at the FP64 pipe for the same values
+    // r = hypot(x, y), (c0, s0) = (x, y) / r  (Calculations-Parallel.c:769-771)
+    const double phi1 = p.phi[c1], psi1 = p.psi[c1], phi2 = p.phi[c2], psi2 = p.psi[c2];
+    const double rx = bk1 * psi1, ry = bk2 * phi2;
+    const double r2 = fma(rx, rx, ry * ry);
+    double r, c0, s0;
+    if (!kBits && bits(r2) > bits(1e-280) && bits(r2) < bits(1e280)) {
+      const double ri = rsqrt(r2);
+      r = r2 * ri;
+      c0 = rx * ri;
+      s0 = ry * ri;
+    } else {
+      r = hypot(rx, ry);
+      c0 = (r > 0.0) ? quot_rn(rx, r) : 1.0;
+      s0 = (r > 0.0) ? quot_rn(ry, r) : 0.0;
+    }
+    zb = max(zb, max_bits(r));
+    if (t == 0) {
+      ds[0] = 0.0; zs[0] = r; hfs[0] = c0 * phi1; hls[0] = s0 * psi2;
+      p.phi[node] = -s0 * phi1;  // Calculations-Parallel.c:807-808 (normalised in P5)
+      p.psi[node] = c0 * psi2;
+    }
   }
   // the children's values ascend, so the largest d is one of their last
   zb = max(grp.maxbits(zb), max(n1 > 0 ? max_bits(s1[n1 - 1]) : 0ll, n2 > 0 ? max_bits(s2[n2 - 1]) : 0ll));
@@ -395,12 +430,10 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
       doff++;
     }
   }
-  double zz = grp.sum(zzl);
+  const double zz = grp.template sum<kBits>(zzl);
   if (t == 0) {
     p.nq[node] = tot;
     p.zz[node] = zz;
-    p.phi[node] = -s0 * phi1;  // Calculations-Parallel.c:807-808 (normalised in P5)
-    p.psi[node] = c0 * psi2;
   }
 }
 
@@ -553,7 +586,7 @@ __device__ __forceinline__ double step_sqrt(double x) { return sqrt(x); }
 
 template <bool kBits, typename T>
 __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T dphi, T da0, T db0, T eps,
-                                         T& lo, T& hi, T& tau) {
+                                         T& lo, T& hi, T& tau, bool& halved) {
   const T err = last ? T(8) * (T(1) + fabs(psi)) + fabs(tau) * dpsi
                      : T(8) * (T(1) + fabs(psi) + fabs(phi)) + fabs(tau) * (dpsi + dphi);
   if (fabs(f) <= eps * err) return true;
@@ -577,7 +610,8 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
     else eta = step_quot<kBits>(T(2) * cq, bq + disc);
     tn = tau + eta;
   }
-  if (!(tn > lo && tn < hi)) tn = T(0.5) * (lo + hi);
+  halved = !(tn > lo && tn < hi);
+  if (halved) tn = T(0.5) * (lo + hi);
   tau = tn;
   return false;
 }
@@ -585,6 +619,21 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
 #ifdef DDCSVD_PHASE_TRACE
 __device__ unsigned g_dc_iters[64 * 84];  // [depth][FP64 iterations 0..80, 81: FP32 phase gave up early]
 #endif
+
+// 1 and the poles other than o at tau = 0: c in c - z_o^2 / tau, the equation
+// a root much nearer to its pole than any other pole solves
+template <int kG>
+__device__ __forceinline__ float sec_rest32(int q, const float2* d, const float* z, int o, const LaneGroup<kG>& g) {
+  const float2 dorg = d[o];
+  float s = 0.f;
+  for (int j = g.lg; j < q; j += g.size()) {
+    const float2 dj = d[j];
+    const float t = z[j] * z[j] * rcp32(pair_diff(dj, dorg) * (dj.x + dorg.x));
+    if (j != o) s += t;
+  }
+  gsum(g, s);
+  return 1.f + s;
+}
 
 // f at the midpoint of (d_i, d_i+1) on the float pairs, with a bound on its
 // error: del_j = (d_j - d_o)(d_j + d_o) - tau carries a relative error of a few
@@ -704,18 +753,26 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
       if (ts > lo32 && ts < hi32) t32 = ts;
     }
   }
-  bool fine = false;
+  bool fine = false, tried = false, halved;
   for (int it = 0; it < 40; it++) {
     float f3, ps3, dps3, ph3, dph3;
     sec_eval32<kBits>(q, df, zf, od, t32, split, g, f3, ps3, dps3, ph3, dph3);
     if (!(fabsf(f3) < INFINITY) || !(dps3 < INFINITY) || !(dph3 < INFINITY)) break;
-    if (sec_step<kBits, float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32)) {
+    if (sec_step<kBits, float>(last, f3, ps3, dps3, ph3, dph3, da32, db32, 4.f * FLT_EPSILON, lo32, hi32, t32,
+                               halved)) {
       if (!kBits) {
         const float tn = t32 - f3 / (dps3 + dph3);  // the evaluation's own Newton step is free
         if (tn > lo32 && tn < hi32) t32 = tn;
       }
       fine = true;
       break;
+    }
+    if (!kBits && halved && !tried) {
+      // out of the model's reach: mostly a root at z_o^2 / c with a tiny z_o
+      tried = true;
+      const float c = sec_rest32(q, df, zf, o, g);
+      const float t = zf[o] * zf[o] * rcp32(c);  // left: c > 0, right: c < 0
+      if (t > lo32 && t < hi32) t32 = t;
     }
   }
   // ---- phase 2: one FP64 evaluation and a third-order step
@@ -756,7 +813,7 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
   for (; it < maxit; it++) {
     sec_eval(q, d, z, dorg, tau, split, g, f, psi, dpsi, phi, dphi);
     const double prev = tau;
-    if (sec_step<kBits, double>(last, f, psi, dpsi, phi, dphi, da0, db0, DBL_EPSILON, lo, hi, tau)) {
+    if (sec_step<kBits, double>(last, f, psi, dpsi, phi, dphi, da0, db0, DBL_EPSILON, lo, hi, tau, halved)) {
       conv = true;
       break;
     }
@@ -895,6 +952,7 @@ __device__ void dc_finish_node(const DcParams& p, int node, int par, bool rows, 
   double* L = p.L[par] + slot;
   double nf = 1.0, nl = 1.0;
   if (rows && !kBits) {  // the norms first, then one write of the scaled rows
+    const double ph = p.phi[node], ps = p.psi[node];
     double sf = 0.0, sl = 0.0;
     for (int k = t; k < q; k += nt) {
       const double f = p.rF[slot + k], l = p.rL[slot + k];
@@ -906,10 +964,9 @@ __device__ void dc_finish_node(const DcParams& p, int node, int par, bool rows, 
       sf += f * f;
       sl += l * l;
     }
-    nf = grp.sum(sf);
-    nl = grp.sum(sl);
-    const double ph = p.phi[node], ps = p.psi[node];
-    grp.inv_norms(&nf, ph, &nl, ps);
+    nf = sf;
+    nl = sl;
+    grp.template norms<true>(&nf, ph, &nl, ps);
     if (t == 0) {
       p.phi[node] = ph * nf;
       p.psi[node] = ps * nl;
@@ -938,10 +995,8 @@ __device__ void dc_finish_node(const DcParams& p, int node, int par, bool rows, 
   grp.sync();
   double sf = 0.0, sl = 0.0;
   for (int k = t; k < nn; k += nt) { sf += F[k] * F[k]; sl += L[k] * L[k]; }
-  sf = grp.sum(sf);
-  sl = grp.sum(sl);
   const double ph = p.phi[node], ps = p.psi[node];
-  grp.norms(&sf, ph, &sl, ps);
+  grp.template norms<false>(&sf, ph, &sl, ps);
   for (int k = t; k < nn; k += nt) {
     if (sf > 0.0) F[k] = quot_rn(F[k], sf);
     if (sl > 0.0) L[k] = quot_rn(L[k], sl);
