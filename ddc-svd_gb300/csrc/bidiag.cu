@@ -292,29 +292,6 @@ __device__ __forceinline__ void stage_vec(float* dst, const float* __restrict__ 
 
 constexpr int kLD = kPanel + 1;  // padded row length of the cached panel blocks
 
-// Warp reduce-scatter of B per-lane values (B a power of two, at most 32):
-// lane l returns the warp sum of v[l / (32 / B)].  Partners add in the order
-// (own + received), which gives the same sum on both sides, so all 32 / B
-// lanes of a group return the same value.  B - 1 + log2(32 / B) shuffles,
-// against 5 B for B separate warp sums.
-template <int B>
-__device__ __forceinline__ float warp_reduce_scatter(float (&v)[B], int lane) {
-#pragma unroll
-  for (int nv = B, off = 16; nv > 1; nv >>= 1, off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int h = 0; h < nv / 2; h++) {
-      const float send = up ? v[h] : v[h + nv / 2];
-      const float keep = up ? v[h + nv / 2] : v[h];
-      v[h] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  float s = v[0];
-#pragma unroll
-  for (int off = 16 / B; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  return s;
-}
-
 // Columns per batch of the fused pass for RPT4 float4 rows per thread (two
 // batches of B * RPT4 float4s in registers).  Measured on the 4096^2 and
 // 8192^2 factorisations: B * RPT4 = 4 at up to 4096 rows, B = 2 at up to 8192
@@ -1252,6 +1229,13 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   for (int k0 = 0; k0 < n; k0 += kPanel) {
+    // the columns down to the tail with the trailing block in the grid's registers
+    while (const int cols = bidiag_resident_columns(ctx, m, n, k0, P)) {
+      ktimer_begin(ctx, KC_BIDIAG);
+      DDC_TRY(bidiag_resident(ctx, m, n, k0, cols, W, ldw, d, e, tauq, taup, w));
+      ktimer_end(ctx);
+      k0 += cols;
+    }
     // the remaining columns on one thread-block cluster once they fit
     if (bidiag_tail_columns(ctx, m, n, k0) > 0) {
       ktimer_begin(ctx, KC_BIDIAG);

@@ -218,6 +218,29 @@ __device__ __forceinline__ FF warp_sum_ff(FF v) {
   return v;
 }
 
+// Warp reduce-scatter of B per-lane values (B a power of two, at most 32):
+// lane l returns the warp sum of v[l / (32 / B)].  Partners add in the order
+// (own + received), which gives the same sum on both sides, so all 32 / B
+// lanes of a group return the same value.  B - 1 + log2(32 / B) shuffles,
+// against 5 B for B separate warp sums.
+template <int B>
+__device__ __forceinline__ float warp_reduce_scatter(float (&v)[B], int lane) {
+#pragma unroll
+  for (int nv = B, off = 16; nv > 1; nv >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int h = 0; h < nv / 2; h++) {
+      const float send = up ? v[h] : v[h + nv / 2];
+      const float keep = up ? v[h + nv / 2] : v[h];
+      v[h] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  float s = v[0];
+#pragma unroll
+  for (int off = 16 / B; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  return s;
+}
+
 // Householder parameters (reference convention alpha = -sign(x0) ||x||,
 // sign(0) = +1) from x0 and a compensated (float-float) ||tail||^2, in FP32
 // only.  The input matrix is scaled so that max|a| lies in [2^-40, 2^40] (or is left

@@ -178,6 +178,11 @@ int bidiag_coop_ctas(ddcsvd_context* ctx, int m, int n);
 // Columns from k0 on that the cluster tail can finish (0 = none: knob off,
 // no co-schedulable cluster, or the trailing block does not fit), and the
 // launch: the trailing block W[k0:m, k0:n] bidiagonalised on one cluster.
+// Columns from k0 that the grid-resident kernel takes in one launch (a multiple of
+// kPanel; 0: not its shape), and the launch.
+int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P);
+int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* W, int ldw, float* d, float* e,
+                    float* tauq, float* taup, const BidiagWork& w);
 int bidiag_tail_columns(ddcsvd_context* ctx, int m, int n, int k0);
 int bidiag_tail(ddcsvd_context* ctx, int m, int n, int k0, float* W, int ldw, float* d, float* e, float* tauq,
                 float* taup);

@@ -1,0 +1,37 @@
+"""The grid-resident columns of the bidiagonalisation at the edges of their
+configurations (8, 12 or 16 rows per CTA, 2 or 4 columns per thread, hand-over
+to the cluster tail), and next to shapes that start in the panels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n", [(513, 513), (514, 513), (545, 544), (1216, 520), (1217, 1024), (1024, 1024),
+                                 (1025, 1025), (1824, 600), (1825, 1025), (2432, 700), (2433, 540), (2048, 2048),
+                                 (2049, 2049), (2500, 1800)])
+@pytest.mark.parametrize("kind", ["normal", "rank"])
+def test_resident_edges(lib, cuda, m, n, kind):
+    rng = np.random.default_rng(m * 7 + n)
+    A = rng.standard_normal((m, n))
+    if kind == "rank":  # zero rows, columns and reflectors on the way
+        r = max(1, n // 3)
+        A = A[:, :r] @ rng.standard_normal((r, n))
+        A[:, n // 2] = 0.0
+        A[0, :] = 0.0
+    A = A.astype(np.float32)
+    W, d, e, tq, tp = lib.bidiag_device(cuda.from_numpy(A).cuda(), mode="tf32x6")
+    B = np.diag(d.double().cpu().numpy()) + np.diag(e.double().cpu().numpy(), 1)
+    want = cuda.linalg.svdvals(cuda.from_numpy(A).double()).numpy()
+    got = cuda.linalg.svdvals(cuda.from_numpy(B)).numpy()
+    # backward error of n FP32 reflections on each side
+    assert np.max(np.abs(got - want)) <= 4 * 2.0 ** -24 * np.sqrt(n + 8) * np.linalg.norm(A)
+    # the stored reflectors: H = I - tau u u^T with ||u||^2 = 2 / tau wherever tau is not zero
+    Wm = W.double().cpu().numpy().T[:m]
+    tq, tp = tq.double().cpu().numpy(), tp.double().cpu().numpy()
+    for i in range(n):
+        u = np.r_[1.0, Wm[i + 1:, i]]
+        assert tq[i] == 0.0 or abs(tq[i] * (u @ u) - 2.0) <= 1e-4
+        if i + 1 < n:
+            v = np.r_[1.0, Wm[i, i + 2:]]
+            assert tp[i] == 0.0 or abs(tp[i] * (v @ v) - 2.0) <= 1e-4
