@@ -1204,6 +1204,8 @@ void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWo
   const int k0_last = ((n - 1) / kPanel) * kPanel;
   w->ldxp = ldw;
   w->xpart = (m - k0_last <= kFusedRows) ? a.take<float>((size_t)P * ldw + 4) : nullptr;
+  w->rwords = bidiag_resident_words(m, n, P, &w->ldr);
+  w->rpart = w->rwords ? a.take<uint2>(w->rwords) : nullptr;
 }
 
 static int launch_coop(const void* fn, int P, int threads, size_t smem, void* args,
@@ -1228,9 +1230,12 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
   range_apply_kernel<<<sg, 256, 0, ctx->stream>>>(m, n, W, ldw, w.amax);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
+  bool cleared = false;
   for (int k0 = 0; k0 < n; k0 += kPanel) {
     // the columns down to the tail with the trailing block in the grid's registers
-    while (const int cols = bidiag_resident_columns(ctx, m, n, k0, P)) {
+    while (const int cols = w.rpart ? bidiag_resident_columns(ctx, m, n, k0, P) : 0) {
+      if (!cleared) DDC_CUDA_TRY(cudaMemsetAsync(w.rpart, 0, sizeof(uint2) * w.rwords, ctx->stream));
+      cleared = true;  // (no tag of an earlier call; within this one they ascend)
       ktimer_begin(ctx, KC_BIDIAG);
       DDC_TRY(bidiag_resident(ctx, m, n, k0, cols, W, ldw, d, e, tauq, taup, w));
       ktimer_end(ctx);

@@ -164,6 +164,9 @@ struct BidiagWork {
   float *Apk, *Bpk;  // K-major packed trailing-update operands (tensor-core modes)
   float* xpart;      // fused panel pass: P partial products x = A w (ld ldxp), or null
   int ldxp;
+  uint2* rpart;      // exchange buffer of the resident columns (rwords words, records ldr apart), or null
+  size_t rwords;
+  int ldr;
 };
 constexpr int kPanel = 32;       // bidiagonalisation panel width
 constexpr int kFusedRows = 8192; // fused panel pass: rows (from the first staged float4) it covers
@@ -181,6 +184,7 @@ int bidiag_coop_ctas(ddcsvd_context* ctx, int m, int n);
 // Columns from k0 that the grid-resident kernel takes in one launch (a multiple of
 // kPanel; 0: not its shape), and the launch.
 int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P);
+size_t bidiag_resident_words(int m, int n, int P, int* ld);
 int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* W, int ldw, float* d, float* e,
                     float* tauq, float* taup, const BidiagWork& w);
 int bidiag_tail_columns(ddcsvd_context* ctx, int m, int n, int k0);

@@ -40,27 +40,96 @@ struct ResParams {
   int ldw, ldp, ldr;
   float* W;  // trailing block
   float *d, *e, *tauq, *taup;
-  float* part;      // P x ldp: x^T A by CTA
-  float* y;         // tau y
-  float* row;       // 2 x ldr: row i, by column parity
-  float2 *cn, *rn;  // P: compensated parts of ||x||^2 and ||w||^2
+  unsigned tag0;  // tag of the first column
+  // exchanged words (value, tag of the column)
+  uint2* part;      // P x ldp: x^T A by CTA
+  uint2* y;         // tau y
+  uint2* row;       // 2 x ldr: row i, by column parity
+  uint2 *cn, *rn;   // P x 2: compensated parts of ||x||^2 and ||w||^2
   GridBarrier* bar;
   DevStatus* st;
 };
 
+// Exchanged words carry their column's tag beside the value: one 8-byte store
+// publishes both, and a reader polls until the tag is there.  No word is
+// overwritten before its readers are through:
+//  * parts, norms cn and row of column i + 1 are written after their CTA has read
+//    the norms rn of column i from every CTA, and a CTA writes its rn after it has
+//    read the parts, cn and its slice of the row of column i;
+//  * y and rn of column i + 1 are written after their CTA has read cn of column
+//    i + 1 from every CTA, and a CTA writes its cn after it has read y, rn and the
+//    row of column i;
+//  * the row of column i may still be read while its successor is written: one
+//    buffer per parity.
+__device__ __forceinline__ void put(uint2* w, float v, unsigned tag) {
+  const unsigned long long x = __float_as_uint(v) | ((unsigned long long)tag << 32);
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(w), "l"(x) : "memory");
+}
+__device__ __forceinline__ uint2 get(const uint2* w) {
+  unsigned long long x;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(x) : "l"(w) : "memory");
+  return make_uint2((unsigned)x, (unsigned)(x >> 32));
+}
+// One unsuccessful poll: false when the wait is over (another CTA's error, or the limit).
+struct Waiter {
+  DevStatus* st;
+  unsigned polls = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool again() {
+    if ((++polls & 31u) != 0) return true;
+    const uint4 s = ld_status(st);
+    if (s.x != 0) return false;
+    const unsigned long long now = global_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 <= (s.z ? 1000ull * s.z : kWaitLimitNs)) return true;
+    set_error(st, DDCSVD_ERR_TIMEOUT, 50);
+    return false;
+  }
+};
+// Reads the words at(0..N-1) that `want` asks for (others: zero); those missing are
+// polled together.  False: gave up.
+// Without kTag a grid barrier has ordered the words already, and their values are
+// read alone.
+template <bool kTag, int N, class At, class Want>
+__device__ __forceinline__ bool take(float (&v)[N], unsigned tag, Waiter& wt, At at, Want want) {
+  if constexpr (!kTag) {
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = want(u) ? __ldcg(reinterpret_cast<const float*>(at(u))) : 0.f;
+  } else {
+    uint2 w[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) w[u] = make_uint2(0u, want(u) ? tag - 1u : tag);
+    while (true) {
+      bool all = true;
+#pragma unroll
+      for (int u = 0; u < N; u++)
+        if (w[u].y != tag) w[u] = get(at(u));
+#pragma unroll
+      for (int u = 0; u < N; u++) all = all && w[u].y == tag;
+      if (all) break;
+      if (!wt.again()) return false;
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = __uint_as_float(w[u].x);
+  }
+  return true;
+}
+
 // entry q of a float4 held in registers (q a constant after unrolling)
 __device__ __forceinline__ float el(const float4& v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
 
-// the sum of P compensated records in one warp
-__device__ __forceinline__ FF sum_records(const float2* rec, int P, int lane) {
+// the sum of P compensated records (two words each) in one warp
+template <bool kTag>
+__device__ __forceinline__ FF sum_records(const uint2* rec, int P, unsigned tag, int lane, Waiter& wt, bool& ok) {
   FF n{0.f, 0.f};
   for (int q = lane; q < P; q += 32 * 5) {
-    float2 v[5];
+    float v[10];
+    ok = take<kTag, 10>(v, tag, wt, [&](int u) { return rec + 2 * (q + 32 * (u >> 1)) + (u & 1); },
+                  [&](int u) { return q + 32 * (u >> 1) < P; }) && ok;
 #pragma unroll
-    for (int u = 0; u < 5; u++) v[u] = (q + 32 * u < P) ? __ldcg(rec + q + 32 * u) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < 5; u++) n = ff_add(n, FF{v[u].x, v[u].y});
+    for (int u = 0; u < 5; u++) n = ff_add(n, FF{v[2 * u], v[2 * u + 1]});
   }
+  __syncwarp();
   return warp_sum_ff(n);
 }
 
@@ -70,14 +139,17 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   constexpr int W = T / 32, R4 = R / 4;
   constexpr int B = R > 16 ? 32 : R > 8 ? 16 : 8;  // rows of the reduce-scatter
   constexpr int U = T > 256 ? 6 : 11;              // slice loads in flight per thread
+  // 24 rows leave no registers to poll from: barriers there (4096^2: stage 1 40.2 ms
+  // against 43.1 polling; below 2432 rows 2048^2 takes 9.5 ms polling against 10.8)
+  constexpr bool kTag = T > 256;
   static_assert(R % 4 == 0 && R <= 32, "rows come in float4s");
-  extern __shared__ __align__(16) float4 s_a[];                 // [R4][S], then S floats: w of these columns
+  extern __shared__ __align__(16) float4 s_a[];                 // [R4][S], then w and y of these columns
   __shared__ __align__(16) float s_x[R], s_u[R], s_z[R];        // own rows of x, u and of the right update
   __shared__ float s_c1[R], s_red[W][B], s_sl[W][kResSlice], s_q[2], s_p[2];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, b = blockIdx.x, P = gridDim.x;
   const bool main = t < T;
   const int mt = p.mt, nt = p.nt, S = p.S, r0 = b * R, ldw = p.ldw;
-  float* s_w = reinterpret_cast<float*>(s_a + (size_t)R4 * S);
+  float *s_w = reinterpret_cast<float*>(s_a + (size_t)R4 * S), *s_y = s_w + S;
   float a[R][K];
   auto load4 = [&](int c, int r) {  // rows r0 + r .. + 3 of column c (the last ones may be padding: ldw is a multiple of 4)
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -114,8 +186,11 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   for (int i = -1; i < p.cols; i++) {
     const bool own = i >= r0 && i < r0 + R;  // row i is here
     if (i >= 0) {
-      float* row = p.row + (i & 1) * p.ldr;
-      if (!grid_sync(p.bar, P, p.st, 50)) return;
+      uint2* row = p.row + (i & 1) * p.ldr;
+      const unsigned tag = p.tag0 + i;
+      Waiter wt{p.st};
+      bool ok = true;
+      if (!kTag && !grid_sync(p.bar, P, p.st, 50)) return;
       // ---- left reflector; tau y and the new row on the CTA's slice of the columns
       const int ncol = nt - (i + 1), cc = (ncol + P - 1) / P;  // (at most kResSlice: the host's choice of shapes)
       const int c0 = i + 1 + b * cc, nc = max(0, min(cc, nt - c0));
@@ -123,22 +198,28 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
       float wic = 0.f;
       if (main) {
         const int cl = t & (w - 1), nrec = T >> lg;
-        if (wid == 0 && lane < nc) wic = __ldcg(row + c0 + lane);
         float s = 0.f;
         for (int q = t >> lg; q < P; q += U * nrec) {
           float v[U];
-#pragma unroll
-          for (int u = 0; u < U; u++)
-            v[u] = (cl < nc && q + u * nrec < P) ? __ldcg(p.part + (size_t)(q + u * nrec) * p.ldp + c0 + cl) : 0.f;
+          ok = take<kTag, U>(v, tag, wt, [&](int u) { return p.part + (size_t)(q + u * nrec) * p.ldp + c0 + cl; },
+                       [&](int u) { return cl < nc && q + u * nrec < P; }) && ok;
 #pragma unroll
           for (int u = 0; u < U; u++) s += v[u];
         }
+        if (wid == 0) {
+          float v[1];
+          ok = take<kTag, 1>(v, tag, wt, [&](int) { return row + c0 + lane; }, [&](int) { return lane < nc; }) && ok;
+          wic = v[0];
+        }
+        __syncwarp();
         for (int o = 16; o >= w; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane < w) s_sl[wid][lane] = s;
       } else {
         float alpha, tq, sq;
-        const float x0 = __ldcg(row + i);
-        householder_ff(x0, sum_records(p.cn, P, lane), &alpha, &tq, &sq);
+        float x0[1];
+        const FF n2 = sum_records<kTag>(p.cn, P, tag, lane, wt, ok);
+        ok = take<kTag, 1>(x0, tag, wt, [&](int) { return row + i; }, [](int) { return true; }) && ok;
+        householder_ff(x0[0], n2, &alpha, &tq, &sq);
         if (lane == 0) {
           s_q[0] = tq;
           s_q[1] = sq;
@@ -148,7 +229,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
           }
         }
       }
-      __syncthreads();
+      if (__syncthreads_or(!ok)) return;
       const float tq = s_q[0], sq = s_q[1];
       if (wid == 0) {
         // the warps' sums: two lanes per column share them while a slice has at most 16
@@ -166,42 +247,57 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
         FF n{0.f, 0.f};
         if (lane < nc) {
           const float y = tq * (wic + sq * s);
-          p.y[c0 + lane] = y;
+          put(p.y + c0 + lane, y, tag);
           if (c0 + lane > i + 1) n = ff_add_sq(n, wic - y);
         }
         n = warp_sum_ff(n);
-        if (lane == 0) p.rn[b] = make_float2(n.hi, n.lo);
+        if (lane < 2) put(p.rn + 2 * b + lane, lane ? n.lo : n.hi, tag);
       } else if (wid == 1 && lane < R) {
         const int r = r0 + lane;
         const float u = s_x[lane] * sq;
         s_u[lane] = r > i ? u : 0.f;
         if (r >= i && r < mt) p.W[r + (size_t)i * ldw] = r > i ? u : 1.f;
       }
-      if (!grid_sync(p.bar, P, p.st, 51)) return;
+      if (!kTag) {
+        if (!grid_sync(p.bar, P, p.st, 51)) return;
+      } else {
+        __syncthreads();  // s_u
+      }
       // ---- left update and products with the new row
       if (main) {
         float z[B];
 #pragma unroll
         for (int r = 0; r < B; r++) z[r] = 0.f;
         float y[K], v[K];
+        const auto reg_at = [&](int k) { return S + t + k * T; };
+        const auto reg_want = [&](int k) { return reg_at(k) > i && reg_at(k) < nt; };
+        {
+          float yw[2 * K];
+          ok = take<kTag, 2 * K>(yw, tag, wt, [&](int u) { return (u < K ? p.y : row) + reg_at(u < K ? u : u - K); },
+                           [&](int u) { return reg_want(u < K ? u : u - K); }) && ok;
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-          const int c = S + t + k * T;
-          const bool in = c > i && c < nt;
-          y[k] = in ? __ldcg(p.y + c) : 0.f;
-          rw[k] = in ? __ldcg(row + c) : 0.f;
-        }
-        // (columns in shared memory: the next one's y and w are on their way while one is swept)
-        int c = t + (t <= i ? (i - t + T) / T * T : 0);  // the thread's first column beyond i
-        float yn = c < S ? __ldcg(p.y + c) : 0.f, wn = c < S ? __ldcg(row + c) : 0.f;
-        for (; c < S; c += T) {
-          const float yc = yn, wc = wn - yc;
-          if (c + T < S) {
-            yn = __ldcg(p.y + c + T);
-            wn = __ldcg(row + c + T);
+          for (int k = 0; k < K; k++) {
+            y[k] = yw[k];
+            rw[k] = yw[K + k];
           }
+        }
+        // columns in shared memory: y and w of a few at a time
+        constexpr int C = T > 256 ? 2 : 5;
+        const int c1 = t + (t <= i ? (i - t + T) / T * T : 0);  // the thread's first column beyond i
+        for (int c = c1; c < S; c += C * T) {
+          float yw[2 * C];
+          ok = take<kTag, 2 * C>(yw, tag, wt, [&](int u) { return (u < C ? p.y : row) + c + (u < C ? u : u - C) * T; },
+                                 [&](int u) { return c + (u < C ? u : u - C) * T < S; }) && ok;
+#pragma unroll
+          for (int u = 0; u < C; u++)
+            if (c + u * T < S) {
+              s_y[c + u * T] = yw[u];
+              s_w[c + u * T] = yw[C + u] - yw[u];
+            }
+        }
+        for (int c = c1; c < S; c += T) {
+          const float yc = s_y[c], wc = s_w[c];
           const float vc = c > i + 1 ? wc : 0.f;
-          s_w[c] = wc;
 #pragma unroll
           for (int q = 0; q < R4; q++) {
             const float4 uv = *reinterpret_cast<const float4*>(s_u + 4 * q);
@@ -214,6 +310,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
             }
           }
         }
+        __syncwarp();
 #pragma unroll
         for (int k = 0; k < K; k++) {
           rw[k] -= y[k];  // the new row
@@ -241,8 +338,10 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
         if (lane % G == 0) s_red[wid][lane / G] = zs;
       } else {
         float beta, tp, sp;
-        const float x0 = __ldcg(row + i + 1) - __ldcg(p.y + i + 1);
-        householder_ff(x0, sum_records(p.rn, P, lane), &beta, &tp, &sp);
+        float x0[2];
+        const FF n2 = sum_records<kTag>(p.rn, P, tag, lane, wt, ok);
+        ok = take<kTag, 2>(x0, tag, wt, [&](int u) { return (u ? p.y : row) + i + 1; }, [](int) { return true; }) && ok;
+        householder_ff(x0[0] - x0[1], n2, &beta, &tp, &sp);
         if (lane == 0) {
           s_p[0] = tp;
           s_p[1] = sp;
@@ -252,7 +351,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
           }
         }
       }
-      __syncthreads();
+      if (__syncthreads_or(!ok)) return;
       {  // one warp per row finishes its product; column i + 1 follows from it
         const float tp = s_p[0], sp = s_p[1];
         for (int r = wid; r < R; r += W + 1) {
@@ -272,8 +371,9 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
     const float tp = s_p[0], sp = s_p[1];
     const int i1 = i + 1;
     const bool more = i1 < p.cols;
-    float* row1 = p.row + (i1 & 1) * p.ldr;
-    float* part = p.part + (size_t)b * p.ldp;
+    uint2* row1 = p.row + (i1 & 1) * p.ldr;
+    uint2* part = p.part + (size_t)b * p.ldp;
+    const unsigned tag1 = p.tag0 + i1;
     const bool own1 = more && i1 >= r0 && i1 < r0 + R;
     if (main) {
       for (int c = t; c < S; c += T) {
@@ -291,8 +391,8 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
 #pragma unroll
           for (int h = 0; h < 4; h++) s += (r0 + 4 * q + h > i1) ? el(av, h) * el(xv, h) : 0.f;
         }
-        if (more && c > i1) part[c] = s;
-        if (own1) row1[c] = reinterpret_cast<const float*>(s_a + ((i1 - r0) >> 2) * S + c)[(i1 - r0) & 3];
+        if (more && c > i1) put(part + c, s, tag1);
+        if (own1) put(row1 + c, reinterpret_cast<const float*>(s_a + ((i1 - r0) >> 2) * S + c)[(i1 - r0) & 3], tag1);
       }
       float s[K];
 #pragma unroll
@@ -319,7 +419,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int c = S + t + k * T;
-        if (more && c > i1 && c < nt) part[c] = s[k];
+        if (more && c > i1 && c < nt) put(part + c, s[k], tag1);
       }
       if (own1) {
 #pragma unroll
@@ -328,7 +428,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
 #pragma unroll
             for (int k = 0; k < K; k++) {
               const int c = S + t + k * T;
-              if (c >= i1 && c < nt) row1[c] = a[r][k];
+              if (c >= i1 && c < nt) put(row1 + c, a[r][k], tag1);
             }
           }
       }
@@ -336,7 +436,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
       FF n{0.f, 0.f};
       if (lane < R && r0 + lane > i1) n = ff_add_sq(n, s_x[lane]);
       n = warp_sum_ff(n);
-      if (lane == 0) p.cn[b] = make_float2(n.hi, n.lo);
+      if (lane < 2) put(p.cn + 2 * b + lane, lane ? n.lo : n.hi, tag1);
     }
   }
   // ---- the rest back (the columns taken are stored already)
@@ -369,7 +469,7 @@ ResConfig res_entry() {
 }
 
 size_t res_smem(const ResConfig& g, int nt) {
-  return (size_t)std::max(0, nt - g.K * g.T) * (g.R + 1) * sizeof(float);
+  return (size_t)std::max(0, nt - g.K * g.T) * (g.R + 2) * sizeof(float);
 }
 
 // The smallest configuration that has the rows and keeps all but a few columns in
@@ -410,33 +510,41 @@ int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P) {
   return tail ? cols : 0;
 }
 
+// Words of the exchange buffer for all launches of one factorisation (none for
+// matrices so small that the tail takes them whole, or with too many rows).
+size_t bidiag_resident_words(int m, int n, int P, int* ld) {
+  *ld = (int)round_up(std::min(n, kResSlice * P), 32);  // the most columns a launch starts with
+  if ((long long)m * n <= 400000 || m - n > 24 * P) return 0;
+  return (size_t)(P + 3) * *ld + 4 * (size_t)P;
+}
+
 int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* W, int ldw, float* d, float* e,
                     float* tauq, float* taup, const BidiagWork& w) {
   const ResConfig* g = res_config(m - k0, n - k0, w.P, res_smem_max(ctx));
-  if (!g || !w.xpart) return DDCSVD_ERR_UNSUPPORTED;
+  if (!g || !w.rpart) return DDCSVD_ERR_UNSUPPORTED;
   ResParams p;
   p.mt = m - k0;
   p.nt = n - k0;
   p.cols = cols;
   p.S = std::max(0, p.nt - g->K * g->T);
   p.ldw = ldw;
-  p.ldp = w.ldxp;
-  p.ldr = w.ldn;
+  p.ldp = p.ldr = w.ldr;
   p.W = W + k0 + (size_t)k0 * ldw;
   p.d = d + k0;
   p.e = e + k0;
   p.tauq = tauq + k0;
   p.taup = taup + k0;
-  p.part = w.xpart;  // the panels' buffers: none is in use between panels
-  p.y = w.Y;
-  p.row = w.VT;
-  p.cn = reinterpret_cast<float2*>(w.colpart);
-  p.rn = reinterpret_cast<float2*>(w.rowpart);
+  p.tag0 = (unsigned)k0 + 1u;
+  p.part = w.rpart;
+  p.y = p.part + (size_t)w.P * p.ldp;
+  p.row = p.y + p.ldr;
+  p.cn = p.row + 2 * p.ldr;
+  p.rn = p.cn + 2 * w.P;
   p.bar = w.bar;
   p.st = ctx->d_status;
+  DDC_CUDA_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), ctx->stream));
   const size_t smem = res_smem(*g, p.nt);
   DDC_CUDA_TRY(cudaFuncSetAttribute(g->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  DDC_CUDA_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), ctx->stream));
   void* args[] = {&p};
   DDC_CUDA_TRY(cudaLaunchCooperativeKernel(g->fn, dim3(w.P), dim3(g->T + 32), args, smem, ctx->stream));
   count_launch();
