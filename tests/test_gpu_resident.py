@@ -36,3 +36,20 @@ def test_resident_edges(lib, cuda, m, n, kind):
         if i + 1 < n:
             v = np.r_[1.0, Wm[i, i + 2:]]
             assert tp[i] == 0.0 or abs(tp[i] * (v @ v) - 2.0) <= 1e-4
+
+
+@pytest.mark.parametrize("m,n", [(900, 700), (2600, 2500)])  # polled words; grid barriers
+def test_waits_that_run_out_end_with_a_status(lib, cuda, m, n):
+    """One CTA's arrival is missing: every wait ends at the 2 ms limit, the call
+    returns DDCSVD_ERR_TIMEOUT and the handle works again afterwards."""
+    rng = np.random.default_rng(3)
+    A = cuda.from_numpy(rng.standard_normal((m, n)).astype(np.float32)).cuda()
+    h = lib.Handle()
+    want = lib.svd_device(A, handle=h)[0].cpu().numpy()
+    keep = h.limits
+    h.limits = {"wait_us": 2000, "barrier_extra_arrivals": 1}
+    with pytest.raises(lib.DdcsvdError) as ei:
+        lib.svd_device(A, handle=h)
+    assert ei.value.status == 5
+    h.limits = keep
+    assert np.array_equal(lib.svd_device(A, handle=h)[0].cpu().numpy(), want)
