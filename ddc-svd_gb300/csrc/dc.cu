@@ -497,8 +497,13 @@ __device__ __forceinline__ void sec_eval(int q, const double* d, const double* z
     const double dj = d[j];
     const double del = (dj - dorg) * (dj + dorg) - tau;
     const double tt = quot_rn(z[j], del);
-    if (j <= split) { ps += z[j] * tt; dps += tt * tt; }
-    else { ph += z[j] * tt; dph += tt * tt; }
+    // (the side's sums by selects: a branch here sent most warps down both sides)
+    const bool le = j <= split;
+    const double a = (le ? ps : ph) + z[j] * tt, da = (le ? dps : dph) + tt * tt;
+    ps = le ? a : ps;
+    dps = le ? da : dps;
+    ph = le ? ph : a;
+    dph = le ? dph : da;
   }
   gsum(g, ps, dps, ph, dph);
   psi = ps; dpsi = dps; phi = ph; dphi = dph;
@@ -584,14 +589,27 @@ __device__ __forceinline__ float step_sqrt(float x) { return kBits ? sqrtf(x) : 
 template <bool kBits>
 __device__ __forceinline__ double step_sqrt(double x) { return sqrt(x); }
 
+// |a| <= b for b >= 0, a < 0 and the larger magnitude; in FP64 by the bits (a
+// comparison takes the FP64 pipe as long as a product)
+__device__ __forceinline__ bool abs_le(float a, float b) { return fabsf(a) <= b; }
+__device__ __forceinline__ bool abs_le(double a, double b) {
+  return abs_bits(a) <= bits(b) && bits(b) <= 0x7ff0000000000000ll;  // (false for a NaN)
+}
+__device__ __forceinline__ bool negative(float a) { return a < 0.f; }
+__device__ __forceinline__ bool negative(double a) { return bits(a) < 0 && abs_bits(a) > 0; }
+__device__ __forceinline__ float max_abs(float a, float b) { return fmaxf(fabsf(a), fabsf(b)); }
+__device__ __forceinline__ double max_abs(double a, double b) {
+  return __longlong_as_double(max(abs_bits(a), abs_bits(b)));
+}
+
 template <bool kBits, typename T>
 __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T dphi, T da0, T db0, T eps,
                                          T& lo, T& hi, T& tau, bool& halved) {
   const T err = last ? T(8) * (T(1) + fabs(psi)) + fabs(tau) * dpsi
                      : T(8) * (T(1) + fabs(psi) + fabs(phi)) + fabs(tau) * (dpsi + dphi);
-  if (fabs(f) <= eps * err) return true;
-  if (f < T(0)) lo = tau; else hi = tau;
-  if (hi - lo <= T(4) * eps * fmax(fabs(lo), fabs(hi))) return true;
+  if (abs_le(f, eps * err)) return true;
+  if (negative(f)) lo = tau; else hi = tau;
+  if (abs_le(hi - lo, T(4) * eps * max_abs(lo, hi))) return true;
   T tn;
   if (last) {
     const T da = -tau;
@@ -604,11 +622,14 @@ __device__ __forceinline__ bool sec_step(bool last, T f, T psi, T dpsi, T phi, T
     const T c = f - step_quot<kBits>(s1, da) - step_quot<kBits>(s2, db);
     const T aq = c, bq = c * (da + db) + s1 + s2, cq = da * db * f;
     const T disc = step_sqrt<kBits>(fabs(bq * bq - T(4) * aq * cq));
-    T eta;
-    if (aq == T(0)) eta = step_quot<kBits>(cq, bq);
-    else if (bq <= T(0)) eta = step_quot<kBits>(bq - disc, T(2) * aq);
-    else eta = step_quot<kBits>(T(2) * cq, bq + disc);
-    tn = tau + eta;
+    // the smaller root of the model's quadratic, one quotient for its three forms
+    const bool low = !(bq > T(0));
+    T num = low ? bq - disc : T(2) * cq, den = low ? T(2) * aq : bq + disc;
+    if (aq == T(0)) {
+      num = cq;
+      den = bq;
+    }
+    tn = tau + step_quot<kBits>(num, den);
   }
   halved = !(tn > lo && tn < hi);
   if (halved) tn = T(0.5) * (lo + hi);
