@@ -1162,7 +1162,11 @@ struct DcTrees {
   const int* order;      // trees, largest first
   int* counter;
 };
+// 256 threads, or 128 where every node is a warp's: a batch of small problems has
+// more trees than 2 x 152 CTAs of the larger size (400 of 36 columns: 443 -> 309 us).  Nodes
+// above a warp's keep 256, which is part of the order of their sums.
 constexpr int kDcTreeThreads = 256;
+constexpr int kDcTreeSmall = 128;
 
 // merge node of segment [lo, mid) containing slot position pos (or -1)
 __device__ __forceinline__ int seg_find(const DcParams& p, const int* nodes, int lo, int mid, int pos) {
@@ -1194,7 +1198,8 @@ __device__ __forceinline__ void dc_tree_phase(const DcParams& p, const int* node
   }
 }
 
-__global__ void __launch_bounds__(kDcTreeThreads, 2) dc_tree_kernel(DcParams p, DcTrees tr) {
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 512 / kThreads) dc_tree_kernel(DcParams p, DcTrees tr) {
   __shared__ int shi[40];
   __shared__ double shd[40];
   __shared__ int s_tree;
@@ -1460,10 +1465,13 @@ int dc_sigma(ddcsvd_context* ctx, int N, const double* b1, const double* b2, dou
     tr.order = dints + q2;
     tr.counter = reinterpret_cast<int*>(bar);
     int occ = 0;
-    DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dc_tree_kernel, kDcTreeThreads, 0));
+    const bool small = H->maxtree <= kWarpNode;
+    const int threads = small ? kDcTreeSmall : kDcTreeThreads;
+    const auto kern = small ? dc_tree_kernel<kDcTreeSmall> : dc_tree_kernel<kDcTreeThreads>;
+    DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0));
     const int grid = std::max(1, std::min(nt, ctx->num_sms * std::max(occ, 1)));
     ktimer_begin(ctx, KC_DC);
-    dc_tree_kernel<<<grid, kDcTreeThreads, 0, ctx->stream>>>(p, tr);
+    kern<<<grid, threads, 0, ctx->stream>>>(p, tr);
     ktimer_end(ctx);
     count_launch();
     DDC_CUDA_TRY(cudaGetLastError());
