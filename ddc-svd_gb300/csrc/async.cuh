@@ -44,6 +44,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// Untiled bulk copy global -> shared (16-byte aligned addresses and size).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
 // Orders this thread's generic-proxy shared-memory writes before later
 // async-proxy (TMA) reads of them.
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -36,6 +36,7 @@
 //
 // Loads of data that other CTAs write during the kernel go through L2 only
 // (ld.global.cg) so that no SM reads a stale L1 line.
+#include "async.cuh"
 #include "internal.hpp"
 
 namespace ddcsvd {
@@ -77,6 +78,7 @@ struct PanelParams {
   int rpt4;
   float* xpart;
   int ldxp;
+  int ring_own, ring_slot4;  // column ring (rpt4 = 4): own slots, float4s per slot
   // two-GEMV form with more rows than shared memory holds next to the panel
   // blocks: y = A^T u reads the column from xcol (global, L2-resident)
   // instead of a staged copy, and the staging buffer holds only the row
@@ -415,6 +417,153 @@ __device__ __forceinline__ void fused_col_pass(const float* __restrict__ W, int 
   }
 }
 
+// The same pass with the columns brought to shared memory by bulk copies, for
+// blocks that come from HBM (more than 4096 rows).  Two batches of B columns in
+// registers keep 64 KB on the way to an SM, and a batch's loads only start when
+// the one before is used; HBM's latency under load wants more (8192^2: 4.5 TB/s).
+// A ring of NS column slots keeps NS columns on the way.  The first `own` slots are
+// the ring's alone, and their first columns of a step are asked for when the step
+// begins: the trailing block does not change within the panel, so they arrive
+// behind the two barriers.  The last two slots lie over the staged column and the
+// row products of S5, which the pass does not need; theirs start with the pass.
+constexpr int kRingMax = 8;
+struct ColumnRing {
+  float4* base;   // own slots
+  float4* alias0; // and the two that share memory
+  float4* alias1;
+  int own, NS, slot4;  // slots, float4s per slot
+  uint64_t* bar;       // one per slot
+  unsigned phase;      // parity of each slot's next completion
+  int waiting;         // columns asked for and not yet used
+  DevStatus* st;
+  __device__ __forceinline__ float4* slot(int s) const {
+    return s < own ? base + (size_t)s * slot4 : s == own ? alias0 : alias1;
+  }
+  // thread 0: column cl of the step
+  __device__ __forceinline__ void ask(const float* col, int cl, int nq) const {
+    const int s = cl % NS;
+    mbar_arrive_expect_tx(bar + s, 16u * nq);
+    bulk_load(slot(s), col, 16u * nq, bar + s);
+  }
+  __device__ __forceinline__ void wait(int s) {
+    unsigned long long t0 = 0;
+    for (unsigned polls = 1; !mbar_try_wait(bar + s, (phase >> s) & 1u); polls++)
+      if ((polls & 255u) == 0) {
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 > kWaitLimitNs) {
+          set_error(st, DDCSVD_ERR_TIMEOUT, 60);
+          break;
+        }
+      }
+    phase ^= 1u << s;
+  }
+  // the copies under way land before the kernel gives its shared memory back
+  __device__ __forceinline__ void drain(int used) {
+    for (int cl = used; cl < used + waiting; cl++) wait(cl % NS);
+  }
+};
+
+template <int RPT4, int B, typename Prologue>
+__device__ __forceinline__ void fused_ring_pass(ColumnRing& ring, const float* __restrict__ W, int ldw, int m, int sa,
+                                                int nq, int c_s, int ncol, int ca, int i, int j, const float* xsb,
+                                                float* red, const float* c1s, const float* c2s, const float* pre,
+                                                float tq, float sq, float* Y, int ldn, float* YS, float* owncol,
+                                                float* xrow, float* xp, Prologue prologue) {
+  constexpr int G = 32 / B;  // lanes per column after the reduce-scatter
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5, nt = blockDim.x;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int mt = m - sa - 4 * (nq - 1);  // valid rows of the last float4, 1..4
+  auto msk = [&](float4 v, int k) {
+    if (t + k * nt == nq - 1 && mt < 4) {
+      if (mt < 2) v.y = 0.f;
+      if (mt < 3) v.z = 0.f;
+      v.w = 0.f;
+    }
+    return v;
+  };
+  float4 xs[RPT4], acc[RPT4];
+#pragma unroll
+  for (int k = 0; k < RPT4; k++) {
+    const int q = t + k * nt;
+    xs[k] = q < nq ? reinterpret_cast<const float4*>(xsb + sa)[q] : z4;
+    acc[k] = z4;
+  }
+  prologue();
+  __syncthreads();
+  if (t == 0) {
+    fence_proxy_async_smem();
+    for (int cl = ring.own; cl < min(ring.NS, ncol); cl++) ring.ask(W + (size_t)(c_s + cl) * ldw + sa, cl, nq);
+  }
+  int s0 = 0;  // slot of the batch's first column
+  for (int c0 = 0, par = 0; c0 < ncol; c0 += B, par ^= 1) {
+    float4 cur[B][RPT4];
+    float pd[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      const bool cin = c0 + u < ncol;
+      const float4* col = ring.slot(s0);
+      if (cin) {
+        ring.wait(s0);
+        s0 = s0 + 1 == ring.NS ? 0 : s0 + 1;
+      }
+      float a = 0.f;
+#pragma unroll
+      for (int k = 0; k < RPT4; k++) {
+        const int q = t + k * nt;
+        const float4 v = msk((cin && q < nq) ? col[q] : z4, k);
+        cur[u][k] = v;
+        a += v.x * xs[k].x + v.y * xs[k].y + v.z * xs[k].z + v.w * xs[k].w;
+      }
+      pd[u] = a;
+    }
+    const float ws = warp_reduce_scatter<B>(pd, lane);
+    const int u = lane / G, sub = lane % G;
+    float* rp = red + par * (B * nw);  // [column][warp]
+    if (sub == 0) rp[u * nw + wid] = ws;
+    __syncthreads();  // (every thread has the batch in registers: its slots are free)
+    if (t == 0)
+      for (int cl = c0 + ring.NS; cl < min(c0 + ring.NS + B, ncol); cl++)
+        ring.ask(W + (size_t)(c_s + cl) * ldw + sa, cl, nq);
+    float tot = 0.f;
+    for (int w2 = sub; w2 < nw; w2 += G) tot += rp[u * nw + w2];
+#pragma unroll
+    for (int off = G / 2; off > 0; off >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, off);
+    const int cl = c0 + u;
+    float wv = 0.f;
+    if (cl < ncol) {
+      const float wic = pre[cl];
+      const float ycj = tq * (wic + sq * tot - c1s[cl]);
+      wv = wic - ycj - c2s[cl];
+      if (wid == 0 && sub == 0) {
+        const int c = c_s + cl;
+        Y[c + (size_t)j * ldn] = ycj;
+        YS[(c - ca) * kLD + j] = ycj;
+        owncol[cl] = wv;
+        xrow[c] = wv;
+      }
+      if (c_s + cl < i + 2) wv = 0.f;
+    }
+#pragma unroll
+    for (int uu = 0; uu < B; uu++) {
+      const float wb = __shfl_sync(0xffffffffu, wv, uu * G);
+#pragma unroll
+      for (int k = 0; k < RPT4; k++) {
+        acc[k].x += cur[uu][k].x * wb;
+        acc[k].y += cur[uu][k].y * wb;
+        acc[k].z += cur[uu][k].z * wb;
+        acc[k].w += cur[uu][k].w * wb;
+      }
+    }
+  }
+  float4* xp4 = reinterpret_cast<float4*>(xp + sa);
+#pragma unroll
+  for (int k = 0; k < RPT4; k++) {
+    const int q = t + k * nt;
+    if (q < nq) xp4[q] = acc[k];
+  }
+}
+
 // Shared-memory layout of the panel kernel (floats unless noted).
 struct PanelSmem {
   float* big;     // max(m, n) + 4: xcol / xrow by absolute index
@@ -433,6 +582,7 @@ struct PanelSmem {
   float* redp;    // (threads / 32) * (kPS + 4): per-warp partial sums
   float* scal;    // 8
   float* xr;      // fused pass: P * rc, the P partial products of the own rows
+  float* ring;    // own slots of the column ring
 };
 
 __device__ PanelSmem carve(float* smem, int bigsz, int rc, int cc, int P, bool fused) {
@@ -472,6 +622,7 @@ __device__ PanelSmem carve(float* smem, int bigsz, int rc, int cc, int P, bool f
   p += (blockDim.x / 32) * (kPS + 4);
   p = reinterpret_cast<float*>(round_up(reinterpret_cast<uintptr_t>(p), 16));
   s.xr = fused ? p : nullptr;
+  s.ring = fused ? p + P * rc : nullptr;  // (rc is a multiple of 4)
   return s;
 }
 
@@ -501,6 +652,18 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
   const int ra = rbase + b * p.rc, rb = min(m, ra + p.rc);
   const int ca = k0 + 1 + b * p.cc, cb = min(n, ca + p.cc);
   float prev_taup = 0.f;  // tau of the previous step's right reflector
+  constexpr bool kRing = kRpt4 == 4;
+  __shared__ uint64_t ring_bar[kRingMax];
+  ColumnRing ring;
+  if constexpr (kRing) {
+    ring = ColumnRing{reinterpret_cast<float4*>(S.ring), reinterpret_cast<float4*>(S.big),
+                      reinterpret_cast<float4*>(S.xr), p.ring_own, p.ring_own + 2, p.ring_slot4, ring_bar, 0u, 0, p.st};
+    if (t == 0) {
+      for (int s = 0; s < ring.NS; s++) mbar_init(ring_bar + s, 1);
+      fence_proxy_async_smem();
+    }
+    __syncthreads();
+  }
   PMARK_K(12);
 
   for (int j = 0; j < p.nb; j++) {
@@ -509,6 +672,13 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
     // ---------------- S1: update column i on own rows, partial sums
     const int r_s = max(ra, i);
     const int nrow = max(0, rb - r_s);
+    if constexpr (kRing) {
+      const int c_s = max(ca, i + 1), sa = (i + 1) & ~3;
+      ring.waiting = min(ring.own, max(0, cb - c_s));
+      if (t == 0)
+        for (int cl = 0; cl < ring.waiting; cl++)
+          ring.ask(W + (size_t)(c_s + cl) * ldw + sa, cl, (m - sa + 3) >> 2);
+    }
     // Row i of Y (S.Yi), of VT (S.VTi) and the own rows of column i (S.pre,
     // indexed r - ra) were loaded by the previous step's S5; only the first
     // column of a panel loads here.  VT[i, j-1] is the previous right
@@ -551,7 +721,10 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
       }
     }
     PMARK(1);
-    if (!grid_sync(p.bar, p.P, p.st, 1)) return;
+    if (!grid_sync(p.bar, p.P, p.st, 1)) {
+      if constexpr (kRing) ring.drain(0);
+      return;
+    }
     PMARK(2);
 
     // ---------------- S2: column reflector
@@ -658,7 +831,10 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
       float* xp = p.xpart + (size_t)b * p.ldxp;
       float* red = reinterpret_cast<float*>(S.red);
       constexpr int kR = fx ? kRpt4 : 1;
-      fused_col_pass<kR, fused_cols(kR)>(W, ldw, m, sa, nq, c_s, ncol, ca, i, j, S.big, red, c1s, c2s, S.pre, tq, sq,
+      if constexpr (kRing)
+        fused_ring_pass<kR, 2>(ring, W, ldw, m, sa, nq, c_s, ncol, ca, i, j, S.big, red, c1s, c2s, S.pre, tq, sq, Y,
+                               ldn, S.YS, S.owncol, p.xrow, xp, corr);
+      else fused_col_pass<kR, fused_cols(kR)>(W, ldw, m, sa, nq, c_s, ncol, ca, i, j, S.big, red, c1s, c2s, S.pre, tq, sq,
                                          Y, ldn, S.YS, S.owncol, p.xrow, xp, corr);
       PMARK(5);
     } else {
@@ -1280,6 +1456,14 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
       pp.ldxp = w.ldxp;
     }
     size_t smem = panel_smem_bytes(std::max(m, n), pp.rc, pp.cc, kBidiagThreads, P, pp.rpt4 > 0);
+    pp.ring_own = pp.ring_slot4 = 0;
+    if (pp.rpt4 == 4) {  // the column ring: as many slots as the rest of the shared memory holds
+      pp.ring_slot4 = (m - ((k0 + 1) & ~3) + 3) >> 2;
+      const size_t slot = sizeof(float4) * (size_t)pp.ring_slot4;
+      const size_t rest = ctx->smem_optin > smem + 1024 ? ctx->smem_optin - smem - 1024 : 0;
+      pp.ring_own = (int)std::min<size_t>(kRingMax - 2, rest / slot);
+      smem += slot * pp.ring_own;
+    }
     pp.ucol_global = 0;
     if (smem > ctx->smem_optin && pp.rpt4 == 0) {
       pp.ucol_global = 1;
