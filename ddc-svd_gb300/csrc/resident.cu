@@ -138,6 +138,7 @@ template <int R, int K, int T>
 __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p) {
   constexpr int W = T / 32, R4 = R / 4;
   constexpr int B = R > 16 ? 32 : R > 8 ? 16 : 8;  // rows of the reduce-scatter
+  constexpr int NG = R > 16 ? 3 : 2;               // columns in shared memory swept together
   constexpr int U = T > 256 ? 6 : 11;              // slice loads in flight per thread
   // 24 rows leave no registers to poll from: barriers there (4096^2: stage 1 40.2 ms
   // against 43.1 polling; below 2432 rows 2048^2 takes 9.5 ms polling against 10.8)
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   static_assert(R % 4 == 0 && R <= 32, "rows come in float4s");
   extern __shared__ __align__(16) float4 s_a[];                 // [R4][S], then w and y of these columns
   __shared__ __align__(16) float s_x[R], s_u[R], s_z[R];        // own rows of x, u and of the right update
-  __shared__ float s_c1[R], s_red[W][B], s_sl[W][kResSlice], s_q[2], s_p[2];
+  __shared__ float s_c1[R], s_red[W][B], s_sl[W][kResSlice], s_q[2], s_p[2], s_row[kResSlice];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, b = blockIdx.x, P = gridDim.x;
   const bool main = t < T;
   const int mt = p.mt, nt = p.nt, S = p.S, r0 = b * R, ldw = p.ldw;
@@ -175,18 +176,19 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
         a[4 * q][k] = v.x; a[4 * q + 1][k] = v.y; a[4 * q + 2][k] = v.z; a[4 * q + 3][k] = v.w;
       }
   } else if (lane < R4) {
-    *reinterpret_cast<float4*>(s_x + 4 * lane) = load4(0, 4 * lane);
-    *reinterpret_cast<float4*>(s_z + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x = load4(0, 4 * lane);
+    if (b == 0 && lane == 0) x.x = 0.f;
+    *reinterpret_cast<float4*>(s_x + 4 * lane) = x;
+    *reinterpret_cast<float4*>(s_u + 4 * lane) = *reinterpret_cast<float4*>(s_z + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (t == 0) s_p[0] = s_p[1] = 0.f;
   __syncthreads();
   float rw[K];
 #pragma unroll
   for (int k = 0; k < K; k++) rw[k] = 0.f;
-  for (int c = t; main && c < S; c += T) s_w[c] = 0.f;
+  for (int c = t; main && c < S; c += T) s_w[c] = s_y[c] = 0.f;
   // i = -1: only the second sweep (nothing to update), for column 0
   for (int i = -1; i < p.cols; i++) {
-    const bool own = i >= r0 && i < r0 + R;  // row i is here
     if (i >= 0) {
       uint2* row = p.row + (i & 1) * p.ldr;
       const unsigned tag = p.tag0 + i;
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
         if (lane < nc) {
           const float y = tq * (wic + sq * s);
           put(p.y + c0 + lane, y, tag);
+          s_row[lane] = wic - y;
           if (c0 + lane > i + 1) n = ff_add_sq(n, wic - y);
         }
         n = warp_sum_ff(n);
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
       } else if (wid == 1 && lane < R) {
         const int r = r0 + lane;
         const float u = s_x[lane] * sq;
-        s_u[lane] = r > i ? u : 0.f;
+        s_u[lane] = u;
         if (r >= i && r < mt) p.W[r + (size_t)i * ldw] = r > i ? u : 1.f;
       }
       if (!kTag) {
@@ -297,19 +300,39 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
               s_w[c + u * T] = yw[C + u] - yw[u];
             }
         }
-        for (int c = c1; c < S; c += T) {
-          const float yc = s_y[c], wc = s_w[c];
-          const float vc = c > i + 1 ? wc : 0.f;
+        // (NG columns at a time share the reads of u; the updated entries are not
+        // written here but formed again in the second sweep: a read and a write
+        // less of the port that bounds both)
+        for (int c = c1; c < S; c += NG * T) {
+          float yc[NG], vc[NG];
+          const float4* col[NG];  // (beyond S: the first column again, times zero)
+#pragma unroll
+          for (int g = 0; g < NG; g++) {
+            const int cg = c + g * T;
+            const bool in = cg < S;
+            yc[g] = in ? s_y[cg] : 0.f;
+            vc[g] = in && cg > i + 1 ? s_w[cg] : 0.f;
+            col[g] = s_a + (in ? cg : c);
+          }
 #pragma unroll
           for (int q = 0; q < R4; q++) {
             const float4 uv = *reinterpret_cast<const float4*>(s_u + 4 * q);
-            float4 av = s_a[q * S + c];
-            av.x -= uv.x * yc; av.y -= uv.y * yc; av.z -= uv.z * yc; av.w -= uv.w * yc;
-            z[4 * q] += av.x * vc; z[4 * q + 1] += av.y * vc; z[4 * q + 2] += av.z * vc; z[4 * q + 3] += av.w * vc;
-            s_a[q * S + c] = av;
-            if (c == i + 1) {
-              s_c1[4 * q] = av.x; s_c1[4 * q + 1] = av.y; s_c1[4 * q + 2] = av.z; s_c1[4 * q + 3] = av.w;
+#pragma unroll
+            for (int g = 0; g < NG; g++) {
+              float4 av = col[g][q * S];
+              av.x -= uv.x * yc[g]; av.y -= uv.y * yc[g]; av.z -= uv.z * yc[g]; av.w -= uv.w * yc[g];
+              z[4 * q] += av.x * vc[g]; z[4 * q + 1] += av.y * vc[g];
+              z[4 * q + 2] += av.z * vc[g]; z[4 * q + 3] += av.w * vc[g];
             }
+          }
+        }
+        if (i + 1 < S && c1 == i + 1) {  // column i + 1, updated on the left
+          const float yc = s_y[i + 1];
+#pragma unroll
+          for (int q = 0; q < R4; q++) {
+            const float4 uv = *reinterpret_cast<const float4*>(s_u + 4 * q), av = s_a[q * S + i + 1];
+            s_c1[4 * q] = av.x - uv.x * yc; s_c1[4 * q + 1] = av.y - uv.y * yc;
+            s_c1[4 * q + 2] = av.z - uv.z * yc; s_c1[4 * q + 3] = av.w - uv.w * yc;
           }
         }
         __syncwarp();
@@ -341,8 +364,10 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
       } else {
         float beta, tp, sp;
         float x0[2];
-        const FF n2 = sum_records<kTag>(p.rn, P, tag, lane, wt, ok);
+        // (y first: it comes earlier than the norms, and the wait for it keeps 152 warps
+        // from polling the norms' words while they are written: 2048^2 9.8 -> 8.4 ms)
         ok = take<kTag, 2>(x0, tag, wt, [&](int u) { return (u ? p.y : row) + i + 1; }, [](int) { return true; }) && ok;
+        const FF n2 = sum_records<kTag>(p.rn, P, tag, lane, wt, ok);
         householder_ff(x0[0] - x0[1], n2, &beta, &tp, &sp);
         if (lane == 0) {
           s_p[0] = tp;
@@ -363,7 +388,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
           if (lane == 0) {
             const float z = (r0 + r > i) ? tp * (s_c1[r] + sp * s) : 0.f;
             s_z[r] = z;
-            s_x[r] = tp != 0.f ? s_c1[r] - z : s_c1[r];
+            s_x[r] = (r0 + r > i + 1) ? (tp != 0.f ? s_c1[r] - z : s_c1[r]) : 0.f;  // (rows below i + 1)
           }
         }
       }
@@ -378,30 +403,46 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
     const unsigned tag1 = p.tag0 + i1;
     const bool own1 = more && i1 >= r0 && i1 < r0 + R;
     if (main) {
-      for (int c = t; c < S; c += T) {
-        if (c <= i) continue;
-        const float vc = c > i1 ? s_w[c] * sp : tp != 0.f ? 1.f : 0.f;
-        if (own) p.W[i + (size_t)c * ldw] = vc;
-        float s = 0.f;
+      for (int c = t + (t <= i ? (i - t + T) / T * T : 0); c < S; c += NG * T) {
+        float vc[NG], yc[NG], s[NG];
+        float4* col[NG];
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          const int cg = c + g * T;
+          const bool in = cg < S;
+          vc[g] = in && cg > i1 ? s_w[cg] * sp : tp != 0.f ? 1.f : 0.f;
+          yc[g] = in ? s_y[cg] : 0.f;
+          s[g] = 0.f;
+          col[g] = s_a + (in ? cg : c);
+        }
 #pragma unroll
         for (int q = 0; q < R4; q++) {
+          const float4 uv = *reinterpret_cast<const float4*>(s_u + 4 * q);
           const float4 zv = *reinterpret_cast<const float4*>(s_z + 4 * q);
           const float4 xv = *reinterpret_cast<const float4*>(s_x + 4 * q);
-          float4 av = s_a[q * S + c];
-          av.x -= zv.x * vc; av.y -= zv.y * vc; av.z -= zv.z * vc; av.w -= zv.w * vc;
-          s_a[q * S + c] = av;
 #pragma unroll
-          for (int h = 0; h < 4; h++) s += (r0 + 4 * q + h > i1) ? el(av, h) * el(xv, h) : 0.f;
+          for (int g = 0; g < NG; g++) {
+            float4 av = col[g][q * S];
+            av.x -= uv.x * yc[g]; av.y -= uv.y * yc[g]; av.z -= uv.z * yc[g]; av.w -= uv.w * yc[g];
+            av.x -= zv.x * vc[g]; av.y -= zv.y * vc[g]; av.z -= zv.z * vc[g]; av.w -= zv.w * vc[g];
+            if (c + g * T < S) col[g][q * S] = av;
+            s[g] += av.x * xv.x + av.y * xv.y + av.z * xv.z + av.w * xv.w;
+          }
         }
-        if (more && c > i1) put(part + c, s, tag1);
-        if (own1) put(row1 + c, reinterpret_cast<const float*>(s_a + ((i1 - r0) >> 2) * S + c)[(i1 - r0) & 3], tag1);
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          const int cg = c + g * T;
+          if (!more || cg >= S) continue;
+          if (cg > i1) put(part + cg, s[g], tag1);
+          if (own1)
+            put(row1 + cg, reinterpret_cast<const float*>(s_a + ((i1 - r0) >> 2) * S + cg)[(i1 - r0) & 3], tag1);
+        }
       }
       float s[K];
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int c = S + t + k * T;
         rw[k] = c > i1 ? rw[k] * sp : (c == i1 && tp != 0.f) ? 1.f : 0.f;  // v
-        if (own && c > i && c < nt) p.W[i + (size_t)c * ldw] = rw[k];
         s[k] = 0.f;
       }
 #pragma unroll
@@ -410,11 +451,10 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
         const float4 xv = *reinterpret_cast<const float4*>(s_x + 4 * q);
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-          const float x = (r0 + 4 * q + h > i1) ? el(xv, h) : 0.f;
 #pragma unroll
           for (int k = 0; k < K; k++) {
             a[4 * q + h][k] -= el(zv, h) * rw[k];
-            s[k] += a[4 * q + h][k] * x;
+            s[k] += a[4 * q + h][k] * el(xv, h);
           }
         }
       }
@@ -434,9 +474,13 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
             }
           }
       }
+      if (wid == 1 && i >= 0) {  // the slice's part of the right reflector into row i
+        const int cc = (nt - i1 + P - 1) / P, c = i1 + b * cc + lane;
+        if (lane < cc && c < nt) p.W[i + (size_t)c * ldw] = c > i1 ? s_row[lane] * sp : tp != 0.f ? 1.f : 0.f;
+      }
     } else if (more) {
       FF n{0.f, 0.f};
-      if (lane < R && r0 + lane > i1) n = ff_add_sq(n, s_x[lane]);
+      if (lane < R) n = ff_add_sq(n, s_x[lane]);
       n = warp_sum_ff(n);
       if (lane < 2 && !lost) put(p.cn + 2 * b + lane, lane ? n.lo : n.hi, tag1);
     }
