@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kBatchBidiagThreads) batch_bidiag_kernel(const
   }
 }
 
-// Applies reflectors j = jhi-1 ... 0 to kCW columns held in registers (lane
+// Applies reflectors j = jhi-1 ... jlo to kCW columns held in registers (lane
 // owns rows lane + 32 k, k < KR).  Reflector j is the vector v(r) = vec(j, r)
 // for rows r >= j + shift (unit leading entry stored), zero above.  KR is the
 // problem's row count in 32-row slices (1, 2, 4 or 8), so small problems do
@@ -388,10 +388,10 @@ __global__ void __launch_bounds__(kBatchBidiagThreads) batch_bidiag_kernel(const
 // sums (17 shuffles instead of 5 per column).
 constexpr int kCW = 8;  // columns per warp at a time
 template <int KR, typename VecFn>
-__device__ __forceinline__ void apply_reflectors_regs(float (&c)[kCW][KR], int rows, int jhi, int shift,
+__device__ __forceinline__ void apply_reflectors_regs(float (&c)[kCW][KR], int rows, int jhi, int jlo, int shift,
                                                       const float* __restrict__ tau, VecFn vec, int lane) {
   const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4;
-  for (int j = jhi - 1; j >= 0; j--) {
+  for (int j = jhi - 1; j >= jlo; j--) {
     const float t = tau[j];
     if (t == 0.f) continue;
     float u[KR];
@@ -428,51 +428,59 @@ __device__ __forceinline__ void apply_reflectors_regs(float (&c)[kCW][KR], int r
   }
 }
 
-// Left side of one problem up to 256 rows: U_core = Q [Y; 0], kCW columns per
-// warp at a time in registers, left reflectors n-1 .. 0 (column j of R).
-template <int KR>
-__device__ void bx_left(float* Uc, int m, int n, const float* R, const float* tauq, int lane, int wid, int nw) {
-  for (int c0 = wid * kCW; c0 < n; c0 += nw * kCW) {
+// One side of one problem up to 256 rows: C (rows x n, its first n rows given,
+// the others zero) becomes H_0 ... H_nref-1 C, kCW columns per warp at a time in
+// registers.  Left (kRight false): reflector j is column j of W; right: row j from
+// column j + 1.  The reflectors come through shared memory in blocks, each a row
+// of odd length there: read as they lie, a right reflector is one sector per
+// entry from L2, or up to 32 words of one bank, and of the problems of 16 to 256
+// rows most of the work has W beyond the room (2048 of them: 1.86 -> 1.68 ms).
+template <int KR, bool kRight>
+__device__ void bx_side(float* C, int rows, int n, int nref, const float* __restrict__ W, int ldw,
+                        const float* __restrict__ tau, float* sm, int room, int lane, int wid, int nw) {
+  constexpr int shift = kRight ? 1 : 0;
+  const int ldt = rows | 1, nb = min(nref, room / ldt);
+  for (int base = 0; base < n; base += nw * kCW) {
+    const int c0 = base + wid * kCW;
     float c[kCW][KR];
 #pragma unroll
     for (int qq = 0; qq < kCW; qq++)
 #pragma unroll
       for (int k = 0; k < KR; k++) {
         const int r = lane + 32 * k, col = c0 + qq;
-        c[qq][k] = (col < n && r < n) ? Uc[r + (size_t)col * m] : 0.f;
+        c[qq][k] = (col < n && r < n) ? C[r + (size_t)col * rows] : 0.f;
       }
-    apply_reflectors_regs<KR>(c, m, n, 0, tauq, [&](int j, int r) { return R[r + (size_t)j * m]; }, lane);
+    for (int j1 = nref; j1 > 0; j1 -= nb) {
+      const int j0 = max(0, j1 - nb);
+      if (base == 0 || nb < nref) {  // (all of them stay for the next columns)
+        const int cnt = j1 - j0;
+        __syncthreads();
+        if (kRight) {
+          for (int x = threadIdx.x; x < cnt * rows; x += blockDim.x) {
+            const int r = x / cnt, j = x - r * cnt;
+            sm[j * ldt + r] = W[j0 + j + (size_t)r * ldw];
+          }
+        } else {
+          for (int x = threadIdx.x; x < cnt * rows; x += blockDim.x) {
+            const int j = x / rows, r = x - j * rows;
+            sm[j * ldt + r] = W[r + (size_t)(j0 + j) * ldw];
+          }
+        }
+        __syncthreads();
+      }
+      if (c0 < n)
+        apply_reflectors_regs<KR>(c, rows, j1, j0, shift, tau, [&](int j, int r) { return sm[(j - j0) * ldt + r]; },
+                                  lane);
+    }
 #pragma unroll
     for (int qq = 0; qq < kCW; qq++)
 #pragma unroll
       for (int k = 0; k < KR; k++) {
         const int r = lane + 32 * k, col = c0 + qq;
-        if (col < n && r < m) Uc[r + (size_t)col * m] = c[qq][k];
+        if (col < n && r < rows) C[r + (size_t)col * rows] = c[qq][k];
       }
   }
-}
-
-// Right side: V_core = P X, right reflectors n-3 .. 0 (row j of R from column j+1).
-template <int KR>
-__device__ void bx_right(float* Vc, int m, int n, const float* R, const float* taup, int lane, int wid, int nw) {
-  for (int c0 = wid * kCW; c0 < n; c0 += nw * kCW) {
-    float c[kCW][KR];
-#pragma unroll
-    for (int qq = 0; qq < kCW; qq++)
-#pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = lane + 32 * k, col = c0 + qq;
-        c[qq][k] = (col < n && r < n) ? Vc[r + (size_t)col * n] : 0.f;
-      }
-    apply_reflectors_regs<KR>(c, n, n - 2, 1, taup, [&](int j, int k) { return R[j + (size_t)k * m]; }, lane);
-#pragma unroll
-    for (int qq = 0; qq < kCW; qq++)
-#pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = lane + 32 * k, col = c0 + qq;
-        if (col < n && r < n) Vc[r + (size_t)col * n] = c[qq][k];
-      }
-  }
+  __syncthreads();  // (the next side or problem takes the room)
 }
 
 // U_core = Q [Y; 0], V_core = P X for one problem per CTA (multU / multV).
@@ -480,8 +488,7 @@ __device__ void bx_right(float* Vc, int m, int n, const float* R, const float* t
 // size-sorted order (a static round robin left the largest problems to the
 // last wave).  Problems up to 256 rows keep kCW columns per warp in
 // registers, sized to the problem's rows, and read the reflectors from
-// shared memory (or L1): one warp-wide reduction per reflector for kCW
-// columns at once.  Larger problems use the plain column loop (one column
+// shared memory: one warp-wide reduction per reflector for kCW columns at once.  Larger problems use the plain column loop (one column
 // per warp, in global memory).
 __global__ void __launch_bounds__(kBatchThreads) batch_backxform_kernel(const BatchTask* __restrict__ tasks,
                                                                         const int* __restrict__ order, int ntask,
@@ -501,7 +508,7 @@ __global__ void __launch_bounds__(kBatchThreads) batch_backxform_kernel(const Ba
     const int m = T.m, n = T.n;
     const bool fits = (long long)m * n <= smem_floats;
     const float* Wg = W + T.offW;
-    if (fits)
+    if (fits && m > 256)
       for (int idx = threadIdx.x; idx < m * n; idx += blockDim.x) sm[idx] = Wg[idx];
     const float* R = fits ? sm : Wg;
     // core U / V of a transposed problem are the caller's V / U
@@ -511,17 +518,18 @@ __global__ void __launch_bounds__(kBatchThreads) batch_backxform_kernel(const Ba
     const float* tauq = tq + T.offD;
     const float* taup = tp + T.offD;
     if (m <= 256) {
+      const int nr = n - 2;
       switch (row_slices(m)) {
-        case 1: bx_left<1>(Uc, m, n, R, tauq, lane, wid, nw); break;
-        case 2: bx_left<2>(Uc, m, n, R, tauq, lane, wid, nw); break;
-        case 4: bx_left<4>(Uc, m, n, R, tauq, lane, wid, nw); break;
-        default: bx_left<8>(Uc, m, n, R, tauq, lane, wid, nw); break;
+        case 1: bx_side<1, false>(Uc, m, n, n, Wg, m, tauq, sm, smem_floats, lane, wid, nw); break;
+        case 2: bx_side<2, false>(Uc, m, n, n, Wg, m, tauq, sm, smem_floats, lane, wid, nw); break;
+        case 4: bx_side<4, false>(Uc, m, n, n, Wg, m, tauq, sm, smem_floats, lane, wid, nw); break;
+        default: bx_side<8, false>(Uc, m, n, n, Wg, m, tauq, sm, smem_floats, lane, wid, nw); break;
       }
-      switch (row_slices(n)) {
-        case 1: bx_right<1>(Vc, m, n, R, taup, lane, wid, nw); break;
-        case 2: bx_right<2>(Vc, m, n, R, taup, lane, wid, nw); break;
-        case 4: bx_right<4>(Vc, m, n, R, taup, lane, wid, nw); break;
-        default: bx_right<8>(Vc, m, n, R, taup, lane, wid, nw); break;
+      if (nr > 0) switch (row_slices(n)) {
+        case 1: bx_side<1, true>(Vc, n, n, nr, Wg, m, taup, sm, smem_floats, lane, wid, nw); break;
+        case 2: bx_side<2, true>(Vc, n, n, nr, Wg, m, taup, sm, smem_floats, lane, wid, nw); break;
+        case 4: bx_side<4, true>(Vc, n, n, nr, Wg, m, taup, sm, smem_floats, lane, wid, nw); break;
+        default: bx_side<8, true>(Vc, n, n, nr, Wg, m, taup, sm, smem_floats, lane, wid, nw); break;
       }
     } else {
       // rows n..m-1 of [Y; 0]
@@ -739,7 +747,8 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
     DDC_TRY(bd_vectors(h, Ntot, P.store, P.b1, P.b2, sig_slot, &P.L, sig, c, false));
   }
   // ---- stage 5 and sigma
-  const size_t smem5 = sizeof(float) * (size_t)std::min<long long>(maxmn, smem_floats);
+  const int room5 = (int)std::min<long long>(maxmn + 512, smem_floats);  // (a reflector's odd length, and all of a small problem's)
+  const size_t smem5 = sizeof(float) * (size_t)room5;
   DDC_CUDA_TRY(cudaFuncSetAttribute(batch_backxform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)std::max<size_t>(smem5, 16)));
   ktimer_begin(h, KC_BACKXFORM);
@@ -747,7 +756,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
   DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ5, batch_backxform_kernel, kBatchThreads,
                                                             std::max<size_t>(smem5, 16)));
   batch_backxform_kernel<<<std::min(batch, h->num_sms * std::max(occ5, 1)), kBatchThreads, smem5, h->stream>>>(
-      dt, dord, batch, counter + 1, W, tq, tp, dU, dV, smem_floats);
+      dt, dord, batch, counter + 1, W, tq, tp, dU, dV, room5);
   count_launch();
   ktimer_end(h);
   batch_sigma_out_kernel<<<std::min(batch, 1024), 128, 0, h->stream>>>(dt, batch, P.L.sorted ? sig_slot : sig, dSigma);
