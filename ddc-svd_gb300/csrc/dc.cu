@@ -445,17 +445,24 @@ __device__ void dc_setup_node(const DcParams& p, int node, int par, const Grp& g
 // rounds with a constant mask, several sums to a round.  With the size and mask
 // read at run time and one loop per sum, the four sums of one FP32 evaluation
 // took most of its 2900 cycles (48 to 128 poles).  kG = 0: any size up to 16.
+//
+// kG = -V: any size, each lane with the terms of V lanes of a group V times as
+// large, V partial sums apart and then added in the order that group's reduction
+// has: the same bits.  V times as many roots share a warp's instructions for what
+// is done once per root (75 FP64 instructions a step, against 11 a term), which is
+// what a forest of many trees wants; a single tree has lanes to spare.
 template <int kG>
 struct LaneGroup {
   int G;          // lanes per group
   int lg;         // lane within the group
   unsigned mask;  // lanes of this group within the warp
-  __device__ __forceinline__ int size() const { return kG ? kG : G; }
+  static constexpr int kV = kG < 0 ? -kG : 1;
+  __device__ __forceinline__ int size() const { return kG > 0 ? kG : G; }
 };
 template <int kG>
 __device__ __forceinline__ LaneGroup<kG> make_group(int G, int lane) {
   LaneGroup<kG> g;
-  g.G = kG ? kG : G;
+  g.G = kG > 0 ? kG : G;
   g.lg = lane & (g.size() - 1);
   g.mask = (kG == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
   return g;
@@ -469,6 +476,37 @@ __device__ __forceinline__ void gsum(const LaneGroup<kG>& g, T&... v) {
   } else {
     for (int o = g.G >> 1; o > 0; o >>= 1) ((v += __shfl_xor_sync(g.mask, v, o)), ...);
   }
+}
+// acc: the group's sums of body over the terms 0 .. q - 1
+template <int kG, int N, typename T, class F>
+__device__ __forceinline__ void group_sums(const LaneGroup<kG>& g, int q, T (&acc)[N], F body) {
+  constexpr int V = LaneGroup<kG>::kV;
+  static_assert(N == 3 || N == 4, "");
+#pragma unroll
+  for (int u = 0; u < N; u++) acc[u] = T(0);
+  if constexpr (V == 1) {
+    for (int j = g.lg; j < q; j += g.size()) body(j, acc);
+  } else {
+    T part[V][N];
+#pragma unroll
+    for (int k = 0; k < V; k++)
+#pragma unroll
+      for (int u = 0; u < N; u++) part[k][u] = T(0);
+    for (int j = g.lg; j < q; j += V * g.size())
+#pragma unroll
+      for (int k = 0; k < V; k++)
+        if (k == 0 || j + k * g.size() < q) body(j + k * g.size(), part[k]);
+#pragma unroll
+    for (int h = V / 2; h > 0; h /= 2)
+#pragma unroll
+      for (int k = 0; k < h; k++)
+#pragma unroll
+        for (int u = 0; u < N; u++) part[k][u] += part[k + h][u];
+#pragma unroll
+    for (int u = 0; u < N; u++) acc[u] = part[0][u];
+  }
+  if constexpr (N == 4) gsum(g, acc[0], acc[1], acc[2], acc[3]);
+  else gsum(g, acc[0], acc[1], acc[2]);
 }
 // the product of v and the sum of e over the group
 template <int kG>
@@ -492,21 +530,20 @@ template <int kG>
 __device__ __forceinline__ void sec_eval(int q, const double* d, const double* z, double dorg,
                                          double tau, int split, const LaneGroup<kG>& g, double& f, double& psi,
                                          double& dpsi, double& phi, double& dphi) {
-  double ps = 0.0, dps = 0.0, ph = 0.0, dph = 0.0;
-  for (int j = g.lg; j < q; j += g.size()) {
+  double acc[4];
+  group_sums(g, q, acc, [&](int j, double (&a)[4]) {
     const double dj = d[j];
     const double del = (dj - dorg) * (dj + dorg) - tau;
     const double tt = quot_rn(z[j], del);
     // (the side's sums by selects: a branch here sent most warps down both sides)
     const bool le = j <= split;
-    const double a = (le ? ps : ph) + z[j] * tt, da = (le ? dps : dph) + tt * tt;
-    ps = le ? a : ps;
-    dps = le ? da : dps;
-    ph = le ? ph : a;
-    dph = le ? dph : da;
-  }
-  gsum(g, ps, dps, ph, dph);
-  psi = ps; dpsi = dps; phi = ph; dphi = dph;
+    const double v = (le ? a[0] : a[2]) + z[j] * tt, dv = (le ? a[1] : a[3]) + tt * tt;
+    a[0] = le ? v : a[0];
+    a[1] = le ? dv : a[1];
+    a[2] = le ? a[2] : v;
+    a[3] = le ? a[3] : dv;
+  });
+  psi = acc[0]; dpsi = acc[1]; phi = acc[2]; dphi = acc[3];
   f = 1.0 + psi + phi;
 }
 
@@ -528,17 +565,16 @@ template <bool kBits, int kG>
 __device__ __forceinline__ void sec_eval32(int q, const float2* d, const float* z, float2 dorg, float tau, int split,
                                            const LaneGroup<kG>& g, float& f, float& psi, float& dpsi, float& phi,
                                            float& dphi) {
-  float ps = 0.f, dps = 0.f, ph = 0.f, dph = 0.f;
-  for (int j = g.lg; j < q; j += g.size()) {
+  float acc[4];
+  group_sums(g, q, acc, [&](int j, float (&a)[4]) {
     const float2 dj = d[j];
     const float zj = z[j];
     const float del = (kBits ? dj.x - dorg.x : pair_diff(dj, dorg)) * (dj.x + dorg.x) - tau;
     const float tt = kBits ? zj / del : zj * rcp32(del);
-    if (j <= split) { ps += zj * tt; dps += tt * tt; }
-    else { ph += zj * tt; dph += tt * tt; }
-  }
-  gsum(g, ps, dps, ph, dph);
-  psi = ps; dpsi = dps; phi = ph; dphi = dph;
+    if (j <= split) { a[0] += zj * tt; a[1] += tt * tt; }
+    else { a[2] += zj * tt; a[3] += tt * tt; }
+  });
+  psi = acc[0]; dpsi = acc[1]; phi = acc[2]; dphi = acc[3];
   f = 1.f + psi + phi;
 }
 
@@ -668,8 +704,8 @@ template <int kG>
 __device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z, float2 dorg, float tau,
                                           const LaneGroup<kG>& g, float& f, float& err) {
   constexpr float e32 = FLT_EPSILON;
-  float s = 0.f, sa = 0.f, ea = 0.f;
-  for (int j = g.lg; j < q; j += g.size()) {
+  float acc[3];
+  group_sums(g, q, acc, [&](int j, float (&a)[3]) {
     const float2 dj = d[j];
     const float ad = fabsf(dj.x) + fabsf(dorg.x);
     const float dif = pair_diff(dj, dorg);
@@ -678,12 +714,12 @@ __device__ __forceinline__ void sec_mid32(int q, const float2* d, const float* z
     const float tt = z[j] * z[j] * ir;
     const float ed = 4.f * e32 * (fabsf(dif) * ad + fabsf(tau)) + 0x1p-44f * ad * ad;
     const float at = fabsf(tt), adel = fabsf(del);
-    s += tt;
-    sa += at;
-    ea += (ed < 0.5f * adel && adel >= 0x1p-100f && adel <= 0x1p100f) ? at * (2.5f * ed * fabsf(ir) + 6.f * e32)
-                                                                     : INFINITY;
-  }
-  gsum(g, s, sa, ea);
+    a[0] += tt;
+    a[1] += at;
+    a[2] += (ed < 0.5f * adel && adel >= 0x1p-100f && adel <= 0x1p100f) ? at * (2.5f * ed * fabsf(ir) + 6.f * e32)
+                                                                       : INFINITY;
+  });
+  const float s = acc[0], sa = acc[1], ea = acc[2];
   f = 1.f + s;
   err = ea + (float)(q + 2) * e32 * (1.f + sa);
 }
@@ -884,20 +920,32 @@ __device__ __forceinline__ void dc_zhat(const DcParams& p, int slot, int pos, in
   const double* tau = p.tau + slot;
   const double* dor = p.dor + slot;
   const double dj = dq[j];
-  double prod, pn = 1.0, pd = 1.0;
+  constexpr int V = LaneGroup<kG>::kV;
+  double prod, pn[V], pd = 1.0;
   int en = 0, ed = 0;
-  for (int k = g.lg; k < q - 1; k += g.size()) {
-    const double dk = dor[k], dd = dq[(k < j) ? k : k + 1];
-    const double num = tau[k] - (dj - dk) * (dj + dk);
-    const double den = (dd - dj) * (dd + dj);
-    if (kBits) {
-      pn *= quot_rn(num, den);
-    } else {
-      pn = take_exponent(pn * num, en);
-      pd = take_exponent(pd * den, ed);
+#pragma unroll
+  for (int v = 0; v < V; v++) pn[v] = 1.0;
+  for (int k0 = g.lg; k0 < q - 1; k0 += V * g.size()) {
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+      const int k = k0 + v * g.size();
+      if (v > 0 && k >= q - 1) continue;
+      const double dk = dor[k], dd = dq[(k < j) ? k : k + 1];
+      const double num = tau[k] - (dj - dk) * (dj + dk);
+      const double den = (dd - dj) * (dd + dj);
+      if (kBits) {
+        pn[v] *= quot_rn(num, den);
+      } else {
+        pn[v] = take_exponent(pn[v] * num, en);
+        pd = take_exponent(pd * den, ed);
+      }
     }
   }
-  prod = kBits ? pn : quot(pn, pd);
+#pragma unroll
+  for (int h = V / 2; h > 0; h /= 2)
+#pragma unroll
+    for (int v = 0; v < h; v++) pn[v] *= pn[v + h];
+  prod = kBits ? pn[0] : quot(pn[0], pd);
   int ex = en - ed;  // (0 with kBits)
   gprod(g, prod, ex);
   if (g.lg == 0) {
@@ -923,16 +971,17 @@ __device__ __forceinline__ void dc_rows(const DcParams& p, int slot, int pos, in
   const double* fq = p.fq + slot;
   const double* lq = p.lq + slot;
   const double dorg = p.dor[pos], ti = p.tau[pos];
-  double nv = 0.0, sf = 0.0, sl = 0.0;
-  for (int j = g.lg; j < q; j += g.size()) {
+  double acc[3];
+  group_sums(g, q, acc, [&](int j, double (&a)[3]) {
     const double dj = dq[j];
     const double del = (dj - dorg) * (dj + dorg) - ti;
     const double v = quotient<kBits>(zh[j], del);
-    nv += v * v;
-    sf += v * fq[j];
-    sl += v * lq[j];
-  }
-  gsum(g, nv, sf, sl);
+    a[0] += v * v;
+    a[1] += v * fq[j];
+    a[2] += v * lq[j];
+  });
+  double nv = acc[0];
+  const double sf = acc[1], sl = acc[2];
   if (g.lg == 0) {
     if (kBits) {
       nv = sqrt(nv);
@@ -1203,6 +1252,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) dc_tree_kernel(DcPar
   __shared__ int shi[40];
   __shared__ double shd[40];
   __shared__ int s_tree;
+  constexpr int kV = kThreads == kDcTreeSmall ? 2 : 4;
   const int t = threadIdx.x, wid = t >> 5, nw = blockDim.x >> 5;
   while (true) {
     if (t == 0) s_tree = atomicAdd(tr.counter, 1);
@@ -1240,7 +1290,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) dc_tree_kernel(DcPar
       __syncthreads();
       const int G = tr.seg_G[k];
       for (int ph = 0; ph < (rows ? 3 : 1); ph++) {  // secular roots, z-hat, rows
-        if (G == 32) dc_tree_phase<32>(p, tr.nodes, lo, mid, ph, d, G);
+        if (G >= kV) dc_tree_phase<-kV>(p, tr.nodes, lo, mid, ph, d, G / kV);
         else dc_tree_phase<0>(p, tr.nodes, lo, mid, ph, d, G);
         __syncthreads();
       }
