@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   constexpr int W = T / 32, R4 = R / 4;
   constexpr int B = R > 16 ? 32 : R > 8 ? 16 : 8;  // rows of the reduce-scatter
   constexpr int NG = R > 16 ? 3 : 2;               // columns in shared memory swept together
-  constexpr int U = T > 256 ? 6 : 11;              // slice loads in flight per thread
+  constexpr int U = T > 256 ? 6 : 22;              // slice loads in flight per thread (24 rows: all of them)
   // 24 rows leave no registers to poll from: barriers there (4096^2: stage 1 40.2 ms
   // against 43.1 polling; below 2432 rows 2048^2 takes 9.5 ms polling against 10.8)
   constexpr bool kTag = T > 256;
