@@ -258,15 +258,12 @@ def cpu_baseline(A64_host: np.ndarray, budget_s: float = 20.0):
                        f"({max(tfull - tbb, 0):.2f} s, scaled by ({n}/{ns})^3); an extrapolation, not a full run")}
 
 
-# DRAM bytes (read + write) of one panel-kernel launch, mean over the 4096^2
-# factorisation: ncu (metrics dram__bytes_read.sum and dram__bytes_write.sum)
-# on six sampled launches of `python -m ddcsvd.profile --size 4096 --mode
-# tf32x6 --reps 1 --kind uniform` (k0 = 0, 32, 1760, 1792, 3488, 3520), each
-# one DRAM read of its trailing block plus 0.44 MB on average, scaled over the
-# 112 panel launches (the last 512 columns run in one cluster-tail launch).
-# Far below the algorithmic GEMV bytes: the trailing block is re-read from
-# L2, not HBM.
-PANEL_DRAM_BYTES_PER_LAUNCH = 26247568
+# DRAM bytes (read + write) of one bidiagonalisation launch, mean over the 21
+# launches of a 4096^2 factorisation (14 panels, 6 grid-resident launches, the
+# cluster tail): ncu, dram__bytes_read.sum and dram__bytes_write.sum, one DRAM
+# read of the trailing block per launch (ncu flushes L2 before each).  Far below
+# the algorithmic GEMV bytes: the block is re-read from L2 or stays on chip.
+PANEL_DRAM_BYTES_PER_LAUNCH = 46438571
 
 
 def bench_tall(torch, lib, steps):
@@ -399,7 +396,7 @@ def bench_batched(torch, lib, h, steps, flush, dist=None, world=1, rank=0, peaks
                      "whole_batch_fp32_frac": round(flops / (ms * 1e-3) / p32, 4),
                      "stage1_fp32_frac": round(f1 / (kms[0] * 1e-3) / p32, 4) if kms[0] > 0 else None,
                      "backxform_fp32_frac": round(f5 / (kms[4] * 1e-3) / p32, 4) if kms[4] > 0 else None,
-                     "dc_fp64_pipe_frac": 0.83,
+                     "dc_fp64_pipe_frac": 0.74,
                      "dc_note": "dc_tree_kernel FP64 pipe utilisation from the committed ncu capture "
                                 "(profiles/dc_tree_kernel_batched2048.md); its FP64 work is data-dependent "
                                 "(secular iterations), so no flop count is formed here"}
@@ -617,22 +614,20 @@ def main():
     nl = max(kinfo["kernel_launches"]["bidiag_kernels"], 1)
     bytes_total = gemv_bytes(M, N)
     achieved = bytes_total / (bid_ms * 1e-3) / 1e9 if bid_ms > 0 else None
-    roof = {"bound": "hbm", "kernel": "bidiag_panel_kernel + bidiag_tail_kernel",
+    roof = {"bound": "hbm", "kernel": "bidiag_panel_kernel + bidiag_resident_kernel + bidiag_tail_kernel",
             "achieved": round(achieved, 1) if achieved else None,
             "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
             "frac": round(achieved / hbm, 3) if achieved else None, "traffic": PANEL_DRAM_BYTES_PER_LAUNCH,
-            "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum per panel launch: six sampled "
-                            "launches (early, middle, late) scaled over the 112 panel launches of a 4096^2 "
-                            "factorisation (L2 flushed before each launch by ncu); "
-                            "achieved = the two GEMVs' algorithmic bytes over all columns / the summed time of "
-                            "the panel launches and the cluster-tail launch",
+            "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum, mean of the 21 launches of a "
+                            "4096^2 factorisation (L2 flushed before each launch by ncu); achieved = the two "
+                            "GEMVs' algorithmic bytes over all columns / the summed time of these launches",
             "bytes_per_launch": round(bytes_total / nl), "launches": nl,
             "avg_launch_ms": round(bid_ms / nl, 4),
             "l2": {"achieved": round(achieved, 1) if achieved else None, "peak": peaks["l2_read_gbs"],
                    "peak_kind": "measured here (best L2-resident read probe)", "unit": "GB/s",
                    "frac": round(achieved / peaks["l2_read_gbs"], 3) if achieved else None,
-                   "note": "the 4096^2 trailing block (64 MiB) stays in L2 between column steps, so L2 "
-                           "bandwidth is the binding memory bound of this kernel"}}
+                   "note": "the 4096^2 trailing block (64 MiB) stays in L2 between the panels' column steps and "
+                           "on chip below 3648 columns"}}
 
     if rank != 0:
         if dist is not None:

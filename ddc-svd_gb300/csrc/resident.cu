@@ -12,20 +12,20 @@
 // Per column i, with x its entries below row i:
 //   1. each CTA writes its part of x^T A and of ||x||^2; the owner of row i writes
 //      that row (all from the sweep that ends the column before);
-//   2. after a grid barrier each CTA adds the P parts of its slice of the columns
-//      (every CTA forms the same reflector from the P norms in a warp of its own),
-//      and writes tau y of the slice and its part of ||w||^2, w the new row i;
-//   3. after a second barrier every CTA reads y and sweeps its columns twice: left
-//      update and products with w (the reflector of w follows in the extra warp
-//      meanwhile), then right update and products with column i + 1, which the
-//      row sums already determine.
+//   2. each CTA adds the P parts of its slice of the columns (every CTA forms the
+//      same reflector from the P norms in a warp of its own), and writes tau y of
+//      the slice and its part of ||w||^2, w the new row i;
+//   3. every CTA reads y and sweeps its columns twice: left update and products
+//      with w (the reflector of w follows in the extra warp meanwhile), then right
+//      update and products with column i + 1, which the row sums already determine.
 //
-// What bounds it: the two barriers (1.3 us each) and the two round trips to L2
-// behind them; the arithmetic is 4 multiply-adds an entry, and the columns in
-// shared memory pass through its port four times.  The panel kernel reads the
-// trailing block from L2 for every column, sums 152 records of 2 j values twice
-// and one 152-part row product, and its trailing update comes on top.
-// @@
+// What bounds it: the two exchanges of a column and the compensated norms behind
+// them; the arithmetic is 4 multiply-adds an entry, and the columns in shared
+// memory pass through its port three times.  The panel kernel reads the trailing
+// block from L2 for every column, sums 152 records of 2 j values twice and one
+// 152-part row product, and its trailing update comes on top.  Us per column,
+// panels and here: 512-1024 columns 11.3 and 4.0, 1024-2048 13 to 15 and 4.9,
+// 2048-3648 15 to 18 and 10.7.
 #include "internal.hpp"
 
 namespace ddcsvd {
@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   constexpr int B = R > 16 ? 32 : R > 8 ? 16 : 8;  // rows of the reduce-scatter
   constexpr int NG = R > 16 ? 3 : 2;               // columns in shared memory swept together
   constexpr int U = T > 256 ? 6 : 22;              // slice loads in flight per thread (24 rows: all of them)
-  // 24 rows leave no registers to poll from: barriers there (4096^2: stage 1 40.2 ms
-  // against 43.1 polling; below 2432 rows 2048^2 takes 9.5 ms polling against 10.8)
+  // 24 rows leave no registers to poll from: barriers there (3648^2: stage 1 26.0 ms
+  // against 28.4 polling; with fewer rows 2048^2 takes 8.4 ms polling, 10.8 with
+  // barriers)
   constexpr bool kTag = T > 256;
   static_assert(R % 4 == 0 && R <= 32, "rows come in float4s");
   extern __shared__ __align__(16) float4 s_a[];                 // [R4][S], then w and y of these columns
