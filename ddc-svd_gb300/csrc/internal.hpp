@@ -187,6 +187,7 @@ int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P);
 size_t bidiag_resident_words(int m, int n, int P, int* ld);
 int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* W, int ldw, float* d, float* e,
                     float* tauq, float* taup, const BidiagWork& w);
+int tail_cluster_size(ddcsvd_context* ctx);  // CTAs of the largest cluster the GPU co-schedules (16, 8 or 0)
 int bidiag_tail_columns(ddcsvd_context* ctx, int m, int n, int k0);
 int bidiag_tail(ddcsvd_context* ctx, int m, int n, int k0, float* W, int ldw, float* d, float* e, float* tauq,
                 float* taup);

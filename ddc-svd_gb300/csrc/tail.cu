@@ -437,7 +437,7 @@ static const void* tail_kernel(int R, int K) {
 }
 
 // Cluster size the device can co-schedule (16, else 8, else 0), cached.
-static int tail_cluster_size(ddcsvd_context* ctx) {
+int tail_cluster_size(ddcsvd_context* ctx) {
   if (ctx->tail_cluster >= 0) return ctx->tail_cluster;
   int best = 0;
   for (int c : {16, 8}) {
