@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(T + 32, 1) bidiag_resident_kernel(ResParams p)
   constexpr int B = R > 16 ? 32 : R > 8 ? 16 : 8;  // rows of the reduce-scatter
   constexpr int NG = R > 16 ? 3 : 2;               // columns in shared memory swept together
   constexpr int U = T > 256 ? 6 : 22;              // slice loads in flight per thread (24 rows: all of them)
-  // 24 rows leave no registers to poll from: barriers there (3648^2: stage 1 26.0 ms
+  // 20 and 24 rows leave no registers to poll from: barriers there (3648^2: stage 1 26.0 ms
   // against 28.4 polling; with fewer rows 2048^2 takes 8.4 ms polling, 10.8 with
   // barriers)
   constexpr bool kTag = T > 256;
@@ -522,12 +522,13 @@ size_t res_smem(const ResConfig& g, int nt) {
 // The smallest configuration that has the rows and keeps all but a few columns in
 // registers, else the largest with the rest of them in shared memory.  Up to 16
 // rows run on 15 + 1 warps (128 registers a thread; 16 + 1 leave 96, and 16 x 4
-// entries then spill: 2048^2 12.0 ms against 11.3), 24 on 7 + 1 (255).
+// entries then spill: 2048^2 12.0 ms against 11.3), 20 and 24 on 7 + 1 (255;
+// 2900^2 16.6 ms with 24 alone, 16.1 with 20 before it).
 const ResConfig* res_config(int mt, int nt, int P, size_t smem_max) {
   static const ResConfig tab[] = {res_entry<8, 2, 480>(),  res_entry<8, 3, 480>(),  res_entry<8, 4, 480>(),
                                   res_entry<12, 2, 480>(), res_entry<12, 3, 480>(), res_entry<12, 4, 480>(),
                                   res_entry<16, 2, 480>(), res_entry<16, 3, 480>(), res_entry<16, 4, 480>(),
-                                  res_entry<24, 7, 224>()};
+                                  res_entry<20, 7, 224>(), res_entry<24, 7, 224>()};
   for (const ResConfig& g : tab)
     if ((long long)g.R * P >= mt && nt <= kResSlice * P && res_smem(g, nt) <= smem_max &&
         (g.K < 4 ? nt <= g.K * g.T + 64 : true))

@@ -1,5 +1,5 @@
 """The grid-resident columns of the bidiagonalisation at the edges of their
-configurations (8, 12, 16 or 24 rows per CTA, columns in registers and in shared
+configurations (8, 12, 16, 20 or 24 rows per CTA, columns in registers and in shared
 memory, hand-over to the cluster tail), and next to shapes that start in the
 panels."""
 import numpy as np
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("m,n", [(513, 513), (514, 513), (545, 544), (1216, 520), (1217, 1024), (1024, 1024),
                                  (1025, 1025), (1216, 1216), (1300, 1217), (1824, 600), (1825, 1025), (2432, 700), (2433, 540), (2048, 2048),
-                                 (2049, 2049), (2500, 1800), (3648, 900), (3649, 600), (2700, 2600)])
+                                 (2049, 2049), (2500, 1800), (3648, 900), (3649, 600), (2700, 2600), (3040, 560), (3041, 580)])
 @pytest.mark.parametrize("kind", ["normal", "rank"])
 def test_resident_edges(lib, cuda, m, n, kind):
     rng = np.random.default_rng(m * 7 + n)
