@@ -117,9 +117,16 @@ __host__ __device__ inline long long ut_offset(int b, int rows_total) {
 // 1.3 ms for an 8192-row block.  NB = 32 (QR panels) or 128 (QR super-blocks
 // and the back-transformation: half the passes over C of 64-reflector blocks).
 constexpr int kPrepRows = 32;    // rows per shared-memory tile
-constexpr int kChunkRows = 512;  // rows per CTA of the chunked kernels (many blocks)
-constexpr int kChunkRowsFew = 128;  // the same when a call has at most two blocks (QR panels / super-blocks)
-__host__ __device__ inline int wy_chunk_rows(int nblk) { return nblk <= 2 ? kChunkRowsFew : kChunkRows; }
+constexpr int kChunkRows = 512;     // rows per CTA of the chunked kernels
+constexpr int kChunkRowsFew = 128;  // the same when a call has few blocks (QR panels, a thousand columns)
+constexpr int kChunkFill = 152;     // CTAs (one per SM)
+// 128 rows where 512 would leave much of the GPU idle: a launch has blocks x chunks
+// CTAs, and those above the diagonal return at once (1500 x 1001: 24 CTAs of 152; with
+// the conflict-free reads below its SVD and product take 5.48 ms instead of 5.97,
+// 1100 x 900 likewise 10% less; 4096^2 fills the GPU with 512).
+inline int wy_chunk_rows(int nblk, int rows) {
+  return nblk <= 2 || nblk * ceil_div(rows, kChunkRows) < kChunkFill ? kChunkRowsFew : kChunkRows;
+}
 constexpr int kWYT = 128;        // reflectors per WY block of the tensor-core back-transformation
 
 template <int NB>
@@ -140,6 +147,10 @@ __device__ __forceinline__ void wy_load_tile(float (*sU)[NB + 1], const float* U
 }
 
 // 256 threads as 16 x 16, each an (NB/16) x (NB/16) tile of G.
+// A thread holds (NB / 16)^2 entries, 16 apart in both directions: the lanes of a
+// half warp then read neighbouring words of a row of U (side by side in groups
+// of NB / 16 they met in the same banks, 4 ways for NB = 128, and the kernel was
+// bound by shared memory, not by its multiply-adds).
 template <int NB>
 __global__ void __launch_bounds__(256) wy_gram_kernel(int rows_total, int nref, const float* __restrict__ Uc, int ldu,
                                                       float* Gp, int nchunk, int chunk) {
@@ -166,8 +177,8 @@ __global__ void __launch_bounds__(256) wy_gram_kernel(int rows_total, int nref, 
       float x[R], y[R];
 #pragma unroll
       for (int a = 0; a < R; a++) {
-        x[a] = sU[k][R * ti + a];
-        y[a] = sU[k][R * tj + a];
+        x[a] = sU[k][ti + 16 * a];
+        y[a] = sU[k][tj + 16 * a];
       }
 #pragma unroll
       for (int a = 0; a < R; a++)
@@ -179,7 +190,7 @@ __global__ void __launch_bounds__(256) wy_gram_kernel(int rows_total, int nref, 
 #pragma unroll
   for (int a = 0; a < R; a++)
 #pragma unroll
-    for (int c = 0; c < R; c++) G[(R * ti + a) + (size_t)(R * tj + c) * NB] = acc[a][c];
+    for (int c = 0; c < R; c++) G[(ti + 16 * a) + (size_t)(tj + 16 * c) * NB] = acc[a][c];
 }
 
 // G of every block: the chunk partials of each entry added in chunk order
@@ -261,7 +272,11 @@ __global__ void __launch_bounds__(256) wy_ut_kernel(int rows_total, int nref, co
   float* out = UT + ut_offset<NB>(blockIdx.x, rows_total);
   const int t = threadIdx.x;
   const float* T = Tin + (size_t)blockIdx.x * NB * NB;
-  for (int idx = t; idx < NB * NB; idx += blockDim.x) sT[idx % NB][idx / NB] = T[idx];
+  for (int idx = t; idx < NB * NB / 4; idx += blockDim.x) {  // four k of a column at a time: neighbouring lanes, neighbouring banks
+    const int c = idx % NB, k = idx / NB * 4;
+    const float4 v = *reinterpret_cast<const float4*>(T + k + (size_t)c * NB);
+    sT[k][c] = v.x; sT[k + 1][c] = v.y; sT[k + 2][c] = v.z; sT[k + 3][c] = v.w;
+  }
   const int cg = t % CG, rg = t / CG;
   for (int r0 = c0; r0 < c1; r0 += kPrepRows) {
     __syncthreads();
@@ -294,7 +309,7 @@ __global__ void __launch_bounds__(256) wy_ut_kernel(int rows_total, int nref, co
 template <int NB = kWY>
 static size_t wy_scratch_floats(int rows_total, int nref) {
   const int nblk = ceil_div(std::max(nref, 1), NB);
-  const int nchunk = ceil_div(std::max(rows_total, 1), wy_chunk_rows(nblk));
+  const int nchunk = ceil_div(std::max(rows_total, 1), wy_chunk_rows(nblk, rows_total));
   return (size_t)nblk * nchunk * NB * NB + 2 * (size_t)nblk * NB * NB + 64;
 }
 
@@ -302,7 +317,7 @@ template <int NB>
 static int wy_prepare_all(ddcsvd_context* ctx, int rows_total, int nref, const float* Uc, int ldu, const float* tau,
                           float* UT, bool transT, float* scratch, bool with_ut = true) {
   const int nblk = ceil_div(nref, NB);
-  const int chunk = wy_chunk_rows(nblk);
+  const int chunk = wy_chunk_rows(nblk, rows_total);
   const int nchunk = ceil_div(rows_total, chunk);
   float* Gp = scratch;
   float* G = scratch + (size_t)nblk * nchunk * NB * NB;
@@ -403,8 +418,8 @@ __global__ void __launch_bounds__(256) wy_xgram_kernel(int rows_total, int nref,
         float x[R], y[R];
 #pragma unroll
         for (int q = 0; q < R; q++) {
-          x[q] = sA[k][R * ti + q];
-          y[q] = sB[k][R * tj + q];
+          x[q] = sA[k][ti + 16 * q];
+          y[q] = sB[k][tj + 16 * q];
         }
 #pragma unroll
         for (int q = 0; q < R; q++)
@@ -417,7 +432,7 @@ __global__ void __launch_bounds__(256) wy_xgram_kernel(int rows_total, int nref,
 #pragma unroll
   for (int q = 0; q < R; q++)
 #pragma unroll
-    for (int c = 0; c < R; c++) X[(R * ti + q) + (size_t)(R * tj + c) * NB] = acc[q][c];
+    for (int c = 0; c < R; c++) X[(ti + 16 * q) + (size_t)(tj + 16 * c) * NB] = acc[q][c];
 }
 
 // X of every pair: the chunk partials added in chunk order (thread per entry).
@@ -431,8 +446,8 @@ __global__ void __launch_bounds__(256) wy_xsum_kernel(const float* __restrict__ 
   X[(size_t)blockIdx.y * NB * NB + idx] = g;
 }
 
-// T_ab = -T_a X T_b for one pair per CTA (256 threads, each an 8 x 8 tile of
-// the 128 x 128 result); sTa, sX and sTb in dynamic shared memory.
+// T_ab = -T_a X T_b for one pair per CTA (256 threads, each 8 x 8 entries
+// of the 128 x 128 result, 16 apart as in wy_gram_kernel); sTa, sX and sTb in dynamic shared memory.
 __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* __restrict__ T, const float* __restrict__ X,
                                                         float* Tab) {
   constexpr int NB = kWYT, R = NB / 16;
@@ -468,8 +483,8 @@ __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* _
     float x[R], y[R];
 #pragma unroll
     for (int q = 0; q < R; q++) {
-      x[q] = sX[R * ti + q][k];
-      y[q] = sTb[k][R * tj + q];
+      x[q] = sX[ti + 16 * q][k];
+      y[q] = sTb[k][tj + 16 * q];
     }
 #pragma unroll
     for (int q = 0; q < R; q++)
@@ -480,7 +495,7 @@ __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* _
 #pragma unroll
   for (int q = 0; q < R; q++)
 #pragma unroll
-    for (int c = 0; c < R; c++) sX[R * ti + q][R * tj + c] = acc[q][c];
+    for (int c = 0; c < R; c++) sX[ti + 16 * q][tj + 16 * c] = acc[q][c];
   __syncthreads();
   // T_ab = -T_a Y
 #pragma unroll
@@ -491,8 +506,8 @@ __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* _
     float x[R], y[R];
 #pragma unroll
     for (int q = 0; q < R; q++) {
-      x[q] = sTa[R * ti + q][k];
-      y[q] = sX[k][R * tj + q];
+      x[q] = sTa[ti + 16 * q][k];
+      y[q] = sX[k][tj + 16 * q];
     }
 #pragma unroll
     for (int q = 0; q < R; q++)
@@ -502,23 +517,26 @@ __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* _
 #pragma unroll
   for (int q = 0; q < R; q++)
 #pragma unroll
-    for (int c = 0; c < R; c++) out[(R * ti + q) + (size_t)(R * tj + c) * NB] = -acc[q][c];
+    for (int c = 0; c < R; c++) out[(ti + 16 * q) + (size_t)(tj + 16 * c) * NB] = -acc[q][c];
 }
 
 // UT of every pair, row-major with 256 columns over rows [j0, rows_total):
 // half 0 (columns 0-127) = U_a T_a, half 1 = U_a T_ab + U_b T_b, i.e. the
 // rows of [U_a U_b] times the half's 256 x 128 slice of the pair's T (grid
-// (pair, row chunk, half); sU [32][257] and the slice in dynamic shared
+// (pair, row chunk, half); sU [64][260] and the slice in dynamic shared
 // memory).  256 threads in 32 column groups of 4 columns and 8 row groups of
-// 4 rows of a 32-row tile, as wy_ut_kernel.
+// 8 rows of a 64-row tile: per four k a thread reads 8 broadcast float4s of U
+// and 4 of T for 128 multiply-adds, which then bound it (one k and four rows at
+// a time: 8 reads' worth of the shared-memory port for 16 multiply-adds).
+constexpr int kUtRows = 64;
+constexpr int kUtLd = kPairNB + 4;
 __global__ void __launch_bounds__(256) wy_ut2_kernel(int rows_total, int nref, const float* __restrict__ Uc, int ldu,
                                                      const float* __restrict__ T, const float* __restrict__ Tab,
                                                      float* UT2, int chunk) {
-  constexpr int NB = kWYT, KP = kPairNB, CG = NB / 4, RPT = 4;
-  static_assert(256 / CG * RPT == kPrepRows, "row groups must cover the tile");
+  constexpr int NB = kWYT, KP = kPairNB, CG = NB / 4, RPT = kUtRows * CG / 256;
   extern __shared__ __align__(16) float wsm[];
-  float(*sU)[KP + 1] = reinterpret_cast<float(*)[KP + 1]>(wsm);
-  float(*sT)[NB] = reinterpret_cast<float(*)[NB]>(wsm + kPrepRows * (KP + 1));
+  float(*sU)[kUtLd] = reinterpret_cast<float(*)[kUtLd]>(wsm);
+  float(*sT)[NB] = reinterpret_cast<float(*)[NB]>(wsm + kUtRows * kUtLd);
   const int p = blockIdx.x, half = blockIdx.z, t = threadIdx.x;
   int j0, bsa, bsb;
   pair_geom(p, nref, j0, bsa, bsb);
@@ -531,38 +549,44 @@ __global__ void __launch_bounds__(256) wy_ut2_kernel(int rows_total, int nref, c
   const float* Ta = T + (size_t)(2 * p) * NB * NB;
   const float* Tb = T + (size_t)(2 * p + 1) * NB * NB;
   const float* Tx = Tab + (size_t)p * NB * NB;
-  for (int idx = t; idx < kin * NB; idx += blockDim.x) {
-    const int k = idx % kin, c = idx / kin;
-    float v;
-    if (half == 0) v = Ta[k + (size_t)c * NB];
-    else v = (k < NB) ? Tx[k + (size_t)c * NB] : Tb[(k - NB) + (size_t)c * NB];
-    sT[k][c] = v;
+  for (int idx = t; idx < kin * NB / 4; idx += blockDim.x) {
+    const int c = idx % NB, k = idx / NB * 4;
+    const float* src = half == 0 ? Ta + k : k < NB ? Tx + k : Tb + (k - NB);
+    const float4 v = *reinterpret_cast<const float4*>(src + (size_t)c * NB);
+    sT[k][c] = v.x; sT[k + 1][c] = v.y; sT[k + 2][c] = v.z; sT[k + 3][c] = v.w;
   }
   const int cg = t % CG, rg = t / CG;
+  const int nuse = bsa + (half == 0 ? 0 : bsb);  // b has columns only where a is full
   float* out = UT2 + ut2_offset(p, rows_total);
-  for (int r0 = c0; r0 < c1; r0 += kPrepRows) {
+  for (int r0 = c0; r0 < c1; r0 += kUtRows) {
     __syncthreads();
-    for (int idx = t; idx < kPrepRows * kin; idx += blockDim.x) {
-      const int rr = idx & (kPrepRows - 1), k = idx / kPrepRows;
-      const int r = r0 + rr;
-      const int bs = (k < NB) ? bsa : bsb;
-      const int col = j0 + k;  // reflector index (b's columns follow a's)
-      sU[rr][k] = (r < c1 && (k % NB) < bs) ? Uc[r + (size_t)col * ldu] : 0.f;
+#pragma unroll 2
+    for (int idx = t; idx < kUtRows * kin / 4; idx += blockDim.x) {
+      const int rr = idx % kUtRows, k = idx / kUtRows * 4, r = r0 + rr;
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] = (r < c1 && k + q < nuse) ? Uc[r + (size_t)(j0 + k + q) * ldu] : 0.f;
+      *reinterpret_cast<float4*>(&sU[rr][k]) = make_float4(v[0], v[1], v[2], v[3]);
     }
     __syncthreads();
     float4 acc[RPT];
 #pragma unroll
     for (int q = 0; q < RPT; q++) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int k = 0; k < kin; k++) {
-      const float4 y = *reinterpret_cast<const float4*>(&sT[k][4 * cg]);
+    for (int k = 0; k < kin; k += 4) {
+      float4 y[4];
+#pragma unroll
+      for (int h = 0; h < 4; h++) y[h] = *reinterpret_cast<const float4*>(&sT[k + h][4 * cg]);
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
-        const float x = sU[rg * RPT + q][k];
-        acc[q].x += x * y.x;
-        acc[q].y += x * y.y;
-        acc[q].z += x * y.z;
-        acc[q].w += x * y.w;
+        const float4 u = *reinterpret_cast<const float4*>(&sU[rg * RPT + q][k]);
+        const float x[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          acc[q].x += x[h] * y[h].x;
+          acc[q].y += x[h] * y[h].y;
+          acc[q].z += x[h] * y[h].z;
+          acc[q].w += x[h] * y[h].w;
+        }
       }
     }
 #pragma unroll
@@ -573,14 +597,14 @@ __global__ void __launch_bounds__(256) wy_ut2_kernel(int rows_total, int nref, c
   }
 }
 
-static size_t ut2_smem_bytes() { return sizeof(float) * ((size_t)kPrepRows * (kPairNB + 1) + (size_t)kPairNB * kWYT); }
+static size_t ut2_smem_bytes() { return sizeof(float) * ((size_t)kUtRows * kUtLd + (size_t)kPairNB * kWYT); }
 
 void bx_plan(int rows_total, int nref, int ncols, GemmKind kind, Arena& a, BxPrepared* out) {
   constexpr int NB = kWYT;
   BxPrepared& w = *out;
   w.ldu = (int)round_up(rows_total, 32);
   const int npair = ceil_div(std::max(nref, 1), kPairNB);
-  const int nchunk = ceil_div(std::max(rows_total, 1), kChunkRows);
+  const int nchunk = ceil_div(std::max(rows_total, 1), wy_chunk_rows(npair, rows_total));
   w.Uc = a.take<float>((size_t)w.ldu * std::max(nref, 1));
   w.UT = a.take<float>((size_t)ut2_offset(npair, rows_total) + 64);
   w.W1s = a.take<float>((size_t)kPairNB * ncols + 64);
@@ -601,15 +625,16 @@ int bx_prepare(ddcsvd_context* ctx, int side, int rows_total, int nref, const fl
   // T of every 128-block (wy_prepare_all's layout: Gram partials, G, then T)
   DDC_TRY(wy_prepare_all<NB>(ctx, rows_total, nref, w.Uc, w.ldu, tau, nullptr, false, w.wys, false));
   const int nblk = ceil_div(nref, NB);
-  const int nchunk_g = ceil_div(rows_total, wy_chunk_rows(nblk));
+  const int nchunk_g = ceil_div(rows_total, wy_chunk_rows(nblk, rows_total));
   const float* T = w.wys + (size_t)nblk * nchunk_g * NB * NB + (size_t)nblk * NB * NB;
   const int npair = ceil_div(nref, kPairNB);
-  const int nchunk = ceil_div(rows_total, kChunkRows);
+  const int chunk = wy_chunk_rows(npair, rows_total);
+  const int nchunk = ceil_div(rows_total, chunk);
   float* Xp = w.wys + wy_scratch_floats<NB>(rows_total, nref);
   float* X = Xp + (size_t)npair * nchunk * NB * NB;
   float* Tab = X + (size_t)npair * NB * NB;
   wy_xgram_kernel<<<dim3(npair, nchunk), 256, 0, ctx->stream>>>(rows_total, nref, w.Uc, w.ldu, Xp, nchunk,
-                                                                kChunkRows);
+                                                                chunk);
   wy_xsum_kernel<<<dim3(ceil_div(NB * NB, 256), npair), 256, 0, ctx->stream>>>(Xp, nchunk, X);
   const int tm_smem = 3 * NB * (NB + 1) * (int)sizeof(float);
   DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)wy_tmerge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -619,7 +644,7 @@ int bx_prepare(ddcsvd_context* ctx, int side, int rows_total, int nref, const fl
   DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)wy_ut2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     ut_smem));
   wy_ut2_kernel<<<dim3(npair, nchunk, 2), 256, ut_smem, ctx->stream>>>(rows_total, nref, w.Uc, w.ldu, T, Tab, w.UT,
-                                                                      kChunkRows);
+                                                                      chunk);
   count_launch(4);
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;
