@@ -209,39 +209,90 @@ __global__ void __launch_bounds__(256) wy_gsum_kernel(int rows_total, int nref, 
   G[(size_t)blockIdx.y * NB * NB + idx] = g;
 }
 
-// 4 * NB threads, four per row of T; sG and sT in dynamic shared memory
-// (2 NB (NB + 1) floats).
+// A column-major NB x NB matrix from L2 into rows of NB + 1 floats: four rows of a
+// column per load, neighbouring lanes in neighbouring columns (and banks).
+template <int NB>
+__device__ __forceinline__ void wy_load_square(float (*dst)[NB + 1], const float* __restrict__ src) {
+#pragma unroll 8
+  for (int idx = threadIdx.x; idx < NB * NB / 4; idx += blockDim.x) {
+    const int c = idx % NB, r = idx / NB * 4;
+    const float4 v = *reinterpret_cast<const float4*>(src + r + (size_t)c * NB);
+    dst[r][c] = v.x; dst[r + 1][c] = v.y; dst[r + 2][c] = v.z; dst[r + 3][c] = v.w;
+  }
+}
+
+// T of neighbouring diagonal blocks a and b of W reflectors joined, for all pairs
+// of them: T_ab = -T_a G_ab T_b (4 NB threads; a thread W / 8 entries of a column).
+template <int NB, int W>
+__device__ __forceinline__ void wy_join(float (*sT)[NB + 1], float (*sG)[NB + 1]) {
+  constexpr int E = W / 8;
+  const int u = threadIdx.x % (8 * W), a0 = threadIdx.x / (8 * W) * 2 * W, b0 = a0 + W;
+  const int c = u % W, r = u / W;
+  float v[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) v[e] = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < W; k++) {
+    const float y = sT[b0 + k][b0 + c];
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] += sG[a0 + r + 8 * e][b0 + k] * y;
+  }
+#pragma unroll
+  for (int e = 0; e < E; e++) sT[a0 + r + 8 * e][b0 + c] = v[e];
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; e++) v[e] = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < W; k++) {
+    const float y = sT[a0 + k][b0 + c];
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] += sT[a0 + r + 8 * e][a0 + k] * y;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; e++) sT[a0 + r + 8 * e][b0 + c] = -v[e];
+  __syncthreads();
+}
+
+// 4 * NB threads; sG and sT in dynamic shared memory (2 NB (NB + 1) floats).  A row
+// of T depends on itself alone, T[r, l] = -tau_l T[r, r:l] G[r:l, l], so a lane
+// keeps its row of a 32 x 32 diagonal block in registers and needs no one else;
+// the blocks are then joined, 32 to 64 to 128.  (Column by column over the CTA, a
+// barrier each, a block of 128 took 66 us; this 21.)
 template <int NB>
 __global__ void __launch_bounds__(4 * NB) wy_tfactor_kernel(int rows_total, int nref, const float* __restrict__ tau,
                                                             const float* __restrict__ G, float* Tout, int transT) {
+  static_assert(NB == 32 || NB == 64 || NB == 128, "blocks of 32, joined");
   extern __shared__ float wsm[];
   float(*sG)[NB + 1] = reinterpret_cast<float(*)[NB + 1]>(wsm);
   float(*sT)[NB + 1] = reinterpret_cast<float(*)[NB + 1]>(wsm + NB * (NB + 1));
   int j0, bs, rows;
   wy_block_geom<NB>(blockIdx.x, rows_total, nref, j0, bs, rows);
   if (bs <= 0 || rows <= 0) return;
-  const int t = threadIdx.x;
-  const float* Gb = G + (size_t)blockIdx.x * NB * NB;
-  for (int idx = t; idx < NB * NB; idx += blockDim.x) {
-    const int r = idx % NB, c = idx / NB;
-    sG[r][c] = Gb[idx];
-    sT[r][c] = 0.f;
-  }
+  const int t = threadIdx.x, lane = t & 31;
+  for (int idx = t; idx < NB * (NB + 1); idx += blockDim.x) sT[0][idx] = 0.f;
+  wy_load_square<NB>(sG, G + (size_t)blockIdx.x * NB * NB);
   __syncthreads();
-  {  // column l from the finished columns 0..l-1; four threads per row
-    const int row = t >> 2, part = t & 3;
-    for (int l = 0; l < bs; l++) {
-      float sum = 0.f;
-      if (row < l)
-        for (int k = row + part; k < l; k += 4) sum += sT[row][k] * sG[k][l];
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      const float tl = tau[j0 + l];
-      if (part == 0 && row < l) sT[row][l] = -tl * sum;
-      if (t == 0) sT[l][l] = tl;
-      __syncthreads();
+  if (t < NB) {
+    const int d0 = t & ~31;
+    const float tl = d0 + lane < bs ? tau[j0 + d0 + lane] : 0.f;
+    float row[32];
+#pragma unroll
+    for (int l = 0; l < 32; l++) {
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int k = 0; k < l; k++) {
+        if (k & 1) s1 += row[k] * sG[d0 + k][d0 + l];
+        else s0 += row[k] * sG[d0 + k][d0 + l];
+      }
+      const float tc = __shfl_sync(0xffffffffu, tl, l);
+      row[l] = lane < l ? -tc * (s0 + s1) : lane == l ? tc : 0.f;
+      sT[d0 + lane][d0 + l] = row[l];
     }
   }
+  __syncthreads();
+  if constexpr (NB >= 64) wy_join<NB, 32>(sT, sG);
+  if constexpr (NB >= 128) wy_join<NB, 64>(sT, sG);
   // T (or T^T for a block applied as a transpose) to global, [row + col * NB]
   float* T = Tout + (size_t)blockIdx.x * NB * NB;
   for (int idx = t; idx < NB * NB; idx += blockDim.x) {
@@ -466,12 +517,9 @@ __global__ void __launch_bounds__(256) wy_tmerge_kernel(int nref, const float* _
   const float* Ta = T + (size_t)(2 * p) * NB * NB;  // [r + c NB]
   const float* Tb = T + (size_t)(2 * p + 1) * NB * NB;
   const float* Xg = X + (size_t)p * NB * NB;
-  for (int idx = t; idx < NB * NB; idx += blockDim.x) {
-    const int r = idx % NB, c = idx / NB;
-    sTa[r][c] = Ta[idx];
-    sX[r][c] = Xg[idx];
-    sTb[r][c] = Tb[idx];
-  }
+  wy_load_square<NB>(sTa, Ta);
+  wy_load_square<NB>(sX, Xg);
+  wy_load_square<NB>(sTb, Tb);
   __syncthreads();
   float acc[R][R];
   // Y = X T_b
