@@ -451,11 +451,17 @@ static int bgemm(ddcsvd_context* ctx, int batch, const BGemm<double>& g0, const 
 // us of kernels with cold caches (bound by shared-memory reads), the call 111 ->
 // 78 us.  Rows of every matrix are an odd number of floats apart, so
 // walks along rows and along columns both spread over the banks.
-constexpr int kFusedThreads = 256;
+constexpr int kFusedThreadsMax = 512;
 static size_t fused_floats(int m, int n) {
   const size_t ld = (size_t)(n | 1);
   return 2 * m * ld + 4 * n * ld + n;
 }
+
+// 512 threads where the m x n products have a tile for each: shared memory holds one
+// or two such problems per SM, and 8 warps each leave its latency open (call on 400 x
+// (128 x 64) 172 -> 135 us, 1500 x (200 x 60) 748 -> 580, 20 x (150 x 80) 122 -> 100).
+// Smaller problems fill the SM with CTAs of 256 (1500 x (64 x 32) 101 us, 122 with 512).
+static int fused_threads(int m, int n) { return ceil_div(m, 4) * ceil_div(n, 4) >= 512 ? 512 : 256; }
 
 // out(i, j) for i < MI, j < NJ in 4 x 4 register tiles: sum over q < K of a(i, q) b(q, j)
 template <typename FA, typename FB, typename FO>
@@ -491,11 +497,11 @@ __device__ __forceinline__ void fused_product(int MI, int NJ, int K, int t0, int
   }
 }
 
-__global__ void __launch_bounds__(kFusedThreads) adjoint_fused_kernel(int m, int n, BMat<float> U, const float* S,
+__global__ void __launch_bounds__(kFusedThreadsMax) adjoint_fused_kernel(int m, int n, BMat<float> U, const float* S,
                                                                       BMat<float> V, BMat<float> gU, const float* gS,
                                                                       BMat<float> gV, float* gA) {
   extern __shared__ __align__(16) float fsm[];
-  const int t = threadIdx.x, ld = n | 1;
+  const int t = threadIdx.x, nt = blockDim.x, ld = n | 1;
   const long long b = blockIdx.x;
   float* sU = fsm;
   float* sP = sU + m * ld;  // gU, then P
@@ -508,7 +514,7 @@ __global__ void __launch_bounds__(kFusedThreads) adjoint_fused_kernel(int m, int
     if (!x.p) return;
     const float* p = x.p + b * x.b;
     const bool rfast = x.r == 1 && x.c != 1;
-    for (int idx = t; idx < rows * n; idx += kFusedThreads) {
+    for (int idx = t; idx < rows * n; idx += nt) {
       const int r = rfast ? idx % rows : idx / n, c = rfast ? idx / rows : idx % n;
       dst[r * ld + c] = p[r * x.r + c * x.c];
     }
@@ -517,20 +523,20 @@ __global__ void __launch_bounds__(kFusedThreads) adjoint_fused_kernel(int m, int
   load(sP, gU, m);
   load(sV, V, n);
   load(sW, gV, n);
-  for (int c = t; c < n; c += kFusedThreads) ss[c] = S[b * n + c];
+  for (int c = t; c < n; c += nt) ss[c] = S[b * n + c];
   __syncthreads();
   // J = U^T gU on one half of the threads, K = V^T gV on the other
-  constexpr int h = kFusedThreads / 2;
+  const int h = nt / 64 * 32;
   if (t < h) {
     if (gU.p)
       fused_product(n, n, m, t, h, [&](int i, int q) { return sU[q * ld + i]; },
                     [&](int q, int j) { return sP[q * ld + j]; }, [&](int i, int j, float v) { sJ[i * ld + j] = v; });
   } else if (gV.p) {
-    fused_product(n, n, n, t - h, h, [&](int i, int q) { return sV[q * ld + i]; },
+    fused_product(n, n, n, t - h, nt - h, [&](int i, int q) { return sV[q * ld + i]; },
                   [&](int q, int j) { return sW[q * ld + j]; }, [&](int i, int j, float v) { sK[i * ld + j] = v; });
   }
   __syncthreads();
-  for (int idx = t; idx < n * n; idx += kFusedThreads) {  // M in place of J, a pair at a time
+  for (int idx = t; idx < n * n; idx += nt) {  // M in place of J, a pair at a time
     const int i = idx / n, j = idx % n;
     if (i > j) continue;
     const float si = ss[i], sj = ss[j];
@@ -556,12 +562,12 @@ __global__ void __launch_bounds__(kFusedThreads) adjoint_fused_kernel(int m, int
     sJ[j * ld + i] = vji;
   }
   __syncthreads();
-  fused_product(m, n, n, t, kFusedThreads, [&](int i, int q) { return sU[i * ld + q]; },
+  fused_product(m, n, n, t, nt, [&](int i, int q) { return sU[i * ld + q]; },
                 [&](int q, int j) { return sJ[q * ld + j]; },
                 [&](int i, int j, float v) { sP[i * ld + j] = gU.p ? v + sP[i * ld + j] / ss[j] : v; });
   __syncthreads();
   float* out = gA + b * m * n;
-  fused_product(m, n, n, t, kFusedThreads, [&](int i, int q) { return sP[i * ld + q]; },
+  fused_product(m, n, n, t, nt, [&](int i, int q) { return sP[i * ld + q]; },
                 [&](int q, int j) { return sV[j * ld + q]; },
                 [&](int i, int j, float v) { out[i + (size_t)j * m] = v; });
 }
@@ -645,7 +651,7 @@ static int svd_backward_f32(ddcsvd_context* h, int batch, int m, int n, BMat<flo
   DDC_TRY(reset_status(h));
   DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)adjoint_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)bytes));
-  adjoint_fused_kernel<<<batch, kFusedThreads, bytes, h->stream>>>(m, n, U, S, V, gU, gS, gV, gA);
+  adjoint_fused_kernel<<<batch, fused_threads(m, n), bytes, h->stream>>>(m, n, U, S, V, gU, gS, gV, gA);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   return check_status(h, "svd_backward");
