@@ -258,12 +258,12 @@ def cpu_baseline(A64_host: np.ndarray, budget_s: float = 20.0):
                        f"({max(tfull - tbb, 0):.2f} s, scaled by ({n}/{ns})^3); an extrapolation, not a full run")}
 
 
-# DRAM bytes (read + write) of one bidiagonalisation launch, mean over the 21
-# launches of a 4096^2 factorisation (14 panels, 6 grid-resident launches, the
+# DRAM bytes (read + write) of one bidiagonalisation launch, mean over the 22
+# launches of a 4096^2 factorisation (14 panels, 7 grid-resident launches, the
 # cluster tail): ncu, dram__bytes_read.sum and dram__bytes_write.sum, one DRAM
 # read of the trailing block per launch (ncu flushes L2 before each).  Far below
 # the algorithmic GEMV bytes: the block is re-read from L2 or stays on chip.
-PANEL_DRAM_BYTES_PER_LAUNCH = 46438571
+PANEL_DRAM_BYTES_PER_LAUNCH = 45927889
 
 
 def bench_tall(torch, lib, steps):
@@ -618,7 +618,7 @@ def main():
             "achieved": round(achieved, 1) if achieved else None,
             "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
             "frac": round(achieved / hbm, 3) if achieved else None, "traffic": PANEL_DRAM_BYTES_PER_LAUNCH,
-            "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum, mean of the 21 launches of a "
+            "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum, mean of the 22 launches of a "
                             "4096^2 factorisation (L2 flushed before each launch by ncu); achieved = the two "
                             "GEMVs' algorithmic bytes over all columns / the summed time of these launches",
             "bytes_per_launch": round(bytes_total / nl), "launches": nl,
