@@ -49,6 +49,7 @@ namespace ddcsvd {
 constexpr int kTailThreads = 256;
 constexpr int kTailWarps = kTailThreads / 32;
 constexpr int kTailMaxC = 16;
+constexpr int kEx1Bars = 2;  // barriers of exchange 1 (the kernel says why not one)
 
 struct TailParams {
   int mt, nt;  // trailing block: rows, columns (mt >= nt)
@@ -164,9 +165,14 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
   __shared__ float s_part[kTailWarps][32 * K];  // per warp: products of the next column with every column
   __shared__ FF s_nw[kTailWarps];               // per warp: ||x||^2 of the own rows
   __shared__ float s_own[32 * K];               // row i, in the CTA that holds it
-  // exchange 1, by column parity: a CTA may send column i + 1's records while
-  // a slower one still reads column i's (never i + 2's: it has then received
-  // something that every CTA sends after its last read of column i)
+  // exchange 1, records and barrier by column parity.  A CTA may send column
+  // i + 1's records to one that still reads column i's, or still waits for some
+  // of them: it has come through exchange 2 of column i, for which the owners of
+  // the slices left needed every CTA's record of column i at themselves, but
+  // nobody needed it at a CTA without a slice.  On one barrier its bytes would
+  // count for those still missing.  It cannot send column i + 2's: the owners
+  // then had that CTA's record of column i + 1, sent after its last read of
+  // column i.
   __shared__ __align__(16) float s_in[2][kTailMaxC][32];  // partial products of the own slice by sender
   __shared__ __align__(16) float s_row[2][32];            // row i of the own slice
   __shared__ __align__(16) FF s_n1[2][kTailMaxC];         // ||x||^2 by sender
@@ -175,7 +181,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
   // the previous column's)
   __shared__ __align__(16) float2 s_yw[32 * K];  // (tau y, w) of every column
   __shared__ __align__(16) FF s_n2[kTailMaxC];   // ||w||^2 over the columns > i + 1 by slice
-  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ __align__(8) uint64_t s_bar[kEx1Bars + 1];  // exchange 1 by column parity, exchange 2
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -183,13 +189,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
   const int GW = kTailWarps * C, gw = wid * C + rank;  // row r: warp r mod GW, slot r / GW
   const int c_own = 32 * rank + lane;                  // the lane's column of the CTA's slice
   const int slice_cols = min(32, nt - 32 * rank);      // (<= 0: no slice)
-  const uint32_t bar1 = smem_u32(&s_bar[0]), bar2 = smem_u32(&s_bar[1]);
+  const uint32_t bar0 = smem_u32(&s_bar[0]), bar2 = smem_u32(&s_bar[kEx1Bars]);
   // a shared address of this CTA plus such a difference is the same place in
   // CTA lane's / CTA (wid + 8 j)'s shared memory
-  const uint32_t to_lane = map_rank(bar1, min(lane, C - 1)) - bar1;
+  const uint32_t to_lane = map_rank(bar0, min(lane, C - 1)) - bar0;
   uint32_t to_cta[NT];
 #pragma unroll
-  for (int j = 0; j < NT; j++) to_cta[j] = map_rank(bar1, min(wid + 8 * j, C - 1)) - bar1;
+  for (int j = 0; j < NT; j++) to_cta[j] = map_rank(bar0, min(wid + 8 * j, C - 1)) - bar0;
   bool dead = false;
 
   float A[R][K];
@@ -217,8 +223,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
   for (int q = t; q < 2 * kTailMaxC * 32; q += kTailThreads) (&s_in[0][0][0])[q] = 0.f;
   if (t < 2 * kTailMaxC) (&s_n1[0][0])[t] = FF{0.f, 0.f};
   if (t == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
+    for (int q = 0; q <= kEx1Bars; q++) mbar_init(&s_bar[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   cluster.sync();  // every CTA runs and is ready before the first remote store
@@ -226,16 +231,18 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
   int islot = 0, iwarp = 0;  // slot and warp of row i
   for (int i = 0; i < nt; i++) {
     const int b = i & 1;
-    const unsigned ph = (unsigned)(i & 1);  // both barriers complete one phase per column
+    const uint32_t bar1 = smem_u32(&s_bar[b]);
+    const unsigned ph1 = (unsigned)(i >> 1) & 1u;  // a phase of it every other column
+    const unsigned ph2 = (unsigned)b;              // and of exchange 2's in each
     const int kf = (i + 1) >> 5;            // first slice with a column > i
     const bool mine = gw == iwarp;          // this warp holds row i
     // ---- exchange 1: products of column i, its norm, row i
     if (t == 0) {
       unsigned bytes = 8u * C + 4u;
       if (rank >= kf && slice_cols > 0) bytes += 4u * (C + 1) * slice_cols;
-      mbar_arrive_expect_tx(&s_bar[0], bytes);
+      mbar_arrive_expect_tx(&s_bar[b], bytes);
       if (i < nt - 1)
-        mbar_arrive_expect_tx(&s_bar[1], 8u * (unsigned)((nt + 31) / 32 - kf) + 8u * (unsigned)(nt - 32 * kf));
+        mbar_arrive_expect_tx(&s_bar[kEx1Bars], 8u * (unsigned)((nt + 31) / 32 - kf) + 8u * (unsigned)(nt - 32 * kf));
     }
 #pragma unroll
     for (int k = 0; k < K; k++) s_part[wid][lane + 32 * k] = acc[k];
@@ -278,7 +285,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
         if (holds) st_async(smem_u32(&s_x0[b]) + to_lane, s_own[i], bar1 + to_lane);
       }
     }
-    tail_wait(bar1, ph, dead, p.st);
+    tail_wait(bar1, ph1, dead, p.st);
     // ---- left reflector, and exchange 2: tau y and the new row of the own
     // slice (every warp forms them; warp w sends them to the CTAs w, w + 8)
     float alpha, tq, sq, w = 0.f;
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
       if (lane < R && r >= i && r < mt) p.W[r + (size_t)i * ldw] = (r == i) ? 1.f : v;
     }
     if (i == nt - 1) break;
-    tail_wait(bar2, ph, dead, p.st);
+    tail_wait(bar2, ph2, dead, p.st);
     // ---- right reflector (every warp); row i of W
     float tp = 0.f, sp = 0.f;
     {
