@@ -120,29 +120,45 @@ __global__ void __launch_bounds__(256) bgemm_kernel(BGemm<T> g0, BGemm<T> g1, in
 // The Ozaki scheme (Ozaki, Ogita, Oishi, Rump, "Error-free transformations of
 // matrix multiplication", Numer. Algorithms 59, 2012; on FP16 tensor cores:
 // Mukunoki, Ozaki, Ogita, Imamura, ISC 2020): every row of A and column of B is
-// scaled by a power of two and rounded to a 54-bit integer, the integer written
-// in seven signed base-256 digits, and each pair of digit matrices multiplied in
-// FP16 with FP32 accumulation.  Digits are at most 128 in magnitude, so a sum of
-// up to seven pairs over K = 128 stays below 2^24 and every accumulation is
-// exact; the 34 pairs of weight 256^12 .. 256^5 are kept and put together in
-// 64-bit integers.  What is lost is the rounding to 54 bits of a row's or
-// column's largest entry and the pairs below, together below the rounding
-// errors of an FP64 sum of the same products (against quadruple precision, the
-// adjoint of 128 x 64, 200 x 100 and 16 x 16 problems is 2.7e-16, 3.0e-16 and
-// 2.2e-16 off, where FP64 sums gave 5.3e-16, 6.5e-16 and 2.8e-16).  Rows or columns that hold Inf or NaN take plain
-// FP64 sums.  The FP64 pipe bounded the direct form (0.98 ms for the four
-// products of 256 x (128 x 64), 0.85 ms at cuBLAS's DGEMM rate); this one is
-// bound by the tensor pipe and the digit extraction (integer instructions).
+// scaled by a power of two and rounded to a 62-bit integer, the integer written
+// in eight signed base-256 digits, and each pair of digit matrices multiplied in
+// FP16 with FP32 accumulation.  Digits are at most 128 in magnitude (the first
+// 64), so a sum of up to eight pairs over K = 128 stays below 2^24 and every
+// accumulation is exact; the 36 pairs of weight 256^14 .. 256^7 are kept and put
+// together in 64-bit integers.
+//
+// What is lost, the pairs below and the bits beyond 62, is relative to the
+// largest entries of the row and of the column: about 2^-59 sqrt(K) of their
+// product.  An FP64 sum keeps the bits of each of its products, however small
+// beside those entries, so the digits stand in for it only where they are as
+// good: the first digits' magnitudes are multiplied too, and an element whose
+// sum of |a| |b| falls below 2^-11 sqrt(K) of the product of the largest entries
+// (where the loss reaches four roundings of that sum) is formed as an FP64 sum
+// after all -- by its warp, or by the CTA where a tile has more than a few of them
+// or holds Inf or NaN.  (Seven digits of 54 bits without that test lost the
+// columns of an unevenly scaled problem: A = X diag(scale) with V near the
+// identity, 8 decades, 3e-9 of a column instead of 5e-16.)  Against extended
+// precision the worst column of the adjoint is 0.3 to 1 times as far off as with
+// FP64 sums, for even and graded values, V or U near the identity, and each
+// gradient alone.
+//
+// The FP64 pipe bounded the direct form (0.98 ms for the four products of 256 x
+// (128 x 64), 0.85 ms at cuBLAS's DGEMM rate); this one is bound by the tensor
+// pipe and the digit extraction (integer instructions).
 //
 // 64 x 32 tile per CTA, eight warps of 16 x 16, two CTAs per SM (one extracts
 // digits while the other multiplies), K in slabs of 32 through two stages.
 constexpr int kOzThreads = 256;
 constexpr int kOzM = 64, kOzN = 32, kOzK = 32;           // tile, slab
-constexpr int kOzD = 7, kOzS = 8;                        // digits, diagonals
-constexpr int kOzLd = kOzK + 8;                          // halves per staged row: ldmatrix rows on distinct banks
+constexpr int kOzD = 8, kOzS = 8;                        // digits, diagonals
 constexpr int kOzChunk = 128;                            // K per exact accumulation
-constexpr int kOzStage = kOzD * (kOzM + kOzN) * kOzLd;   // halves per stage: A's digits, then B's
+constexpr int kOzStage = kOzD * (kOzM + kOzN) * kOzK;    // halves per stage: A's digits, then B's
 constexpr int kOzSmem = 2 * kOzStage * (int)sizeof(__half);
+constexpr int kOzFew = 64;                               // elements of a tile that warps sum in FP64 one by one
+
+// Place of the eight halves k .. k + 7 of a staged row: rows are 64 bytes, their
+// 16-byte parts exchanged so that eight rows of ldmatrix meet distinct banks.
+__device__ __forceinline__ int oz_at(int row, int k) { return row * kOzK + ((((k >> 3) ^ (row >> 1)) & 3) << 3); }
 
 // One operand of the tile: R rows (of A, or columns of B) by K.
 struct OzOp {
@@ -191,22 +207,22 @@ __device__ __forceinline__ bool oz_max(const OzOp& o, int* e) {  // exponents of
   }
   return bad;
 }
-// v 2^(54 - e) rounded to an integer, where |v| < 2^e, plus 128 in each of the
-// seven low bytes: byte t is then digit t + 128
+// v 2^(62 - e) rounded to an integer, where |v| < 2^e, plus 128 in each byte:
+// byte t is then digit t + 128
 __device__ __forceinline__ unsigned long long oz_digits(double v, int e) {
   const long long b = __double_as_longlong(v);
   const int ex = (int)((b >> 52) & 0x7ff);
   unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
   if (ex) m |= 0x10000000000000ull;
-  const int sh = (ex ? ex : 1) - 1075 + 54 - e;  // at most 1
+  const int sh = (ex ? ex : 1) - 1075 + 62 - e;  // at most 9
   unsigned long long x;
   if (sh >= 0) x = m << sh;
   else if (sh > -64) x = (m + (1ull << (-sh - 1))) >> -sh;
   else x = 0;
-  return (b < 0 ? 0ull - x : x) + 0x0080808080808080ull;
+  return (b < 0 ? 0ull - x : x) + 0x8080808080808080ull;
 }
 // digits of one slab into a stage: digit d (0 = most significant) of row r at
-// dst + (d R + r) kOzLd + k
+// dst + oz_at(d R + r, k)
 template <int R>
 __device__ __forceinline__ void oz_stage(const OzOp& o, const int* e, int k0, __half* dst) {
   for (int u = threadIdx.x; u < 4 * R; u += kOzThreads) {
@@ -218,7 +234,7 @@ __device__ __forceinline__ void oz_stage(const OzOp& o, const int* e, int k0, __
     unsigned long long y[8];
 #pragma unroll
     for (int h = 0; h < 8; h++) y[h] = oz_digits(v[h], er);
-    __half* q = dst + r * kOzLd + k;
+    __half* q = dst + oz_at(r, k);
 #pragma unroll
     for (int d = 0; d < kOzD; d++) {
       const int t = kOzD - 1 - d;  // byte
@@ -233,7 +249,7 @@ __device__ __forceinline__ void oz_stage(const OzOp& o, const int* e, int k0, __
         const __half2 hv = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2half2(__ushort_as_half(0x6480)));
         w[h] = *reinterpret_cast<const unsigned*>(&hv);
       }
-      *reinterpret_cast<uint4*>(q + d * R * kOzLd) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(q + d * R * kOzK) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
 }
@@ -250,11 +266,51 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// the same on magnitudes, FP16 sums (infinite beyond its range)
+__device__ __forceinline__ void mma16816_abs(unsigned (&c)[2], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  constexpr unsigned m = 0x7fff7fffu;
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3, %4, %5}, {%6, %7}, {%0, %1};"
+      : "+r"(c[0]), "+r"(c[1])
+      : "r"(a[0] & m), "r"(a[1] & m), "r"(a[2] & m), "r"(a[3] & m), "r"(b0 & m), "r"(b1 & m));
+}
+
+// The tile's eight elements of a thread as FP64 sums, k ascending; `sm` holds a
+// slab of both operands.
+__device__ __forceinline__ void oz_plain(const OzOp& A, const OzOp& B, double* sm, int lr, int lc, double (&run)[8]) {
+  double(*sa)[kOzM + 1] = reinterpret_cast<double(*)[kOzM + 1]>(sm);
+  double(*sb)[kOzN + 1] = reinterpret_cast<double(*)[kOzN + 1]>(sm + kOzK * (kOzM + 1));
+  static_assert(kOzThreads == 4 * kOzM, "a unit of A per thread");
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int x = 0; x < 8; x++) run[x] = 0.0;
+  for (int k0 = 0; k0 < A.K; k0 += kOzK) {
+    double v[8];
+    int r, k;
+    __syncthreads();
+    oz_load<kOzM>(A, k0, t, v);
+    oz_place<kOzM>(A, t, r, k);
+#pragma unroll
+    for (int h = 0; h < 8; h++) sa[k + h][r] = v[h];
+    if (t < 4 * kOzN) {
+      oz_load<kOzN>(B, k0, t, v);
+      oz_place<kOzN>(B, t, r, k);
+#pragma unroll
+      for (int h = 0; h < 8; h++) sb[k + h][r] = v[h];
+    }
+    __syncthreads();
+    for (k = 0; k < min(kOzK, A.K - k0); k++)
+#pragma unroll
+      for (int x = 0; x < 8; x++)
+        run[x] = fma(sa[k][lr + 8 * ((x >> 1) & 1)], sb[k][lc + 8 * (x >> 2) + (x & 1)], run[x]);
+  }
+}
+
 __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0, BGemm<double> g1, int batch) {
   extern __shared__ __align__(16) __half ozm[];  // [stage][A digits, B digits]
   __shared__ int s_ea[kOzM], s_eb[kOzN];         // exponent bound of each row of A / column of B
   __shared__ double s_rs[kOzN];                  // 1 / s of each column
-  __shared__ int s_bad;
+  __shared__ int s_bad, s_weak;
   const bool first = (int)blockIdx.z < batch;
   const BGemm<double>& g = first ? g0 : g1;
   const int b = first ? blockIdx.z : blockIdx.z - batch;
@@ -266,13 +322,13 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
   // ---- exponent of the largest entry of each row / column
   if (t < kOzM) s_ea[t] = 1;
   if (t < kOzN) s_eb[t] = 1;
-  if (t == 0) s_bad = 0;
+  if (t == 0) s_bad = s_weak = 0;
   __syncthreads();
   const bool bada = oz_max<kOzM>(A, s_ea), badb = oz_max<kOzN>(B, s_eb);
   if (bada || badb) s_bad = 1;
   if (g.X.p && t < B.rows) s_rs[t] = adj_quot(1.0, g.s[b * g.sb + c0 + t]);
   __syncthreads();
-  const bool bad = s_bad != 0;
+  bool plain = s_bad != 0;
   if (t < kOzM) s_ea[t] -= 1022;  // |v| < 2^(exponent - 1022)
   if (t < kOzN) s_eb[t] -= 1022;
   __syncthreads();
@@ -282,18 +338,13 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
   double run[8];
 #pragma unroll
   for (int x = 0; x < 8; x++) run[x] = 0.0;
-  if (bad) {
-    for (int k = 0; k < g.K; k++)
-#pragma unroll
-      for (int x = 0; x < 8; x++) {
-        const int r = lr + 8 * ((x >> 1) & 1), c = lc + 8 * (x >> 2) + (x & 1);
-        if (r < A.rows && c < B.rows) run[x] += A.p[r * A.s_r + k * A.s_k] * B.p[c * B.s_r + k * B.s_k];
-      }
-  } else {
-    auto stage = [&](int s, int op) { return ozm + (size_t)s * kOzStage + op * kOzD * kOzM * kOzLd; };
+  unsigned weak = 0;  // elements left to FP64 sums
+  if (!plain) {
+    auto stage = [&](int s, int op) { return ozm + (size_t)s * kOzStage + op * kOzD * kOzM * kOzK; };
     oz_stage<kOzM>(A, s_ea, 0, stage(0, 0));
     oz_stage<kOzN>(B, s_eb, 0, stage(0, 1));
     float acc[kOzS][2][4];
+    unsigned mag[2][2] = {{0u, 0u}, {0u, 0u}};  // sums of the first digits' |a| |b|
 #pragma unroll
     for (int s = 0; s < kOzS; s++)
 #pragma unroll
@@ -302,17 +353,21 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
     for (int k0 = 0; k0 < g.K; k0 += kOzK, buf ^= 1) {
       const bool more = k0 + kOzK < g.K;
       __syncthreads();  // stage `buf` written; the other one's readers are done
-      const __half* sa = stage(buf, 0) + (wm + (lane & 15)) * kOzLd + 8 * (lane >> 4);
-      const __half* sb = stage(buf, 1) + (wn + (lane & 7) + 8 * (lane >> 4)) * kOzLd + 8 * ((lane >> 3) & 1);
 #pragma unroll
       for (int kk = 0; kk < kOzK; kk += 16) {
+        const __half* sa = stage(buf, 0) + oz_at(wm + (lane & 15), kk + 8 * (lane >> 4));
+        const __half* sb = stage(buf, 1) + oz_at(wn + (lane & 7) + 8 * (lane >> 4), kk + 8 * ((lane >> 3) & 1));
         unsigned bf[kOzD][4];
 #pragma unroll
-        for (int j = 0; j < kOzD; j++) ldsm4(bf[j], sb + j * kOzN * kOzLd + kk);
+        for (int j = 0; j < kOzD; j++) ldsm4(bf[j], sb + j * kOzN * kOzK);
 #pragma unroll
         for (int i = 0; i < kOzD; i++) {
           unsigned af[4];
-          ldsm4(af, sa + i * kOzM * kOzLd + kk);
+          ldsm4(af, sa + i * kOzM * kOzK);
+          if (i == 0) {
+            mma16816_abs(mag[0], af, bf[0][0], bf[0][1]);
+            mma16816_abs(mag[1], af, bf[0][2], bf[0][3]);
+          }
 #pragma unroll
           for (int j = 0; j < kOzD; j++) {
             if (i + j >= kOzS) continue;
@@ -326,7 +381,7 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
         oz_stage<kOzN>(B, s_eb, k0 + kOzK, stage(buf ^ 1, 1));
       }
       if (!more || (k0 + kOzK) % kOzChunk == 0) {
-        // the exact sums of this chunk, weights 2^96 .. 2^72 and 2^64 .. 2^40; each
+        // the exact sums of this chunk, weights 2^112 .. 2^88 and 2^80 .. 2^56; each
         // half is below 2^49, so an integer added to the bits of 1.5 2^52 is its double
 #pragma unroll
         for (int x = 0; x < 8; x++) {
@@ -347,6 +402,34 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
         }
       }
     }
+    // 2^-11 sqrt(K) of the largest product, 64 x 64 of the first digits (a row or
+    // column of zeros or subnormals is exact)
+    const float least = 2.f * sqrtf((float)g.K);
+#pragma unroll
+    for (int x = 0; x < 8; x++) {
+      const int r = lr + 8 * ((x >> 1) & 1), c = lc + 8 * (x >> 2) + (x & 1);
+      const unsigned h = mag[x >> 2][(x >> 1) & 1] >> (16 * (x & 1));
+      const bool strong = __half2float(__ushort_as_half((unsigned short)h)) >= least || s_ea[r] == 1 - 1022 ||
+                          s_eb[c] == 1 - 1022 || r >= A.rows || c >= B.rows;
+      weak |= strong ? 0u : 1u << x;
+    }
+    if (weak) atomicAdd(&s_weak, __popc(weak));
+    __syncthreads();
+    plain = s_weak > kOzFew;
+  }
+  if (plain) {
+    oz_plain(A, B, reinterpret_cast<double*>(ozm), lr, lc, run);
+  } else if (s_weak) {
+#pragma unroll
+    for (int x = 0; x < 8; x++)
+      for (unsigned w = __ballot_sync(0xffffffffu, (weak >> x) & 1u); w; w &= w - 1) {
+        const int src = __ffs(w) - 1;  // the warp forms lane src's element
+        const int r = wm + (src >> 2) + 8 * ((x >> 1) & 1), c = wn + 2 * (src & 3) + 8 * (x >> 2) + (x & 1);
+        double v = 0.0;
+        for (int k = lane; k < g.K; k += 32) v = fma(A.p[r * A.s_r + k * A.s_k], B.p[c * B.s_r + k * B.s_k], v);
+        v = warp_sum(v);
+        if (lane == src) run[x] = v;
+      }
   }
   double* Cb = g.C + b * g.cb;
 #pragma unroll
@@ -354,7 +437,7 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
     const int r = lr + 8 * ((x >> 1) & 1), c = lc + 8 * (x >> 2) + (x & 1);
     if (r < A.rows && c < B.rows) {
       double v = run[x];
-      if (!bad) {  // v 2^(e_r + e_c - 68), in the exponent field where both ends are normal
+      if (!plain && !((weak >> x) & 1u)) {  // v 2^(e_r + e_c - 68), in the exponent field where both ends are normal
         const int sh = s_ea[r] + s_eb[c] - 68, ex = (__double2hiint(v) >> 20) & 0x7ff;
         if (ex != 0 && ex + sh > 0 && ex + sh < 0x7ff)
           v = __hiloint2double(__double2hiint(v) + (sh << 20), __double2loint(v));
