@@ -25,6 +25,14 @@ namespace ddcsvd {
 
 __device__ __forceinline__ float adj_quot(float a, float x) { return a / x; }
 __device__ __forceinline__ double adj_quot(double a, double x) { return quot_rn(a, x); }
+// a / x with rx = 1 / x at hand: the quotient and one correction by its remainder
+// (the product alone is up to an ulp worse than a division)
+__device__ __forceinline__ float adj_quot(float a, float x, float) { return a / x; }
+__device__ __forceinline__ double adj_quot(double a, double x, double rx) {
+  if (!(mid_range(a) && mid_range(rx))) return a / x;
+  const double q = a * rx;
+  return fma(fma(-x, q, a), rx, q);
+}
 
 // A matrix of every problem: element (r, c) of problem b at p + b*b_ + r*r_ + c*c_.
 template <typename T>
@@ -446,8 +454,7 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
       }
       if (g.X.p) {
         const double xv = g.X.p[b * g.X.b + (r0 + r) * g.X.r + (c0 + c) * g.X.c];
-        const double rs = s_rs[c];
-        v += mid_range(rs) ? xv * rs : adj_quot(xv, g.s[b * g.sb + c0 + c]);
+        v += adj_quot(xv, g.s[b * g.sb + c0 + c], s_rs[c]);
       }
       Cb[(r0 + r) + (size_t)(c0 + c) * g.ldc] = v;
     }
@@ -459,8 +466,6 @@ __global__ void __launch_bounds__(kOzThreads, 2) ozgemm_kernel(BGemm<double> g0,
 // Columns a and k - 1 - a of the upper triangle hold k + 1 entries together, so
 // the pairs fill a rectangle and no lane idles through an FP64 instruction.
 constexpr int kCoreCols = 512;
-__device__ __forceinline__ bool adj_mid(double x) { return mid_range(x); }
-__device__ __forceinline__ bool adj_mid(float) { return false; }  // FP32 divisions cost nothing that matters here
 
 template <typename T>
 __global__ void __launch_bounds__(256) adjoint_core_kernel(int k, const T* __restrict__ J, const T* __restrict__ Kv,
@@ -470,13 +475,12 @@ __global__ void __launch_bounds__(256) adjoint_core_kernel(int k, const T* __res
   const T* Kb = Kv ? Kv + (size_t)b * k * k : nullptr;
   const T* sb = s + (size_t)b * k;
   T* Mb = Mo + (size_t)b * k * k;
-  // 1 / s of every column once per CTA; columns whose reciprocal leaves the
-  // normal range (or beyond the table) divide
+  // 1 / s of every column once per CTA (columns beyond the table divide)
   __shared__ T s_rs[kCoreCols];
   for (int c = threadIdx.x; c < min(k, kCoreCols); c += blockDim.x) s_rs[c] = adj_quot(T(1), sb[c]);
   __syncthreads();
   auto over = [&](T x, int c) {  // x / s_c
-    return (c < kCoreCols && adj_mid(s_rs[c])) ? x * s_rs[c] : adj_quot(x, sb[c]);
+    return c < kCoreCols ? adj_quot(x, sb[c], s_rs[c]) : adj_quot(x, sb[c]);
   };
   const int half = (k + 1) / 2;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < half * (k + 1); idx += gridDim.x * blockDim.x) {

@@ -107,3 +107,18 @@ def test_columns_and_rows(lib, cuda, kind, loss, m, n):
     # roundings of the result where the FP64 sums happen to be nearly exact
     for g, w in zip(got, sums):
         assert g <= 4.0 * w + 4.0 * 2.0 ** -53, (got, sums)
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -300, 2.0 ** -520])
+def test_quotients_are_rounded_once(lib, cuda, scale):
+    """U = [I; 0], V = I and gU in U's complement: the gradient is gU / s, and each entry the
+    quotient that a division gives (operands within and beyond the range of the short form)."""
+    rng = np.random.default_rng(5)
+    B, n = 16, 40
+    U, V = np.zeros((B, 2 * n, n)), np.broadcast_to(np.eye(n), (B, n, n)).copy()
+    U[:, :n] = np.eye(n)
+    s = np.sort(rng.uniform(1.0, 3.0, (B, n)), axis=1)
+    gU = np.zeros((B, 2 * n, n))
+    gU[:, n:] = rng.uniform(0.5, 1.0, (B, n, n)) * scale
+    got = lib.svd_backward_device(*(cuda.from_numpy(x).cuda() for x in (U, s, V, gU)), None, None).cpu().numpy()
+    assert np.array_equal(got, gU / s[:, None, :])
