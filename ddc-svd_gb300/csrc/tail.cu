@@ -127,10 +127,12 @@ __device__ __forceinline__ void householder_fast(float x0, FF t2, float* alpha, 
   *scale = zero ? 0.f : sg * q;
 }
 
-// Waits for the phase of the given parity.  Bounded: after kTailWaitNs the
-// status word holds DDCSVD_ERR_TIMEOUT, `dead` stays set in this thread and no
-// later wait of it waits (the column loop runs out with meaningless values).
-constexpr unsigned long long kTailWaitNs = 2000000000ull;
+// Waits for the phase of the given parity.  Bounded by the handle's limit: when
+// it runs out the status word holds DDCSVD_ERR_TIMEOUT, and then or when it holds
+// another CTA's error `dead` is set in this thread: it waits, sends and arms
+// barriers no more, and the column loop runs out with meaningless values (leaving
+// it instead takes a barrier that agrees on `dead`, 0.1 us a column).
+constexpr unsigned long long kTailLateNs = 20000;  // from here on the status word is read (a column takes 1.5-3 us)
 __device__ __forceinline__ void tail_wait(uint32_t bar, unsigned parity, bool& dead, DevStatus* st) {
   unsigned long long t0 = 0;
   for (unsigned polls = 0; !dead; polls++) {
@@ -146,7 +148,11 @@ __device__ __forceinline__ void tail_wait(uint32_t bar, unsigned parity, bool& d
     if ((polls & 63u) == 63u) {
       const unsigned long long now = global_ns();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > kTailWaitNs) {
+      if (now - t0 < kTailLateNs) continue;
+      const uint4 s = ld_status(st);
+      if (s.x != 0) {
+        dead = true;
+      } else if (now - t0 > (s.z ? 1000ull * s.z : kWaitLimitNs)) {
         set_error(st, DDCSVD_ERR_TIMEOUT, 700);
         dead = true;
       }
@@ -197,6 +203,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
 #pragma unroll
   for (int j = 0; j < NT; j++) to_cta[j] = map_rank(bar0, min(wid + 8 * j, C - 1)) - bar0;
   bool dead = false;
+  // the handle's extra arrivals stand for a CTA whose norm never comes (tests of the bounded waits)
+  const bool lost = rank == 0 && ld_status(p.st).w != 0;
 
   float A[R][K];
 #pragma unroll
@@ -237,7 +245,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
     const int kf = (i + 1) >> 5;            // first slice with a column > i
     const bool mine = gw == iwarp;          // this warp holds row i
     // ---- exchange 1: products of column i, its norm, row i
-    if (t == 0) {
+    if (t == 0 && !dead) {
       unsigned bytes = 8u * C + 4u;
       if (rank >= kf && slice_cols > 0) bytes += 4u * (C + 1) * slice_cols;
       mbar_arrive_expect_tx(&s_bar[b], bytes);
@@ -269,7 +277,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
 #pragma unroll
     for (int j = 0; j < NS; j++) {
       const int c = t + kTailThreads * j;  // warp wid: slice wid + 8 j
-      if (c >= 32 * kf && c < nt) {
+      if (c >= 32 * kf && c < nt && !dead) {
         float v[kTailWarps];
 #pragma unroll
         for (int w = 0; w < kTailWarps; w++) v[w] = s_part[w][c];
@@ -280,8 +288,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
     }
     if (wid == kTailWarps - 1) {
       const FF n = ff_lanes<kTailWarps>(s_nw[lane & (kTailWarps - 1)]);
-      if (lane < C) {
-        st_async(smem_u32(&s_n1[b][rank]) + to_lane, n.hi, n.lo, bar1 + to_lane);
+      if (lane < C && !dead) {
+        if (!lost) st_async(smem_u32(&s_n1[b][rank]) + to_lane, n.hi, n.lo, bar1 + to_lane);
         if (holds) st_async(smem_u32(&s_x0[b]) + to_lane, s_own[i], bar1 + to_lane);
       }
     }
@@ -306,12 +314,12 @@ __global__ void __launch_bounds__(kTailThreads, 1) bidiag_tail_kernel(TailParams
       if (i < nt - 1 && rank >= kf && slice_cols > 0) {
 #pragma unroll
         for (int j = 0; j < NT; j++)
-          if (c_own < nt && wid + 8 * j < C)
+          if (c_own < nt && wid + 8 * j < C && !dead)
             st_async(smem_u32(&s_yw[c_own]) + to_cta[j], ty, w, bar2 + to_cta[j]);
         const FF n2 = ff_lanes<32>(c_own > i + 1 ? ff_square(w) : FF{0.f, 0.f});
 #pragma unroll
         for (int j = 0; j < NT; j++)
-          if (lane == 0 && wid + 8 * j < C)
+          if (lane == 0 && wid + 8 * j < C && !dead)
             st_async(smem_u32(&s_n2[rank]) + to_cta[j], n2.hi, n2.lo, bar2 + to_cta[j]);
       }
     }
