@@ -112,7 +112,8 @@ __global__ void status_init_kernel(DevStatus* st, unsigned wait_us, unsigned ext
 }
 
 int reset_status(ddcsvd_context* ctx) {
-  status_init_kernel<<<1, 32, 0, ctx->stream>>>(ctx->d_status, ctx->wait_us, ctx->barrier_extra);
+  status_init_kernel<<<1, 32, 0, ctx->stream>>>(ctx->d_status, ctx->wait_us,
+                                                 ctx->barrier_extra == kLostCopy ? 0u : ctx->barrier_extra);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());
   return DDCSVD_OK;

@@ -79,6 +79,7 @@ struct PanelParams {
   float* xpart;
   int ldxp;
   int ring_own, ring_slot4;  // column ring (rpt4 = 4): own slots, float4s per slot
+  int ring_lost;             // first columns that CTA 0 does not ask for (tests of the bounded waits)
   // two-GEMV form with more rows than shared memory holds next to the panel
   // blocks: y = A^T u reads the column from xcol (global, L2-resident)
   // instead of a staged copy, and the staging buffer holds only the row
@@ -434,33 +435,49 @@ struct ColumnRing {
   int own, NS, slot4;  // slots, float4s per slot
   uint64_t* bar;       // one per slot
   unsigned phase;      // parity of each slot's next completion
-  int waiting;         // columns asked for and not yet used
+  unsigned sent;       // parity of each slot's copies asked for
+  bool asks;           // thread 0
   DevStatus* st;
   __device__ __forceinline__ float4* slot(int s) const {
     return s < own ? base + (size_t)s * slot4 : s == own ? alias0 : alias1;
   }
-  // thread 0: column cl of the step
-  __device__ __forceinline__ void ask(const float* col, int cl, int nq) const {
+  // column cl of the step
+  __device__ __forceinline__ void ask(const float* col, int cl, int nq) {
     const int s = cl % NS;
+    sent ^= 1u << s;
     mbar_arrive_expect_tx(bar + s, 16u * nq);
     bulk_load(slot(s), col, 16u * nq, bar + s);
   }
-  __device__ __forceinline__ void wait(int s) {
+  // until the slot's phase of the given parity ends, the handle's limit runs out or
+  // the status word holds an error (an earlier wait's, say)
+  __device__ __forceinline__ bool landed(int s, unsigned parity) const {
     unsigned long long t0 = 0;
-    for (unsigned polls = 1; !mbar_try_wait(bar + s, (phase >> s) & 1u); polls++)
+    for (unsigned polls = 1; !mbar_try_wait(bar + s, parity); polls++)
       if ((polls & 255u) == 0) {
+        const uint4 v = ld_status(st);
         const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
-        if (now - t0 > kWaitLimitNs) {
+        if (v.x != 0) return false;
+        if (now - t0 > (v.z ? 1000ull * v.z : kWaitLimitNs)) {
           set_error(st, DDCSVD_ERR_TIMEOUT, 60);
-          break;
+          return false;
         }
       }
+    return true;
+  }
+  // after a wait that did not end well no column is asked for; the next grid
+  // barrier ends the kernel
+  __device__ __forceinline__ void wait(int s) {
+    if (!landed(s, (phase >> s) & 1u)) asks = false;
     phase ^= 1u << s;
   }
   // the copies under way land before the kernel gives its shared memory back
-  __device__ __forceinline__ void drain(int used) {
-    for (int cl = used; cl < used + waiting; cl++) wait(cl % NS);
+  __device__ __forceinline__ void drain() const {
+    if (threadIdx.x != 0) return;
+    const unsigned long long t0 = global_ns();
+    for (int s = 0; s < NS; s++)
+      while (!mbar_try_wait(bar + s, ((sent >> s) & 1u) ^ 1u) && global_ns() - t0 < kWaitLimitNs) {
+      }
   }
 };
 
@@ -522,7 +539,7 @@ __device__ __forceinline__ void fused_ring_pass(ColumnRing& ring, const float* _
     float* rp = red + par * (B * nw);  // [column][warp]
     if (sub == 0) rp[u * nw + wid] = ws;
     __syncthreads();  // (every thread has the batch in registers: its slots are free)
-    if (t == 0)
+    if (ring.asks)
       for (int cl = c0 + ring.NS; cl < min(c0 + ring.NS + B, ncol); cl++)
         ring.ask(W + (size_t)(c_s + cl) * ldw + sa, cl, nq);
     float tot = 0.f;
@@ -657,7 +674,7 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
   ColumnRing ring;
   if constexpr (kRing) {
     ring = ColumnRing{reinterpret_cast<float4*>(S.ring), reinterpret_cast<float4*>(S.big),
-                      reinterpret_cast<float4*>(S.xr), p.ring_own, p.ring_own + 2, p.ring_slot4, ring_bar, 0u, 0, p.st};
+                      reinterpret_cast<float4*>(S.xr), p.ring_own, p.ring_own + 2, p.ring_slot4, ring_bar, 0u, 0u, t == 0, p.st};
     if (t == 0) {
       for (int s = 0; s < ring.NS; s++) mbar_init(ring_bar + s, 1);
       fence_proxy_async_smem();
@@ -674,9 +691,8 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
     const int nrow = max(0, rb - r_s);
     if constexpr (kRing) {
       const int c_s = max(ca, i + 1), sa = (i + 1) & ~3;
-      ring.waiting = min(ring.own, max(0, cb - c_s));
-      if (t == 0)
-        for (int cl = 0; cl < ring.waiting; cl++)
+      if (ring.asks)
+        for (int cl = (j == 0 && b == 0) ? p.ring_lost : 0; cl < min(ring.own, cb - c_s); cl++)
           ring.ask(W + (size_t)(c_s + cl) * ldw + sa, cl, (m - sa + 3) >> 2);
     }
     // Row i of Y (S.Yi), of VT (S.VTi) and the own rows of column i (S.pre,
@@ -722,7 +738,7 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
     }
     PMARK(1);
     if (!grid_sync(p.bar, p.P, p.st, 1)) {
-      if constexpr (kRing) ring.drain(0);
+      if constexpr (kRing) ring.drain();
       return;
     }
     PMARK(2);
@@ -897,7 +913,10 @@ __global__ void __launch_bounds__(kBidiagThreads, 1) bidiag_panel_kernel(PanelPa
       }
     }
     PMARK(6);
-    if (!grid_sync(p.bar, p.P, p.st, 2)) return;
+    if (!grid_sync(p.bar, p.P, p.st, 2)) {
+      if constexpr (kRing) ring.drain();
+      return;
+    }
     PMARK(7);
 
     // ---------------- S5: row reflector
@@ -1457,6 +1476,7 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
     }
     size_t smem = panel_smem_bytes(std::max(m, n), pp.rc, pp.cc, kBidiagThreads, P, pp.rpt4 > 0);
     pp.ring_own = pp.ring_slot4 = 0;
+    pp.ring_lost = ctx->barrier_extra == kLostCopy;
     if (pp.rpt4 == 4) {  // the column ring: as many slots as the rest of the shared memory holds
       pp.ring_slot4 = (m - ((k0 + 1) & ~3) + 3) >> 2;
       const size_t slot = sizeof(float4) * (size_t)pp.ring_slot4;

@@ -11,6 +11,8 @@
 
 #include "common.cuh"
 
+constexpr unsigned kLostCopy = 1024;
+
 struct ddcsvd_context {
   int device = 0;
   int num_sms = 0;
@@ -65,7 +67,7 @@ struct ddcsvd_context {
   int sec_maxit = 80;
   unsigned wait_us = 0;
   size_t ws_cap = 0;
-  unsigned barrier_extra = 0;
+  unsigned barrier_extra = 0;  // DevStatus::extra, or kLostCopy: a bulk copy is not started instead
   // set while an SVD of the R factor runs inside the tall-matrix path
   bool nested = false;
   std::mutex mu;

@@ -278,14 +278,15 @@ int ddcsvd_autotune_batched(ddcsvd_handle_t handle, int batch, const int *m, con
  *   [0] FP64 iterations per secular root in stage 2 (1..80, default 80);
  *       a root that has not converged by then gives DDCSVD_ERR_NOCONV
  *   [1] wall-clock limit of one device-side wait of the cooperative kernels
- *       (grid barriers) in microseconds (0..4000000; 0 = the built-in 4 s);
+ *       (grid barriers, exchanged records, copies) in microseconds (0..4000000; 0 = the built-in 4 s);
  *       a wait that runs out gives DDCSVD_ERR_TIMEOUT and the kernel returns
  *   [2] device workspace budget of the handle in bytes (0 = none); a call
  *       whose workspace would exceed it gives DDCSVD_ERR_ALLOC
  *   [3] fault injection for tests of the timeout path (0 in normal use):
  *       the first grid barrier of every cooperative launch waits for this
  *       many arrivals beyond its own CTAs, so its waits run out after limit
- *       [1] and the call returns DDCSVD_ERR_TIMEOUT
+ *       [1] and the call returns DDCSVD_ERR_TIMEOUT (kernels that exchange
+ *       records leave one out; 1024: a copy is not started)
  * After any of these failures the handle stays usable.  get/set copy up to
  * `count` limits; set checks the ranges (DDCSVD_ERR_ARG, nothing changed). */
 int ddcsvd_set_limits(ddcsvd_handle_t handle, const long long *values, int count);

@@ -29,3 +29,9 @@ def run_out(lib, cuda, m, n, extra, mode="tf32x6"):
 def test_cluster_tail(lib, cuda, m, n):
     """Clusters of 1 to 16 CTAs, with and without slices of their own."""
     run_out(lib, cuda, m, n, 1)
+
+
+@pytest.mark.parametrize("m,n", [(4500, 300), (8190, 200)])
+def test_column_ring(lib, cuda, m, n):
+    """A column that is never asked for, with several slots of the ring's own and with one."""
+    run_out(lib, cuda, m, n, 1024)
