@@ -736,8 +736,7 @@ static int svd_backward_f32(ddcsvd_context* h, int batch, int m, int n, BMat<flo
   std::lock_guard<std::mutex> g(h->mu);
   DDC_CUDA_TRY(cudaSetDevice(h->device));
   DDC_TRY(reset_status(h));
-  DDC_CUDA_TRY(cudaFuncSetAttribute((const void*)adjoint_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)bytes));
+  DDC_TRY(allow_smem(h, (const void*)adjoint_fused_kernel));
   adjoint_fused_kernel<<<batch, fused_threads(m, n), bytes, h->stream>>>(m, n, U, S, V, gU, gS, gV, gA);
   count_launch();
   DDC_CUDA_TRY(cudaGetLastError());

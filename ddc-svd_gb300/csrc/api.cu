@@ -105,6 +105,15 @@ int ensure_pinned(ddcsvd_context* ctx, size_t bytes) {
   return DDCSVD_OK;
 }
 
+int allow_smem(const ddcsvd_context* ctx, const void* kernel) {
+  cudaFuncAttributes a;
+  DDC_CUDA_TRY(cudaFuncGetAttributes(&a, kernel));
+  const int most = (int)(ctx->smem_optin - a.sharedSizeBytes);
+  if (a.maxDynamicSharedSizeBytes < most)
+    DDC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  return DDCSVD_OK;
+}
+
 // Clears the error code and writes the handle's limits (kernel arguments, so
 // the host values may change right after the launch).
 __global__ void status_init_kernel(DevStatus* st, unsigned wait_us, unsigned extra) {

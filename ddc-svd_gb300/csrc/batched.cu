@@ -685,7 +685,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
                                 ? std::max(1024, (max_optin - 2048) / (int)sizeof(float) - vrow_floats)
                                 : smem_floats;
   const size_t smem = sizeof(float) * ((size_t)vrow_floats + bidiag_floats);
-  DDC_CUDA_TRY(cudaFuncSetAttribute(batch_bidiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DDC_TRY(allow_smem(h, (const void*)batch_bidiag_kernel));
   int occ = 1;
   DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_bidiag_kernel, bthreads, smem));
   const int grid1 = std::max(1, std::min(batch, h->num_sms * std::max(occ, 1)));
@@ -749,8 +749,7 @@ extern "C" int ddcsvd_svd_batched_f32_device(ddcsvd_handle_t h, int batch, const
   // ---- stage 5 and sigma
   const int room5 = (int)std::min<long long>(maxmn + 512, smem_floats);  // (a reflector's odd length, and all of a small problem's)
   const size_t smem5 = sizeof(float) * (size_t)room5;
-  DDC_CUDA_TRY(cudaFuncSetAttribute(batch_backxform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::max<size_t>(smem5, 16)));
+  DDC_TRY(allow_smem(h, (const void*)batch_backxform_kernel));
   ktimer_begin(h, KC_BACKXFORM);
   int occ5 = 1;
   DDC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ5, batch_backxform_kernel, kBatchThreads,

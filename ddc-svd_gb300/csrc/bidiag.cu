@@ -1403,11 +1403,10 @@ void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWo
   w->rpart = w->rwords ? a.take<uint2>(w->rwords) : nullptr;
 }
 
-static int launch_coop(const void* fn, int P, int threads, size_t smem, void* args,
-                       cudaStream_t s) {
-  DDC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+static int launch_coop(ddcsvd_context* ctx, const void* fn, int P, int threads, size_t smem, void* args) {
+  DDC_TRY(allow_smem(ctx, fn));
   void* argv[] = {args};
-  DDC_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(P), dim3(threads), argv, smem, s));
+  DDC_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(P), dim3(threads), argv, smem, ctx->stream));
   count_launch();
   return DDCSVD_OK;
 }
@@ -1500,7 +1499,7 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
                       : pp.rpt4 == 2 ? (const void*)bidiag_panel_kernel<2>
                       : pp.rpt4 == 4 ? (const void*)bidiag_panel_kernel<4>
                                      : (const void*)bidiag_panel_kernel<0>;
-    DDC_TRY(launch_coop(kfn, P, kBidiagThreads, smem, &pp, ctx->stream));
+    DDC_TRY(launch_coop(ctx, kfn, P, kBidiagThreads, smem, &pp));
     ktimer_end(ctx);
     const int kn = k0 + nb;
     if (kn < n) {
@@ -1557,7 +1556,7 @@ int bidiag_plain(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d,
     return DDCSVD_ERR_ARG;
   }
   ktimer_begin(ctx, KC_BIDIAG);
-  int rc = launch_coop((const void*)bidiag_plain_kernel, w.P, kBidiagThreads, smem, &pp, ctx->stream);
+  int rc = launch_coop(ctx, (const void*)bidiag_plain_kernel, w.P, kBidiagThreads, smem, &pp);
   ktimer_end(ctx);
   return rc;
 }
@@ -1626,8 +1625,8 @@ int qr_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* tau,
         return DDCSVD_ERR_ARG;
       }
       DDC_CUDA_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), ctx->stream));
-      DDC_TRY(launch_coop((const void*)qr_panel_kernel, w.P, kBidiagThreads, qr_smem_bytes(q.rc, kBidiagThreads), &q,
-                          ctx->stream));
+      DDC_TRY(launch_coop(ctx, (const void*)qr_panel_kernel, w.P, kBidiagThreads, qr_smem_bytes(q.rc, kBidiagThreads),
+                          &q));
       ktimer_end(ctx);
       if (k0 + nb < K0 + NB) {
         // the super-block's remaining columns: W[k0:, k0+nb:K0+NB] := (I - V T^T V^T) W[...]

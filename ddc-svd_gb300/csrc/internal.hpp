@@ -119,6 +119,10 @@ void ktimer_collect(ddcsvd_context* ctx);        // after a stream sync
 
 int ensure_workspace(ddcsvd_context* ctx, size_t bytes);
 int ensure_pinned(ddcsvd_context* ctx, size_t bytes);
+// Lets a kernel have all the dynamic shared memory that its static one leaves.  The
+// attribute belongs to the function and the device, so a size of one call's set here
+// could refuse another handle's launch in another thread: it is never lowered.
+int allow_smem(const ddcsvd_context* ctx, const void* kernel);
 int check_status(ddcsvd_context* ctx, const char* stage);  // syncs the stream
 int reset_status(ddcsvd_context* ctx);
 

@@ -592,7 +592,7 @@ int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* 
   p.st = ctx->d_status;
   DDC_CUDA_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), ctx->stream));
   const size_t smem = res_smem(*g, p.nt);
-  DDC_CUDA_TRY(cudaFuncSetAttribute(g->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DDC_TRY(allow_smem(ctx, g->fn));
   void* args[] = {&p};
   DDC_CUDA_TRY(cudaLaunchCooperativeKernel(g->fn, dim3(w.P), dim3(g->T + 32), args, smem, ctx->stream));
   count_launch();
