@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
 #pragma unroll
         for (int u = 0; u < kB; u++) {
           const double dp = v.x[0][u] + s;
-          ok = ok && mid_range(dp) && mid_range(v.x[1][u]);
-          const double L = quot_mid(v.x[1][u], dp);
+          bool sure;
+          const double L = quot_mid(v.x[1][u], dp, sure);
+          ok = ok && sure && mid_range(dp) && mid_range(v.x[1][u]);
           p.Lp[at(i0 + u)] = L;
           p.S[at(i0 + u)] = s;
           s = L * v.x[2][u] * s - lam;
@@ -185,8 +186,9 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
 #pragma unroll
         for (int u = 0; u < kB; u++) {
           const double dm = v.x[0][u] + pv;
-          ok = ok && mid_range(dm) && mid_range(v.x[1][u]);
-          const double tt = quot_mid(v.x[1][u], dm);
+          bool sure;
+          const double tt = quot_mid(v.x[1][u], dm, sure);
+          ok = ok && sure && mid_range(dm) && mid_range(v.x[1][u]);
           p.Um[at(i0 - u)] = v.x[2][u] * tt;
           pv = pv * tt - lam;
           p.Pp[at(i0 - u)] = pv;
