@@ -264,6 +264,58 @@ __device__ __forceinline__ void householder_ff(float x0, FF t2, float* alpha, fl
   *scale = sg / (ax + nrm);  // 1 / (x0 - alpha)
 }
 
+// Compensated sums without the final renormalisation of ff_add: the heads by
+// two-sum, the errors added to the tails.  Head, error and tail do not depend
+// on the operands' order, so lanes that add the same pair agree bit for bit.
+__device__ __forceinline__ FF ff_acc(FF a, FF b) {
+  const float s = __fadd_rn(a.hi, b.hi);
+  const float bb = __fsub_rn(s, a.hi);
+  const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));
+  return FF{s, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
+}
+__device__ __forceinline__ FF ff_square(float x) {
+  const float p = __fmul_rn(x, x);
+  return FF{p, __fmaf_rn(x, x, -p)};
+}
+// sum over aligned groups of N lanes
+template <int N>
+__device__ __forceinline__ FF ff_lanes(FF v) {
+#pragma unroll
+  for (int o = N >> 1; o > 0; o >>= 1)
+    v = ff_acc(v, FF{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+  return v;
+}
+
+__device__ __forceinline__ float rcp_approx_f32(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// householder_ff with approximate reciprocal and reciprocal square root and one
+// Newton correction each (the square root's from the compensated sum itself, which
+// householder_ff rounds first) in place of the IEEE square root and quotients, whose
+// ~300 cycles stood twice in every column's chain.  Largest errors of alpha, tau
+// and scale in units of 2^-24: 1.0, 1.3 and 2.5 (householder_ff 1.5, 2.3 and 3.0).
+__device__ __forceinline__ void householder_fast(float x0, FF t2, float* alpha, float* tau, float* scale) {
+  const FF n2 = ff_add_sq(t2, x0);
+  const float s = n2.hi;
+  const float r = rsqrtf(s);
+  float nrm = s * r;
+  const float d2 = __fadd_rn(__fmaf_rn(-nrm, nrm, s), n2.lo);
+  nrm = fmaf(0.5f * r, d2, nrm);
+  const float ax = fabsf(x0), den = ax + nrm;
+  float q = rcp_approx_f32(den);
+  q = fmaf(q, fmaf(-den, q, 1.f), q);
+  float ri = r;  // 1 / nrm
+  ri = fmaf(ri, fmaf(-nrm, ri, 1.f), ri);
+  const float sg = x0 < 0.f ? -1.f : 1.f;
+  const bool zero = !(s > 0.f);
+  *alpha = zero ? 0.f : -sg * nrm;
+  *tau = zero ? 0.f : fmaf(ax, ri, 1.f);
+  *scale = zero ? 0.f : sg * q;
+}
+
 // 2^k with max|a| * 2^k in [0.5, 1) when max|a| is outside [2^-40, 2^40], else 1
 __device__ __forceinline__ float range_scale(unsigned bits) {
   const float a = __uint_as_float(bits);
