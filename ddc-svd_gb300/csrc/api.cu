@@ -335,7 +335,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
     Arena a;
     region_a(a, pl);
     Arena b1 = a;
-    plan_bidiag(b1, m, n, ldw, nctas, kind, &pl.bw);
+    plan_bidiag(ctx, b1, m, n, ldw, nctas, kind, &pl.bw);
     b1.take<char>(gsc);
     Arena b2 = a;
     DDC_TRY(dc_sigma(ctx, n, nullptr, nullptr, nullptr, nullptr, nullptr, b2, true, false));
@@ -362,7 +362,7 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
   DDC_TRY(stage_event(ctx, 0));
   {
     Arena b = a;
-    plan_bidiag(b, m, n, ldw, nctas, kind, &pl.bw);
+    plan_bidiag(ctx, b, m, n, ldw, nctas, kind, &pl.bw);
     if (!plain) DDC_CUDA_TRY(cudaMemsetAsync(pl.bw.amax, 0, sizeof(unsigned), ctx->stream));
     copy_pad_kernel<<<dim3(std::min(ceil_div(ldw, 256), 4), n), 256, 0, ctx->stream>>>(
         m, n, dA, lda, pl.W, ldw, check_finite ? ctx->d_status : nullptr, plain ? nullptr : pl.bw.amax);
@@ -797,7 +797,7 @@ static int bidiag_device(ddcsvd_context* h, int m, int n, float* dA, int lda, fl
     Arena a;
     a.plan = pass == 0;
     a.base = (char*)h->ws;
-    plan_bidiag(a, m, n, lda, bidiag_coop_ctas(h, m, n), kind, &bw);
+    plan_bidiag(h, a, m, n, lda, bidiag_coop_ctas(h, m, n), kind, &bw);
     sc = a.take<char>(scb);
     if (pass == 0) DDC_TRY(ensure_workspace(h, a.off + 4096));
   }

@@ -1378,7 +1378,7 @@ int bidiag_coop_ctas(ddcsvd_context* ctx, int m, int n) {
   return ctx->num_sms;
 }
 
-void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWork* w) {
+void plan_bidiag(ddcsvd_context* ctx, Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWork* w) {
   w->ldn = (int)round_up(n, 32);
   w->P = P;
   w->X = a.take<float>((size_t)ldw * kPanel);
@@ -1399,7 +1399,7 @@ void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWo
   const int k0_last = ((n - 1) / kPanel) * kPanel;
   w->ldxp = ldw;
   w->xpart = (m - k0_last <= kFusedRows) ? a.take<float>((size_t)P * ldw + 4) : nullptr;
-  w->rwords = bidiag_resident_words(m, n, P, &w->ldr);
+  w->rwords = bidiag_resident_words(ctx, m, n, P, &w->ldr);
   w->rpart = w->rwords ? a.take<uint2>(w->rwords) : nullptr;
 }
 

@@ -177,7 +177,7 @@ struct BidiagWork {
 constexpr int kPanel = 32;       // bidiagonalisation panel width
 constexpr int kFusedRows = 8192; // fused panel pass: rows (from the first staged float4) it covers
 constexpr int kBidiagThreads = 512;
-void plan_bidiag(Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWork* w);
+void plan_bidiag(ddcsvd_context* ctx, Arena& a, int m, int n, int ldw, int P, GemmKind kind, BidiagWork* w);
 int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d, float* e,
                    float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch, bool scanned = false);
 // (scanned: w.amax already holds the largest |a|, and the caller scales d and e back)
@@ -190,7 +190,7 @@ int bidiag_coop_ctas(ddcsvd_context* ctx, int m, int n);
 // Columns from k0 that the grid-resident kernel takes in one launch (a multiple of
 // kPanel; 0: not its shape), and the launch.
 int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P);
-size_t bidiag_resident_words(int m, int n, int P, int* ld);
+size_t bidiag_resident_words(ddcsvd_context* ctx, int m, int n, int P, int* ld);
 int bidiag_resident(ddcsvd_context* ctx, int m, int n, int k0, int cols, float* W, int ldw, float* d, float* e,
                     float* tauq, float* taup, const BidiagWork& w);
 int tail_cluster_size(ddcsvd_context* ctx);  // CTAs of the largest cluster the GPU co-schedules (16, 8 or 0)

@@ -558,11 +558,11 @@ int bidiag_resident_columns(ddcsvd_context* ctx, int m, int n, int k0, int P) {
   return tail ? cols : 0;
 }
 
-// Words of the exchange buffer for all launches of one factorisation (none for
-// matrices so small that the tail takes them whole, or with too many rows).
-size_t bidiag_resident_words(int m, int n, int P, int* ld) {
+// Words of the exchange buffer for all launches of one factorisation (none where
+// the tail is off or takes the matrix whole, or with too many rows).
+size_t bidiag_resident_words(ddcsvd_context* ctx, int m, int n, int P, int* ld) {
   *ld = (int)round_up(std::min(n, kResSlice * P), 32);  // the most columns a launch starts with
-  if ((long long)m * n <= 400000 || m - n > 24 * P) return 0;
+  if (ctx->tune[TK_PANEL_TAIL] <= 0 || m - n > 24 * P || bidiag_tail_columns(ctx, m, n, 0) > 0) return 0;
   return (size_t)(P + 3) * *ld + 4 * (size_t)P;
 }
 
