@@ -843,13 +843,15 @@ __device__ bool sec_root(int q, const double* d, const double* z, const float2* 
     const double t0 = (double)t32;
     sec_eval_newton(q, d, z, dorg, t0, g, f, fp, g2);
     const double u = quot(f, fp);
-    const float uf = (float)u, un = uf / t32, gr = g2 / (float)fp;
-    const float corr = uf * gr * un;
-    const float rest = fabsf(uf) * un * un * (2.f * gr * gr + 1.f);  // size of the third-order term
-    const double tau = t0 - (u + (double)corr);
+    // (everything relative to tau: in absolute terms the test underflowed or overflowed
+    // for inputs far from 1 and let any step through)
+    const float fpf = (float)fp, at = fabsf(t32), un = (float)u / t32, gr = g2 / fpf;
+    const float rest = fabsf(un) * un * un * (2.f * gr * gr + 1.f);  // size of the third-order term
+    const double tau = t0 - fma(u, (double)(gr * un), u);
     const float tf = left ? (float)tau : -(float)tau;
     const float far32 = last ? 1.001f * (float)zz : 0.501f * dd32;
-    if (fabsf(un) <= 1e-3f && rest <= 0x1p-55f * (od.x * od.x + t32) && tf > 0.f && tf <= far32) {
+    const bool range = at >= 0x1p-100f && at <= 0x1p100f && fpf >= 0x1p-100f && fpf <= 0x1p100f;
+    if (range && fabsf(un) <= 1e-3f && rest <= 0x1p-55f * fabsf(od.x * (od.x / t32) + 1.f) && tf > 0.f && tf <= far32) {
       if (iters) *iters = 1;
       *tau_out = tau;
       return true;
