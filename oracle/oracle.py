@@ -17,6 +17,7 @@ from __future__ import annotations
 import ctypes
 import os
 import subprocess
+import sys
 
 import numpy as np
 
@@ -30,11 +31,15 @@ _dp = ctypes.POINTER(ctypes.c_double)
 def build(with_ref: bool | None = None, ref_src: str | None = None) -> None:
     """Compile the oracle (always) and the reference build from the reference's
     sources in `ref_src` (else the DDCSVD_REF_SRC environment variable): when
-    with_ref is True, or None and that directory holds them."""
+    with_ref is True, or None and that directory exists and is not empty (an empty
+    one is named on stderr; the comparisons with the reference build are skipped then)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
     src = ref_src or os.environ.get("DDCSVD_REF_SRC", "")
     if with_ref is None:
-        with_ref = bool(src) and os.path.exists(os.path.join(src, "matrix_helper.c"))
+        with_ref = bool(src) and os.path.isdir(src)
+        if with_ref and not os.listdir(src):
+            with_ref = False
+            print(f"oracle: {src} is empty, no reference build", file=sys.stderr)
     if with_ref:
         if not (src and os.path.isdir(src)):
             raise RuntimeError("the reference build needs its sources: pass ref_src or set DDCSVD_REF_SRC")
