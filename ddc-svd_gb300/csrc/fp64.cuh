@@ -66,6 +66,11 @@ __device__ __forceinline__ double quot_rn(double a, double x) {
 // order of non-negative values = order of their bit patterns
 __device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
 __device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
+// the order of any values (-0 and 0 equal) as integers
+__device__ __forceinline__ long long order_bits(double x) {
+  const long long b = bits(x);
+  return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
 // |x|'s bits for a maximum that ignores NaN, as fmax does
 __device__ __forceinline__ long long max_bits(double x) {
   const long long b = abs_bits(x);

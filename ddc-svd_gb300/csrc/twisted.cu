@@ -557,7 +557,7 @@ constexpr int kRankTile = 1024;
 
 __global__ void __launch_bounds__(kRankThreads) tw_rank_count_kernel(int N, const double* __restrict__ sigma,
                                                                    VecLayout L, int* rank, int seg) {
-  __shared__ long long tile[kRankTile];  // bit patterns: order as the (non-negative) values do
+  __shared__ long long tile[kRankTile];  // integers in the values' order (a caller's may be negative)
   __shared__ int s_lo, s_hi;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   int glo = N, ghi = 0;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(kRankThreads) tw_rank_count_kernel(int N, cons
     const int g = L.grp[k];
     glo = L.g_lo[g];
     ghi = glo + L.g_n[g];
-    v = bits(sigma[k]);
+    v = order_bits(sigma[k]);
   }
   if (threadIdx.x == 0) {
     s_lo = N;
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kRankThreads) tw_rank_count_kernel(int N, cons
   int cnt = 0;
   for (int t0 = j0; t0 < j1; t0 += kRankTile) {
     const int t1 = min(j1, t0 + kRankTile);
-    for (int j = t0 + threadIdx.x; j < t1; j += blockDim.x) tile[j - t0] = bits(sigma[j]);
+    for (int j = t0 + threadIdx.x; j < t1; j += blockDim.x) tile[j - t0] = order_bits(sigma[j]);
     __syncthreads();
     const int a = max(t0, glo), b = min(t1, ghi);
     for (int j = a; j < b; j++) {
