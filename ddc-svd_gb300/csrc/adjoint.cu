@@ -9,9 +9,10 @@
 // + (I - U U^T) gU S^-1 V^T.  (The reference has no derivative; this is the
 // standard SVD adjoint.)  Any of gU, gs, gV may be null (zero).
 //
-// Four launches per call: J and K together, an elementwise kernel for M, then
-// P = U M + gU S^-1 and gA = P V^T, all batched products of any strides.  FP32
-// products run on the FP32 pipe; FP64 ones on the tensor cores, exactly on
+// FP32 problems whose matrices fit one CTA's shared memory take one launch
+// (adjoint_fused_kernel).  Otherwise four: J and K together, an elementwise kernel
+// for M, then P = U M + gU S^-1 and gA = P V^T, all batched products of any
+// strides.  FP32 products run on the FP32 pipe; FP64 ones on the tensor cores, on
 // digits (ozgemm_kernel), because GB300's FP64 pipe is 1/64 of FP32's.
 #include <cudaTypedefs.h>
 

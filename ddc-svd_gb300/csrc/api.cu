@@ -490,8 +490,11 @@ static int svd_core_impl(ddcsvd_context* ctx, int m, int n, const float* dA, int
 static bool use_tall_qr(const ddcsvd_context* ctx, int m, int n, int mode) {
   if (mode < DDCSVD_MODE_BLOCKED_TF32X3 || m < 2 * n || n < 128) return false;
   const int k = ctx->tune[TK_TALL_QR];
-  // auto: when the matrix no longer fits the L2-resident regime of the
-  // one-stage GEMVs (measured: 16384 x 8192 gains 1.3x, 8192 x 4096 loses 10%)
+  // auto: from 64M entries on.  The line was drawn when 8192 x 4096 lost 10% by it;
+  // since R's columns run on chip, QR first is the faster route at every measured
+  // m >= 2 n (direct / QR first, ms: 3500 x 300 3.95 / 3.37, 4096 x 1024 13.8 / 11.5,
+  // 8192 x 2048 41.6 / 27.1, 8192 x 4096 105 / 76, 16384 x 8192 732 / 356), and
+  // knob 5 = 1 takes it there; the default has not moved yet
   return k == 1 || (k == 2 && (long long)m * n >= (64ll << 20));
 }
 

@@ -797,7 +797,7 @@ __host__ __device__ inline int direct_regs(int rows) {
 }
 
 struct BxSide {
-  int rows, nref, off;  // reflector j starts at row j + off
+  int rows, nref;
   int vrows;            // rows of C that hold values on entry (zero below)
   int ncols, ldu, ldc;
   const float *Uc, *T4;
@@ -948,8 +948,8 @@ int bx_direct_prepare(ddcsvd_context* ctx, int m, int n, const float* W, int ldw
 
 int bx_direct_apply(ddcsvd_context* ctx, int m, int n, const BxDirect& w, float* U, int ldu, float* V, int ldv) {
   const int nr = std::max(0, n - 2);
-  const BxSide left{m, n, 0, n, n, w.lduL, ldu, w.UcL, w.T4, U};
-  const BxSide right{n, nr, 1, n, n, w.lduR, ldv, w.UcR, w.T4 + 16 * (size_t)ceil_div(n, 4), V};
+  const BxSide left{m, n, n, n, w.lduL, ldu, w.UcL, w.T4, U};
+  const BxSide right{n, nr, n, n, w.lduR, ldv, w.UcR, w.T4 + 16 * (size_t)ceil_div(n, 4), V};
   const int ctas = ceil_div(n, kDirectW), ctas_r = nr > 0 ? ctas : 0;
   bx_direct_kernel<<<ctas + ctas_r, kDirectThreads, 0, ctx->stream>>>(left, right, ctas);
   count_launch();

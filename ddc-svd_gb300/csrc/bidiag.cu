@@ -1411,6 +1411,16 @@ static int launch_coop(ddcsvd_context* ctx, const void* fn, int P, int threads, 
   return DDCSVD_OK;
 }
 
+// Tall blocks of at most 512 columns (knob 7) that the shared memory of 16 CTAs would
+// hold: their columns stay FP32 throughout, as in the tail's clusters, whose registers
+// end at 3072 rows.  The tensor cores' sums round towards zero and cost sigma a bit
+// (5000 x 64 1.6e-7 of the largest value, 8e-8 in FP32), and such an update is a few
+// microseconds either way.
+static bool fp32_update(const ddcsvd_context* ctx, int mt, int nt) {
+  return nt <= ctx->tune[TK_PANEL_TAIL] &&
+         (long long)mt * (ceil_div(nt, 16) + 6) * (long long)sizeof(float) <= (long long)ctx->smem_optin - 1024;
+}
+
 int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* d, float* e,
                    float* tauq, float* taup, BidiagWork& w, GemmKind kind, Arena* scratch, bool scanned) {
   if (m < n || n <= 0) return DDCSVD_ERR_ARG;
@@ -1458,7 +1468,8 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
     pp.rownrm = reinterpret_cast<double*>(round_up(reinterpret_cast<uintptr_t>(pp.rownrm), 8));
     pp.bar = w.bar;
     pp.st = ctx->d_status;
-    const bool fused_pack = (kind != GEMM_SIMT) && nb == kPanel && k0 + nb < n;
+    const bool simt = kind == GEMM_SIMT || fp32_update(ctx, m - k0, n - k0);
+    const bool fused_pack = !simt && nb == kPanel && k0 + nb < n;
     pp.Apk = fused_pack ? w.Apk : nullptr;
     pp.Bpk = fused_pack ? w.Bpk : nullptr;
     // one read of the trailing block per column when the rows fit 4 float4s
@@ -1510,8 +1521,8 @@ int bidiag_blocked(ddcsvd_context* ctx, int m, int n, float* W, int ldw, float* 
       Mat A2{w.X + kn, 1, ldw};
       Mat B2{w.VT + kn, w.ldn, 1};
       ktimer_begin(ctx, KC_TRAIL_GEMM);
-      if (kind == GEMM_SIMT) {
-        DDC_TRY(gemm(ctx, kind, M, N, nb, A1, B1, nb, A2, B2, -1.f, 1.f, W + kn + (size_t)kn * ldw,
+      if (simt) {
+        DDC_TRY(gemm(ctx, GEMM_SIMT, M, N, nb, A1, B1, nb, A2, B2, -1.f, 1.f, W + kn + (size_t)kn * ldw,
                      ldw, scratch));
       } else {
         // tensor cores read K-major operands: [U_p X] and [Y VT] as rows of 2*nb

@@ -25,7 +25,7 @@
 // block from L2 for every column, sums 152 records of 2 j values twice and one
 // 152-part row product, and its trailing update comes on top.  Us per column,
 // panels and here: 512-1024 columns 11.3 and 4.0, 1024-2048 13 to 15 and 4.9,
-// 2048-3648 15 to 18 and 10.7.
+// 2048-3648 15 to 18 and 6 (16 rows per CTA) to 12 (20 and 24, with grid barriers).
 #include "internal.hpp"
 
 namespace ddcsvd {
