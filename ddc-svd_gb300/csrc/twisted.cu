@@ -81,7 +81,9 @@ constexpr int kTwWarps = 4;
 // Bound by the two transforms' chains: nine FP64 instructions a step, each 64
 // cycles for a warp whatever its active lanes (fp64.cuh); the division was half
 // of them.  Every rounding of S, P and of the division is that of the plain
-// formulas: the twist index, and with it the vector's sign, follows from them.
+// formulas: the twist index, and with it the vector's sign, follows from them (the
+// multiply-adds are written out, for the compiler contracted them in one path of the
+// batches and not in another).
 // Loads are a batch of steps ahead.  N = 3000: 2.18 -> 1.59 ms, of which the
 // transforms 1.15 (745 cycles a step); the batch of 2048 1.26 -> 1.09 ms.
 // A warp whose vectors share one block (uni: every warp of a single unreduced
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
           ok = ok && sure && mid_range(dp) && mid_range(v.x[1][u]);
           p.Lp[at(i0 + u)] = L;
           p.S[at(i0 + u)] = s;
-          s = L * v.x[2][u] * s - lam;
+          s = fma(L * v.x[2][u], s, -lam);
         }
         if (__all_sync(0xffffffffu, ok)) return;
         s = s0;
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
           const double L = quot_rn(p.dl[i], dp);
           p.Lp[at(i)] = L;
           p.S[at(i)] = s;
-          s = L * p.ll[i] * s - lam;
+          s = fma(L * p.ll[i], s, -lam);
         }
       }
     };
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
           const double tt = quot_mid(v.x[1][u], dm, sure);
           ok = ok && sure && mid_range(dm) && mid_range(v.x[1][u]);
           p.Um[at(i0 - u)] = v.x[2][u] * tt;
-          pv = pv * tt - lam;
+          pv = fma(pv, tt, -lam);
           p.Pp[at(i0 - u)] = pv;
         }
         if (__all_sync(0xffffffffu, ok)) return;
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(32 * kTwWarps) twisted_kernel(TwParams p) {
           if (abs_bits(dm) < bits(tiny)) dm = -tiny;
           const double tt = quot_rn(p.dd[i], dm);
           p.Um[at(i)] = p.ll[i] * tt;
-          pv = pv * tt - lam;
+          pv = fma(pv, tt, -lam);
           p.Pp[at(i)] = pv;
         }
       }
@@ -464,7 +466,7 @@ __device__ void cl_refine(const TwParams& p, int k0, double* red) {
         if (i + 1 < hi) {
           const double L = p.dl[i] * is * is / dp;
           Lf[i - lo] = L;
-          s = L * p.ll[i] * s - lam;
+          s = fma(L * p.ll[i], s, -lam);
         }
       }
     }
