@@ -72,12 +72,14 @@ int main() {
   std::vector<double> d(q * nprob), z(q * nprob), zz(nprob);
   for (int p = 0; p < nprob; p++) {
     double* a = &d[(size_t)p * q];
-    for (int j = 0; j < q; j++) a[j] = (p % 3 == 0) ? uni() + j : (p % 3 == 1) ? pow(10.0, 4.0 * uni() - 4.0) : 1.0 + 1e-3 * uni();
+    for (int j = 0; j < q; j++)
+      a[j] = (p % 4 == 0) ? uni() + j : (p % 4 == 1) ? pow(10.0, 4.0 * uni() - 4.0) : (p % 4 == 2) ? 1.0 + 1e-3 * uni() : pow(10.0, 6.0 * uni() - 6.0);
     a[0] = 0.0;
     std::sort(a, a + q);
     double s = 0.0;
     for (int j = 0; j < q; j++) {
-      const double v = (uni() < 0.2 ? 1e-3 : 1.0) * (2.0 * uni() - 1.0) * a[q - 1];
+      // (the last kind: roots so near to their poles that tau leaves FP32's range)
+      const double v = (uni() < 0.2 ? (p % 4 == 3 ? 1e-15 : 1e-3) : 1.0) * (2.0 * uni() - 1.0) * a[q - 1];
       z[(size_t)p * q + j] = v;
       s += v * v;
     }
